@@ -14,17 +14,14 @@ namespace {
 // Environment switches for tests and profiling, read once per process:
 //   KS_B200_W4A16_PATH=general|tcgen05|decode  pins the kernel (tcgen05 / decode refuse
 //                                              shapes they cannot take instead of falling back)
-//   KS_B200_W4A16_OPERAND=smem|tmem            how the tcgen05 kernel passes the weights on
 // KS_B200_ENV_RELOAD=1 makes every call read them again (the test-suite flips them).
 struct EnvChoice {
   int path = 0;      // 0 choose, 1 general, 2 tcgen05, 3 decode
-  int operand = 0;   // 0 choose, 1 shared memory, 2 tensor memory
 };
 EnvChoice read_env() {
   EnvChoice c;
   if (const char* v = std::getenv("KS_B200_W4A16_PATH"))
     c.path = v[0] == 'g' ? 1 : (v[0] == 't' ? 2 : (v[0] == 'd' ? 3 : 0));
-  if (const char* v = std::getenv("KS_B200_W4A16_OPERAND")) c.operand = v[0] == 's' ? 1 : (v[0] == 't' ? 2 : 0);
   return c;
 }
 EnvChoice env_choice() {
@@ -60,7 +57,6 @@ ks_status_t gemm_w4a16_impl(const char* where, bool static_scratch, void* c, con
     sm100::W4A16Args args;
     args.c = c; args.a = a; args.b_packed = b_packed; args.scales = scales; args.zeros = zeros; args.bias = bias;
     args.m = m; args.n = n; args.k = k; args.group_size = gs; args.dtype = dtype;
-    args.operand_path = env.operand;
     args.kernel = env.path == 2 ? 1 : (env.path == 3 ? 2 : 0);
     if (env.path == 3 && !sm100::decode::eligible(args))
       KSB_FAIL(KS_ERROR_UNSUPPORTED_SHAPE, w + ": shape not eligible for the decode kernel");

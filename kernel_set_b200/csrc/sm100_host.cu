@@ -33,6 +33,8 @@ struct Scratch {
   size_t bytes = 0;
   bool dirty = false;
 };
+__global__ void __launch_bounds__(256) full_sm_kernel() {}   // only asked about, never launched
+
 std::mutex g_scratch_mutex;
 std::map<std::pair<std::pair<int, cudaStream_t>, int>, Scratch> g_scratch;
 
@@ -122,6 +124,37 @@ void stream_scratch_release(cudaStream_t stream) {
     }
   }
   cudaGetLastError();
+}
+
+int cluster_capacity(int s) {
+  static std::mutex mu;
+  static int known[64][kMaxClusterSplit + 1] = {};   // capacity + 1
+  constexpr int kSmem = 200 * 1024;                  // one CTA per SM
+  int dev = 0;
+  if (s < 2 || s > kMaxClusterSplit || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  int& slot = known[dev][s];
+  if (slot == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(s);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = kSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = s;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(full_sm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, full_sm_kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    slot = n + 1;
+  }
+  return slot - 1;
 }
 
 bool programmatic_launch_enabled() {

@@ -63,5 +63,39 @@ inline cudaError_t launch_programmatic(void (*kernel)(KArgs...), unsigned grid, 
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// The same with the grid cut into clusters of `cluster` CTAs (1: no clusters).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_programmatic_cluster(void (*kernel)(KArgs...), unsigned grid, unsigned cluster,
+                                               unsigned block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  unsigned n = 0;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (programmatic_launch_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Clusters of `s` CTAs (2 <= s <= kMaxClusterSplit) that the current device runs at a time when
+// a CTA fills an SM: a cluster's CTAs sit in one group of SMs, so 148 SMs hold fewer than
+// 148 / s. 0 when the query fails. Cached per device.
+constexpr int kMaxClusterSplit = 8;   // portable cluster size
+int cluster_capacity(int s);
+
 }  // namespace sm100
 }  // namespace ksb

@@ -70,87 +70,81 @@ namespace sm100 {
 namespace {
 
 constexpr int kTileN = 128;    // weight columns per tile = UMMA M
-constexpr int kStepK = 128;    // k per pipeline step (one scale group when gs % 128 == 0)
+constexpr int kStepK = 128;    // k per pipeline step ("unit" = 128 columns x 128 k)
 constexpr int kRawBytes = (kStepK / 2) * kTileN;      // 8192
-constexpr int kRawStage = kRawBytes + 2 * 256;        // + scales + zeros of the step
-constexpr int kDeqBytes = kStepK * kTileN * 2;        // 32768: dequantised UMMA operand
-constexpr int kDeqGroupWarps = 4;  // a group = one warp per TMEM lane quarter = one unit at a time
-// The numbers of operand stages and of activation stages must be multiples of the number
-// of issuers: an issuer's wait on a stage's `full` barrier is ordered after the stage's
-// previous use only because the same issuer consumed that use. (Three issuers with four
-// stages let an issuer pass a fresh barrier one phase early: intermittent bounded-wait
-// timeouts on the GPU, and a deadlock in the protocol model under tests/.)
-#ifndef KSB_W4_TMEM_ISSUERS
-#define KSB_W4_TMEM_ISSUERS 2
-#endif
-#ifndef KSB_W4_TMEM_STAGES
-#define KSB_W4_TMEM_STAGES 4
-#endif
-#ifndef KSB_W4_TMEM_GROUPS
-#define KSB_W4_TMEM_GROUPS 4
-#endif
+constexpr int kRawStageBytes = 2 * kRawBytes;         // one TMA box: two K-steps
+// Dequantisation: two groups of eight warps on alternate units; a warp takes one TMEM lane quarter
+// (32 columns) and one 64-k half of its group's unit. With four operand stages each group then has
+// two of its own, and fills one while the MMAs read the other. (Four groups of four warps
+// are each tied to one stage: a group's next unit waits for the MMAs of its last, and the two
+// times add up.)
+constexpr int kGroups = 2;
+constexpr int kDeqGroupWarps = 8;
+constexpr int kDeqWarps = kGroups * kDeqGroupWarps;
+constexpr int kDeqStages = 4;      // operand stages in tensor memory
+constexpr int kDeqTmemCols = kStepK / 2;   // 64 columns of two k each
+constexpr int kAtomK = 64;         // k per 128-byte swizzle atom of the activations
 
-// TA: the dequantised weights are handed to the tensor core through tensor memory
-// (tcgen05.st, A operand in TMEM) instead of shared memory. Decode shapes only
-// (MTMAX == 32): the accumulators of wider token tiles need all 512 TMEM columns.
-template <int MTMAX, bool TA>
+// Everything that depends on the width of the token tile. The numbers of operand stages and
+// of activation stages must be multiples of the number of issuers: an issuer's wait on a
+// stage's `full` barrier is ordered after the stage's previous use only because the same
+// issuer consumed that use. (Three issuers with four stages let an issuer pass a fresh barrier
+// one phase early: intermittent bounded-wait timeouts on the GPU, and a deadlock in the
+// protocol model under tests/.)
+template <int MTMAX>
 struct Cfg {
-  static_assert(!TA || MTMAX <= 32, "the TMEM operand path is built for token tiles of at most 32 rows");
-  // TA: a stage is one TMA box of two K-steps (16 KB); scales and zero-points do not
-  // travel through it. A warp keeps only about three TMA loads in flight, so the box
-  // has to be large for one producer warp to cover HBM latency.
-  // Dequantisation groups working on different units at the same time. The tensor-memory
-  // path is a chain of waits per unit (~1900 cycles per group); more groups in flight hide
-  // it until tcgen05.st bandwidth (~400 cycles per unit) becomes the limit.
-  static constexpr int kGroups = TA ? KSB_W4_TMEM_GROUPS : 2;
-  static constexpr int kDeqWarps = kGroups * kDeqGroupWarps;
-  // MMA issuers: warps 1 and 3, plus (TA) extra warps after the epilogue warps. An issuer
-  // spends ~1000 cycles per unit it owns (barrier tests, eight MMAs, commits).
-  static constexpr int kIssuers = TA ? KSB_W4_TMEM_ISSUERS : 2;
-  static_assert(!TA || (KSB_W4_TMEM_STAGES % KSB_W4_TMEM_ISSUERS == 0 && 8 % KSB_W4_TMEM_ISSUERS == 0),
-                "stage counts must be multiples of the number of issuers");
-  static constexpr int kExtraIssuerWarp0 = 4 + kDeqWarps + 4;   // first warp index after the epilogue warps
-  static constexpr int kThreads = 128 + kDeqWarps * 32 + 128 + (kIssuers - 2) * 32;
-  static constexpr int kRawStages = TA ? 8 : (MTMAX <= 32 ? 9 : 6);
-  static constexpr int kRawStageBytes = TA ? 2 * kRawBytes : kRawStage;
-  static constexpr int kActStages = TA ? 8 : (MTMAX <= 32 ? 4 : 3);
-  // TA: more operand stages than groups, so that a group can fill its next stage while the
-  // MMAs of its previous unit are still queued
-  static constexpr int kDeqStages = TA ? KSB_W4_TMEM_STAGES : (MTMAX <= 32 ? 3 : 2);
-  // shared memory per dequantised stage; with TA a stage is 64 TMEM columns instead
-  static constexpr int kDeqSmem = TA ? 0 : kDeqBytes;
-  static constexpr int kDeqTmemCols = kStepK / 2;
-  // Consecutive K=16 instructions of a step go to different TMEM accumulators:
-  // an instruction that accumulates into the result of the previous one waits
-  // for it, and with 16..32 token columns that latency, not throughput, would
-  // set the pace. The epilogue adds the accumulators up.
-  // TA: accumulators per issuer times issuers; the operand stages take the rest of TMEM
-  static constexpr int kAccsPerIssuer = (TA && (KSB_W4_TMEM_STAGES > 4 || KSB_W4_TMEM_ISSUERS > 2)) ? 1 : 2;
-  static constexpr int kAccs = TA ? kAccsPerIssuer * kIssuers : (MTMAX <= 32 ? 8 : 2);
-  static constexpr int kAccCols = 2 * kAccs * MTMAX;   // two segment buffers
-  static constexpr int kTmemCols = TA ? 512 : kAccCols;
-  static constexpr int kOperandCol0 = kAccCols;         // TA: first column of the operand ring
-  static_assert(!TA || kAccCols + kDeqStages * kDeqTmemCols <= 512, "TMEM holds 512 columns");
-  static constexpr int kActStage = MTMAX * kStepK * 2;  // bytes reserved per activation stage
-  static constexpr int kRing = kDeqStages * kDeqSmem + kActStages * kActStage + kRawStages * kRawStageBytes;
-  static constexpr int kNumBars = 2 * kRawStages + 2 * kActStages + 2 * kDeqStages + 4;
+  // Issuing a tcgen05.mma costs its thread ~55 cycles. Up to 64 token columns the tensor core
+  // needs less than that, at 128 about as much; two issuers take alternate units into accumulators
+  // of their own. 256 columns are bound by the tensor core (128 cycles per instruction).
+  static constexpr int kIssuers = MTMAX <= 128 ? 2 : 1;
+  // Consecutive instructions into one accumulator wait for one another; with 32 columns that
+  // latency would set the pace, so an issuer alternates between two.
+  static constexpr int kAccsPerIssuer = MTMAX <= 32 ? 2 : 1;
+  static constexpr int kAccs = kIssuers * kAccsPerIssuer;
+  // Tensor memory: 256 columns of operand ring, 256 of accumulators: two segment buffers up to
+  // 64 token columns, one above (the epilogue of a tile, ~2 % of a K = 4096 tile, is then
+  // not overlapped with the next tile's MMAs).
+  static constexpr int kAccBufs = MTMAX <= 64 ? 2 : 1;
+  static constexpr int kAccCols = kAccBufs * kAccs * MTMAX;
+  static constexpr int kOperandCol0 = kAccCols;
+  static constexpr int kTmemCols = 512;
+  static_assert(kAccCols + kDeqStages * kDeqTmemCols <= 512, "TMEM holds 512 columns");
+  // Activations: a stage is a whole unit (both 64-k atoms), or one atom at 256 tokens, where
+  // a whole unit (64 KB) would leave room for two stages only.
+  static constexpr int kActAtoms = MTMAX <= 128 ? 2 : 1;      // atoms per stage
+  static constexpr int kActPerUnit = 2 / kActAtoms;           // stages per unit
+  static constexpr int kActStage = MTMAX * kAtomK * 2 * kActAtoms;
+  static constexpr int kActStages = MTMAX <= 32 ? 8 : (MTMAX <= 64 ? 6 : 4);
+  static constexpr int kRawStages = MTMAX <= 32 ? 8 : (MTMAX <= 64 ? 7 : 5);
+  static_assert(kDeqStages % kIssuers == 0 && kActStages % (kIssuers * kActPerUnit) == 0, "see above");
+  static constexpr int kEpiWarps = MTMAX <= 128 ? 4 : 8;      // 256 tokens: two warps share a lane quarter
+  static constexpr int kEpiThreads = kEpiWarps * 32;
+  static constexpr int kThreads = 128 + kDeqWarps * 32 + kEpiThreads;
+  static constexpr int kRing = kActStages * kActStage + kRawStages * kRawStageBytes;
+  static constexpr int kNumBars = 2 * kRawStages + 2 * kActStages + 2 * kDeqStages + 2 * kAccBufs;
   static constexpr int kSmemBytes = kRing + 1024 + 512;
+  static_assert(8 * kNumBars + 16 <= 512 && kSmemBytes <= 232448, "shared memory layout");
 };
 
 struct Params {
   void* c;
   const void* bias;
-  const void* scales;       // read directly by the tensor-memory path
+  const void* scales;
   const void* zeros;
-  float* slots;             // [tiles][max_parts][mt][128] fp32 partials
-  unsigned int* counters;   // [tiles]
+  float* slots;             // fp32 partials, [slot][mt / 4][128][4]
+  unsigned int* counters;
   unsigned int* fault_word;
   int m, n, k;
   int mt;                   // token tile, multiple of 16, <= MTMAX
   int m_tiles;
-  int n_tiles, k_steps;
-  int gs_steps;             // K-steps per scale group (group_size / 128)
-  int max_parts;
+  int n_tiles;
+  int k_steps;              // 128-k steps, rounded up to an even number (a box holds two)
+  int gs_steps;             // K-steps per scale group (group_size / 128); FINE: unused
+  int sub_shift;            // FINE: log2 of the 32-k quarters per scale group (group_size 32: 0, 64: 1)
+  int groups;               // rows of scales and zeros
+  int split;                // 1: equal runs of units, tiles may be shared by CTAs; 0: whole tiles
+  int cluster_s;            // > 1: every tile is one cluster's, its K range cut over the cluster's CTAs
+  int c_vec;                // C is 8-byte aligned
   int has_zeros;
   uint32_t idesc;
 };
@@ -185,34 +179,79 @@ __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-template <typename T, int MTMAX, bool TA>
-__global__ void __launch_bounds__((Cfg<MTMAX, TA>::kThreads), 1)
-w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_s,
-                  const __grid_constant__ CUtensorMap tm_z, const __grid_constant__ CUtensorMap tm_a,
+// Weight column (inside a warp's 32) that TMEM lane `lane` of the warp's quarter holds: the
+// store shape of the dequantised operand puts columns 2g and 2g + 1 of a block of 16 in lanes
+// g and g + 8 (see the dequantisation role).
+__device__ __forceinline__ int column_of_lane(int lane) { return (lane & 16) + 2 * (lane & 7) + ((lane >> 3) & 1); }
+
+// Stores 16 token rows x the warp's 32 columns: a lane holds its column of token j in v[j].
+// Two exchanges with the lanes of the neighbouring columns turn that into four adjacent columns
+// of four tokens per lane, so that a store instruction writes 64 contiguous bytes of four rows
+// instead of 64 bytes of one. `c` points at (first token, first column of the warp).
+template <typename T>
+__device__ __forceinline__ void store_tokens16(T* c, int ld, const float (&v)[16], int lane, int rows_ok, int cols_ok,
+                                               bool vec) {
+  if (!vec) {
+    const int col = column_of_lane(lane);
+    if (col < cols_ok) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (j < rows_ok) c[static_cast<size_t>(j) * ld + col] = from_f32<T>(v[j]);
+    }
+    return;
+  }
+  using P = Pack16<T>;
+  // w[i] = tokens (2i, 2i + 1) of this lane's column
+  uint32_t w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) w[i] = P::bits(P::make(v[2 * i], v[2 * i + 1]));
+  // columns 2g and 2g + 1 (lanes g, g + 8): the first lane keeps token 2i of both, the other token 2i + 1
+  const bool odd = (lane & 8) != 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, w[i], 8);
+    w[i] = odd ? __byte_perm(other, w[i], 0x7632) : __byte_perm(w[i], other, 0x5410);
+  }
+  // column pairs g and g + 1: even lanes keep the pairs i < 4, odd lanes i >= 4
+  const bool up = (lane & 1) != 0;
+  const int col = (lane & 16) + 2 * (lane & 6);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t give = up ? w[i] : w[i + 4];
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, give, 1);
+    const uint32_t keep = up ? w[i + 4] : w[i];
+    const int token = 2 * (i + (up ? 4 : 0)) + (odd ? 1 : 0);
+    if (token < rows_ok && col < cols_ok)
+      *reinterpret_cast<uint2*>(c + static_cast<size_t>(token) * ld + col) =
+          up ? make_uint2(got, keep) : make_uint2(keep, got);
+  }
+}
+
+// FINE: scale groups of 32 or 64 k (several per K-step); otherwise multiples of 128.
+template <typename T, int MTMAX, bool FINE>
+__global__ void __launch_bounds__((Cfg<MTMAX>::kThreads), 1)
+w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a,
                   const Params p) {
-  using C = Cfg<MTMAX, TA>;
+  using C = Cfg<MTMAX>;
   using P16 = Pack16<T>;
   using V2 = typename P16::V2;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - raw_addr);
-  // ring: dequantised operand stages | activation stages | raw stages | barriers
-  const uint32_t deq_base = base;
-  const uint32_t act_base = deq_base + C::kDeqStages * C::kDeqSmem;
+  // ring: activation stages | raw stages | barriers
+  const uint32_t act_base = base;
   const uint32_t rawst_base = act_base + C::kActStages * C::kActStage;
-  const uint32_t bar_base = rawst_base + C::kRawStages * C::kRawStageBytes;
-  uint8_t* deq_ptr = base_ptr;
-  uint8_t* rawst_ptr = base_ptr + (rawst_base - base);
+  const uint32_t bar_base = rawst_base + C::kRawStages * kRawStageBytes;
   uint8_t* ctrl_ptr = base_ptr + (bar_base - base);
   const uint32_t bar_raw_full = bar_base;
   const uint32_t bar_raw_empty = bar_raw_full + 8 * C::kRawStages;
   const uint32_t bar_act_full = bar_raw_empty + 8 * C::kRawStages;
   const uint32_t bar_act_empty = bar_act_full + 8 * C::kActStages;
   const uint32_t bar_deq_full = bar_act_empty + 8 * C::kActStages;
-  const uint32_t bar_deq_empty = bar_deq_full + 8 * C::kDeqStages;
-  const uint32_t bar_acc_full = bar_deq_empty + 8 * C::kDeqStages;
-  const uint32_t bar_acc_empty = bar_acc_full + 16;
+  const uint32_t bar_deq_empty = bar_deq_full + 8 * kDeqStages;
+  const uint32_t bar_acc_full = bar_deq_empty + 8 * kDeqStages;
+  const uint32_t bar_acc_empty = bar_acc_full + 8 * C::kAccBufs;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(ctrl_ptr + 8 * C::kNumBars);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* last_flag = tmem_slot + 2;
@@ -224,26 +263,24 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kRawStages; ++s) {
       mbar_init(bar_raw_full + 8 * s, 1);
-      mbar_init(bar_raw_empty + 8 * s, TA ? 2 * kDeqGroupWarps : kDeqGroupWarps);   // TA: both halves of a box
+      mbar_init(bar_raw_empty + 8 * s, 2 * kDeqGroupWarps);   // both halves of a box
     }
     for (int s = 0; s < C::kActStages; ++s) {
       mbar_init(bar_act_full + 8 * s, 1);
-      mbar_init(bar_act_empty + 8 * s, TA ? 1 : 2);   // TA: the issuer that owns the unit; else both
+      mbar_init(bar_act_empty + 8 * s, 1);   // the issuer that owns the unit
     }
-    for (int s = 0; s < C::kDeqStages; ++s) {
+    for (int s = 0; s < kDeqStages; ++s) {
       mbar_init(bar_deq_full + 8 * s, kDeqGroupWarps);
-      mbar_init(bar_deq_empty + 8 * s, TA ? 1 : 2);
+      mbar_init(bar_deq_empty + 8 * s, 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < C::kAccBufs; ++b) {
       mbar_init(bar_acc_full + 8 * b, C::kIssuers);
-      mbar_init(bar_acc_empty + 8 * b, 4);
+      mbar_init(bar_acc_empty + 8 * b, C::kEpiWarps);
     }
     *abort_flag = 0u;
     fence_barrier_init();
     prefetch_tensormap(&tm_w);
-    prefetch_tensormap(&tm_s);
     prefetch_tensormap(&tm_a);
-    if (p.has_zeros) prefetch_tensormap(&tm_z);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), C::kTmemCols);
@@ -254,23 +291,28 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  // Unit space: (token tile, column tile, K-step), K-step fastest. With one
-  // token tile the units are dealt in exact equal runs (column tiles may be
-  // split between CTAs); with several, runs are snapped to whole column tiles
-  // so that no partial sums arise.
-  const long long units = static_cast<long long>(p.n_tiles) * p.k_steps;   // per token tile
+  // Unit space: (column tile, token tile, K-step), K-step fastest; a "tile" below is a
+  // (column tile, token tile) pair. Token tiles of one column tile are neighbours, so the
+  // CTAs in flight share weights. Units are dealt in equal contiguous runs (tiles may be
+  // split between CTAs), or in runs of whole tiles (split == 0), or, where there are few
+  // tiles, a tile's units over the CTAs of a cluster.
+  const long long tiles = static_cast<long long>(p.n_tiles) * p.m_tiles;
+  const long long units = tiles * p.k_steps;
   const int ctas = gridDim.x;
   long long u_begin, u_end;
-  if (p.m_tiles == 1) {
+  if (p.cluster_s > 1) {
+    // (parts are whole boxes of two steps)
+    const int part = static_cast<int>(blockIdx.x) % p.cluster_s;
+    const long long tile_begin = static_cast<long long>(blockIdx.x) / p.cluster_s * p.k_steps;
+    u_begin = tile_begin + 2 * (part * (p.k_steps / 2) / p.cluster_s);
+    u_end = tile_begin + 2 * ((part + 1) * (p.k_steps / 2) / p.cluster_s);
+  } else if (p.split) {
     u_begin = run_start(units, ctas, blockIdx.x);
     u_end = run_start(units, ctas, blockIdx.x + 1);
   } else {
-    const long long tiles_total = static_cast<long long>(p.m_tiles) * p.n_tiles;
-    u_begin = run_start(tiles_total, ctas, blockIdx.x) * p.k_steps;
-    u_end = run_start(tiles_total, ctas, blockIdx.x + 1) * p.k_steps;
+    u_begin = run_start(tiles, ctas, blockIdx.x) * p.k_steps;
+    u_end = run_start(tiles, ctas, blockIdx.x + 1) * p.k_steps;
   }
-  const uint32_t act_tx = static_cast<uint32_t>(p.mt) * kStepK * 2;
-  const uint32_t raw_tx = kRawBytes + 256 + (p.has_zeros ? 256 : 0);
   // The next kernel on the stream may start its prologue now. This one touches what the
   // kernel before it may have produced or may still read (activations, C, the split-K
   // scratch) only behind grid_dependency_wait(): the activation producer and the epilogue.
@@ -278,457 +320,451 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 
   if (warp == 0) {
     // ------------------------- weight producer (TMA) -------------------------
-    if constexpr (TA) {
-      // boxes of two K-steps; k_steps is even here, so a box never straddles two column
-      // tiles, and with a single token tile u indexes (tile, step) directly
-      const long long b_end = (u_end + 1) >> 1;
-      uint32_t itb = 0;
-      // (tile, step) advance with the loop: a 64-bit division per box would cost hundreds of cycles
-      int tile = static_cast<int>((u_begin & ~1ll) / p.k_steps);
-      int step = static_cast<int>((u_begin & ~1ll) - static_cast<long long>(tile) * p.k_steps);
-      for (long long b = u_begin >> 1; b < b_end; ++b, ++itb, step += 2) {
-        if (step >= p.k_steps) { step -= p.k_steps; ++tile; }
-        const uint32_t sr = itb % C::kRawStages, pr = (itb / C::kRawStages) & 1u;
-        if (!mbar_wait(wctx, bar_raw_empty + 8 * sr, pr ^ 1u, 0x100u + sr)) break;
-        const uint32_t full = bar_raw_full + 8 * sr;
-        mbar_arrive_expect_tx_elect(full, 2 * kRawBytes);
-        tma_load_2d_elect(rawst_base + sr * C::kRawStageBytes, &tm_w, full, tile * kTileN, step * (kStepK / 2));
+    // boxes of two K-steps; k_steps is even, so a box never straddles two tiles
+    const long long b_end = (u_end + 1) >> 1;
+    uint32_t itb = 0;
+    // (tile, step) advance with the loop: a 64-bit division per box would cost hundreds of cycles
+    const long long t0 = (u_begin & ~1ll) / p.k_steps;
+    int step = static_cast<int>((u_begin & ~1ll) - t0 * p.k_steps);
+    int ntile = static_cast<int>(t0 / p.m_tiles);
+    int mtile = static_cast<int>(t0 - static_cast<long long>(ntile) * p.m_tiles);
+    for (long long b = u_begin >> 1; b < b_end; ++b, ++itb, step += 2) {
+      if (step >= p.k_steps) {
+        step -= p.k_steps;
+        if (++mtile == p.m_tiles) { mtile = 0; ++ntile; }
       }
-    } else {
-    uint32_t it = 0;
-    for (long long u = u_begin; u < u_end; ++u, ++it) {
-      const long long ul = u % units;
-      const int tile = static_cast<int>(ul / p.k_steps);
-      const int step = static_cast<int>(ul - static_cast<long long>(tile) * p.k_steps);
-      const uint32_t sr = it % C::kRawStages, pr = (it / C::kRawStages) & 1u;
+      const uint32_t sr = itb % C::kRawStages, pr = (itb / C::kRawStages) & 1u;
       if (!mbar_wait(wctx, bar_raw_empty + 8 * sr, pr ^ 1u, 0x100u + sr)) break;
-      {
-        const uint32_t full = bar_raw_full + 8 * sr;
-        const uint32_t dst = rawst_base + sr * kRawStage;
-        mbar_arrive_expect_tx_elect(full, raw_tx);
-        tma_load_2d_elect(dst, &tm_w, full, tile * kTileN, step * (kStepK / 2));
-        tma_load_2d_elect(dst + kRawBytes, &tm_s, full, tile * kTileN, step / p.gs_steps);
-        if (p.has_zeros) tma_load_2d_elect(dst + kRawBytes + 256, &tm_z, full, tile * kTileN, step / p.gs_steps);
-      }
-    }
+      const uint32_t full = bar_raw_full + 8 * sr;
+      mbar_arrive_expect_tx_elect(full, 2 * kRawBytes);
+      tma_load_2d_elect(rawst_base + sr * kRawStageBytes, &tm_w, full, ntile * kTileN, step * (kStepK / 2));
+      // The dequantising warps fetch scales and zero-points only one unit ahead, which can be less
+      // than the latency of HBM under load: this warp, a ring of boxes ahead, brings their lines
+      // into L2. Lane: 64 bytes of a 256-byte row piece (lane % 4), scales or zero-points
+      // (lane / 4 % 2), row (lane / 8).
+      const int rows = FINE ? 8 >> p.sub_shift : 2;          // of the box's two K-steps
+      const int row0 = FINE ? (step * 4) >> p.sub_shift : step / p.gs_steps;
+      const char* table = static_cast<const char*>((lane & 4) ? p.zeros : p.scales);
+      const int n = ntile * kTileN + (lane & 3) * 32;
+      for (int r = row0 + (lane >> 3); r < row0 + rows; r += 4)
+        if (r < p.groups && n < p.n && table != nullptr) prefetch_l2(table + (static_cast<size_t>(r) * p.n + n) * 2);
+      __syncwarp();
     }
   } else if (warp == 2) {
     // ----------------------- activation producer (TMA) -----------------------
     grid_dependency_wait();
-    uint32_t it = 0;
-    int mtile = static_cast<int>(u_begin / units);
-    int step = static_cast<int>((u_begin - static_cast<long long>(mtile) * units) % p.k_steps);
-    long long next_mtile_at = (static_cast<long long>(mtile) + 1) * units;
-    for (long long u = u_begin; u < u_end; ++u, ++it, step = (step + 1 == p.k_steps) ? 0 : step + 1) {
-      if (u == next_mtile_at) { ++mtile; next_mtile_at += units; }
-      const uint32_t sa = it % C::kActStages, pa = (it / C::kActStages) & 1u;
-      if (!mbar_wait(wctx, bar_act_empty + 8 * sa, pa ^ 1u, 0x180u + sa)) break;
-      {
+    const uint32_t act_tx = static_cast<uint32_t>(p.mt) * kAtomK * 2 * C::kActAtoms;
+    const long long t0 = u_begin / p.k_steps;
+    int step = static_cast<int>(u_begin - t0 * p.k_steps);
+    int mtile = static_cast<int>(t0 % p.m_tiles);
+    uint32_t ita = 0;
+    bool ok = true;
+    for (long long u = u_begin; ok && u < u_end; ++u) {
+#pragma unroll
+      for (int h = 0; h < C::kActPerUnit; ++h, ++ita) {
+        const uint32_t sa = ita % C::kActStages, pa = (ita / C::kActStages) & 1u;
+        if (!mbar_wait(wctx, bar_act_empty + 8 * sa, pa ^ 1u, 0x180u + sa)) { ok = false; break; }
         const uint32_t full = bar_act_full + 8 * sa;
-        const uint32_t dst = act_base + sa * C::kActStage;
         mbar_arrive_expect_tx_elect(full, act_tx);
-        if constexpr (TA) {
-          // one load for both 64-k atoms: the map views A as [K/64][M][64]
-          tma_load_3d_elect(dst, &tm_a, full, 0, mtile * p.mt, step * 2);
-        } else {
-          tma_load_2d_elect(dst, &tm_a, full, step * kStepK, mtile * p.mt);
-          tma_load_2d_elect(dst + p.mt * 128, &tm_a, full, step * kStepK + 64, mtile * p.mt);
-        }
+        // the map views A as [K/64][M][64]
+        tma_load_3d_elect(act_base + sa * C::kActStage, &tm_a, full, 0, mtile * p.mt, step * 2 + h);
+      }
+      if (++step == p.k_steps) {
+        step = 0;
+        if (++mtile == p.m_tiles) mtile = 0;
       }
     }
-  } else if (warp == 1 || warp == 3 || (warp >= C::kExtraIssuerWarp0 && warp < C::kExtraIssuerWarp0 + C::kIssuers - 2)) {
+  } else if (warp == 1 || (warp == 3 && C::kIssuers == 2)) {
     // ------------------------------ MMA issuers ------------------------------
-    // Issuing one tcgen05.mma costs its thread ~55 cycles; eight per unit from one
-    // thread would set the pace of the whole kernel. Two warps issue four each,
-    // into disjoint accumulators (an accumulator must have a single issuer).
-    const int mma_half = warp == 1 ? 0 : (warp == 3 ? 1 : 2 + (warp - C::kExtraIssuerWarp0));   // issuer index
-    constexpr int kHalfAccs = TA ? C::kAccsPerIssuer : C::kAccs / 2;
+    // The issuers take the units in turn (unit it -> issuer it % kIssuers): per unit an
+    // issuer pays its barrier tests (~100 cycles each), eight MMAs and the commits; sharing
+    // every unit between all issuers made each of them pay the fixed part for every unit. An
+    // issuer owns its accumulator(s) of the segment buffer and tells the epilogue "done" after
+    // its last unit of the segment; an issuer without a unit in a short segment arrives
+    // without a commit, and the epilogue skips its accumulators.
+    const int me = warp == 1 ? 0 : 1;
     uint32_t it = 0, seg = 0;
-    if constexpr (TA) {
-      // The issuers take the units in turn (unit it -> issuer it % kIssuers): per unit an
-      // issuer pays its barrier tests (~100 cycles each), eight MMAs (~55 each) and the
-      // commits; sharing every unit between all issuers made each of them pay the fixed part
-      // for every unit. An issuer owns its accumulator(s) of the segment buffer and tells the
-      // epilogue "done" after its last unit of the segment; an issuer without a unit in a
-      // short segment arrives without a commit, and the epilogue skips its accumulators.
-      int step = static_cast<int>(u_begin % p.k_steps);
-      uint32_t n_in_seg = 0;
-      for (long long u = u_begin; u < u_end; ++u, ++it, step = (step + 1 == p.k_steps) ? 0 : step + 1) {
-        const bool seg_first = (u == u_begin) || (step == 0);
-        const bool seg_last = (u + 1 == u_end) || (step == p.k_steps - 1);
-        // last unit of this segment: end of the column tile or of this CTA's run
-        const long long tile_last = u - step + p.k_steps - 1;
-        const long long seg_last_u = tile_last < u_end - 1 ? tile_last : u_end - 1;
-        const bool mine = static_cast<int>(it % C::kIssuers) == mma_half;
-        const bool my_last = u + C::kIssuers > seg_last_u;   // no later unit of mine in this segment
-        const uint32_t sd = it % C::kDeqStages, pd = (it / C::kDeqStages) & 1u;
-        const uint32_t sa = it % C::kActStages, pa = (it / C::kActStages) & 1u;
-        const uint32_t buf = seg & 1u, pacc = (seg >> 1) & 1u;
-        if (seg_first) n_in_seg = 0;
-        if (mine) {
-          if (n_in_seg == 0 && !mbar_wait(wctx, bar_acc_empty + 8 * buf, pacc ^ 1u, 0x200u + buf)) break;
-          if (!mbar_wait_both(wctx, bar_deq_full + 8 * sd, pd, 0x280u + sd, bar_act_full + 8 * sa, pa, 0x300u + sa)) break;
+    int step = static_cast<int>(u_begin % p.k_steps);
+    uint32_t n_in_seg = 0;
+    bool ok = true;
+    for (long long u = u_begin; ok && u < u_end; ++u, ++it, step = (step + 1 == p.k_steps) ? 0 : step + 1) {
+      const bool seg_first = (u == u_begin) || (step == 0);
+      const bool seg_last = (u + 1 == u_end) || (step == p.k_steps - 1);
+      // last unit of this segment: end of the tile or of this CTA's run
+      const long long tile_last = u - step + p.k_steps - 1;
+      const long long seg_last_u = tile_last < u_end - 1 ? tile_last : u_end - 1;
+      const bool mine = static_cast<int>(it % C::kIssuers) == me;
+      const bool my_last = u + C::kIssuers > seg_last_u;   // no later unit of mine in this segment
+      const uint32_t sd = it % kDeqStages, pd = (it / kDeqStages) & 1u;
+      const uint32_t buf = seg % C::kAccBufs, pacc = (seg / C::kAccBufs) & 1u;
+      if (seg_first) n_in_seg = 0;
+      if (mine) {
+        if (n_in_seg == 0 && !mbar_wait(wctx, bar_acc_empty + 8 * buf, pacc ^ 1u, 0x200u + buf)) break;
+        const uint32_t d_tmem = tmem_base + buf * (C::kAccs * MTMAX);
+        const uint32_t w_stage = tmem_base + C::kOperandCol0 + sd * kDeqTmemCols;
+#pragma unroll
+        for (int h = 0; h < C::kActPerUnit; ++h) {
+          const uint32_t ita = it * C::kActPerUnit + h;
+          const uint32_t sa = ita % C::kActStages, pa = (ita / C::kActStages) & 1u;
+          if (h == 0) {
+            if (!mbar_wait_both(wctx, bar_deq_full + 8 * sd, pd, 0x280u + sd, bar_act_full + 8 * sa, pa, 0x300u + sa)) {
+              ok = false;
+              break;
+            }
+          } else {
+            if (!mbar_wait(wctx, bar_act_full + 8 * sa, pa, 0x300u + sa)) { ok = false; break; }
+          }
           tc_fence_after_sync();
           const uint32_t a_src = act_base + sa * C::kActStage;
-          const uint32_t d_tmem = tmem_base + buf * (C::kAccs * MTMAX);
-          const uint32_t w_stage = tmem_base + C::kOperandCol0 + sd * C::kDeqTmemCols;
 #pragma unroll
-          for (int kk = 0; kk < kStepK / 16; ++kk) {
-            // tokens: K-major, two 64-k atoms of mt rows, 32 B per instruction inside an atom;
+          for (int k4 = 0; k4 < 4 * C::kActAtoms; ++k4) {
+            // tokens: K-major, 64-k atoms of mt rows, 32 B per instruction inside an atom;
             // weights: 16 k = 8 columns of the operand stage in tensor memory
-            const uint64_t a_desc = umma_smem_desc_sw128(a_src + (kk >> 2) * (p.mt * 128) + (kk & 3) * 32, 16, 1024);
-            const uint32_t d_acc = d_tmem + (mma_half * kHalfAccs + (kk % kHalfAccs)) * MTMAX;
-            umma_f16_tmem_a_elect(d_acc, w_stage + kk * 8, a_desc, p.idesc, (n_in_seg == 0 && kk < kHalfAccs) ? 0u : 1u);
+            const int kk = h * 4 + k4;
+            const uint64_t a_desc = umma_smem_desc_sw128(a_src + (k4 >> 2) * (p.mt * 128) + (k4 & 3) * 32, 16, 1024);
+            const uint32_t d_acc = d_tmem + (me * C::kAccsPerIssuer + (kk % C::kAccsPerIssuer)) * MTMAX;
+            umma_f16_tmem_a_elect(d_acc, w_stage + kk * 8, a_desc, p.idesc,
+                                  (n_in_seg == 0 && kk < C::kAccsPerIssuer) ? 0u : 1u);
           }
-          ++n_in_seg;
-          tc_commit_elect(bar_deq_empty + 8 * sd);
+          if (h == C::kActPerUnit - 1) tc_commit_elect(bar_deq_empty + 8 * sd);
           tc_commit_elect(bar_act_empty + 8 * sa);
-          if (my_last) tc_commit_elect(bar_acc_full + 8 * buf);   // my last unit of the segment
-        } else if (seg_last && n_in_seg == 0) {
-          // A short segment without a unit of mine. Like an issuer with work, wait until the
-          // epilogue has drained this buffer's previous segment: otherwise this arrival could
-          // overtake my own (asynchronous) commit for that segment and complete its phase early.
-          if (!mbar_wait(wctx, bar_acc_empty + 8 * buf, pacc ^ 1u, 0x200u + buf)) break;
-          mbar_arrive_elect(bar_acc_full + 8 * buf);
         }
-        if (seg_last) ++seg;
+        if (!ok) break;
+        ++n_in_seg;
+        if (my_last) tc_commit_elect(bar_acc_full + 8 * buf);   // my last unit of the segment
+      } else if (seg_last && n_in_seg == 0) {
+        // A short segment without a unit of mine. Like an issuer with work, wait until the
+        // epilogue has drained this buffer's previous segment: otherwise this arrival could
+        // overtake my own (asynchronous) commit for that segment and complete its phase early.
+        if (!mbar_wait(wctx, bar_acc_empty + 8 * buf, pacc ^ 1u, 0x200u + buf)) break;
+        mbar_arrive_elect(bar_acc_full + 8 * buf);
       }
-    } else {
-      int step = static_cast<int>(u_begin % p.k_steps);
-      for (long long u = u_begin; u < u_end; ++u, ++it, step = (step + 1 == p.k_steps) ? 0 : step + 1) {
-        const bool seg_first = (u == u_begin) || (step == 0);
-        const bool seg_last = (u + 1 == u_end) || (step == p.k_steps - 1);
-        const uint32_t sd = it % C::kDeqStages, pd = (it / C::kDeqStages) & 1u;
-        const uint32_t sa = it % C::kActStages, pa = (it / C::kActStages) & 1u;
-        const uint32_t buf = seg & 1u, pacc = (seg >> 1) & 1u;
-        if (seg_first && !mbar_wait(wctx, bar_acc_empty + 8 * buf, pacc ^ 1u, 0x200u + buf)) break;
-        if (!mbar_wait(wctx, bar_deq_full + 8 * sd, pd, 0x280u + sd)) break;
-        if (!mbar_wait(wctx, bar_act_full + 8 * sa, pa, 0x300u + sa)) break;
-        tc_fence_after_sync();
-        {
-          // all 32 lanes run this code; each instruction elects its one issuing lane
-          const uint32_t w_src = deq_base + sd * C::kDeqSmem;
-          const uint32_t a_src = act_base + sa * C::kActStage;
-          const uint32_t d_tmem = tmem_base + buf * (C::kAccs * MTMAX);
-#pragma unroll
-          for (int kq = 0; kq < kStepK / 32; ++kq) {
-            const int kk = mma_half * (kStepK / 32) + kq;
-            // Weights: MN-major, 64-column atoms 16 KB apart, 8-k groups 1024 B
-            // apart, 16 k = 2048 B per instruction. Tokens: K-major, two 64-k
-            // atoms of mt rows, 32 B per instruction inside an atom.
-            const uint64_t a_desc = umma_smem_desc_sw128(a_src + (kk >> 2) * (p.mt * 128) + (kk & 3) * 32, 16, 1024);
-            const uint32_t d_acc = d_tmem + (mma_half * kHalfAccs + (kq % kHalfAccs)) * MTMAX;
-            const uint32_t first = (seg_first && kq < kHalfAccs) ? 0u : 1u;
-            const uint64_t w_desc = umma_smem_desc_sw128(w_src + kk * 2048, 16384, 1024);
-            umma_f16_elect(d_acc, w_desc, a_desc, p.idesc, first);
-          }
-          tc_commit_elect(bar_deq_empty + 8 * sd);
-          tc_commit_elect(bar_act_empty + 8 * sa);
-          if (seg_last) tc_commit_elect(bar_acc_full + 8 * buf);
-        }
-        if (seg_last) ++seg;
-      }
+      if (seg_last) ++seg;
     }
-  } else if (warp >= 4 && warp < 4 + C::kDeqWarps) {
+  } else if (warp >= 4 && warp < 4 + kDeqWarps) {
     // ----------------------------- dequantisation -----------------------------
-    const int group = (warp - 4) >> 2;          // which units of this CTA's run: u % kGroups == group
-    const int tt = (threadIdx.x - 128) & 127;   // thread inside its group
-    const int oct = tt & 15;   // 8 weight columns: n_local = 8*oct .. 8*oct+7
-    const int rg = tt >> 4;    // 8 packed byte-rows: k_local = 16*rg .. 16*rg+15
-    const uint32_t atom_off = (oct >> 3) * 16384u;
-    const uint32_t chunk = oct & 7;
+    // A packed byte holds the codes of k and k+1 of one column, which is exactly one 32-bit
+    // operand cell. ldmatrix.trans hands lane (g = lane / 4, s = lane % 4) a word with the bytes
+    // (row 2s, columns 2g, 2g + 1) and (row 2s + 1, columns 2g, 2g + 1) of an 8-row x 16-column
+    // block; tcgen05.st.16x256b takes from it the cells (TMEM lane g, columns 2s, 2s + 1) and
+    // (lane g + 8, columns 2s, 2s + 1). So TMEM lanes g and g + 8 stand for the weight columns 2g
+    // and 2g + 1, and no byte crosses a lane. Per cell: one byte permute (code k to byte 0, code
+    // k+1, from the word shifted by four, to byte 2), one mask-or with the exponent bits of
+    // magic, subtract (magic + zero), multiply by the scale.
+    // (Reading one byte per lane and row instead takes a full shared-memory cycle for 32 bytes,
+    // 256 per unit, on the port through which the MMAs read 64 KB and TMA writes 72 KB per unit.)
+    const int half = (warp - 4) >> 3;           // group = K-step half of every box = parity of its units
+    const int khalf = ((warp - 4) >> 2) & 1;    // 64-k half of the unit
     const V2 magic2 = P16::splat(P16::kMagic);
-    if constexpr (TA) {
-      // A thread owns one weight column (= one TMEM lane; warp w may only touch the lane
-      // quarter w % 4) and walks down its 64 packed bytes. A byte holds the codes of k and
-      // k+1, which is exactly one 32-bit operand cell: b * 0x1001 puts the low nibble at bit
-      // 0 and the high nibble at bit 16, one mask-and-or makes the pair (magic + q), and
-      // two packed operations subtract (magic + zero) and apply the scale.
-      const int quarter = warp & 3;
-      const int n_local = quarter * 32 + lane;
-      constexpr uint32_t kMagic2 = P16::kMagicBytes & 0xFF00FF00u;
-      // Group g owns the units u with u % kGroups == g: K-step half (g & 1) of every box b
-      // with b % (kGroups / 2) == g >> 1. Scales and zero-points come straight from global
-      // memory, fetched one unit of the group ahead; (tile, step) of the unit being fetched
-      // advance without any 64-bit division (k_steps and kGroups are even, so the parity of
-      // step is fixed).
-      constexpr int kBoxStride = C::kGroups / 2;
-      const int half = group & 1;
-      const unsigned short* gscales = static_cast<const unsigned short*>(p.scales);
-      const unsigned short* gzeros = static_cast<const unsigned short*>(p.zeros);
-      const long long b_begin = u_begin >> 1, b_end = (u_end + 1) >> 1;
-      long long b_first = b_begin;
-      while ((b_first % kBoxStride) != (group >> 1)) ++b_first;
-      long long u_first = (b_first << 1) + half;
-      if (u_first < u_begin) u_first += C::kGroups;
-      int f_tile = static_cast<int>(u_first / p.k_steps);
-      int f_step = static_cast<int>(u_first - static_cast<long long>(f_tile) * p.k_steps);
-      int f_row = f_step / p.gs_steps, f_in_row = f_step - f_row * p.gs_steps;
-      auto fetch_sz = [&](uint32_t* s_out, uint32_t* z_out) {
-        const int n = f_tile * kTileN + n_local;
-        const size_t idx = static_cast<size_t>(f_row) * p.n + n;
-        const bool n_ok = n < p.n;
-        *s_out = n_ok ? __ldg(gscales + idx) : 0u;
-        *z_out = (n_ok && p.has_zeros) ? __ldg(gzeros + idx) : 0u;
-        f_step += C::kGroups;
-        f_in_row += C::kGroups;
-        if (f_step >= p.k_steps) {
-          while (f_step >= p.k_steps) { f_step -= p.k_steps; ++f_tile; }
+    const int quarter = warp & 3;
+    constexpr uint32_t kMagic2 = P16::kMagicBytes & 0xFF00FF00u;
+    // Scales and zero-points come straight from global memory, fetched one unit of the group
+    // ahead; (tile, step) of the unit being fetched advance without any 64-bit division
+    // (k_steps and kGroups are even, so the parity of step is fixed).
+    constexpr int kSz = FINE ? 2 : 1;           // scale rows of this warp's 64 k: one per 32 k, or one
+    const int col0 = quarter * 32 + 2 * (lane >> 2);   // this lane's columns: col0, col0 + 1, col0 + 16, col0 + 17
+    const long long b_begin = u_begin >> 1, b_end = (u_end + 1) >> 1;
+    long long u_first = (b_begin << 1) + half;
+    if (u_first < u_begin) u_first += kGroups;
+    const long long f_t0 = u_first / p.k_steps;
+    int f_step = static_cast<int>(u_first - f_t0 * p.k_steps);
+    int f_ntile = static_cast<int>(f_t0 / p.m_tiles);
+    int f_mtile = static_cast<int>(f_t0 - static_cast<long long>(f_ntile) * p.m_tiles);
+    int f_row = FINE ? 0 : f_step / p.gs_steps, f_in_row = FINE ? 0 : f_step - f_row * p.gs_steps;
+    uint32_t s_pair[kSz][2], z_pair[kSz][2];   // [scale row][block of 16 columns]: columns 2g (low half), 2g + 1
+    auto fetch = [&]() {
+      const int n = f_ntile * kTileN + col0;
+#pragma unroll
+      for (int i = 0; i < kSz; ++i) {
+        const int row = FINE ? ((f_step * 4 + khalf * 2 + i) >> p.sub_shift) : f_row;
+        const size_t idx = static_cast<size_t>(row) * p.n + n;
+        const unsigned short* gs = static_cast<const unsigned short*>(p.scales) + idx;
+        const unsigned short* gz = static_cast<const unsigned short*>(p.zeros) + idx;
+#pragma unroll
+        for (int cb = 0; cb < 2; ++cb) {
+          // (the step that rounds k_steps up to an even number has no row: codes and activations
+          // are zero-filled there, and zero scales keep the product zero)
+          const bool in = n + 16 * cb < p.n && row < p.groups;
+          s_pair[i][cb] = in ? __ldg(reinterpret_cast<const unsigned int*>(gs + 16 * cb)) : 0u;
+          z_pair[i][cb] = (in && p.has_zeros) ? __ldg(reinterpret_cast<const unsigned int*>(gz + 16 * cb)) : 0u;
+        }
+      }
+    };
+    auto fetch_advance = [&]() {
+      f_step += kGroups;
+      if constexpr (!FINE) f_in_row += kGroups;
+      if (f_step >= p.k_steps) {
+        f_step -= p.k_steps;
+        if (++f_mtile == p.m_tiles) { f_mtile = 0; ++f_ntile; }
+        if constexpr (!FINE) {
           f_row = 0;
           f_in_row = f_step;
         }
-        while (f_in_row >= p.gs_steps) { f_in_row -= p.gs_steps; ++f_row; }
-      };
-      uint32_t s_next = 0u, z_next = 0u;
-      if (u_first < u_end) fetch_sz(&s_next, &z_next);
-      for (long long b = b_first; b < b_end; b += kBoxStride) {
-        const uint32_t itb = static_cast<uint32_t>(b - b_begin);
-        const uint32_t sr = itb % C::kRawStages, pr = (itb / C::kRawStages) & 1u;
-        const long long u = (b << 1) + half;
-        if (u < u_begin || u >= u_end) {
-          // this half of the box belongs to a neighbouring CTA's run
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_raw_empty + 8 * sr);
-          continue;
-        }
-        const uint32_t it = static_cast<uint32_t>(u - u_begin);
-        const uint32_t sd = it % C::kDeqStages, pd = (it / C::kDeqStages) & 1u;
-        const uint32_t s16 = s_next, z16 = z_next;
-        if (u + C::kGroups < u_end) fetch_sz(&s_next, &z_next);
-        if (!mbar_wait_both(wctx, bar_raw_full + 8 * sr, pr, 0x400u + sr, bar_deq_empty + 8 * sd, pd ^ 1u, 0x480u + sd)) break;
-        const uint8_t* col = rawst_ptr + sr * C::kRawStageBytes + half * kRawBytes + n_local;
-        const V2 sc = P16::from_bits(s16 | (s16 << 16));
-        const uint32_t zw = z16 | (z16 << 16);
-        const V2 zz = __hadd2(P16::from_bits(zw), magic2);
-        // (magic + zero) exact and |q - zero| exact: non-negative integer zero-points up to kMaxZero
-        const uint32_t back = P16::bits(__hsub2(zz, magic2));
-        const bool simple = ((back ^ zw) | (zw & 0x80008000u)) == 0u && z16 <= P16::kMaxZeroBits;
-        const uint32_t t_dst = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::kOperandCol0 +
-                               sd * C::kDeqTmemCols;
-#pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4) {
-          uint32_t cells[16];
-          if (simple) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const uint32_t b = col[(c4 * 16 + j) * kTileN];
-              const uint32_t x = ((b * 0x1001u) & 0x000F000Fu) | kMagic2;
-              cells[j] = P16::bits(__hmul2(__hsub2(P16::from_bits(x), zz), sc));
-            }
-          } else {
-            // zero-points that are not small integers: the fp32 statement, verbatim
-            const float z0 = P16::lo(P16::from_bits(zw)), s0 = P16::lo(sc);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const uint32_t b = col[(c4 * 16 + j) * kTileN];
-              cells[j] = P16::bits(P16::make(__fmul_rn(__fsub_rn(static_cast<float>(b & 15u), z0), s0),
-                                             __fmul_rn(__fsub_rn(static_cast<float>(b >> 4), z0), s0)));
-            }
-          }
-          tmem_st(t_dst + c4 * 16, cells);
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_raw_empty + 8 * sr);   // every byte of the packed stage has been read
-        tmem_wait_st();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_deq_full + 8 * sd);
       }
-    } else {
-      for (long long u = u_begin + group; u < u_end; u += 2) {
-        const uint32_t it = static_cast<uint32_t>(u - u_begin);
-        const uint32_t sr = it % C::kRawStages, pr = (it / C::kRawStages) & 1u;
-        const uint32_t sd = it % C::kDeqStages, pd = (it / C::kDeqStages) & 1u;
-        if (!mbar_wait(wctx, bar_raw_full + 8 * sr, pr, 0x400u + sr)) break;
-        const uint8_t* raw = rawst_ptr + sr * kRawStage;
-        // the packed bytes this thread owns, and the group constants of its 8 columns
-        uint2 pk[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) pk[i] = *reinterpret_cast<const uint2*>(raw + (rg * 8 + i) * kTileN + oct * 8);
-        const uint4 s4 = *reinterpret_cast<const uint4*>(raw + kRawBytes + oct * 16);
-        uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
-        if (p.has_zeros) z4 = *reinterpret_cast<const uint4*>(raw + kRawBytes + 256 + oct * 16);
+      if constexpr (!FINE) {
+        while (f_in_row >= p.gs_steps) { f_in_row -= p.gs_steps; ++f_row; }
+      }
+    };
+    if (u_first < u_end) fetch();
+    // ldmatrix row addresses: lanes 0-7 / 8-15 rows 0-7 of the first / second block of 16
+    // columns, lanes 16-31 the same of rows 8-15; 128-byte rows with the 16-byte chunks swizzled
+    const uint32_t lane_off =
+        static_cast<uint32_t>(half * kRawBytes + khalf * (32 * 128) + ((lane >> 4) * 8 + (lane & 7)) * 128 +
+                              (((quarter * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+    const uint32_t lane_dst = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::kOperandCol0 + khalf * 32;
+    for (long long b = b_begin; b < b_end; ++b) {
+      const uint32_t itb = static_cast<uint32_t>(b - b_begin);
+      const uint32_t sr = itb % C::kRawStages, pr = (itb / C::kRawStages) & 1u;
+      const long long u = (b << 1) + half;
+      if (u < u_begin || u >= u_end) {
+        // this half of the box belongs to a neighbouring CTA's run
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_raw_empty + 8 * sr);  // the packed stage is in registers
-        const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w};
-        const uint32_t zw[4] = {z4.x, z4.y, z4.z, z4.w};
-        V2 sc[4], zz[4];
-        // (magic + zero) must be exact and |q - zero| small enough to be exact too:
-        // true for non-negative integer zero-points up to kMaxZero, which a packed
-        // add / subtract round trip plus two range checks establish.
-        uint32_t bad = 0;
+        if (lane == 0) mbar_arrive(bar_raw_empty + 8 * sr);
+        continue;
+      }
+      const uint32_t it = static_cast<uint32_t>(u - u_begin);
+      const uint32_t sd = it % kDeqStages, pd = (it / kDeqStages) & 1u;
+      // constants of the unit: columns 2g, 2g + 1 of the first block of 16, then of the second
+      V2 sc[kSz][4], zz[kSz][4];
+      uint32_t zw[kSz][4];
+      uint32_t bad = 0;
+#pragma unroll
+      for (int i = 0; i < kSz; ++i) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          sc[j] = P16::from_bits(sw[j]);
-          const V2 z = P16::from_bits(zw[j]);
-          zz[j] = __hadd2(z, magic2);
-          const uint32_t back = P16::bits(__hsub2(zz[j], magic2));
-          bad |= (back ^ zw[j]) | (zw[j] & 0x80008000u);
-          bad |= ((zw[j] & 0xFFFFu) > P16::kMaxZeroBits) ? 1u : 0u;
-          bad |= ((zw[j] >> 16) > P16::kMaxZeroBits) ? 1u : 0u;
+          const uint32_t sel = (j & 1) ? 0x3232u : 0x1010u;
+          sc[i][j] = P16::from_bits(__byte_perm(s_pair[i][j >> 1], 0u, sel));
+          zw[i][j] = __byte_perm(z_pair[i][j >> 1], 0u, sel);
+          zz[i][j] = __hadd2(P16::from_bits(zw[i][j]), magic2);
+          // (magic + zero) exact and |q - zero| exact: non-negative integer zero-points up to kMaxZero
+          bad |= (P16::bits(__hsub2(zz[i][j], magic2)) ^ zw[i][j]) | (zw[i][j] & 0x80008000u);
+          bad |= (zw[i][j] & 0xFFFFu) > P16::kMaxZeroBits ? 1u : 0u;
         }
-        const bool simple = bad == 0u;
-        if (!mbar_wait(wctx, bar_deq_empty + 8 * sd, pd ^ 1u, 0x480u + sd)) break;
-        uint8_t* deq = deq_ptr + sd * kDeqBytes + atom_off;
+      }
+      const bool simple = __all_sync(0xffffffffu, bad == 0u);   // (both forms agree to the bit where both apply)
+      if (u + kGroups < u_end) {
+        fetch_advance();
+        fetch();
+      }
+      if (!mbar_wait_both(wctx, bar_raw_full + 8 * sr, pr, 0x400u + sr, bar_deq_empty + 8 * sd, pd ^ 1u, 0x480u + sd)) break;
+      const uint32_t src = rawst_base + sr * kRawStageBytes + lane_off;
+      uint32_t w[2][4];                // [32-k part][8-row block, block of 16 columns]
+      ldmatrix_x4_trans(src, w[0]);
+      ldmatrix_x4_trans(src + 16 * 128, w[1]);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r_even = rg * 16 + 2 * i;
-          uint32_t even[4], odd[4];
-          if (simple) {
-            const uint32_t words[2] = {pk[i].x, pk[i].y};
+      for (int cb = 0; cb < 2; ++cb) {
+        uint32_t cells[16];            // 64 k = 32 operand columns of this block's 16 weight columns
+        if (simple) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const uint32_t e = words[h] & 0x0F0F0F0Fu;
-              const uint32_t o = (words[h] >> 4) & 0x0F0F0F0Fu;
-              // bytes (q0,q1,q2,q3) -> 16-bit patterns magic|q for (q0,q1) and (q2,q3)
-              const V2 e01 = P16::from_bits(__byte_perm(e, P16::kMagicBytes, 0x4140));
-              const V2 e23 = P16::from_bits(__byte_perm(e, P16::kMagicBytes, 0x4342));
-              const V2 o01 = P16::from_bits(__byte_perm(o, P16::kMagicBytes, 0x4140));
-              const V2 o23 = P16::from_bits(__byte_perm(o, P16::kMagicBytes, 0x4342));
-              even[2 * h] = P16::bits(__hmul2(__hsub2(e01, zz[2 * h]), sc[2 * h]));
-              even[2 * h + 1] = P16::bits(__hmul2(__hsub2(e23, zz[2 * h + 1]), sc[2 * h + 1]));
-              odd[2 * h] = P16::bits(__hmul2(__hsub2(o01, zz[2 * h]), sc[2 * h]));
-              odd[2 * h + 1] = P16::bits(__hmul2(__hsub2(o23, zz[2 * h + 1]), sc[2 * h + 1]));
-            }
-          } else {
-            // zero-points that are not small integers: the fp32 statement, verbatim
-            const uint64_t w64 = (static_cast<uint64_t>(pk[i].y) << 32) | pk[i].x;
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t w0 = w[q >> 1][2 * (q & 1) + cb], w4 = w0 >> 4;
+            const int r = FINE ? q >> 1 : 0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const V2 z = P16::from_bits(zw[j]);
-              const float z0 = P16::lo(z), z1 = P16::hi(z);
-              const float s0 = P16::lo(sc[j]), s1 = P16::hi(sc[j]);
-              const uint32_t b0 = static_cast<uint32_t>(w64 >> (16 * j)) & 0xFFu;
-              const uint32_t b1 = static_cast<uint32_t>(w64 >> (16 * j + 8)) & 0xFFu;
-              even[j] = P16::bits(P16::make(__fmul_rn(__fsub_rn(static_cast<float>(b0 & 15u), z0), s0),
-                                            __fmul_rn(__fsub_rn(static_cast<float>(b1 & 15u), z1), s1)));
-              odd[j] = P16::bits(P16::make(__fmul_rn(__fsub_rn(static_cast<float>(b0 >> 4), z0), s0),
-                                           __fmul_rn(__fsub_rn(static_cast<float>(b1 >> 4), z1), s1)));
+            for (int i = 0; i < 4; ++i) {
+              // byte i: column 2g + (i & 1), row 2s + (i >> 1)
+              const uint32_t sel = i | (i << 4) | ((4 + i) << 8) | ((4 + i) << 12);
+              const uint32_t x = (__byte_perm(w0, w4, sel) & 0x000F000Fu) | kMagic2;
+              cells[4 * q + 2 * (i & 1) + (i >> 1)] =
+                  P16::bits(__hmul2(__hsub2(P16::from_bits(x), zz[r][2 * cb + (i & 1)]), sc[r][2 * cb + (i & 1)]));
             }
           }
-          // rows r_even and r_even+1 of the operand: 128 B per 64 columns, 16-byte
-          // chunks xor-swizzled with the row index inside each group of 8 rows
-          *reinterpret_cast<uint4*>(deq + r_even * 128 + ((chunk ^ (r_even & 7)) << 4)) =
-              make_uint4(even[0], even[1], even[2], even[3]);
-          *reinterpret_cast<uint4*>(deq + (r_even + 1) * 128 + ((chunk ^ ((r_even + 1) & 7)) << 4)) =
-              make_uint4(odd[0], odd[1], odd[2], odd[3]);
+        } else {
+          // zero-points that are not small integers: the fp32 statement, verbatim
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t w0 = w[q >> 1][2 * (q & 1) + cb];
+            const int r = FINE ? q >> 1 : 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t b8 = (w0 >> (8 * i)) & 0xFFu;
+              const float z0 = P16::lo(P16::from_bits(zw[r][2 * cb + (i & 1)])), s0 = P16::lo(sc[r][2 * cb + (i & 1)]);
+              cells[4 * q + 2 * (i & 1) + (i >> 1)] =
+                  P16::bits(P16::make(__fmul_rn(__fsub_rn(static_cast<float>(b8 & 15u), z0), s0),
+                                      __fmul_rn(__fsub_rn(static_cast<float>(b8 >> 4), z0), s0)));
+            }
+          }
         }
-        fence_proxy_async_smem();  // generic-proxy writes -> visible to the tensor core's reads
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_deq_full + 8 * sd);
+        tmem_st_16x256b(lane_dst + sd * kDeqTmemCols + (static_cast<uint32_t>(16 * cb) << 16), cells);
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_raw_empty + 8 * sr);   // every byte of the packed stage has been read
+      tmem_wait_st();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_deq_full + 8 * sd);
     }
-  } else if (warp >= 4 + C::kDeqWarps) {
+  } else if (warp >= 4 + kDeqWarps) {
     // -------------------------------- epilogue --------------------------------
     const int quarter = warp & 3;
-    const int n_local = quarter * 32 + lane;   // TMEM lane = weight column inside the tile
-    const int et = threadIdx.x - (128 + C::kDeqWarps * 32);
+    const int n_local = quarter * 32 + column_of_lane(lane);   // weight column inside the tile
+    const int et = threadIdx.x - (128 + kDeqWarps * 32);
+    // token columns of this warp: all of the tile, or one half of it
+    const int half = (warp - (4 + kDeqWarps)) >> 2;
+    const int cc_half = C::kEpiWarps == 4 ? p.mt : ((p.mt >> 1) + 15) & ~15;
+    const int cc_begin = half * cc_half;
+    const int cc_end = cc_begin + cc_half < p.mt ? cc_begin + cc_half : p.mt;
     grid_dependency_wait();
     T* c = static_cast<T*>(p.c);
     const T* bias = static_cast<const T*>(p.bias);
+    const size_t slot_floats = static_cast<size_t>(p.mt) * kTileN;
     uint32_t seg = 0;
-    {
-      long long u = u_begin;
-      while (u < u_end) {
-        const int mtile = static_cast<int>(u / units);
-        const int m0 = mtile * p.mt;
-        const long long ul = u - static_cast<long long>(mtile) * units;
-        const int tile = static_cast<int>(ul / p.k_steps);
-        const int step0 = static_cast<int>(ul - static_cast<long long>(tile) * p.k_steps);
-        const long long tile_end = u - step0 + p.k_steps;
-        const long long seg_end = tile_end < u_end ? tile_end : u_end;
-        const bool whole = (step0 == 0) && (seg_end == tile_end);
-        // TA: the MMA issuers take alternate units of the CTA's run; in a one-unit segment
-        // only one of them has written its accumulators
-        bool issuer_has_units[C::kIssuers];
+    long long u = u_begin;
+    while (u < u_end) {
+      const long long tile = u / p.k_steps;
+      const int ntile = static_cast<int>(tile / p.m_tiles);
+      const int m0 = static_cast<int>(tile - static_cast<long long>(ntile) * p.m_tiles) * p.mt;
+      const long long tile_begin = tile * p.k_steps;
+      const long long tile_end = tile_begin + p.k_steps;
+      const long long seg_end = tile_end < u_end ? tile_end : u_end;
+      const bool whole = (u == tile_begin) && (seg_end == tile_end);
+      // the MMA issuers take alternate units of the CTA's run; in a one-unit segment only one
+      // of them has written its accumulators
+      bool issuer_has_units[C::kIssuers];
 #pragma unroll
-        for (int i = 0; i < C::kIssuers; ++i) {
-          // units of the segment are it0 .. it0 + len - 1; issuer i owns those with it % kIssuers == i
-          const long long it0 = u - u_begin, len = seg_end - u;
-          const long long first = it0 + ((i - it0 % C::kIssuers) + C::kIssuers) % C::kIssuers;
-          issuer_has_units[i] = first < it0 + len;
+      for (int i = 0; i < C::kIssuers; ++i) {
+        // units of the segment are it0 .. it0 + len - 1; issuer i owns those with it % kIssuers == i
+        const long long it0 = u - u_begin, len = seg_end - u;
+        const long long first = it0 + ((i - it0 % C::kIssuers) + C::kIssuers) % C::kIssuers;
+        issuer_has_units[i] = first < it0 + len;
+      }
+      const uint32_t buf = seg % C::kAccBufs, pacc = (seg / C::kAccBufs) & 1u;
+      ++seg;
+      // Where a partial segment goes. Cluster: this CTA's shared memory (the ring is idle once
+      // the accumulators of its only segment are complete). Equal runs: a slot in scratch;
+      // a CTA's run holds at most two partial segments, slot 2c if the tile began in an earlier
+      // CTA and slot 2c + 1 if it begins in c. The tile's arrival counter is its first CTA's.
+      const bool shared_in_cluster = p.cluster_s > 1;
+      const bool local = whole || shared_in_cluster;
+      const int first_cta = local ? 0 : cta_of_unit(units, ctas, tile_begin);
+      const int last_cta = local ? 0 : cta_of_unit(units, ctas, tile_end - 1);
+      const int parts = last_cta - first_cta + 1;
+      auto slot_of = [&](int part) {
+        return p.slots + static_cast<size_t>(2 * (first_cta + part) + (part == 0 ? 1 : 0)) * slot_floats;
+      };
+      unsigned int* counter = p.counters + first_cta;
+      const int n = ntile * kTileN + n_local;
+      const bool n_ok = n < p.n;
+      const int cols_ok = p.n - (ntile * kTileN + quarter * 32);   // of this warp's 32 columns
+      const float bias_v = (bias != nullptr && n_ok) ? to_f32<T>(bias[n]) : 0.f;
+      T* c_warp = c + static_cast<size_t>(m0) * p.n + ntile * kTileN + quarter * 32;
+      const bool begins_tile = u == tile_begin;
+      u = seg_end;
+      if (!mbar_wait_long(wctx, bar_acc_full + 8 * buf, pacc, 0x500u + buf)) break;
+      tc_fence_after_sync();
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * (C::kAccs * MTMAX);
+      float* slot = whole ? nullptr
+                    : shared_in_cluster ? reinterpret_cast<float*>(base_ptr)
+                                        : slot_of(begins_tile ? 0 : static_cast<int>(blockIdx.x) - first_cta);
+      for (int cc = cc_begin; cc < cc_end; cc += 16) {
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = 0.f;
+#pragma unroll
+        for (int acc = 0; acc < C::kAccs; ++acc) {
+          if (C::kIssuers > 1 && !issuer_has_units[acc / C::kAccsPerIssuer]) continue;   // stale accumulators
+          uint32_t r[16];
+          tmem_ld(taddr + acc * MTMAX + cc, r);
+          tmem_wait_ld(r);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
         }
-        const uint32_t buf = seg & 1u, pacc = (seg >> 1) & 1u;
-        ++seg;
-        u = seg_end;
-        if (!mbar_wait_long(wctx, bar_acc_full + 8 * buf, pacc, 0x500u + buf)) break;
-        tc_fence_after_sync();
-        const int n = tile * kTileN + n_local;
-        const bool n_ok = n < p.n;
-        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * (C::kAccs * MTMAX);
-        // which slot of the tile this CTA's segment is
-        // (only reached with a single token tile, where u indexes `units` directly)
-        const int first_cta = whole ? 0 : cta_of_unit(units, ctas, static_cast<long long>(tile) * p.k_steps);
-        const int last_cta = whole ? 0 : cta_of_unit(units, ctas, tile_end - 1);
-        const int parts = last_cta - first_cta + 1;
-        const int part = static_cast<int>(blockIdx.x) - first_cta;
-        float* slot = p.slots + (static_cast<size_t>(tile) * p.max_parts + part) * (static_cast<size_t>(p.mt) * kTileN);
-        const float bias_v = (whole && bias != nullptr && n_ok) ? to_f32<T>(bias[n]) : 0.f;
-        for (int cc = 0; cc < p.mt; cc += 16) {
-          float v[16];
+        if (whole) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = 0.f;
+          for (int j = 0; j < 16; ++j) v[j] += bias_v;
+          store_tokens16<T>(c_warp + static_cast<size_t>(cc) * p.n, p.n, v, lane, p.m - (m0 + cc), cols_ok,
+                            p.c_vec != 0);
+        } else {
 #pragma unroll
-          for (int acc = 0; acc < C::kAccs; ++acc) {
-            if (TA && !issuer_has_units[acc / (C::kAccs / C::kIssuers)]) continue;   // stale accumulators
-            uint32_t r[16];
-            tmem_ld(taddr + acc * MTMAX + cc, r);
-            tmem_wait_ld(r);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
-          }
-          if (whole) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int m = m0 + cc + j;
-              if (m < p.m && n_ok) c[static_cast<size_t>(m) * p.n + n] = from_f32<T>(v[j] + bias_v);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) slot[(cc + j) * kTileN + n_local] = v[j];
-          }
-        }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
-        if (!whole) {
-          // publish the partial, then find out whether this CTA completes the tile
-          __threadfence();
-          named_barrier_sync(1, 128);
-          if (et == 0) {
-            const unsigned int prev = atomicAdd(p.counters + tile, 1u);
-            *last_flag = (prev == static_cast<unsigned int>(parts - 1)) ? 1u : 0u;
-            if (prev == static_cast<unsigned int>(parts - 1)) p.counters[tile] = 0u;  // ready for the next launch
-          }
-          named_barrier_sync(1, 128);
-          if (*last_flag != 0u) {
-            __threadfence();
-            const float* tile_slots = p.slots + static_cast<size_t>(tile) * p.max_parts * (static_cast<size_t>(p.mt) * kTileN);
-            const float bv = (bias != nullptr && n_ok) ? to_f32<T>(bias[n]) : 0.f;
-            // eight rows at a time, all their loads issued before any is consumed
-            for (int mm0 = 0; mm0 < p.mt && m0 + mm0 < p.m; mm0 += 8) {
-              float sum[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) sum[j] = 0.f;
-              for (int q = 0; q < parts; ++q) {
-                const float* src = tile_slots + (static_cast<size_t>(q) * p.mt + mm0) * kTileN + n_local;
-                float v[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = __ldcg(src + j * kTileN);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) sum[j] += v[j];
-              }
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const int m = m0 + mm0 + j;
-                if (m < p.m && n_ok) c[static_cast<size_t>(m) * p.n + n] = from_f32<T>(sum[j] + bv);
-              }
-            }
-          }
-          named_barrier_sync(1, 128);  // last_flag may be rewritten only after everyone has read it
+          for (int q = 0; q < 4; ++q)
+            reinterpret_cast<float4*>(slot)[((cc >> 2) + q) * kTileN + n_local] =
+                make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
         }
       }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
+      if (!local) {
+        // publish the partial, then find out whether this CTA completes the tile
+        __threadfence();
+        named_barrier_sync(1, C::kEpiThreads);
+        if (et == 0) {
+          const unsigned int prev = atomicAdd(counter, 1u);
+          *last_flag = (prev == static_cast<unsigned int>(parts - 1)) ? 1u : 0u;
+          if (prev == static_cast<unsigned int>(parts - 1)) *counter = 0u;  // ready for the next launch
+        }
+        named_barrier_sync(1, C::kEpiThreads);
+        if (*last_flag != 0u) {
+          __threadfence();
+          // sixteen rows at a time; the loads of a part are issued before any is consumed
+          for (int cc = cc_begin; cc < cc_end && m0 + cc < p.m; cc += 16) {
+            float sum[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sum[j] = 0.f;
+#pragma unroll 2
+            for (int q = 0; q < parts; ++q) {
+              const float4* src = reinterpret_cast<const float4*>(slot_of(q)) + (cc >> 2) * kTileN + n_local;
+              float4 v[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) v[j] = __ldcg(src + j * kTileN);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                sum[4 * j] += v[j].x;
+                sum[4 * j + 1] += v[j].y;
+                sum[4 * j + 2] += v[j].z;
+                sum[4 * j + 3] += v[j].w;
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sum[j] += bias_v;
+            store_tokens16<T>(c_warp + static_cast<size_t>(cc) * p.n, p.n, sum, lane, p.m - (m0 + cc), cols_ok,
+                              p.c_vec != 0);
+          }
+        }
+        named_barrier_sync(1, C::kEpiThreads);  // last_flag may be rewritten only after everyone has read it
+      }
     }
+  }
+
+  if (p.cluster_s > 1) {
+    // Every CTA holds the partial sums of its part of K in shared memory. The cluster's warps
+    // share the (16 tokens x 32 columns) blocks of the tile, and add the parts in part order.
+    static_assert(MTMAX * kTileN * 4 <= C::kRing, "the partial tile fits the ring");
+    __syncwarp();
+    cluster_sync();
+    const int part = static_cast<int>(blockIdx.x) % p.cluster_s;
+    const int tile = static_cast<int>(blockIdx.x) / p.cluster_s;
+    const int ntile = tile / p.m_tiles, m0 = (tile - ntile * p.m_tiles) * p.mt;
+    constexpr int kWarps = C::kThreads / 32;
+    for (int i = part * kWarps + warp; i < p.mt / 4; i += p.cluster_s * kWarps) {
+      const int cc = (i >> 2) * 16, quarter = i & 3;
+      if (m0 + cc >= p.m) continue;
+      const int n_local = quarter * 32 + column_of_lane(lane), n = ntile * kTileN + n_local;
+      const T* bias = static_cast<const T*>(p.bias);
+      const uint32_t src = base + ((cc >> 2) * kTileN + n_local) * 16;
+      float sum[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) sum[j] = 0.f;
+      for (int q = 0; q < p.cluster_s; ++q) {
+        const uint32_t peer = cluster_map_shared(src, q);
+        float4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = ld_shared_cluster_f4(peer + j * (kTileN * 16));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sum[4 * j] += v[j].x;
+          sum[4 * j + 1] += v[j].y;
+          sum[4 * j + 2] += v[j].z;
+          sum[4 * j + 3] += v[j].w;
+        }
+      }
+      const float bias_v = (bias != nullptr && n < p.n) ? to_f32<T>(bias[n]) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) sum[j] += bias_v;
+      store_tokens16<T>(static_cast<T*>(p.c) + static_cast<size_t>(m0 + cc) * p.n + ntile * kTileN + quarter * 32, p.n,
+                        sum, lane, p.m - (m0 + cc), p.n - (ntile * kTileN + quarter * 32), p.c_vec != 0);
+    }
+    __syncwarp();
+    cluster_sync();   // nobody reads this CTA's shared memory any more
   }
 
   // ------------------------------- teardown -------------------------------
@@ -744,11 +780,11 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   }
 }
 
-template <typename T, int MTMAX, bool TA>
-ks_status_t launch_t(const W4A16Args& a, const CUtensorMap& tm_w, const CUtensorMap& tm_s, const CUtensorMap& tm_z,
-                     const CUtensorMap& tm_a, const Params& p, int grid, cudaStream_t stream) {
-  using C = Cfg<MTMAX, TA>;
-  auto kernel = w4a16_umma_kernel<T, MTMAX, TA>;
+template <typename T, int MTMAX, bool FINE>
+ks_status_t launch_t(const CUtensorMap& tm_w, const CUtensorMap& tm_a, const Params& p, int grid,
+                     cudaStream_t stream) {
+  using C = Cfg<MTMAX>;
+  auto kernel = w4a16_umma_kernel<T, MTMAX, FINE>;
   static std::mutex mu;
   static bool attr_done[64] = {};
   int dev = 0;
@@ -761,17 +797,29 @@ ks_status_t launch_t(const W4A16Args& a, const CUtensorMap& tm_w, const CUtensor
       attr_done[dev] = true;
     }
   }
-  return cuda_status(launch_programmatic(kernel, static_cast<unsigned>(grid), C::kThreads, C::kSmemBytes, stream, tm_w,
-                                         tm_s, tm_z, tm_a, p),
+  return cuda_status(launch_programmatic_cluster(kernel, static_cast<unsigned>(grid), static_cast<unsigned>(p.cluster_s),
+                                                 C::kThreads, C::kSmemBytes, stream, tm_w, tm_a, p),
                      "ks_gemm_w4a16");
+}
+
+template <typename T, bool FINE>
+ks_status_t launch_mt(int mtmax, const CUtensorMap& tm_w, const CUtensorMap& tm_a, const Params& p, int grid,
+                      cudaStream_t stream) {
+  switch (mtmax) {
+    case 32: return launch_t<T, 32, FINE>(tm_w, tm_a, p, grid, stream);
+    case 64: return launch_t<T, 64, FINE>(tm_w, tm_a, p, grid, stream);
+    case 128: return launch_t<T, 128, FINE>(tm_w, tm_a, p, grid, stream);
+    default: return launch_t<T, 256, FINE>(tm_w, tm_a, p, grid, stream);
+  }
 }
 
 }  // namespace
 
 bool w4a16_eligible(const W4A16Args& a) {
   if (a.k % kStepK != 0) return false;
-  if (a.group_size % kStepK != 0) return false;   // one scale row per 128-k step
-  if (a.n % 16 != 0) return false;                // 16-byte row pitch of the packed weight and of the scales
+  // one scale row per 128-k step, or a whole number of rows per step
+  if (a.group_size % kStepK != 0 && a.group_size != 64 && a.group_size != 32) return false;
+  if (a.n % 16 != 0) return false;                // 16-byte row pitch of the packed weight
   if (!aligned16(a.a) || !aligned16(a.b_packed) || !aligned16(a.scales)) return false;
   if (a.zeros != nullptr && !aligned16(a.zeros)) return false;
   if (a.m > (1 << 24) || a.n > (1 << 28) || a.k > (1 << 28)) return false;
@@ -781,72 +829,107 @@ bool w4a16_eligible(const W4A16Args& a) {
 namespace {
 
 struct Geometry {
-  int mt = 0, mtmax = 0, n_tiles = 0, k_steps = 0, grid = 0, max_parts = 0;
+  int mt = 0, mtmax = 0, m_tiles = 0, n_tiles = 0, k_steps = 0, grid = 0;
+  int cluster_s = 1;
+  bool split = true;
   size_t counter_bytes = 0, slot_bytes = 0;
 };
 
+// Time of one unit (128 columns x 128 k) of a token tile of `mt` rows in a long run, in ns;
+// measured as the slope of time against K with one whole tile per CTA.
+double unit_ns(int mt, bool fine) {
+  const double t = mt <= 64 ? 300.0 : mt <= 128 ? 300.0 + (mt - 64) * 1.6 : 400.0 + (mt - 128) * 2.0;
+  return fine ? t * 1.2 : t;
+}
+
+// Token tiles, and how the units go to the CTAs: whichever finishes first by this estimate.
+//   cluster    a tile's K range over S CTAs, which exchange partial sums through shared memory
+//              (~1.5 us); needs all clusters resident at once
+//   whole      runs of whole tiles: the last round may leave SMs idle
+//   even runs  no SM idles, but a tile's last CTA reads the other parts from L2: ~0.25 us per part and
+//              16 token rows (two warps share that work in 256-row tiles)
+// Fewer token tiles mean fewer dequantisations of a weight; more of them, more tiles to deal out.
 Geometry geometry_of(const W4A16Args& a) {
   Geometry g;
-  const int mt_raw = static_cast<int>(a.m < 128 ? a.m : 128);
-  g.mt = (mt_raw + 15) & ~15;
-  g.mtmax = g.mt <= 32 ? 32 : 128;
-  g.n_tiles = static_cast<int>((a.n + kTileN - 1) / kTileN);
-  g.k_steps = static_cast<int>(a.k / kStepK);
-  const long long units = static_cast<long long>(g.n_tiles) * g.k_steps;
   const int sms = sm_count();
-  g.grid = static_cast<int>(units < sms ? units : sms);
-  const long long per_cta = units / g.grid;  // shortest run
-  g.max_parts = static_cast<int>((g.k_steps + per_cta - 1) / per_cta) + 1;
-  g.slot_bytes = static_cast<size_t>(g.n_tiles) * g.max_parts * g.mt * kTileN * sizeof(float);
-  g.counter_bytes = (static_cast<size_t>(g.n_tiles) * sizeof(unsigned int) + 255) & ~size_t(255);
+  const bool fine = a.group_size % kStepK != 0;
+  g.n_tiles = static_cast<int>((a.n + kTileN - 1) / kTileN);
+  g.k_steps = static_cast<int>((a.k / kStepK + 1) & ~int64_t(1));
+  double best = 0;
+  auto offer = [&](double cost, int mt, int m_tiles, int cluster_s, bool split) {
+    if (best != 0 && cost >= best) return;
+    best = cost;
+    g.mt = mt;
+    g.m_tiles = m_tiles;
+    g.cluster_s = cluster_s;
+    g.split = split;
+  };
+  const int lo = static_cast<int>((a.m + 255) / 256), hi = static_cast<int>((a.m + 31) / 32);
+  for (int want = lo; want <= hi && want < lo + 24; ++want) {
+    const int mt = static_cast<int>(((a.m + want - 1) / want + 15) & ~int64_t(15));
+    const int m_tiles = static_cast<int>((a.m + mt - 1) / mt);
+    const long long tiles = static_cast<long long>(g.n_tiles) * m_tiles;
+    const double unit = unit_ns(mt, fine);
+    const double drain = mt * 8.0;   // accumulators to C
+    offer(static_cast<double>((tiles + sms - 1) / sms) * (g.k_steps * unit + drain), mt, m_tiles, 1, false);
+    for (int s = 2; s <= kMaxClusterSplit && 2 * s <= g.k_steps && tiles * s <= sms; ++s) {
+      if (cluster_capacity(s) < tiles) break;
+      offer(2.0 * ((g.k_steps / 2 + s - 1) / s) * unit + drain + 1500.0, mt, m_tiles, s, false);
+    }
+    const double per_cta = static_cast<double>(tiles) * g.k_steps / (tiles * g.k_steps < sms ? tiles * g.k_steps : sms);
+    const double parts = g.k_steps / per_cta + 1.0;
+    const int chunks = mt <= 128 ? mt / 16 : (mt + 31) / 32;
+    offer(per_cta * unit + 2 * drain + 250.0 * chunks * parts, mt, m_tiles, 1, true);
+  }
+  g.mtmax = g.mt <= 32 ? 32 : (g.mt <= 64 ? 64 : (g.mt <= 128 ? 128 : 256));
+  const long long tiles = static_cast<long long>(g.n_tiles) * g.m_tiles;
+  const long long work = g.split ? tiles * g.k_steps : tiles;
+  g.grid = g.cluster_s > 1 ? static_cast<int>(tiles * g.cluster_s) : static_cast<int>(work < sms ? work : sms);
+  g.slot_bytes = g.split ? static_cast<size_t>(g.grid) * 2 * g.mt * kTileN * sizeof(float) : 0;
+  g.counter_bytes = (static_cast<size_t>(g.grid) * sizeof(unsigned int) + 255) & ~size_t(255);
   return g;
 }
 
+// What the fixed scratch array is held against: counters and slots per (column tile, part) of equal
+// runs with one token tile of up to 128 rows. The shapes that entry point takes do not depend on
+// how a launch is dealt out.
+size_t per_tile_scratch(const W4A16Args& a) {
+  const int sms = sm_count();
+  const long long mt = (a.m + 15) & ~int64_t(15);
+  const long long n_tiles = (a.n + kTileN - 1) / kTileN, k_steps = a.k / kStepK;
+  const long long units = n_tiles * k_steps;
+  const long long per_cta = units / (units < sms ? units : sms);   // shortest run
+  const long long max_parts = (k_steps + per_cta - 1) / per_cta + 1;
+  return static_cast<size_t>(n_tiles * max_parts * mt * kTileN) * sizeof(float) +
+         ((static_cast<size_t>(n_tiles) * sizeof(unsigned int) + 255) & ~size_t(255));
+}
+
 // Encodes the tensor maps and enqueues the kernel on scratch memory the caller of this
-// function has already obtained: the per-tile arrival counters (all zero on entry; the
+// function has already obtained: the arrival counters (all zero on entry; the
 // kernel leaves them zero) and the fp32 partial slots.
 ks_status_t enqueue_w4a16(const W4A16Args& a, const Geometry& g, unsigned int* counters, float* slots,
                           unsigned int* fault_word, cudaStream_t stream) {
   const bool bf16 = a.dtype == KS_DTYPE_BF16;
-  const int mt = g.mt, mtmax = g.mtmax, n_tiles = g.n_tiles, k_steps = g.k_steps, grid = g.grid,
-            max_parts = g.max_parts;
   const CUtensorMapDataType dt16 = bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  // Decode shapes hand the weights over in tensor memory unless told otherwise; that path
-  // loads the packed weight two K-steps at a time.
-  const bool tmem_operand = mtmax == 32 && a.operand_path != 1 && (k_steps % 2 == 0);
-  CUtensorMap tm_w, tm_s, tm_z, tm_a;
+  CUtensorMap tm_w, tm_a;
   {
+    // two K-steps per box; a step past the end of K reads zeros
     const uint64_t dims[2] = {static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.k / 2)};
     const uint64_t str[1] = {static_cast<uint64_t>(a.n)};
-    const uint32_t box[2] = {static_cast<uint32_t>(kTileN), static_cast<uint32_t>(tmem_operand ? kStepK : kStepK / 2)};
-    if (!tma_encode(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a.b_packed, dims, str, box, CU_TENSOR_MAP_SWIZZLE_NONE))
+    const uint32_t box[2] = {static_cast<uint32_t>(kTileN), static_cast<uint32_t>(kStepK)};
+    if (!tma_encode(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a.b_packed, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B))
       KSB_FAIL(KS_ERROR_INTERNAL, "ks_gemm_w4a16: tensor map for the packed weight rejected");
   }
   {
-    const uint64_t dims[2] = {static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.k / a.group_size)};
-    const uint64_t str[1] = {static_cast<uint64_t>(a.n) * 2};
-    const uint32_t box[2] = {static_cast<uint32_t>(kTileN), 1u};
-    if (!tma_encode(&tm_s, dt16, 2, a.scales, dims, str, box, CU_TENSOR_MAP_SWIZZLE_NONE))
-      KSB_FAIL(KS_ERROR_INTERNAL, "ks_gemm_w4a16: tensor map for the scales rejected");
-    if (!tma_encode(&tm_z, dt16, 2, a.zeros != nullptr ? a.zeros : a.scales, dims, str, box,
-                    CU_TENSOR_MAP_SWIZZLE_NONE))
-      KSB_FAIL(KS_ERROR_INTERNAL, "ks_gemm_w4a16: tensor map for the zero-points rejected");
-  }
-  if (tmem_operand) {
-    // A[M,K] seen as [K/64][M][64]: one box brings both 64-k swizzle atoms of a K-step
+    // A[M,K] seen as [K/64][M][64]: a box brings one or both 64-k swizzle atoms of a K-step
     const uint64_t dims[3] = {64u, static_cast<uint64_t>(a.m), static_cast<uint64_t>(a.k / 64)};
     const uint64_t str[2] = {static_cast<uint64_t>(a.k) * 2, 128u};
-    const uint32_t box[3] = {64u, static_cast<uint32_t>(mt), 2u};
+    const uint32_t box[3] = {64u, static_cast<uint32_t>(g.mt), g.mtmax <= 128 ? 2u : 1u};
     if (!tma_encode(&tm_a, dt16, 3, a.a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B))
-      KSB_FAIL(KS_ERROR_INTERNAL, "ks_gemm_w4a16: tensor map for the activations rejected");
-  } else {
-    const uint64_t dims[2] = {static_cast<uint64_t>(a.k), static_cast<uint64_t>(a.m)};
-    const uint64_t str[1] = {static_cast<uint64_t>(a.k) * 2};
-    const uint32_t box[2] = {64u, static_cast<uint32_t>(mt)};
-    if (!tma_encode(&tm_a, dt16, 2, a.a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B))
       KSB_FAIL(KS_ERROR_INTERNAL, "ks_gemm_w4a16: tensor map for the activations rejected");
   }
 
+  const bool fine = a.group_size % kStepK != 0;
   Params p;
   p.c = a.c;
   p.bias = a.bias;
@@ -858,25 +941,26 @@ ks_status_t enqueue_w4a16(const W4A16Args& a, const Geometry& g, unsigned int* c
   p.m = static_cast<int>(a.m);
   p.n = static_cast<int>(a.n);
   p.k = static_cast<int>(a.k);
-  p.mt = mt;
-  p.m_tiles = static_cast<int>((a.m + mt - 1) / mt);
-  p.n_tiles = n_tiles;
-  p.k_steps = k_steps;
-  p.gs_steps = a.group_size / kStepK;
-  p.max_parts = max_parts;
+  p.mt = g.mt;
+  p.m_tiles = g.m_tiles;
+  p.n_tiles = g.n_tiles;
+  p.k_steps = g.k_steps;
+  p.gs_steps = fine ? 1 : a.group_size / kStepK;
+  p.sub_shift = a.group_size == 64 ? 1 : 0;
+  p.groups = static_cast<int>(a.k / a.group_size);
+  p.split = g.split ? 1 : 0;
+  p.cluster_s = g.cluster_s;
+  p.c_vec = (reinterpret_cast<uintptr_t>(a.c) & 7) == 0 ? 1 : 0;
   p.has_zeros = a.zeros != nullptr ? 1 : 0;
   const uint32_t fmt = bf16 ? 1u : 0u;
-  // weights: MN-major in shared memory, K along the columns in tensor memory
-  p.idesc = umma_instr_desc(fmt, fmt, tmem_operand ? 0u : 1u, 0u, 128u, static_cast<uint32_t>(mt));
+  // weights: K along the columns in tensor memory
+  p.idesc = umma_instr_desc(fmt, fmt, 0u, 0u, 128u, static_cast<uint32_t>(g.mt));
 
-  if (bf16) {
-    if (tmem_operand) return launch_t<__nv_bfloat16, 32, true>(a, tm_w, tm_s, tm_z, tm_a, p, grid, stream);
-    return mtmax == 32 ? launch_t<__nv_bfloat16, 32, false>(a, tm_w, tm_s, tm_z, tm_a, p, grid, stream)
-                       : launch_t<__nv_bfloat16, 128, false>(a, tm_w, tm_s, tm_z, tm_a, p, grid, stream);
-  }
-  if (tmem_operand) return launch_t<__half, 32, true>(a, tm_w, tm_s, tm_z, tm_a, p, grid, stream);
-  return mtmax == 32 ? launch_t<__half, 32, false>(a, tm_w, tm_s, tm_z, tm_a, p, grid, stream)
-                     : launch_t<__half, 128, false>(a, tm_w, tm_s, tm_z, tm_a, p, grid, stream);
+  if (bf16)
+    return fine ? launch_mt<__nv_bfloat16, true>(g.mtmax, tm_w, tm_a, p, g.grid, stream)
+                : launch_mt<__nv_bfloat16, false>(g.mtmax, tm_w, tm_a, p, g.grid, stream);
+  return fine ? launch_mt<__half, true>(g.mtmax, tm_w, tm_a, p, g.grid, stream)
+              : launch_mt<__half, false>(g.mtmax, tm_w, tm_a, p, g.grid, stream);
 }
 
 }  // namespace
@@ -970,13 +1054,22 @@ size_t w4a16_static_scratch_capacity() { return kStaticScratchBytes; }
 
 ks_status_t launch_w4a16_static(const W4A16Args& a, cudaStream_t stream) {
   const bool dec = use_decode_kernel(a);
-  const Geometry g = dec ? Geometry{} : geometry_of(a);
+  Geometry g = dec ? Geometry{} : geometry_of(a);
   const decode::Geometry gd = dec ? decode::geometry_of(a) : decode::Geometry{};
   const size_t counter_bytes = dec ? gd.counter_bytes : g.counter_bytes;
-  // With several token tiles the tcgen05 kernel snaps its runs to whole column tiles and
-  // never touches the partial slots.
-  const size_t slot_bytes = dec ? gd.slot_bytes : (a.m > 128 ? 0 : g.slot_bytes);
-  const size_t need = counter_bytes + slot_bytes;
+  size_t need = gd.counter_bytes + gd.slot_bytes;
+  if (!dec) {
+    // more than 128 rows, and scale groups of 32 or 64, are taken at any size
+    const bool any_size = a.m > 128 || a.group_size % kStepK != 0;
+    need = any_size ? 0 : per_tile_scratch(a);
+    if (g.split && g.counter_bytes + g.slot_bytes > kStaticScratchBytes) {
+      // whole tiles per CTA need no slots
+      g.split = false;
+      const long long tiles = static_cast<long long>(g.n_tiles) * g.m_tiles;
+      g.grid = static_cast<int>(tiles < sm_count() ? tiles : sm_count());
+      g.slot_bytes = 0;
+    }
+  }
   if (need > kStaticScratchBytes) {
     char msg[224];
     snprintf(msg, sizeof(msg),

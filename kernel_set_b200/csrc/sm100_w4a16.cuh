@@ -19,10 +19,6 @@ struct W4A16Args {
   int64_t m = 0, n = 0, k = 0;
   int group_size = 128;            // already resolved (> 0, divides k)
   ks_dtype_t dtype = KS_DTYPE_BF16;
-  // How the tcgen05 kernel hands the dequantised weights of decode shapes (at most 32
-  // token rows) to the tensor core: 0 = choose (tensor memory), 1 = shared memory,
-  // 2 = tensor memory.
-  int operand_path = 0;
   // Which fast kernel: 0 = choose, 1 = tcgen05 (sm100_w4a16.cu), 2 = register-operand
   // decode kernel (w4a16_decode.cu).
   int kernel = 0;
@@ -40,8 +36,8 @@ __host__ __device__ __forceinline__ int cta_of_unit(long long units, int ctas, l
   return c;
 }
 
-// True when the tcgen05 kernel can take the problem: K and group_size multiples
-// of 128, N a multiple of 16, 16-byte aligned operands, driver entry point found.
+// True when the tcgen05 kernel can take the problem: K a multiple of 128, group_size a
+// multiple of 128 or 32 or 64, N a multiple of 16, 16-byte aligned operands, driver entry point found.
 bool w4a16_eligible(const W4A16Args& a);
 
 // Encodes the tensor maps, sizes the scratch memory and enqueues one launch.

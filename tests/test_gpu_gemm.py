@@ -592,3 +592,52 @@ def test_grouped_gemm_fp8_256_experts(ks, cuda, n, k):
         check_gemm(out[lo:hi].cpu(), ref32, noise, f"256 experts, expert {i} ({hi - lo} rows) n={n} k={k}")
     # rows of the emptied experts do not exist; the row after them belongs to the next expert
     assert int(offs[4]) == int(offs[3]) and int(offs[201]) == int(offs[200])
+
+
+@pytest.mark.parametrize("m,k,n,gs,dtype,zeros,bias", [
+    (33, 1024, 272, 32, torch.bfloat16, "random", False),    # 48-row token tile, four scale rows per K-step
+    (64, 1152, 528, 64, torch.float16, "random", True),      # odd number of K-steps: the padded half box
+    (65, 640, 1040, 64, torch.bfloat16, "fraction", False),  # fp32 dequantisation
+    (3, 384, 144, 32, torch.float16, None, True),            # narrow tile, no zero-points, odd K-steps
+    (100, 4096, 400, 64, torch.float16, "random", False),    # few column tiles: a cluster per tile
+    (129, 512, 2064, 128, torch.bfloat16, "eight", True),
+    (256, 1152, 1040, 128, torch.float16, "random", False),
+    (257, 768, 656, 128, torch.bfloat16, "random", False),   # several token tiles
+    (700, 256, 16400, 32, torch.bfloat16, "eight", False),   # whole tiles per CTA, several rounds
+    (1001, 2048, 2064, 256, torch.float16, "random", True),  # ragged in every direction
+    (24, 2048, 28688, 128, torch.bfloat16, "random", True),  # equal runs: tiles shared through scratch
+    (128, 1024, 28688, 64, torch.float16, "random", False),
+    (250, 2048, 20496, 128, torch.bfloat16, "eight", False),
+])
+def test_w4a16_tcgen05_token_tiles_and_fine_groups(ks, cuda, m, k, n, gs, dtype, zeros, bias):
+    """Every token-tile width, scale groups narrower than a K-step, odd numbers of K-steps, and each
+    way of dealing the work out (the fixed-scratch entry point never shares tiles through scratch above
+    128 rows), against the general kernel, which multiplies the same rounded weights: summation order only."""
+    g = gen(m + k + n)
+    a = torch.randn(m, k, generator=g).to(dtype).to(cuda)
+    b_packed = torch.randint(0, 256, (k // 2, n), generator=g, dtype=torch.uint8).to(cuda)
+    scales = (torch.randn(k // gs, n, generator=g).mul(0.02).abs() + 1e-3).to(dtype).to(cuda)
+    zp = {"eight": lambda: torch.full((k // gs, n), 8.0), "random": lambda: torch.randint(0, 16, (k // gs, n), generator=g),
+          "fraction": lambda: torch.rand(k // gs, n, generator=g) * 15, None: lambda: None}[zeros]()
+    zp = zp.to(dtype).to(cuda) if zp is not None else None
+    bias_t = torch.randn(n, generator=g).to(dtype).to(cuda) if bias else None
+    ref32 = orc.w4a16(a.cpu(), b_packed.cpu(), scales.cpu(), zp.cpu() if zp is not None else None, gs,
+                      bias_t.cpu() if bias else None, out_dtype=None)
+    w = orc.w4a16_weight(b_packed.cpu(), scales.cpu(), zp.cpu() if zp is not None else None, gs).float()
+    noise = accumulation_noise(a.cpu().float().abs(), w.abs(), k)
+    with w4_path("tcgen05"):
+        out = ks.dispatch.w4a16(a, b_packed, scales, zp, group_size=gs, bias=bias_t)
+        out2 = ks.dispatch.w4a16(a, b_packed, scales, zp, group_size=gs, bias=bias_t)
+        stat = ks.gemm.gemm_w4a16_static_scratch(torch.empty_like(out), a, b_packed, scales, zp, m, n, k, gs, bias=bias_t)
+        # an output that is only 2-byte aligned takes the element-wise stores
+        odd = torch.empty(m * n + 1, dtype=dtype, device=cuda)[1:].view(m, n)
+        ks.gemm.gemm_w4a16(odd, a, b_packed, scales, zp, m, n, k, gs, bias=bias_t)
+        torch.cuda.synchronize()
+        ks.runtime.stream_synchronize(0)
+    check_gemm(out.cpu(), ref32, noise, f"w4a16 {m}x{n}x{k} group {gs}")
+    check_gemm(stat.cpu(), ref32, noise, f"w4a16 fixed scratch {m}x{n}x{k} group {gs}")
+    assert torch.equal(out.view(torch.int16), out2.view(torch.int16)), "not reproducible run to run"
+    assert torch.equal(out.view(torch.int16), odd.view(torch.int16))
+    with w4_path("general"):
+        gen_out = ks.dispatch.w4a16(a, b_packed, scales, zp, group_size=gs, bias=bias_t)
+    assert orc.rel_frobenius(out.cpu().float(), gen_out.cpu().float()) < 2e-3
