@@ -43,6 +43,13 @@
 // better: handing the accumulator over in two 128-column halves (eight N=128 MMAs per
 // K-block read A twice: 232 us), wider loads, more loads in flight, sixteen narrower epilogue
 // warps, 224-wide tiles, scalar FMAs, paced MMA issue, sleeping or spinning waits.
+// Problems with fewer tiles than SMs (decode: M = 16, N = 7168 is 28 tiles of 256 columns) are
+// cut along K as well, over the S <= 8 CTAs of a cluster: each leaves its fp32 partial tile in
+// its own shared memory (the ring is idle by then), and after a cluster barrier every CTA
+// adds the S partials of its share of the tile's rows in part order, over distributed shared
+// memory, and writes them. No scratch memory, no second kernel. S and the tile width are
+// chosen in launch_fp8_blockwise(). Measured (cold L2): M=16, N=K=7168 28.7 -> 22.6 us; M=228,
+// N=944, K=10256 38.9 -> 18.5; M=6, N=624, K=3712 16.4 -> 12.3; M=128, N=2048, K=7168 24.6 -> 16.4.
 // B may be stored [N,K] (K-major UMMA operand) or [K,N] (MN-major operand, the
 // layout of the reference C ABI); both are loaded by TMA without a transpose.
 //
@@ -139,6 +146,7 @@ struct Params {
   int split_items;        // number of K-part items (tail tiles x split_s), at most the grid size
   int split_s;            // 1 = no split
   float4* split_slots;    // [tail tile][part][epilogue warp][16-byte column chunk][lane]
+  int cluster_s;          // > 1: every tile is split (split_from = 0) over the CTAs of a cluster
   // MODE 1 / 2 (one scale per row and per column, the whole K range accumulated in TMEM)
   int64_t as_row_stride, as_kb_stride;   // a_scale[row * as_row_stride + kb * as_kb_stride]
   const void* bias;       // [N] in the output type or NULL
@@ -241,6 +249,26 @@ static_assert(128 * Cfg<256>::kRegsIssue + (Cfg<256>::kThreads - 128) * Cfg<256>
                   Cfg<256>::kThreads * ((65536 / Cfg<256>::kThreads) & ~7),
               "setmaxnreg budgets exceed the register pool the CTA is launched with");
 
+// Four adjacent outputs, rounded once; `valid` of them lie inside the row.
+template <typename OutT>
+__device__ __forceinline__ void store_4(OutT* dst, const float4& v, bool vec_ok, int valid) {
+  const float v4[4] = {v.x, v.y, v.z, v.w};
+  if (vec_ok && valid >= 4) {
+    if constexpr (std::is_same<OutT, float>::value) {
+      *reinterpret_cast<float4*>(dst) = v;
+    } else {
+      OutT o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[j] = from_f32<OutT>(v4[j]);
+      *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < valid) dst[j] = from_f32<OutT>(v4[j]);
+  }
+}
+
 // MODE 0: block-scaled FP8 (a partial per K-block, promoted in registers).
 // MODE 1: FP8 with one scale per row of A and one per column of B: the whole K range
 //         accumulates in tensor memory, the epilogue runs once per tile.
@@ -311,14 +339,22 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
       }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
       int run = 0;
-      for (int e = 0; e < p.num_experts; ++e) {
-        prefix[e] = run;
-        const int rows = ends[e] - offs[e];
-        run += rows > 0 ? (rows + kBM - 1) / kBM : 0;
+      for (int e0 = 0; e0 < p.num_experts; e0 += 32) {
+        const int e = e0 + lane;
+        const int rows = e < p.num_experts ? ends[e] - offs[e] : 0;
+        const int tiles = rows > 0 ? (rows + kBM - 1) / kBM : 0;
+        int inc = tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += t;
+        }
+        if (e < p.num_experts) prefix[e] = run + inc - tiles;
+        run += __shfl_sync(0xffffffffu, inc, 31);
       }
-      prefix[p.num_experts] = run;
+      if (lane == 0) prefix[p.num_experts] = run;
     }
   }
   tc_fence_before_sync();
@@ -546,7 +582,18 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
       }
       bool stored = false;
       if constexpr (!GROUPED) {
-        if (ok && tc.part >= 0) {
+        if (ok && tc.part >= 0 && p.cluster_s > 1) {
+          // One K-part of a tile that the cluster shares: rows of BN + 4 floats (the padding
+          // keeps the 16-byte stores of eight neighbouring lanes on different banks).
+          if (row_ok) {
+            const uint32_t dst = ring + (row_in_tile * (BN + 4) + slice * EC) * 4;
+#pragma unroll
+            for (int c4 = 0; c4 < EC / 4; ++c4)
+              st_shared_v4(dst + c4 * 16, __float_as_uint(acc[2 * c4].x), __float_as_uint(acc[2 * c4].y),
+                           __float_as_uint(acc[2 * c4 + 1].x), __float_as_uint(acc[2 * c4 + 1].y));
+          }
+          stored = true;
+        } else if (ok && tc.part >= 0) {
           // One K-part of a split tile. The warp's 32 x EC partial goes to its slot (16 bytes
           // per lane and column chunk, chunks 512 B apart: every store of the warp is one
           // contiguous 512-byte piece); split_reduce_kernel adds the parts up afterwards.
@@ -614,6 +661,36 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     if constexpr (C::kRebalanceRegs) setmaxnreg_dec<C::kRegsIssue>();
   }
 
+  if constexpr (!GROUPED && MODE == 0) {
+    static_assert(kBM * (BN + 4) * 4 <= C::kStages * C::kStageBytes, "the partial tile fits the ring");
+    if (p.cluster_s > 1) {
+      __syncwarp();
+      cluster_sync();   // every CTA's partial is in its shared memory
+      if (warp >= 4) {
+        // this CTA's share of the tile, in units of four columns
+        TileCoord tc;
+        locate_tile<BN, GROUPED>(p, prefix, offs, static_cast<int>(blockIdx.x), &tc);
+        const int rows = tc.row_end - tc.row0 < kBM ? tc.row_end - tc.row0 : kBM;
+        const int total = rows * (BN / 4);
+        const int begin = (tc.part * total) / p.cluster_s, end = ((tc.part + 1) * total) / p.cluster_s;
+        for (int i = begin + static_cast<int>(threadIdx.x) - 128; i < end; i += C::kEpiWarps * 32) {
+          const int r = i / (BN / 4), col = tc.n0 + (i % (BN / 4)) * 4;
+          if (col >= p.n) continue;
+          const uint32_t src = ring + (r * (BN + 4) + (i % (BN / 4)) * 4) * 4;
+          float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int q = 0; q < p.cluster_s; ++q) {
+            const float4 v = ld_shared_cluster_f4(cluster_map_shared(src, q));
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+          }
+          store_4<OutT>(static_cast<OutT*>(p.out) + static_cast<size_t>(tc.row0 + r) * p.n + col, sum,
+                        p.vec_store != 0, p.n - col);
+        }
+      }
+      __syncwarp();
+      cluster_sync();   // nobody reads this CTA's shared memory any more
+    }
+  }
+
   // ------------------------------- teardown -------------------------------
   tc_fence_before_sync();
   __syncthreads();
@@ -664,22 +741,7 @@ split_reduce_kernel(OutT* __restrict__ out, const float4* __restrict__ slots, in
     sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
   }
   if (row >= m || col >= n) return;
-  OutT* dst = out + static_cast<size_t>(row) * n + col;
-  const float v4[4] = {sum.x, sum.y, sum.z, sum.w};
-  if (vec_ok && col + 4 <= n) {
-    if constexpr (std::is_same<OutT, float>::value) {
-      *reinterpret_cast<float4*>(dst) = sum;
-    } else {
-      OutT o[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) o[j] = from_f32<OutT>(v4[j]);
-      *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (col + j < n) dst[j] = from_f32<OutT>(v4[j]);
-  }
+  store_4<OutT>(out + static_cast<size_t>(row) * n + col, sum, vec_ok != 0, n - col);
 }
 
 // ------------------------------- host side --------------------------------
@@ -741,6 +803,21 @@ ks_status_t launch_one(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUte
   // (Programmatic dependent launch was measured on the quantizer -> GEMM -> reducer chain and
   // lost 1 % there: these kernels have no input-independent prologue worth overlapping, and
   // the dependency wait costs more than an ordinary kernel boundary.)
+  if (p.cluster_s > 1) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(C::kThreads);
+    cfg.dynamicSmemBytes = C::smem_bytes(GROUPED);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = p.cluster_s;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, tm_a, tm_b, tm_cs, p), a.where);
+  }
   kernel<<<grid, C::kThreads, C::smem_bytes(GROUPED), stream>>>(tm_a, tm_b, tm_cs, p);
   if constexpr (!GROUPED) {
     if (p.split_s > 1) {
@@ -819,7 +896,36 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   // back, ~512 / ~300 cycles per K-block, and the wide tile wins whenever it needs no more rounds)
   const int64_t cost256 = ((tiles256 + sms - 1) / sms) * (a.mode == 0 ? 850 : 512);
   const int64_t cost128 = ((tiles128 + sms - 1) / sms) * (a.mode == 0 ? 550 : 300);
-  const int bn = (a.force_bn == 128 || a.force_bn == 256) ? a.force_bn : (cost256 <= cost128 ? 256 : 128);
+  int bn = (a.force_bn == 128 || a.force_bn == 256) ? a.force_bn : (cost256 <= cost128 ? 256 : 128);
+
+  // Fewer tiles than SMs (dense block-scaled problems): cut every tile along K over a cluster of
+  // S CTAs. Same unit of cost; sharing a tile adds two cluster barriers and the exchange
+  // of the partials (~3000 cycles). At least two K-blocks per CTA.
+  int cluster_s = 1;
+  if (!grouped && a.mode == 0 && a.force_split != 0 && a.num_out_parts == 0) {
+    const int64_t nkb = (a.k + kBK - 1) / kBK;
+    int64_t best = INT64_MAX;
+    for (int w = 256; w >= 128; w -= 128) {
+      if ((a.force_bn == 128 || a.force_bn == 256) && a.force_bn != w) continue;
+      const int64_t tiles = w == 256 ? tiles256 : tiles128;
+      const int64_t per_kb = w == 256 ? 850 : 550;
+      const int64_t whole = (tiles + sms - 1) / sms * nkb * per_kb;
+      if (whole < best) {
+        best = whole;
+        bn = w;
+        cluster_s = 1;
+      }
+      for (int s = 2; s <= kMaxClusterSplit && tiles * s <= sms && nkb >= 2 * s; ++s) {
+        if (cluster_capacity(s) < tiles) break;   // all clusters run at once
+        const int64_t cost = (nkb + s - 1) / s * per_kb + 3000;
+        if (cost < best) {
+          best = cost;
+          bn = w;
+          cluster_s = s;
+        }
+      }
+    }
+  }
 
   CUtensorMap tm_a, tm_b;
   // 16-bit operands (mode 3) are described to TMA as bytes: a row of A is 2K bytes, of B 2N
@@ -890,7 +996,7 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   p.vec_store = (out_aligned && (static_cast<size_t>(a.n) * out_elt) % 16 == 0) ? 1 : 0;
 
   int64_t tiles = tiles_m_bound * p.tiles_n;
-  const int grid = static_cast<int>(tiles < sms ? (tiles < 1 ? 1 : tiles) : sms);
+  const int grid = static_cast<int>(cluster_s > 1 ? tiles * cluster_s : (tiles < sms ? (tiles < 1 ? 1 : tiles) : sms));
 
   // K-split of the last partial round (dense problems only). Worth it when the tiles left
   // over after the full rounds occupy at most half of the CTAs and every part keeps at least
@@ -900,7 +1006,12 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   p.split_items = 0;
   p.split_s = 1;
   p.split_slots = nullptr;
-  if (!grouped && a.mode == 0 && a.force_split != 0 && a.num_out_parts == 0 && tiles > grid) {
+  p.cluster_s = cluster_s;
+  if (cluster_s > 1) {
+    p.split_from = 0;
+    p.split_items = grid;
+    p.split_s = cluster_s;
+  } else if (!grouped && a.mode == 0 && a.force_split != 0 && a.num_out_parts == 0 && tiles > grid) {
     const int rem = static_cast<int>(tiles % grid);
     int s = rem > 0 ? grid / rem : 1;
     if (s > 8) s = 8;
