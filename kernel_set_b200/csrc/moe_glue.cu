@@ -92,48 +92,96 @@ gate_softmax_topk_kernel(float* __restrict__ out_w, int32_t* __restrict__ out_i,
 }
 
 // ---------------------------------------------------------------------------------
-// permutation: stable counting sort of the pairs by expert, one CTA, no workspace
+// permutation: stable counting sort of the pairs by expert, no workspace
 // ---------------------------------------------------------------------------------
-// Warp w owns a contiguous chunk of the pairs and walks it 32 pairs at a time.
-// Pass 1 counts pairs per (warp, expert); a scan over warps and then over experts turns
-// the counts into the first output position of every (warp, expert); pass 2 walks the
-// chunks again and places every pair: position = running counter of (warp, expert) +
-// number of lower lanes with the same expert in this step.
+// CTA b places the pairs of chunk b. It needs, per expert, the number of pairs in all chunks
+// (where an expert's rows begin) and in the chunks before its own (where its pairs go in
+// there). Every CTA counts all of that for itself: the ids are 4 bytes a pair and come
+// from L2, so reading them once per CTA costs less than handing counts from CTA to CTA would (a second
+// launch or a grid-wide wait). Inside a chunk, warp w owns a contiguous piece and walks it 32
+// pairs at a time: position = running counter of (warp, expert) + number of lower lanes
+// with the same expert in this step, which keeps the sort stable.
 constexpr int kPermThreads = 1024;
 constexpr int kPermWarps = kPermThreads / 32;
 
+// Adds the pairs [begin, end) to the warp's row of `cnt`. Loads are issued eight at a time.
+__device__ __forceinline__ void count_pairs(int* mine, const int32_t* __restrict__ topk_idx, int64_t begin,
+                                            int64_t end, int experts) {
+  for (int64_t base = begin + threadIdx.x; base < end; base += 8 * kPermThreads) {
+    int e[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int64_t i = base + static_cast<int64_t>(j) * kPermThreads;
+      e[j] = i < end ? __ldg(topk_idx + i) : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (e[j] >= 0 && e[j] < experts) atomicAdd(mine + e[j], 1);
+  }
+}
+
+// Sums `cnt` over the warps into `sum` and clears it.
+__device__ __forceinline__ void fold_counts(int* cnt, int* sum, int experts) {
+  __syncthreads();
+  for (int e = threadIdx.x; e < experts; e += kPermThreads) {
+    int run = 0;
+#pragma unroll 8
+    for (int w = 0; w < kPermWarps; ++w) {
+      run += cnt[w * experts + e];
+      cnt[w * experts + e] = 0;
+    }
+    sum[e] = run;
+  }
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(kPermThreads)
 compute_permutation_kernel(int32_t* __restrict__ sorted_ids, int32_t* __restrict__ offsets,
-                           const int32_t* __restrict__ topk_idx, int64_t pairs, int experts) {
-  extern __shared__ int perm_smem[];       // [warps][experts] counters, then [experts] totals
+                           const int32_t* __restrict__ topk_idx, int64_t pairs, int experts, int64_t chunk) {
+  extern __shared__ int perm_smem[];       // [warps][experts] counters, then two [experts] rows
   int* cnt = perm_smem;
-  int* total = perm_smem + kPermWarps * experts;
+  int* before = perm_smem + kPermWarps * experts;   // pairs of an expert in the chunks before this one
+  int* total = before + experts;                    // ... in the chunks after it, then in all
   __shared__ int warp_sums[kPermWarps];
+  __shared__ int routed_pairs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < kPermWarps * experts; i += kPermThreads) cnt[i] = 0;
+  for (int i = threadIdx.x; i < 2 * experts; i += kPermThreads) before[i] = 0;
   __syncthreads();
-  const int64_t chunk = ((pairs + kPermWarps - 1) / kPermWarps + 31) & ~int64_t(31);
-  const int64_t begin = warp * chunk;
-  const int64_t end = begin + chunk < pairs ? begin + chunk : pairs;
+  const int64_t c_begin = static_cast<int64_t>(blockIdx.x) * chunk;
+  const int64_t c_end = c_begin + chunk < pairs ? c_begin + chunk : pairs;
   int* mine = cnt + warp * experts;
+  if (c_begin > 0) {
+    count_pairs(mine, topk_idx, 0, c_begin, experts);
+    fold_counts(cnt, before, experts);
+  }
+  if (c_end < pairs) {
+    count_pairs(mine, topk_idx, c_end, pairs, experts);
+    fold_counts(cnt, total, experts);
+  }
+  // this CTA's pairs: a piece of chunk / 32 (a multiple of 32) per warp
+  const int64_t piece = chunk / kPermWarps;
+  const int64_t begin = c_begin + warp * piece;
+  const int64_t end = begin + piece < c_end ? begin + piece : c_end;
   for (int64_t base = begin; base < end; base += 32) {
     const int64_t i = base + lane;
-    const int e = i < end ? topk_idx[i] : -1;
+    const int e = i < end ? __ldg(topk_idx + i) : -1;
     const bool valid = e >= 0 && e < experts;
     const unsigned mask = __match_any_sync(0xffffffffu, valid ? e : experts + lane);
     if (valid && lane == __ffs(mask) - 1) mine[e] += __popc(mask);
     __syncwarp();
   }
   __syncthreads();
-  // exclusive scan over warps for every expert
+  // exclusive scan over warps for every expert, starting behind the earlier chunks
   for (int e = threadIdx.x; e < experts; e += kPermThreads) {
-    int run = 0;
+    int run = before[e];
+#pragma unroll 8
     for (int w = 0; w < kPermWarps; ++w) {
       const int c = cnt[w * experts + e];
       cnt[w * experts + e] = run;
       run += c;
     }
-    total[e] = run;
+    total[e] += run;
   }
   __syncthreads();
   // exclusive scan of the totals over experts (experts <= 1024 = one element per thread)
@@ -161,26 +209,28 @@ compute_permutation_kernel(int32_t* __restrict__ sorted_ids, int32_t* __restrict
     const int excl = inc - v + warp_sums[warp];
     if (threadIdx.x < experts) {
       total[threadIdx.x] = excl;
-      offsets[threadIdx.x] = excl;
-      if (threadIdx.x == experts - 1) offsets[experts] = excl + v;
+      if (blockIdx.x == 0) offsets[threadIdx.x] = excl;
+      if (threadIdx.x == experts - 1) {
+        routed_pairs = excl + v;
+        if (blockIdx.x == 0) offsets[experts] = excl + v;
+      }
     }
   }
   __syncthreads();
-  const int routed = offsets[experts];
-  for (int i = threadIdx.x; i < kPermWarps * experts; i += kPermThreads) cnt[i] += total[i % experts];
-  __syncthreads();
   for (int64_t base = begin; base < end; base += 32) {
     const int64_t i = base + lane;
-    const int e = i < end ? topk_idx[i] : -1;
+    const int e = i < end ? __ldg(topk_idx + i) : -1;
     const bool valid = e >= 0 && e < experts;
     const unsigned mask = __match_any_sync(0xffffffffu, valid ? e : experts + lane);
-    if (valid) sorted_ids[mine[e] + __popc(mask & ((1u << lane) - 1u))] = static_cast<int32_t>(i);
+    if (valid) sorted_ids[total[e] + mine[e] + __popc(mask & ((1u << lane) - 1u))] = static_cast<int32_t>(i);
     __syncwarp();
     if (valid && lane == __ffs(mask) - 1) mine[e] += __popc(mask);
     __syncwarp();
   }
   // pairs with an expert id out of range are dropped; their places at the end hold -1
-  for (int64_t i = routed + threadIdx.x; i < pairs; i += kPermThreads) sorted_ids[i] = -1;
+  for (int64_t i = routed_pairs + static_cast<int64_t>(blockIdx.x) * kPermThreads + threadIdx.x; i < pairs;
+       i += static_cast<int64_t>(gridDim.x) * kPermThreads)
+    sorted_ids[i] = -1;
 }
 
 // ---------------------------------------------------------------------------------
@@ -250,11 +300,21 @@ inverse_permutation_kernel(int32_t* __restrict__ inverse, const int32_t* __restr
   if (pair >= 0 && pair < pairs) inverse[pair] = static_cast<int32_t>(r);
 }
 
+// Row of a pair after the sort, -1 for a dropped pair. The inverse map of a dropped pair was not
+// written by this call and holds whatever an earlier one left there, so the row it names is
+// looked up again: only the row that really holds the pair counts. (Clearing the map first was
+// a launch of its own.)
+__device__ __forceinline__ int32_t row_of_pair(const int32_t* __restrict__ inverse, const int32_t* __restrict__ ids,
+                                               int64_t pair, int64_t pairs) {
+  const int32_t row = __ldg(inverse + pair);
+  return (row >= 0 && row < pairs && __ldg(ids + row) == pair) ? row : -1;
+}
+
 // A thread owns 8 consecutive columns (16 bytes of a 16-bit type) of one token; slots are
 // added in slot order in fp32 and the row is written once.
 template <typename T>
 __global__ void __launch_bounds__(256)
-unpermute_vec8_kernel(T* __restrict__ out, const T* __restrict__ permuted, const int32_t* __restrict__ inverse,
+unpermute_vec8_kernel(T* __restrict__ out, const T* __restrict__ permuted, const int32_t* __restrict__ inverse, const int32_t* __restrict__ ids,
                       const float* __restrict__ weights, int64_t tokens, int top_k, int64_t hidden) {
   const int64_t row_vec = hidden / 8;
   const int64_t total = tokens * row_vec;
@@ -265,7 +325,7 @@ unpermute_vec8_kernel(T* __restrict__ out, const T* __restrict__ permuted, const
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
     for (int k = 0; k < top_k; ++k) {
-      const int32_t prow = __ldg(inverse + token * top_k + k);
+      const int32_t prow = row_of_pair(inverse, ids, token * top_k + k, tokens * top_k);
       if (prow < 0) continue;
       const float w = __ldg(weights + token * top_k + k);
       const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(permuted + static_cast<int64_t>(prow) * hidden) + c);
@@ -283,7 +343,7 @@ unpermute_vec8_kernel(T* __restrict__ out, const T* __restrict__ permuted, const
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-unpermute_any_kernel(T* __restrict__ out, const T* __restrict__ permuted, const int32_t* __restrict__ inverse,
+unpermute_any_kernel(T* __restrict__ out, const T* __restrict__ permuted, const int32_t* __restrict__ inverse, const int32_t* __restrict__ ids,
                      const float* __restrict__ weights, int64_t tokens, int top_k, int64_t hidden) {
   const int64_t total = tokens * hidden;
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
@@ -291,7 +351,7 @@ unpermute_any_kernel(T* __restrict__ out, const T* __restrict__ permuted, const 
     const int64_t token = t / hidden, c = t - token * hidden;
     float acc = 0.f;
     for (int k = 0; k < top_k; ++k) {
-      const int32_t prow = inverse[token * top_k + k];
+      const int32_t prow = row_of_pair(inverse, ids, token * top_k + k, tokens * top_k);
       if (prow < 0) continue;
       acc = fmaf(to_f32<T>(permuted[static_cast<int64_t>(prow) * hidden + c]), weights[token * top_k + k], acc);
     }
@@ -466,18 +526,23 @@ ks_status_t ks_moe_compute_permutation(int32_t* sorted_token_ids, int32_t* exper
   st = require_sm100(where);
   if (st != KS_SUCCESS) return st;
   cudaStream_t s = as_stream(stream);
-  const size_t smem = (static_cast<size_t>(kPermWarps) + 1) * num_experts * sizeof(int);
+  const size_t smem = (static_cast<size_t>(kPermWarps) + 2) * num_experts * sizeof(int);
+  // one pair per thread, at most one CTA per SM
+  const int64_t per_cta = (pairs + sm_count() - 1) / sm_count();
+  const int64_t per_thread = (per_cta + kPermThreads - 1) / kPermThreads;
+  const int64_t chunk = (per_thread > 0 ? per_thread : 1) * kPermThreads;
+  const unsigned ctas = pairs > 0 ? static_cast<unsigned>((pairs + chunk - 1) / chunk) : 1u;
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (smem > 48 * 1024 && dev >= 0 && dev < 64 && !attr_done[dev]) {
     cudaError_t e = cudaFuncSetAttribute(compute_permutation_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>((kPermWarps + 1) * kMaxExperts * sizeof(int)));
+                                         static_cast<int>((kPermWarps + 2) * kMaxExperts * sizeof(int)));
     if (e != cudaSuccess) return cuda_status(e, where);
     attr_done[dev] = true;
   }
-  compute_permutation_kernel<<<1, kPermThreads, smem, s>>>(sorted_token_ids, expert_offsets, topk_indices, pairs,
-                                                           num_experts);
+  compute_permutation_kernel<<<ctas, kPermThreads, smem, s>>>(sorted_token_ids, expert_offsets, topk_indices, pairs,
+                                                              num_experts, chunk);
   KSB_CHECK_LAUNCH(where);
   return KS_SUCCESS;
 }
@@ -579,30 +644,28 @@ ks_status_t ks_moe_unpermute(void* out, const void* permuted, const int32_t* sor
   st = require_sm100(where);
   if (st != KS_SUCCESS) return st;
   cudaStream_t s = as_stream(stream);
-  // inverse[pair] = row of the pair after the sort; -1 for dropped pairs. Stream-ordered
+  // inverse[pair] = row of the pair after the sort (not written for dropped pairs). Stream-ordered
   // library workspace: allocated when the stream first needs it (or needs more), never freed
   // or synchronised per call.
   int32_t* inverse = static_cast<int32_t*>(sm100::stream_scratch(s, static_cast<size_t>(pairs) * sizeof(int32_t), 4));
   if (inverse == nullptr) KSB_FAIL(KS_ERROR_OUT_OF_MEMORY, "ks_moe_unpermute: workspace allocation failed");
-  cudaError_t e = cudaMemsetAsync(inverse, 0xFF, static_cast<size_t>(pairs) * sizeof(int32_t), s);
-  if (e != cudaSuccess) return cuda_status(e, where);
   inverse_permutation_kernel<<<static_cast<unsigned>((pairs + 255) / 256), 256, 0, s>>>(inverse, sorted_token_ids, pairs);
   const bool vec = dtype != KS_DTYPE_F32 && hidden % 8 == 0 && aligned16(out) && aligned16(permuted);
   if (dtype == KS_DTYPE_F32) {
     unpermute_any_kernel<float><<<grid_for(num_tokens * hidden), 256, 0, s>>>(
-        static_cast<float*>(out), static_cast<const float*>(permuted), inverse, routing_weights, num_tokens, top_k, hidden);
+        static_cast<float*>(out), static_cast<const float*>(permuted), inverse, sorted_token_ids, routing_weights, num_tokens, top_k, hidden);
   } else if (dtype == KS_DTYPE_F16) {
     if (vec) unpermute_vec8_kernel<__half><<<grid_for(num_tokens * (hidden / 8)), 256, 0, s>>>(
-        static_cast<__half*>(out), static_cast<const __half*>(permuted), inverse, routing_weights, num_tokens, top_k, hidden);
+        static_cast<__half*>(out), static_cast<const __half*>(permuted), inverse, sorted_token_ids, routing_weights, num_tokens, top_k, hidden);
     else unpermute_any_kernel<__half><<<grid_for(num_tokens * hidden), 256, 0, s>>>(
-        static_cast<__half*>(out), static_cast<const __half*>(permuted), inverse, routing_weights, num_tokens, top_k, hidden);
+        static_cast<__half*>(out), static_cast<const __half*>(permuted), inverse, sorted_token_ids, routing_weights, num_tokens, top_k, hidden);
   } else {
     if (vec) unpermute_vec8_kernel<__nv_bfloat16><<<grid_for(num_tokens * (hidden / 8)), 256, 0, s>>>(
-        static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(permuted), inverse, routing_weights,
-        num_tokens, top_k, hidden);
+        static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(permuted), inverse, sorted_token_ids,
+        routing_weights, num_tokens, top_k, hidden);
     else unpermute_any_kernel<__nv_bfloat16><<<grid_for(num_tokens * hidden), 256, 0, s>>>(
-        static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(permuted), inverse, routing_weights,
-        num_tokens, top_k, hidden);
+        static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(permuted), inverse, sorted_token_ids,
+        routing_weights, num_tokens, top_k, hidden);
   }
   KSB_CHECK_LAUNCH(where);
   return KS_SUCCESS;
