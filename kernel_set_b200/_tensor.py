@@ -8,7 +8,6 @@ reference tensor's device (``:205-219``); dtype map ``:81-93``.
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Any, Optional
 
 import torch
@@ -32,6 +31,11 @@ TORCH_TO_KS = {
 KS_TO_TORCH = {v: k for k, v in TORCH_TO_KS.items()}
 
 
+# Handle of the current stream of a device without building a Stream object around it (which takes
+# 5-6 us, a third of a small call); older torch builds lack the function.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def dtype_to_ks(torch_dtype) -> int:
     try:
         return TORCH_TO_KS[torch_dtype]
@@ -48,6 +52,8 @@ def ks_to_torch_dtype(ks_dtype: int):
 
 def ptr(obj: TensorLike, *, name: str = "tensor", allow_none: bool = True) -> int:
     """Raw device address of ``obj`` (tensor, int, or ``None`` -> 0)."""
+    if type(obj) is torch.Tensor and obj.is_cuda and obj.is_contiguous():   # what nearly every call passes
+        return obj.data_ptr()
     if obj is None:
         if allow_none:
             return 0
@@ -68,12 +74,14 @@ def ptr(obj: TensorLike, *, name: str = "tensor", allow_none: bool = True) -> in
                     f"got {type(obj).__name__}")
 
 
-def f32_ptr(obj: TensorLike, *, name: str):
-    return ctypes.cast(ptr(obj, name=name), ctypes.POINTER(ctypes.c_float))
+# Typed pointers cross the boundary as plain addresses: building a ctypes pointer object for
+# each argument costs more than the rest of its checks (about 1 us a call).
+def f32_ptr(obj: TensorLike, *, name: str) -> int:
+    return ptr(obj, name=name)
 
 
-def i32_ptr(obj: TensorLike, *, name: str):
-    return ctypes.cast(ptr(obj, name=name), ctypes.POINTER(ctypes.c_int32))
+def i32_ptr(obj: TensorLike, *, name: str) -> int:
+    return ptr(obj, name=name)
 
 
 def stream_ptr(stream: TensorLike) -> int:
@@ -95,6 +103,8 @@ def default_stream(stream: TensorLike, reference: TensorLike = None) -> int:
     if stream is not None:
         return stream_ptr(stream)
     if isinstance(reference, torch.Tensor) and reference.is_cuda:
+        if _raw_stream is not None:
+            return _raw_stream(reference.device.index)
         return torch.cuda.current_stream(reference.device).cuda_stream
     return 0
 
