@@ -161,6 +161,8 @@ template <> struct Pack16<__nv_bfloat16> {
   __device__ static float lo(V2 v) { return __low2float(v); }
   __device__ static float hi(V2 v) { return __high2float(v); }
   __device__ static V2 make(float a, float b) { return __floats2bfloat162_rn(a, b); }
+  __device__ static V2 low(V2 v) { return __low2bfloat162(v); }    // the low half twice
+  __device__ static V2 high(V2 v) { return __high2bfloat162(v); }
 };
 template <> struct Pack16<__half> {
   using V2 = __half2;
@@ -173,6 +175,8 @@ template <> struct Pack16<__half> {
   __device__ static float lo(V2 v) { return __low2float(v); }
   __device__ static float hi(V2 v) { return __high2float(v); }
   __device__ static V2 make(float a, float b) { return __floats2half2_rn(a, b); }
+  __device__ static V2 low(V2 v) { return __low2half2(v); }
+  __device__ static V2 high(V2 v) { return __high2half2(v); }
 };
 
 __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
@@ -453,31 +457,40 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // magic, subtract (magic + zero), multiply by the scale.
     // (Reading one byte per lane and row instead takes a full shared-memory cycle for 32 bytes,
     // 256 per unit, on the port through which the MMAs read 64 KB and TMA writes 72 KB per unit.)
+    // The loop is bound by instruction issue (the integer pipe at half rate above all), so
+    // everything outside the cells counts: 32-bit counters relative to the CTA's run, ring
+    // positions that advance instead of divisions, addresses of the scale rows that advance, and
+    // zero-points tested two columns at a time.
     const int half = (warp - 4) >> 3;           // group = K-step half of every box = parity of its units
     const int khalf = ((warp - 4) >> 2) & 1;    // 64-k half of the unit
     const V2 magic2 = P16::splat(P16::kMagic);
+    const V2 max_zero2 = P16::from_bits(P16::kMaxZeroBits | (P16::kMaxZeroBits << 16));
+    const V2 zero2 = P16::from_bits(0u);
     const int quarter = warp & 3;
     constexpr uint32_t kMagic2 = P16::kMagicBytes & 0xFF00FF00u;
-    // Scales and zero-points come straight from global memory, fetched one unit of the group
-    // ahead; (tile, step) of the unit being fetched advance without any 64-bit division
-    // (k_steps and kGroups are even, so the parity of step is fixed).
     constexpr int kSz = FINE ? 2 : 1;           // scale rows of this warp's 64 k: one per 32 k, or one
     const int col0 = quarter * 32 + 2 * (lane >> 2);   // this lane's columns: col0, col0 + 1, col0 + 16, col0 + 17
-    const long long b_begin = u_begin >> 1, b_end = (u_end + 1) >> 1;
-    long long u_first = (b_begin << 1) + half;
-    if (u_first < u_begin) u_first += kGroups;
+    const int n_units = static_cast<int>(u_end - u_begin);
+    const int odd0 = static_cast<int>(u_begin & 1);
+    const int n_boxes = (n_units + odd0 + 1) >> 1;
+    // Scales and zero-points come straight from global memory, fetched one unit of the group
+    // ahead (k_steps and kGroups are even, so the parity of step is fixed).
+    int it = half - odd0;                       // unit of box 0, relative to the run; -1: a neighbour's
+    const long long u_first = u_begin + (it < 0 ? it + kGroups : it);
     const long long f_t0 = u_first / p.k_steps;
     int f_step = static_cast<int>(u_first - f_t0 * p.k_steps);
     int f_ntile = static_cast<int>(f_t0 / p.m_tiles);
     int f_mtile = static_cast<int>(f_t0 - static_cast<long long>(f_ntile) * p.m_tiles);
     int f_row = FINE ? 0 : f_step / p.gs_steps, f_in_row = FINE ? 0 : f_step - f_row * p.gs_steps;
     uint32_t s_pair[kSz][2], z_pair[kSz][2];   // [scale row][block of 16 columns]: columns 2g (low half), 2g + 1
+#pragma unroll
+    for (int i = 0; i < kSz; ++i) s_pair[i][0] = s_pair[i][1] = z_pair[i][0] = z_pair[i][1] = 0u;
     auto fetch = [&]() {
       const int n = f_ntile * kTileN + col0;
 #pragma unroll
       for (int i = 0; i < kSz; ++i) {
         const int row = FINE ? ((f_step * 4 + khalf * 2 + i) >> p.sub_shift) : f_row;
-        const size_t idx = static_cast<size_t>(row) * p.n + n;
+        const long long idx = static_cast<long long>(row) * p.n + n;
         const unsigned short* gs = static_cast<const unsigned short*>(p.scales) + idx;
         const unsigned short* gz = static_cast<const unsigned short*>(p.zeros) + idx;
 #pragma unroll
@@ -486,13 +499,12 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           // are zero-filled there, and zero scales keep the product zero)
           const bool in = n + 16 * cb < p.n && row < p.groups;
           s_pair[i][cb] = in ? __ldg(reinterpret_cast<const unsigned int*>(gs + 16 * cb)) : 0u;
-          z_pair[i][cb] = (in && p.has_zeros) ? __ldg(reinterpret_cast<const unsigned int*>(gz + 16 * cb)) : 0u;
+          if (p.has_zeros) z_pair[i][cb] = in ? __ldg(reinterpret_cast<const unsigned int*>(gz + 16 * cb)) : 0u;
         }
       }
     };
     auto fetch_advance = [&]() {
       f_step += kGroups;
-      if constexpr (!FINE) f_in_row += kGroups;
       if (f_step >= p.k_steps) {
         f_step -= p.k_steps;
         if (++f_mtile == p.m_tiles) { f_mtile = 0; ++f_ntile; }
@@ -500,6 +512,8 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           f_row = 0;
           f_in_row = f_step;
         }
+      } else if constexpr (!FINE) {
+        f_in_row += kGroups;
       }
       if constexpr (!FINE) {
         while (f_in_row >= p.gs_steps) { f_in_row -= p.gs_steps; ++f_row; }
@@ -512,37 +526,34 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         static_cast<uint32_t>(half * kRawBytes + khalf * (32 * 128) + ((lane >> 4) * 8 + (lane & 7)) * 128 +
                               (((quarter * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
     const uint32_t lane_dst = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::kOperandCol0 + khalf * 32;
-    for (long long b = b_begin; b < b_end; ++b) {
-      const uint32_t itb = static_cast<uint32_t>(b - b_begin);
-      const uint32_t sr = itb % C::kRawStages, pr = (itb / C::kRawStages) & 1u;
-      const long long u = (b << 1) + half;
-      if (u < u_begin || u >= u_end) {
+    uint32_t sr = 0, pr = 0;
+    for (int b = 0; b < n_boxes; ++b, it += kGroups, sr = sr + 1 == C::kRawStages ? (pr ^= 1u, 0u) : sr + 1) {
+      if (it < 0 || it >= n_units) {
         // this half of the box belongs to a neighbouring CTA's run
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_raw_empty + 8 * sr);
         continue;
       }
-      const uint32_t it = static_cast<uint32_t>(u - u_begin);
-      const uint32_t sd = it % kDeqStages, pd = (it / kDeqStages) & 1u;
+      const uint32_t sd = it & (kDeqStages - 1), pd = (static_cast<uint32_t>(it) / kDeqStages) & 1u;
+      static_assert((kDeqStages & (kDeqStages - 1)) == 0, "a power of two");
       // constants of the unit: columns 2g, 2g + 1 of the first block of 16, then of the second
-      V2 sc[kSz][4], zz[kSz][4];
-      uint32_t zw[kSz][4];
+      V2 sc[kSz][2], zz[kSz][2], zp[kSz][2];
       uint32_t bad = 0;
+      bool in_range = true;
 #pragma unroll
       for (int i = 0; i < kSz; ++i) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t sel = (j & 1) ? 0x3232u : 0x1010u;
-          sc[i][j] = P16::from_bits(__byte_perm(s_pair[i][j >> 1], 0u, sel));
-          zw[i][j] = __byte_perm(z_pair[i][j >> 1], 0u, sel);
-          zz[i][j] = __hadd2(P16::from_bits(zw[i][j]), magic2);
+        for (int cb = 0; cb < 2; ++cb) {
+          sc[i][cb] = P16::from_bits(s_pair[i][cb]);
+          zp[i][cb] = P16::from_bits(z_pair[i][cb]);
+          zz[i][cb] = __hadd2(zp[i][cb], magic2);
           // (magic + zero) exact and |q - zero| exact: non-negative integer zero-points up to kMaxZero
-          bad |= (P16::bits(__hsub2(zz[i][j], magic2)) ^ zw[i][j]) | (zw[i][j] & 0x80008000u);
-          bad |= (zw[i][j] & 0xFFFFu) > P16::kMaxZeroBits ? 1u : 0u;
+          bad |= P16::bits(__hsub2(zz[i][cb], magic2)) ^ z_pair[i][cb];
+          in_range = in_range && __hbge2(zp[i][cb], zero2) && __hble2(zp[i][cb], max_zero2);
         }
       }
-      const bool simple = __all_sync(0xffffffffu, bad == 0u);   // (both forms agree to the bit where both apply)
-      if (u + kGroups < u_end) {
+      const bool simple = __all_sync(0xffffffffu, bad == 0u && in_range);   // (both forms agree to the bit where both apply)
+      if (it + kGroups < n_units) {
         fetch_advance();
         fetch();
       }
@@ -555,17 +566,19 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       for (int cb = 0; cb < 2; ++cb) {
         uint32_t cells[16];            // 64 k = 32 operand columns of this block's 16 weight columns
         if (simple) {
+          const int r0 = 0, r1 = FINE ? 1 : 0;
+          const V2 s_lo[2] = {P16::low(sc[r0][cb]), P16::low(sc[r1][cb])}, s_hi[2] = {P16::high(sc[r0][cb]), P16::high(sc[r1][cb])};
+          const V2 z_lo[2] = {P16::low(zz[r0][cb]), P16::low(zz[r1][cb])}, z_hi[2] = {P16::high(zz[r0][cb]), P16::high(zz[r1][cb])};
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const uint32_t w0 = w[q >> 1][2 * (q & 1) + cb], w4 = w0 >> 4;
-            const int r = FINE ? q >> 1 : 0;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               // byte i: column 2g + (i & 1), row 2s + (i >> 1)
               const uint32_t sel = i | (i << 4) | ((4 + i) << 8) | ((4 + i) << 12);
               const uint32_t x = (__byte_perm(w0, w4, sel) & 0x000F000Fu) | kMagic2;
-              cells[4 * q + 2 * (i & 1) + (i >> 1)] =
-                  P16::bits(__hmul2(__hsub2(P16::from_bits(x), zz[r][2 * cb + (i & 1)]), sc[r][2 * cb + (i & 1)]));
+              const V2 z = (i & 1) ? z_hi[q >> 1] : z_lo[q >> 1], sx = (i & 1) ? s_hi[q >> 1] : s_lo[q >> 1];
+              cells[4 * q + 2 * (i & 1) + (i >> 1)] = P16::bits(__hmul2(__hsub2(P16::from_bits(x), z), sx));
             }
           }
         } else {
@@ -577,7 +590,8 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const uint32_t b8 = (w0 >> (8 * i)) & 0xFFu;
-              const float z0 = P16::lo(P16::from_bits(zw[r][2 * cb + (i & 1)])), s0 = P16::lo(sc[r][2 * cb + (i & 1)]);
+              const float z0 = (i & 1) ? P16::hi(zp[r][cb]) : P16::lo(zp[r][cb]);
+              const float s0 = (i & 1) ? P16::hi(sc[r][cb]) : P16::lo(sc[r][cb]);
               cells[4 * q + 2 * (i & 1) + (i >> 1)] =
                   P16::bits(P16::make(__fmul_rn(__fsub_rn(static_cast<float>(b8 & 15u), z0), s0),
                                       __fmul_rn(__fsub_rn(static_cast<float>(b8 >> 4), z0), s0)));
@@ -855,6 +869,8 @@ Geometry geometry_of(const W4A16Args& a) {
   const bool fine = a.group_size % kStepK != 0;
   g.n_tiles = static_cast<int>((a.n + kTileN - 1) / kTileN);
   g.k_steps = static_cast<int>((a.k / kStepK + 1) & ~int64_t(1));
+  int64_t capacity[kMaxClusterSplit + 1];
+  for (int s = 2; s <= kMaxClusterSplit; ++s) capacity[s] = cluster_capacity(s);
   double best = 0;
   auto offer = [&](double cost, int mt, int m_tiles, int cluster_s, bool split) {
     if (best != 0 && cost >= best) return;
@@ -873,7 +889,7 @@ Geometry geometry_of(const W4A16Args& a) {
     const double drain = mt * 8.0;   // accumulators to C
     offer(static_cast<double>((tiles + sms - 1) / sms) * (g.k_steps * unit + drain), mt, m_tiles, 1, false);
     for (int s = 2; s <= kMaxClusterSplit && 2 * s <= g.k_steps && tiles * s <= sms; ++s) {
-      if (cluster_capacity(s) < tiles) break;
+      if (capacity[s] < tiles) break;
       offer(2.0 * ((g.k_steps / 2 + s - 1) / s) * unit + drain + 1500.0, mt, m_tiles, s, false);
     }
     const double per_cta = static_cast<double>(tiles) * g.k_steps / (tiles * g.k_steps < sms ? tiles * g.k_steps : sms);
@@ -991,6 +1007,8 @@ ks_status_t launch_w4a16(const W4A16Args& a, cudaStream_t stream) {
   const decode::Geometry gd = dec ? decode::geometry_of(a) : decode::Geometry{};
   const size_t slot_bytes = dec ? gd.slot_bytes : g.slot_bytes;
   const size_t counter_bytes = dec ? gd.counter_bytes : g.counter_bytes;
+  // Whole tiles and clusters share nothing through memory.
+  if (!dec && !g.split) return enqueue_w4a16(a, g, nullptr, nullptr, kernel_fault_word(), stream);
   float* slots = static_cast<float*>(stream_scratch(stream, slot_bytes, 0));
   unsigned int* counters = static_cast<unsigned int*>(stream_scratch(stream, counter_bytes, 1));
   if (slots == nullptr || counters == nullptr)
