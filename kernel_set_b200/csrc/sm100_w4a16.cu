@@ -152,9 +152,10 @@ struct Params {
 template <typename T> struct Pack16;
 template <> struct Pack16<__nv_bfloat16> {
   using V2 = __nv_bfloat162;
-  static constexpr uint32_t kMagicBytes = 0x43434343u;  // high byte of bf16(128 + q)
-  static constexpr float kMagic = 128.0f;
-  static constexpr uint32_t kMaxZeroBits = 0x42FEu;     // bf16(127)
+  static constexpr float kMaxZero = 127.0f;             // zero-points up to here: |q - zero| is exact
+  static constexpr float kUnit = 0x1p-133f;             // the bit pattern q is q * 2^-133 (subnormal)
+  static constexpr float kUp = 0x1p127f;                // largest power of two; q * kUnit * kUp = q / kDown
+  static constexpr float kDown = 0x1p6f;
   __device__ static V2 from_bits(uint32_t b) { return *reinterpret_cast<V2*>(&b); }
   __device__ static uint32_t bits(V2 v) { return *reinterpret_cast<uint32_t*>(&v); }
   __device__ static V2 splat(float f) { return __float2bfloat162_rn(f); }
@@ -166,9 +167,10 @@ template <> struct Pack16<__nv_bfloat16> {
 };
 template <> struct Pack16<__half> {
   using V2 = __half2;
-  static constexpr uint32_t kMagicBytes = 0x64646464u;  // high byte of f16(1024 + q)
-  static constexpr float kMagic = 1024.0f;
-  static constexpr uint32_t kMaxZeroBits = 0x63FEu;     // f16(1023)
+  static constexpr float kMaxZero = 1023.0f;
+  static constexpr float kUnit = 0x1p-24f;
+  static constexpr float kUp = 0x1p15f;
+  static constexpr float kDown = 0x1p9f;
   __device__ static V2 from_bits(uint32_t b) { return *reinterpret_cast<V2*>(&b); }
   __device__ static uint32_t bits(V2 v) { return *reinterpret_cast<uint32_t*>(&v); }
   __device__ static V2 splat(float f) { return __float2half2_rn(f); }
@@ -178,6 +180,13 @@ template <> struct Pack16<__half> {
   __device__ static V2 low(V2 v) { return __low2half2(v); }
   __device__ static V2 high(V2 v) { return __high2half2(v); }
 };
+
+// prmt with all four selector bits (bit 3 of a nibble replicates the byte's sign bit).
+__device__ __forceinline__ uint32_t byte_perm_sign(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
 
 __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -452,9 +461,12 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // (row 2s, columns 2g, 2g + 1) and (row 2s + 1, columns 2g, 2g + 1) of an 8-row x 16-column
     // block; tcgen05.st.16x256b takes from it the cells (TMEM lane g, columns 2s, 2s + 1) and
     // (lane g + 8, columns 2s, 2s + 1). So TMEM lanes g and g + 8 stand for the weight columns 2g
-    // and 2g + 1, and no byte crosses a lane. Per cell: one byte permute (code k to byte 0, code
-    // k+1, from the word shifted by four, to byte 2), one mask-or with the exponent bits of
-    // magic, subtract (magic + zero), multiply by the scale.
+    // and 2g + 1, and no byte crosses a lane. The low and the high nibbles of the word are split once;
+    // per cell one byte permute then puts code k into the low half and code k+1 into the high
+    // half. Such a half, read as a 16-bit float, is the subnormal q * kUnit, and one exact
+    // multiply-add makes it (q - zero) / kDown; the product with kDown * scale rounds once, as
+    // (q - zero) * scale does. (Building the float magic + q first costs one more integer
+    // instruction per cell, and the integer pipe is what bounds this loop.)
     // (Reading one byte per lane and row instead takes a full shared-memory cycle for 32 bytes,
     // 256 per unit, on the port through which the MMAs read 64 KB and TMA writes 72 KB per unit.)
     // The loop is bound by instruction issue (the integer pipe at half rate above all), so
@@ -463,11 +475,12 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // zero-points tested two columns at a time.
     const int half = (warp - 4) >> 3;           // group = K-step half of every box = parity of its units
     const int khalf = ((warp - 4) >> 2) & 1;    // 64-k half of the unit
-    const V2 magic2 = P16::splat(P16::kMagic);
-    const V2 max_zero2 = P16::from_bits(P16::kMaxZeroBits | (P16::kMaxZeroBits << 16));
-    const V2 zero2 = P16::from_bits(0u);
+    static_assert(P16::kUnit * P16::kUp * P16::kDown == 1.0f, "the three factors cancel");
+    const V2 up2 = P16::splat(P16::kUp), down2 = P16::splat(P16::kDown), neg_inv_down2 = P16::splat(-1.0f / P16::kDown);
+    const V2 max_zero2 = P16::splat(P16::kMaxZero), zero2 = P16::from_bits(0u);
+    const V2 max_scale2 = P16::splat(P16::kUp);
+    const V2 whole2 = P16::splat(P16::kMaxZero + 1.0f);   // adding it rounds to whole numbers
     const int quarter = warp & 3;
-    constexpr uint32_t kMagic2 = P16::kMagicBytes & 0xFF00FF00u;
     constexpr int kSz = FINE ? 2 : 1;           // scale rows of this warp's 64 k: one per 32 k, or one
     const int col0 = quarter * 32 + 2 * (lane >> 2);   // this lane's columns: col0, col0 + 1, col0 + 16, col0 + 17
     const int n_units = static_cast<int>(u_end - u_begin);
@@ -537,22 +550,24 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       const uint32_t sd = it & (kDeqStages - 1), pd = (static_cast<uint32_t>(it) / kDeqStages) & 1u;
       static_assert((kDeqStages & (kDeqStages - 1)) == 0, "a power of two");
       // constants of the unit: columns 2g, 2g + 1 of the first block of 16, then of the second
-      V2 sc[kSz][2], zz[kSz][2], zp[kSz][2];
-      uint32_t bad = 0;
-      bool in_range = true;
+      V2 sd2[kSz][2], zd2[kSz][2];     // scale * kDown, -zero / kDown
+      uint32_t s_cur[kSz][2], z_cur[kSz][2];
+      bool simple_lane = true;
 #pragma unroll
       for (int i = 0; i < kSz; ++i) {
 #pragma unroll
         for (int cb = 0; cb < 2; ++cb) {
-          sc[i][cb] = P16::from_bits(s_pair[i][cb]);
-          zp[i][cb] = P16::from_bits(z_pair[i][cb]);
-          zz[i][cb] = __hadd2(zp[i][cb], magic2);
-          // (magic + zero) exact and |q - zero| exact: non-negative integer zero-points up to kMaxZero
-          bad |= P16::bits(__hsub2(zz[i][cb], magic2)) ^ z_pair[i][cb];
-          in_range = in_range && __hbge2(zp[i][cb], zero2) && __hble2(zp[i][cb], max_zero2);
+          s_cur[i][cb] = s_pair[i][cb];
+          z_cur[i][cb] = z_pair[i][cb];
+          const V2 sv = P16::from_bits(s_cur[i][cb]), zv = P16::from_bits(z_cur[i][cb]);
+          sd2[i][cb] = __hmul2(sv, down2);
+          zd2[i][cb] = __hmul2(zv, neg_inv_down2);
+          // exact for integer zero-points 0..kMaxZero, and where scale * kDown stays in range
+          simple_lane = simple_lane && __hbge2(zv, zero2) && __hble2(zv, max_zero2) && __hbeq2(__hsub2(__hadd2(zv, whole2), whole2), zv) &&
+                        __hble2(__habs2(sd2[i][cb]), max_scale2);
         }
       }
-      const bool simple = __all_sync(0xffffffffu, bad == 0u && in_range);   // (both forms agree to the bit where both apply)
+      const bool simple = __all_sync(0xffffffffu, simple_lane);   // (both forms agree to the bit where both apply)
       if (it + kGroups < n_units) {
         fetch_advance();
         fetch();
@@ -566,19 +581,21 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       for (int cb = 0; cb < 2; ++cb) {
         uint32_t cells[16];            // 64 k = 32 operand columns of this block's 16 weight columns
         if (simple) {
-          const int r0 = 0, r1 = FINE ? 1 : 0;
-          const V2 s_lo[2] = {P16::low(sc[r0][cb]), P16::low(sc[r1][cb])}, s_hi[2] = {P16::high(sc[r0][cb]), P16::high(sc[r1][cb])};
-          const V2 z_lo[2] = {P16::low(zz[r0][cb]), P16::low(zz[r1][cb])}, z_hi[2] = {P16::high(zz[r0][cb]), P16::high(zz[r1][cb])};
+          const int r1 = FINE ? 1 : 0;
+          const V2 s_lo[2] = {P16::low(sd2[0][cb]), P16::low(sd2[r1][cb])}, s_hi[2] = {P16::high(sd2[0][cb]), P16::high(sd2[r1][cb])};
+          const V2 z_lo[2] = {P16::low(zd2[0][cb]), P16::low(zd2[r1][cb])}, z_hi[2] = {P16::high(zd2[0][cb]), P16::high(zd2[r1][cb])};
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const uint32_t w0 = w[q >> 1][2 * (q & 1) + cb], w4 = w0 >> 4;
+            const uint32_t w0 = w[q >> 1][2 * (q & 1) + cb];
+            const uint32_t lo4 = w0 & 0x0F0F0F0Fu, hi4 = (w0 >> 4) & 0x0F0F0F0Fu;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              // byte i: column 2g + (i & 1), row 2s + (i >> 1)
-              const uint32_t sel = i | (i << 4) | ((4 + i) << 8) | ((4 + i) << 12);
-              const uint32_t x = (__byte_perm(w0, w4, sel) & 0x000F000Fu) | kMagic2;
+              // byte i: column 2g + (i & 1), row 2s + (i >> 1); selector 8 + j replicates the sign of
+              // byte j, which is zero
+              const uint32_t sel = i | ((8 + i) << 4) | ((4 + i) << 8) | ((12 + i) << 12);
+              const V2 x = P16::from_bits(byte_perm_sign(lo4, hi4, sel));
               const V2 z = (i & 1) ? z_hi[q >> 1] : z_lo[q >> 1], sx = (i & 1) ? s_hi[q >> 1] : s_lo[q >> 1];
-              cells[4 * q + 2 * (i & 1) + (i >> 1)] = P16::bits(__hmul2(__hsub2(P16::from_bits(x), z), sx));
+              cells[4 * q + 2 * (i & 1) + (i >> 1)] = P16::bits(__hmul2(__hfma2(x, up2, z), sx));
             }
           }
         } else {
@@ -590,8 +607,9 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const uint32_t b8 = (w0 >> (8 * i)) & 0xFFu;
-              const float z0 = (i & 1) ? P16::hi(zp[r][cb]) : P16::lo(zp[r][cb]);
-              const float s0 = (i & 1) ? P16::hi(sc[r][cb]) : P16::lo(sc[r][cb]);
+              const V2 sv = P16::from_bits(s_cur[r][cb]), zv = P16::from_bits(z_cur[r][cb]);
+              const float z0 = (i & 1) ? P16::hi(zv) : P16::lo(zv);
+              const float s0 = (i & 1) ? P16::hi(sv) : P16::lo(sv);
               cells[4 * q + 2 * (i & 1) + (i >> 1)] =
                   P16::bits(P16::make(__fmul_rn(__fsub_rn(static_cast<float>(b8 & 15u), z0), s0),
                                       __fmul_rn(__fsub_rn(static_cast<float>(b8 >> 4), z0), s0)));
