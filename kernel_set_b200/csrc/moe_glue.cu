@@ -310,6 +310,71 @@ __device__ __forceinline__ int32_t row_of_pair(const int32_t* __restrict__ inver
   return (row >= 0 && row < pairs && __ldg(ids + row) == pair) ? row : -1;
 }
 
+// permute_quant_kernel the other way round, for large problems: a token is read and quantized
+// once and its codes are written to the rows of all its pairs. (Row by row, every row quantizes its token
+// again: 145 instructions per 512 elements, top_k times, made that the bound: 141 us for 4096
+// tokens x 7168 x top 8, where writing the 242 MB takes ~40.) Blocks from `token_blocks` on walk the rows and
+// do those that no token's inverse entry names: ids out of range (a row of zeros) and
+// repeated ids, which the row-by-row kernel takes as they come.
+template <typename T, bool E5M2>
+__global__ void __launch_bounds__(256)
+permute_quant_tokens_kernel(uint8_t* __restrict__ out, float* __restrict__ scale, const T* __restrict__ in,
+                            const int32_t* __restrict__ ids, const int32_t* __restrict__ inverse, int64_t tokens,
+                            int top_k, int64_t hidden, unsigned token_blocks, float qmax) {
+  const int64_t segs_per_row = hidden / 16;
+  const int64_t pairs = tokens * top_k;
+  float v[16];
+  if (blockIdx.x < token_blocks) {
+    const int64_t seg = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t token = seg / segs_per_row;
+    const bool live = token < tokens;
+    const int64_t c = seg - token * segs_per_row;
+    if (live) {
+      quantmath::Vec16<T>::load(in + token * hidden + c * 16, v);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = 0.f;
+    }
+    float sc;
+    const uint4 codes = quantmath::quant_segment_codes<E5M2>(v, qmax, &sc);
+    if (!live) return;
+    for (int k = 0; k < top_k; ++k) {
+      const int32_t row = row_of_pair(inverse, ids, token * top_k + k, pairs);
+      if (row < 0) continue;
+      const int64_t dst = row * segs_per_row + c;
+      if ((c & 7) == 0) scale[dst >> 3] = sc;
+      __stcs(reinterpret_cast<uint4*>(out + dst * 16), codes);
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x - token_blocks) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t mine = warp * 32 + lane;
+  bool left = false;
+  if (mine < pairs) {
+    const int32_t pair = __ldg(ids + mine);
+    left = !(pair >= 0 && pair < pairs && __ldg(inverse + pair) == mine);
+  }
+  unsigned todo = __ballot_sync(0xffffffffu, left);
+  while (todo != 0u) {
+    const int64_t r = warp * 32 + __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int32_t pair = __ldg(ids + r);
+    const bool have = pair >= 0 && pair < pairs;
+    for (int64_t c0 = 0; c0 < segs_per_row; c0 += 32) {   // (segs_per_row is a multiple of 8)
+      const int64_t c = c0 + lane;
+      const bool live = c < segs_per_row;
+      if (have && live) {
+        quantmath::Vec16<T>::load(in + static_cast<int64_t>(pair / top_k) * hidden + c * 16, v);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+      }
+      quantmath::quant_segment<T, E5M2>(out, scale, v, r * segs_per_row + c, live, qmax);
+    }
+  }
+}
+
 // A thread owns 8 consecutive columns (16 bytes of a 16-bit type) of one token; slots are
 // added in slot order in fp32 and the row is written once.
 template <typename T>
@@ -612,6 +677,34 @@ ks_status_t ks_moe_permute_quant_fp8(void* out_fp8, float* out_scale, const void
   const unsigned blocks = static_cast<unsigned>((segs + 255) / 256);
   const bool e5 = fp8_dtype == KS_DTYPE_F8E5M2;
   uint8_t* o = static_cast<uint8_t*>(out_fp8);
+  // Token by token where the quantizing outweighs the extra launch (the inverse map, ~2.5 us): from
+  // about 16 M elements, with at least two pairs per token. The map lives in stream scratch; a
+  // stream under capture, where scratch may not grow, keeps to rows.
+  if (top_k >= 2 && pairs * hidden >= (int64_t(16) << 20)) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) {
+      cudaGetLastError();
+      capturing = cudaStreamCaptureStatusActive;
+    }
+    int32_t* inverse = capturing != cudaStreamCaptureStatusNone
+                           ? nullptr
+                           : static_cast<int32_t*>(sm100::stream_scratch(s, static_cast<size_t>(pairs) * sizeof(int32_t), 4));
+    if (inverse != nullptr) {
+      inverse_permutation_kernel<<<static_cast<unsigned>((pairs + 255) / 256), 256, 0, s>>>(inverse, sorted_token_ids, pairs);
+      const unsigned token_blocks = static_cast<unsigned>((num_tokens * (hidden / 16) + 255) / 256);
+      const unsigned total_blocks = token_blocks + static_cast<unsigned>((pairs + 255) / 256);
+#define KSB_PT(T, E5, QMAX)                                                                                      \
+  permute_quant_tokens_kernel<T, E5><<<total_blocks, 256, 0, s>>>(o, out_scale, static_cast<const T*>(input),    \
+                                                                  sorted_token_ids, inverse, num_tokens, top_k,  \
+                                                                  hidden, token_blocks, QMAX)
+      if (in_dtype == KS_DTYPE_F32) { if (e5) KSB_PT(float, true, 57344.0f); else KSB_PT(float, false, 448.0f); }
+      else if (in_dtype == KS_DTYPE_F16) { if (e5) KSB_PT(__half, true, 57344.0f); else KSB_PT(__half, false, 448.0f); }
+      else { if (e5) KSB_PT(__nv_bfloat16, true, 57344.0f); else KSB_PT(__nv_bfloat16, false, 448.0f); }
+#undef KSB_PT
+      KSB_CHECK_LAUNCH(where);
+      return KS_SUCCESS;
+    }
+  }
 #define KSB_PQ(T)                                                                                               \
   do {                                                                                                          \
     if (e5) permute_quant_kernel<T, true><<<blocks, 256, 0, s>>>(o, out_scale, static_cast<const T*>(input),   \

@@ -279,3 +279,25 @@ def test_peer_dispatch_and_combine_on_one_device(ks, cuda):
                 lo = int(offs_h[s][e])
                 assert torch.equal(back[s][lo:lo + n], ys[d][row:row + n]), (d, el, s)
                 row += n
+
+
+@pytest.mark.parametrize("top_k,dtype", [(2, torch.bfloat16), (4, torch.float32)])
+def test_permute_quant_of_large_problems_takes_any_ids(ks, cuda, top_k, dtype):
+    """From 16 M elements on, tokens are quantized once and written to all their rows; ids out of range and
+    repeated ids are rows that no token writes. Bit for bit what gather + quantizer give."""
+    tokens, hidden = (16 << 20) // 4096 // top_k + 3, 4096
+    pairs = tokens * top_k
+    g = gen(31)
+    ids = torch.randperm(pairs, generator=g).to(torch.int32)
+    ids[5::97] = ids[4::97][:ids[5::97].numel()]     # repeated
+    ids[7::101] = -1                                 # dropped
+    ids[9::103] = pairs + 9                          # out of range
+    x = torch.randn(tokens, hidden, generator=g).to(dtype).to(cuda)
+    ids = ids.to(cuda)
+    q = torch.full((pairs, hidden), 7, dtype=torch.uint8, device=cuda).view(torch.float8_e4m3fn)
+    s = torch.full((pairs, hidden // 128), float("nan"), dtype=torch.float32, device=cuda)
+    ks.moe.permute_quant_fp8(q, s, x, ids, tokens, top_k, hidden)
+    p = torch.empty(pairs, hidden, dtype=dtype, device=cuda)
+    ks.moe.permute(p, x, ids, tokens, top_k, hidden)
+    q2, s2 = ks.dispatch.per_token_group_quant(p)
+    assert torch.equal(q.view(torch.uint8), q2.view(torch.uint8)) and torch.equal(s, s2)
