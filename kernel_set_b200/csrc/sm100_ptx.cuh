@@ -216,11 +216,6 @@ __device__ __forceinline__ float4 ld_shared_cluster_f4(uint32_t addr) {
   return v;
 }
 
-// Brings the cache line of `p` (global memory) into L2.
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
 // ---- TMA (tiled bulk tensor loads, one CTA, completion on an mbarrier) --------
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

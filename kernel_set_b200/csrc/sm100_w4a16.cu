@@ -351,17 +351,6 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       const uint32_t full = bar_raw_full + 8 * sr;
       mbar_arrive_expect_tx_elect(full, 2 * kRawBytes);
       tma_load_2d_elect(rawst_base + sr * kRawStageBytes, &tm_w, full, ntile * kTileN, step * (kStepK / 2));
-      // The dequantising warps fetch scales and zero-points only one unit ahead, which can be less
-      // than the latency of HBM under load: this warp, a ring of boxes ahead, brings their lines
-      // into L2. Lane: 64 bytes of a 256-byte row piece (lane % 4), scales or zero-points
-      // (lane / 4 % 2), row (lane / 8).
-      const int rows = FINE ? 8 >> p.sub_shift : 2;          // of the box's two K-steps
-      const int row0 = FINE ? (step * 4) >> p.sub_shift : step / p.gs_steps;
-      const char* table = static_cast<const char*>((lane & 4) ? p.zeros : p.scales);
-      const int n = ntile * kTileN + (lane & 3) * 32;
-      for (int r = row0 + (lane >> 3); r < row0 + rows; r += 4)
-        if (r < p.groups && n < p.n && table != nullptr) prefetch_l2(table + (static_cast<size_t>(r) * p.n + n) * 2);
-      __syncwarp();
     }
   } else if (warp == 2) {
     // ----------------------- activation producer (TMA) -----------------------
@@ -867,10 +856,11 @@ struct Geometry {
   size_t counter_bytes = 0, slot_bytes = 0;
 };
 
-// Time of one unit (128 columns x 128 k) of a token tile of `mt` rows in a long run, in ns;
-// measured as the slope of time against K with one whole tile per CTA.
+// Time of one unit (128 columns x 128 k) of a token tile of `mt` rows in a long run, in ns:
+// measured as the slope of time against K (2048 to 8192) with one whole tile per CTA, group 128:
+// 420 at 16 rows, 480 at 64, 490 at 128, 710 at 192, 830 at 256; groups of 32 about a fifth more.
 double unit_ns(int mt, bool fine) {
-  const double t = mt <= 64 ? 300.0 : mt <= 128 ? 300.0 + (mt - 64) * 1.6 : 400.0 + (mt - 128) * 2.0;
+  const double t = mt <= 128 ? 420.0 + mt * 0.55 : 490.0 + (mt - 128) * 2.7;
   return fine ? t * 1.2 : t;
 }
 
@@ -878,8 +868,9 @@ double unit_ns(int mt, bool fine) {
 //   cluster    a tile's K range over S CTAs, which exchange partial sums through shared memory
 //              (~1.5 us); needs all clusters resident at once
 //   whole      runs of whole tiles: the last round may leave SMs idle
-//   even runs  no SM idles, but a tile's last CTA reads the other parts from L2: ~0.25 us per part and
-//              16 token rows (two warps share that work in 256-row tiles)
+//   even runs  no SM idles, but a tile's last CTA reads the other parts from L2: ~2.5 us for the
+//              hand-over and ~0.25 us per part and 16 token rows (two warps share that work in
+//              256-row tiles). K = N = 4096, 16 rows: 12.5 us against 10.5 with clusters
 // Fewer token tiles mean fewer dequantisations of a weight; more of them, more tiles to deal out.
 Geometry geometry_of(const W4A16Args& a) {
   Geometry g;
@@ -913,7 +904,7 @@ Geometry geometry_of(const W4A16Args& a) {
     const double per_cta = static_cast<double>(tiles) * g.k_steps / (tiles * g.k_steps < sms ? tiles * g.k_steps : sms);
     const double parts = g.k_steps / per_cta + 1.0;
     const int chunks = mt <= 128 ? mt / 16 : (mt + 31) / 32;
-    offer(per_cta * unit + 2 * drain + 250.0 * chunks * parts, mt, m_tiles, 1, true);
+    offer(per_cta * unit + 2 * drain + 2500.0 + 250.0 * chunks * parts, mt, m_tiles, 1, true);
   }
   g.mtmax = g.mt <= 32 ? 32 : (g.mt <= 64 ? 64 : (g.mt <= 128 ? 128 : 256));
   const long long tiles = static_cast<long long>(g.n_tiles) * g.m_tiles;

@@ -22,11 +22,12 @@ class Bar:
         if s.pending==0: s.phase+=1; s.pending=s.count
     def done(s, parity): return (s.phase & 1) != parity
 def run_start(units, ctas, c): return (units*c)//ctas
-def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None):
+def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1):
+    # AB: accumulator (segment) buffers; AP: activation stages per unit
     raw_full=[Bar(1) for _ in range(RS)]; raw_empty=[Bar(2) for _ in range(RS)]
     act_full=[Bar(1) for _ in range(AS)]; act_empty=[Bar(1) for _ in range(AS)]
     deq_full=[Bar(1) for _ in range(DS)]; deq_empty=[Bar(1) for _ in range(DS)]
-    acc_full=[Bar(K) for _ in range(2)]; acc_empty=[Bar(1) for _ in range(2)]
+    acc_full=[Bar(K) for _ in range(AB)]; acc_empty=[Bar(1) for _ in range(AB)]
     b_begin, b_end = ub>>1, (ue+1)>>1
     def wprod():
         itb=0
@@ -38,10 +39,11 @@ def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None):
     def aprod():
         it=0
         for u in range(ub,ue):
-            sa=it%AS; pa=(it//AS)&1
-            yield ('wait', act_empty[sa], pa^1, it//AS, 'aprod act_empty')
-            act_full[sa].arrive()
-            it+=1
+            for _ in range(AP):
+                sa=it%AS; pa=(it//AS)&1
+                yield ('wait', act_empty[sa], pa^1, it//AS, 'aprod act_empty')
+                act_full[sa].arrive()
+                it+=1
     def issuer(i):
         it=0; seg=0; n_in_seg=0; step=ub%k_steps
         for u in range(ub,ue):
@@ -51,18 +53,21 @@ def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None):
             seg_last_u=min(tile_last,ue-1)
             mine=(it%K)==i
             my_last=u+K>seg_last_u
-            sd=it%DS; pd=(it//DS)&1; sa=it%AS; pa=(it//AS)&1
-            buf=seg&1; pacc=(seg>>1)&1
+            sd=it%DS; pd=(it//DS)&1
+            buf=seg%AB; pacc=(seg//AB)&1
             if seg_first: n_in_seg=0
             if mine:
-                if n_in_seg==0: yield ('wait', acc_empty[buf], pacc^1, seg>>1, f'issuer{i} acc_empty u={u}')
+                if n_in_seg==0: yield ('wait', acc_empty[buf], pacc^1, seg//AB, f'issuer{i} acc_empty u={u}')
                 yield ('wait', deq_full[sd], pd, it//DS+1, f'issuer{i} deq_full u={u}')
-                yield ('wait', act_full[sa], pa, it//AS+1, f'issuer{i} act_full u={u}')
+                for h in range(AP):
+                    ita=it*AP+h; sa=ita%AS; pa=(ita//AS)&1
+                    yield ('wait', act_full[sa], pa, ita//AS+1, f'issuer{i} act_full u={u}')
+                    if h==AP-1: deq_empty[sd].arrive()
+                    act_empty[sa].arrive()
                 n_in_seg+=1
-                deq_empty[sd].arrive(); act_empty[sa].arrive()
                 if my_last: acc_full[buf].arrive()
             elif seg_last and n_in_seg==0:
-                yield ('wait', acc_empty[buf], pacc^1, seg>>1, f'issuer{i} idle acc_empty u={u}')
+                yield ('wait', acc_empty[buf], pacc^1, seg//AB, f'issuer{i} idle acc_empty u={u}')
                 acc_full[buf].arrive()
             if seg_last: seg+=1
             it+=1; step=0 if step+1==k_steps else step+1
@@ -87,9 +92,9 @@ def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None):
             step0=u%k_steps
             tile_end=u-step0+k_steps
             seg_end=min(tile_end,ue)
-            buf=seg&1; pacc=(seg>>1)&1
+            buf=seg%AB; pacc=(seg//AB)&1
             seg+=1; u=seg_end
-            yield ('wait', acc_full[buf], pacc, ((seg-1)>>1)+1, f'epilogue acc_full seg={seg-1}')
+            yield ('wait', acc_full[buf], pacc, (seg-1)//AB+1, f'epilogue acc_full seg={seg-1}')
             acc_empty[buf].arrive()
     procs={'wprod':wprod(),'aprod':aprod(),'epi':epilogue()}
     for i in range(K): procs[f'iss{i}']=issuer(i)
@@ -187,3 +192,14 @@ def test_every_issuer_arrives_once_per_segment():
 def test_three_issuers_are_detected_as_broken():
     """The configuration that failed on the GPU fails in the model too."""
     assert deadlocked_ctas(28, 32, K=3, G=4) != []
+
+
+@pytest.mark.parametrize("n_tiles,k_steps", [(224, 32), (32, 112), (28, 32), (2, 8), (5, 2), (1, 2), (3, 6), (37, 4)])
+@pytest.mark.parametrize("config", [
+    dict(K=2, G=2, RS=8, AS=8, AB=2),          # token tiles of up to 32 rows
+    dict(K=2, G=2, RS=7, AS=6, AB=2),          # 64
+    dict(K=2, G=2, RS=5, AS=4, AB=1),          # 128
+    dict(K=1, G=2, RS=5, AS=4, AB=1, AP=2),    # 256: one issuer, two activation stages per unit
+])
+def test_protocol_of_every_token_tile(n_tiles, k_steps, config):
+    assert deadlocked_ctas(n_tiles, k_steps, **config) == []
