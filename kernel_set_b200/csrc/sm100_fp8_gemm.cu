@@ -173,6 +173,19 @@ struct TileCoord {
   int tail;       // index of the tile among the split tiles
 };
 
+// Tile t of a tiles_m x tiles_n grid: column panels of kPanel tiles, all row tiles of a panel before
+// the next panel. The tiles in flight at any time then share a few B panels and sweep A, so the
+// set that has to stay in L2 between rounds is A (small) instead of all of B.
+__device__ __forceinline__ void place_in_panels(int t, int tiles_m, int tiles_n, int* mt, int* nt) {
+  constexpr int kPanel = KSB_FP8_PANEL;
+  const int per_panel = kPanel * tiles_m;
+  const int panel = t / per_panel;
+  const int r = t - panel * per_panel;
+  const int width = (tiles_n - panel * kPanel) < kPanel ? (tiles_n - panel * kPanel) : kPanel;
+  *mt = r / width;
+  *nt = panel * kPanel + (r - *mt * width);
+}
+
 template <int BN, bool GROUPED>
 __device__ __forceinline__ bool locate_tile(const Params& p, const int* prefix, const int* offs, int t,
                                             TileCoord* tc) {
@@ -190,16 +203,8 @@ __device__ __forceinline__ bool locate_tile(const Params& p, const int* prefix, 
       t = p.split_from + tc->tail;
     }
     if (t >= p.tiles_m * p.tiles_n) return false;
-    // Column panels of kPanel tiles, all row tiles of a panel before the next panel: the
-    // tiles in flight at any time then share a few B panels and sweep A, so the set that has
-    // to stay in L2 between rounds is A (small) instead of all of B.
-    constexpr int kPanel = KSB_FP8_PANEL;
-    const int per_panel = kPanel * p.tiles_m;
-    const int panel = t / per_panel;
-    const int r = t - panel * per_panel;
-    const int width = (p.tiles_n - panel * kPanel) < kPanel ? (p.tiles_n - panel * kPanel) : kPanel;
-    const int mt = r / width;
-    const int nt = panel * kPanel + (r - mt * width);
+    int mt, nt;
+    place_in_panels(t, p.tiles_m, p.tiles_n, &mt, &nt);
     tc->expert = 0;
     tc->row0 = mt * kBM;
     tc->row_end = p.m;
@@ -218,10 +223,15 @@ __device__ __forceinline__ bool locate_tile(const Params& p, const int* prefix, 
       const int mid = (lo + hi + 1) >> 1;
       if (prefix[mid] <= mt) lo = mid; else hi = mid - 1;
     }
+    // The expert's tiles in panels, like a dense problem's: with all columns of one row tile before
+    // the next row tile, the second row tile of an expert found its weights gone from L2 where the
+    // expert's weight is larger (K=4096, N=28672 in 16 bits: 235 MB) and read them from HBM again.
+    int em, en;
+    place_in_panels(t - prefix[lo] * p.tiles_n, prefix[lo + 1] - prefix[lo], p.tiles_n, &em, &en);
     tc->expert = lo;
-    tc->row0 = offs[lo] + (mt - prefix[lo]) * kBM;
+    tc->row0 = offs[lo] + em * kBM;
     tc->row_end = offs[kMaxExperts + 1 + lo];   // ends[lo]
-    tc->n0 = (t - mt * p.tiles_n) * BN;
+    tc->n0 = en * BN;
     return true;
   }
 }
@@ -724,14 +734,8 @@ split_reduce_kernel(OutT* __restrict__ out, const float4* __restrict__ slots, in
   const int c4 = (r / 32) % kChunks;
   const int lane = r & 31;
   // the tile's place in the output: the column-panel order of locate_tile
-  constexpr int kPanel = KSB_FP8_PANEL;
-  const int t = split_from + tail;
-  const int per_panel = kPanel * tiles_m;
-  const int panel = t / per_panel;
-  const int rr = t - panel * per_panel;
-  const int width = (tiles_n - panel * kPanel) < kPanel ? (tiles_n - panel * kPanel) : kPanel;
-  const int mt = rr / width;
-  const int nt = panel * kPanel + (rr - mt * width);
+  int mt, nt;
+  place_in_panels(split_from + tail, tiles_m, tiles_n, &mt, &nt);
   const int row = mt * kBM + (ew & 3) * 32 + lane;
   const int col = nt * BN + (ew >> 2) * EC + 4 * c4;
   float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
