@@ -1,5 +1,5 @@
-// int4 weight-only GEMM for sm_100a, built for the decode regime (few
-// activation rows, the packed weight read once from HBM).
+// int4 weight-only GEMM for sm_100a: any number of rows, scale groups of 32, 64 or a multiple
+// of 128.
 //
 // Computes what ks_gemm_w4a16 declares (reference: kernels/src/gemm/
 // gemm_w4a16.cu:50-130, layout :6-19): C[M,N] = A[M,K] . W + bias with
@@ -9,49 +9,30 @@
 //
 // The GEMM is transposed onto the tensor core: the weight's N dimension is the
 // UMMA M dimension (128 TMEM lanes), the tokens are the UMMA N dimension
-// (16..128 columns), so a CTA streams 128 weight columns x 128 k per step ("unit").
-// Two ways of handing the dequantised weights (the A operand) to the tensor core:
-//
-// Tensor-memory operand (token tiles of at most 32 rows, K a multiple of 256; default there):
+// (16..256 columns), so a CTA streams 128 weight columns x 128 k per step ("unit").
 //   warp 0        weight producer (TMA): boxes of two K-steps, [128 byte-rows x 128
-//                 columns] = 16 KB straight from HBM, eight stages. (A warp keeps only
+//                 columns] = 16 KB straight from HBM. (A warp keeps only
 //                 about three TMA loads in flight whatever their size; 8 KB boxes cap a
 //                 single producer warp near 2.5 TB/s, 16 KB boxes near 4.5 TB/s.)
-//   warp 2        activation producer (TMA): one 3-D box per K-step (both 64-k swizzle
-//                 atoms of the K-slice [tokens x 128], from L2)
-//   warps 4-11    dequantisation, two groups of four warps on alternate units. A thread
-//                 owns ONE weight column (= one TMEM lane) and walks down its 64 packed
-//                 bytes: a byte holds the codes of k and k+1, exactly one 32-bit operand
-//                 cell; b * 0x1001 and one mask-or build the pair (magic + q), two packed
-//                 16-bit operations subtract (magic + zero) and apply the scale, and
-//                 tcgen05.st writes 16 cells at a time. Scales and zero-points are read
-//                 from global memory one unit ahead.
-//   warps 1, 3    MMA issuers: 4 x tcgen05.mma kind::f16 (M128, N=tokens, K16) each per
-//                 unit, A operand in tensor memory, into disjoint accumulators
-// Shared-memory operand (everything else, or KS_B200_W4A16_OPERAND=smem):
-//   warp 0        weight producer: packed tile [64 byte-rows x 128 columns] = 8 KB plus the
-//                 group's 128 scales and zero-points (2 x 256 B) per unit
-//   warp 2        activation producer (two 2-D boxes per unit)
-//   warps 4-11    dequantisation: a thread owns 8 columns x 16 k of a unit, 8 packed bytes
-//                 -> 16 weights per step by byte-permute into the (magic + q) pattern,
-//                 written as the MN-major, 128-byte-swizzled UMMA A operand
-//   warps 1, 3    MMA issuers, both operands from shared memory
-// Both:
-//   warps 12-15   epilogue: TMEM -> registers -> C, or -> an fp32 partial slot
-// Measured on B200, decode shapes: both arrangements take ~39 us for K=4096, N=28672
-// (~1000 cycles per unit against ~300 at the HBM rate). The shared-memory operand moves
-// 64 KB per unit through shared memory (~650 cycles at 128 B/clk); the tensor-memory
-// operand is bounded by tcgen05.st, which sustains only ~20 B/clk per scheduler whatever
-// the store width (~400 cycles per unit), and by its per-unit chain of waits. Processing
-// whole two-K-step boxes per iteration measured slower (48 us: two operand stages are too
-// few), as did sixteen dequantisation warps.
-// Work is cut stream-K style: the (column tile, K-step) units are dealt to the
-// CTAs in equal contiguous runs, so every SM streams the same number of bytes
-// whatever N is. A column tile whose K range is shared by several CTAs is
-// finished by the last CTA to arrive: each writes its fp32 partial to its own
-// slot, bumps the tile's counter, and the one that completes the count sums the
-// slots in slot order (deterministic) and writes C. Slots and counters live in
-// library-owned scratch memory that stays in L2.
+//   warp 2        activation producer (TMA): [tokens x 64 or 128 k] from L2
+//   warps 4-19    dequantisation (see there): shared memory -> tensor memory, where the MMA
+//                 reads the weights as its A operand
+//   warps 1, 3    MMA issuers on alternate units (one at 256 tokens)
+//   the rest      epilogue: tensor memory -> registers -> C, or an fp32 partial
+// Work is dealt out in one of three ways, chosen by estimated time (geometry_of): a tile's
+// K range over a cluster of CTAs that add their partial sums over distributed shared memory; equal
+// contiguous runs of units per CTA, where a tile shared by several CTAs is finished by the last to
+// arrive (fp32 slots in stream scratch, added in slot order: deterministic); runs of whole tiles.
+//
+// What bounds it, from work-skipping builds at K=8192, N=18944 (one tile of 64 units per CTA, 82 MB:
+// 12.6 us at the HBM rate). 16 tokens: 42 us, without the dequantisation arithmetic 26, without the
+// arithmetic and seven of eight MMAs 22: the integer pipe (half rate) and instruction issue of
+// sixteen warps. 256 tokens: 62 us, without arithmetic 51, without MMAs 47, with neither 41: the 72 KB
+// per unit that every SM reads from L2, the MMAs' own 1024 cycles per unit and the arithmetic
+// overlap only partly. (The loop has since lost a third of its integer instructions: 34.6 and 58.9 us.)
+// Measured, start of this design -> now: K=4096 N=28672 M=2048 628 -> 442 us (1.1 PFLOP/s; the weights used
+// to go through shared memory in 128-row tiles), M=192 92 -> 54 us; M=100 N=11008 group 64 730 -> 22.5 us
+// (narrow groups ran on the SIMT kernel); K=N=4096 M=1 12.3 -> 9.4 us.
 //
 // Roofline: HBM-bound for M <= 64; algorithmic bytes per launch
 // K*N/2 + (K/gs)*N*2*(1 or 2) + M*K*2 + M*N*2.
@@ -1080,7 +1061,12 @@ ks_status_t static_scratch_address(uint8_t** out) {
 size_t w4a16_static_scratch_capacity() { return kStaticScratchBytes; }
 
 ks_status_t launch_w4a16_static(const W4A16Args& a, cudaStream_t stream) {
-  const bool dec = use_decode_kernel(a);
+  bool dec = use_decode_kernel(a);
+  if (dec && a.group_size % kStepK != 0 && a.kernel == 0) {
+    // scale groups of 32 or 64 are taken at any size
+    const decode::Geometry d = decode::geometry_of(a);
+    dec = d.counter_bytes + d.slot_bytes <= kStaticScratchBytes;
+  }
   Geometry g = dec ? Geometry{} : geometry_of(a);
   const decode::Geometry gd = dec ? decode::geometry_of(a) : decode::Geometry{};
   const size_t counter_bytes = dec ? gd.counter_bytes : g.counter_bytes;

@@ -58,8 +58,8 @@ struct Geometry {
   int n_tiles = 0, k_steps = 0, grid = 0, max_parts = 0;
   size_t counter_bytes = 0, slot_bytes = 0;
 };
-// K and group_size multiples of 128, N a multiple of 16, at most kMaxTokens rows,
-// 16-byte aligned operands.
+// K a multiple of 128, group_size too (or 32 or 64, with at most 16 rows), N a multiple of 16, at
+// most kMaxTokens rows, 16-byte aligned operands.
 bool eligible(const W4A16Args& a);
 Geometry geometry_of(const W4A16Args& a);
 // Enqueues one launch on scratch the caller owns: `counters` (all zero on entry; the

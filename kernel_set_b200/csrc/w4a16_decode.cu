@@ -67,17 +67,19 @@ constexpr int kWarps = 8;
 constexpr int kThreads = kWarps * 32;
 constexpr int kWBytes = kRows * kTileN; // 16 KB of packed weight per unit
 
-template <int MG>
+// FINE: scale groups of 32 or 64 k, four or two rows of scales and zero-points per unit.
+template <int MG, bool FINE = false>
 struct Cfg {
   static constexpr int kTokens = 8 * MG;
   static constexpr int kXBytes = kTokens * kStepK * 2;   // activation slice of the unit
-  static constexpr int kSZBytes = 2 * kTileN * 2;        // one row of scales, one of zero-points
+  static constexpr int kSZRow = 2 * kTileN * 2;          // a row of scales, then one of zero-points
+  static constexpr int kSZBytes = (FINE ? 4 : 1) * kSZRow;
   static constexpr int kStageBytes = kWBytes + kXBytes + kSZBytes;
   // Two CTAs per SM (16 warps) up to 32 tokens: a warp spends about half of its time
   // between dependent instructions, and the __syncthreads of one CTA overlaps the other's
   // work. Their rings together keep 100+ KB of copies in flight per SM.
   static constexpr int kCtasPerSm = MG <= 4 ? 2 : 1;
-  static constexpr int kStages = MG <= 2 ? 5 : (MG == 4 ? 4 : 6);   // at least 4: units it+2 .. it+S-1 are in flight
+  static constexpr int kStages = MG <= 2 ? (FINE && MG == 2 ? 4 : 5) : (MG == 4 ? 4 : 6);   // at least 4: units it+2 .. it+S-1 are in flight
   static constexpr int kSmemBytes = kStages * kStageBytes + 128;
   static constexpr int kAccRegs = MG * 2 * 4;            // per lane: token groups x column chunks x 4
   static_assert(kSmemBytes * kCtasPerSm + 1024 * kCtasPerSm <= 233472, "stage rings exceed the shared memory of an SM");
@@ -94,7 +96,8 @@ struct Params {
   unsigned int* counters;   // [tiles][warp]
   int m, n, k;
   int n_tiles, k_steps;
-  int gs_steps;             // K-steps per scale group (group_size / 128)
+  int gs_steps;             // K-steps per scale group (group_size / 128); FINE: 1
+  int sz_rows;              // scale rows per unit (FINE: 128 / group_size, else 1)
   int max_parts;
   int has_zeros;
 };
@@ -198,9 +201,9 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-template <typename T, int MG>
-__global__ void __launch_bounds__(kThreads, Cfg<MG>::kCtasPerSm) w4a16_decode_kernel(const Params p) {
-  using C = Cfg<MG>;
+template <typename T, int MG, bool FINE>
+__global__ void __launch_bounds__(kThreads, (Cfg<MG, FINE>::kCtasPerSm)) w4a16_decode_kernel(const Params p) {
+  using C = Cfg<MG, FINE>;
   using P16 = Pack16<T>;
   using V2 = typename P16::V2;
   constexpr int S = C::kStages;
@@ -238,9 +241,12 @@ __global__ void __launch_bounds__(kThreads, Cfg<MG>::kCtasPerSm) w4a16_decode_ke
   const size_t w_step = static_cast<size_t>(kRows) * p.n;          // one K-step further down
   const size_t x_row16 = static_cast<size_t>(16) * p.k * 2;        // 16 tokens further down
   const uint8_t* const a_bytes = static_cast<const uint8_t*>(p.a);
-  const uint8_t* const sz_base = static_cast<const uint8_t*>(warp == 0 ? p.scales : p.zeros);
-  const bool sz_active = warp == 0 || (warp == 1 && p.has_zeros);
-  const uint32_t sz_dst = kWBytes + C::kXBytes + (warp == 1 ? kTileN * 2 : 0) + (lane << 4);
+  // (FINE: warps 2r and 2r + 1 copy the unit's row r)
+  const bool sz_zeros = (warp & 1) != 0;
+  const int sz_row = warp >> 1;
+  const uint8_t* const sz_base = static_cast<const uint8_t*>(sz_zeros ? p.zeros : p.scales);
+  const bool sz_active = sz_row < (FINE ? p.sz_rows : 1) && (!sz_zeros || p.has_zeros);
+  const uint32_t sz_dst = kWBytes + C::kXBytes + sz_row * C::kSZRow + (sz_zeros ? kTileN * 2 : 0) + (lane << 4);
   // tokens this thread stages: ld_r0 + 16 i; rows at or beyond M are written as zeros
   uint32_t x_bytes[kXChunks];
 #pragma unroll
@@ -256,7 +262,8 @@ __global__ void __launch_bounds__(kThreads, Cfg<MG>::kCtasPerSm) w4a16_decode_ke
     w_src = w_ok ? p.w + (static_cast<size_t>(step) * kRows + ld_r0) * p.n + col0 + ld_cc * 16 : p.w;
     const bool s_ok = sz_active && col0 + lane * 8 < p.n;
     sz_bytes = s_ok ? 16u : 0u;
-    sz_src = s_ok ? sz_base + (static_cast<size_t>(grp) * p.n + col0 + lane * 8) * 2 : a_bytes;
+    const int row = FINE ? step * p.sz_rows + sz_row : grp;
+    sz_src = s_ok ? sz_base + (static_cast<size_t>(row) * p.n + col0 + lane * 8) * 2 : a_bytes;
   };
   enter_tile(tile_l, step_l, grp_l);
   // The activations may be the output of the kernel that runs before this one on the stream;
@@ -291,7 +298,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<MG>::kCtasPerSm) w4a16_decode_ke
         if (w_bytes) w_src += w_step;
         if (++in_grp_l == p.gs_steps) {
           in_grp_l = 0; ++grp_l;
-          if (sz_bytes) sz_src += static_cast<size_t>(p.n) * 2;
+          if (sz_bytes) sz_src += static_cast<size_t>(p.n) * 2 * (FINE ? p.sz_rows : 1);
         }
       }
     }
@@ -396,22 +403,24 @@ __global__ void __launch_bounds__(kThreads, Cfg<MG>::kCtasPerSm) w4a16_decode_ke
     // scales and zero-points of this lane's columns: chunk c, columns 2g and 2g+1
     V2 sc[2][2], zz[2][2];
     uint32_t sraw[2], zraw[2];
-    uint32_t bad = 0u;
+    auto load_constants = [&](uint32_t row_off) {   // true: every column's zero-point takes the short form
+      uint32_t bad = 0u;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      sraw[c] = lds32(st + sz_off + 32u * c);
-      zraw[c] = p.has_zeros ? lds32(st + sz_off + 32u * c + kTileN * 2) : 0u;
-      sc[c][0] = P16::from_bits(__byte_perm(sraw[c], sraw[c], 0x1010));
-      sc[c][1] = P16::from_bits(__byte_perm(sraw[c], sraw[c], 0x3232));
-      // (magic + zero) must be exact; then (magic + q) - (magic + zero) is exact too: true for
-      // every non-negative integer zero-point that survives the round trip
-      const V2 zp = __hadd2(P16::from_bits(zraw[c]), magic2);
-      bad |= (P16::bits(__hsub2(zp, magic2)) ^ zraw[c]) | (zraw[c] & 0x80008000u);
-      const uint32_t zb = P16::bits(zp);
-      zz[c][0] = P16::from_bits(__byte_perm(zb, zb, 0x1010));
-      zz[c][1] = P16::from_bits(__byte_perm(zb, zb, 0x3232));
-    }
-    const bool simple = !__any_sync(0xFFFFFFFFu, bad != 0u);
+      for (int c = 0; c < 2; ++c) {
+        sraw[c] = lds32(st + sz_off + row_off + 32u * c);
+        zraw[c] = p.has_zeros ? lds32(st + sz_off + row_off + 32u * c + kTileN * 2) : 0u;
+        sc[c][0] = P16::from_bits(__byte_perm(sraw[c], sraw[c], 0x1010));
+        sc[c][1] = P16::from_bits(__byte_perm(sraw[c], sraw[c], 0x3232));
+        // (magic + zero) must be exact; then (magic + q) - (magic + zero) is exact too: true for
+        // every non-negative integer zero-point that survives the round trip
+        const V2 zp = __hadd2(P16::from_bits(zraw[c]), magic2);
+        bad |= (P16::bits(__hsub2(zp, magic2)) ^ zraw[c]) | (zraw[c] & 0x80008000u);
+        const uint32_t zb = P16::bits(zp);
+        zz[c][0] = P16::from_bits(__byte_perm(zb, zb, 0x1010));
+        zz[c][1] = P16::from_bits(__byte_perm(zb, zb, 0x3232));
+      }
+      return !__any_sync(0xFFFFFFFFu, bad != 0u);
+    };
 
     auto pair_body = [&](int pr, auto fast_tag) {
       constexpr bool kFast = decltype(fast_tag)::value;
@@ -455,7 +464,17 @@ __global__ void __launch_bounds__(kThreads, Cfg<MG>::kCtasPerSm) w4a16_decode_ke
         }
       }
     };
-    if (simple) {
+    if constexpr (FINE) {
+      // pair pr covers 32 k: the unit's scale row pr (group 32) or pr / 2 (group 64)
+      bool simple = false;
+#pragma unroll
+      for (int pr = 0; pr < 4; ++pr) {
+        if (pr == 0 || p.sz_rows == 4 || (pr & 1) == 0)
+          simple = load_constants((p.sz_rows == 4 ? pr : pr >> 1) * C::kSZRow);
+        if (simple) pair_body(pr, std::true_type{});
+        else pair_body(pr, std::false_type{});
+      }
+    } else if (load_constants(0u)) {
 #pragma unroll
       for (int pr = 0; pr < 4; ++pr) pair_body(pr, std::true_type{});
     } else {
@@ -561,10 +580,10 @@ __global__ void __launch_bounds__(kThreads, Cfg<MG>::kCtasPerSm) w4a16_decode_ke
   }
 }
 
-template <typename T, int MG>
+template <typename T, int MG, bool FINE>
 ks_status_t launch_t(const Params& p, int grid, cudaStream_t stream) {
-  using C = Cfg<MG>;
-  auto kernel = w4a16_decode_kernel<T, MG>;
+  using C = Cfg<MG, FINE>;
+  auto kernel = w4a16_decode_kernel<T, MG, FINE>;
   static std::mutex mu;
   static bool attr_done[64] = {};
   int dev = 0;
@@ -585,12 +604,13 @@ ks_status_t launch_t(const Params& p, int grid, cudaStream_t stream) {
 }
 
 template <typename T>
-ks_status_t launch_mg(int mg, const Params& p, int grid, cudaStream_t stream) {
+ks_status_t launch_mg(int mg, bool fine, const Params& p, int grid, cudaStream_t stream) {
+  if (fine) return mg == 1 ? launch_t<T, 1, true>(p, grid, stream) : launch_t<T, 2, true>(p, grid, stream);
   switch (mg) {
-    case 1: return launch_t<T, 1>(p, grid, stream);
-    case 2: return launch_t<T, 2>(p, grid, stream);
-    case 4: return launch_t<T, 4>(p, grid, stream);
-    default: return launch_t<T, 8>(p, grid, stream);
+    case 1: return launch_t<T, 1, false>(p, grid, stream);
+    case 2: return launch_t<T, 2, false>(p, grid, stream);
+    case 4: return launch_t<T, 4, false>(p, grid, stream);
+    default: return launch_t<T, 8, false>(p, grid, stream);
   }
 }
 
@@ -599,7 +619,8 @@ ks_status_t launch_mg(int mg, const Params& p, int grid, cudaStream_t stream) {
 bool eligible(const W4A16Args& a) {
   if (a.m > kMaxTokens) return false;
   if (a.k % kStepK != 0) return false;
-  if (a.group_size % kStepK != 0) return false;   // one scale row per 128-k step
+  // one scale row per 128-k step, or (up to 16 tokens, where this kernel is chosen) two or four
+  if (a.group_size % kStepK != 0 && !((a.group_size == 32 || a.group_size == 64) && a.m <= 16)) return false;
   if (a.n % 16 != 0) return false;                // 16-byte chunks of the packed rows and of the scale rows
   if (!aligned16(a.a) || !aligned16(a.b_packed) || !aligned16(a.scales)) return false;
   if (a.zeros != nullptr && !aligned16(a.zeros)) return false;
@@ -640,11 +661,13 @@ ks_status_t enqueue(const W4A16Args& a, const Geometry& g, unsigned int* counter
   p.k = static_cast<int>(a.k);
   p.n_tiles = g.n_tiles;
   p.k_steps = g.k_steps;
-  p.gs_steps = a.group_size / kStepK;
+  const bool fine = a.group_size < kStepK;
+  p.gs_steps = fine ? 1 : a.group_size / kStepK;
+  p.sz_rows = fine ? kStepK / a.group_size : 1;
   p.max_parts = g.max_parts;
   p.has_zeros = a.zeros != nullptr ? 1 : 0;
-  if (a.dtype == KS_DTYPE_BF16) return launch_mg<__nv_bfloat16>(g.mg, p, g.grid, stream);
-  return launch_mg<__half>(g.mg, p, g.grid, stream);
+  if (a.dtype == KS_DTYPE_BF16) return launch_mg<__nv_bfloat16>(g.mg, fine, p, g.grid, stream);
+  return launch_mg<__half>(g.mg, fine, p, g.grid, stream);
 }
 
 }  // namespace decode

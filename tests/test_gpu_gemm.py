@@ -641,3 +641,38 @@ def test_w4a16_tcgen05_token_tiles_and_fine_groups(ks, cuda, m, k, n, gs, dtype,
     with w4_path("general"):
         gen_out = ks.dispatch.w4a16(a, b_packed, scales, zp, group_size=gs, bias=bias_t)
     assert orc.rel_frobenius(out.cpu().float(), gen_out.cpu().float()) < 2e-3
+
+
+@pytest.mark.parametrize("m,k,n,gs,dtype,zeros,bias", [
+    (1, 128, 256, 32, torch.bfloat16, "random", False),       # one unit
+    (8, 4096, 272, 64, torch.float16, "eight", True),         # a tile split over many CTAs, ragged columns
+    (9, 640, 1040, 32, torch.bfloat16, "fraction", True),     # two token groups, fp32 dequantisation
+    (16, 4096, 14336, 64, torch.bfloat16, "random", False),   # every ring wraps several times
+    (5, 1152, 4112, 32, torch.float16, None, False),          # zeros == NULL, odd number of K-steps
+])
+def test_w4a16_decode_kernel_fine_groups(ks, cuda, m, k, n, gs, dtype, zeros, bias):
+    """The register-operand kernel with two or four scale rows per K-step, against the oracle and the general
+    kernel, and against itself (the second call finds the split-K counters as the first left them)."""
+    g = gen(m + k + n + gs)
+    a = torch.randn(m, k, generator=g).to(dtype)
+    codes = torch.randint(0, 16, (k, n), generator=g).to(torch.int32)
+    scales = (torch.randn(k // gs, n, generator=g).mul(0.02).abs() + 1e-3).to(dtype)
+    zp = {"eight": lambda: torch.full((k // gs, n), 8.0).to(dtype),
+          "random": lambda: torch.randint(0, 16, (k // gs, n), generator=g).to(dtype),
+          "fraction": lambda: (torch.rand(k // gs, n, generator=g) * 15).to(dtype),
+          None: lambda: None}[zeros]()
+    b_packed = orc.pack_int4_bytes(codes)
+    bias_t = torch.randn(n, generator=g).to(dtype) if bias else None
+    ref32 = orc.w4a16(a, b_packed, scales, zp, gs, bias_t, out_dtype=None)
+    noise = accumulation_noise(a.float().abs(), orc.w4a16_weight(b_packed, scales, zp, gs).float().abs(), k)
+    args = (a.to(cuda), b_packed.to(cuda), scales.to(cuda), zp.to(cuda) if zp is not None else None)
+    kw = dict(group_size=gs, bias=bias_t.to(cuda) if bias else None)
+    with w4_path("decode"):
+        out = ks.dispatch.w4a16(*args, **kw)
+        out2 = ks.dispatch.w4a16(*args, **kw)
+        torch.cuda.synchronize()
+    check_gemm(out.cpu(), ref32, noise, f"w4a16 decode {m}x{n}x{k} group {gs}")
+    assert torch.equal(out.cpu().view(torch.int16), out2.cpu().view(torch.int16)), "not reproducible run to run"
+    with w4_path("general"):
+        gen_out = ks.dispatch.w4a16(*args, **kw)
+    assert orc.rel_frobenius(out.cpu().float(), gen_out.cpu().float()) < 2e-3
