@@ -300,14 +300,18 @@ inverse_permutation_kernel(int32_t* __restrict__ inverse, const int32_t* __restr
   if (pair >= 0 && pair < pairs) inverse[pair] = static_cast<int32_t>(r);
 }
 
+// `row` if it is the row of pair `pair`, else -1.
+__device__ __forceinline__ int32_t check_row(int32_t row, const int32_t* __restrict__ ids, int64_t pair, int64_t pairs) {
+  return (row >= 0 && row < pairs && __ldg(ids + row) == pair) ? row : -1;
+}
+
 // Row of a pair after the sort, -1 for a dropped pair. The inverse map of a dropped pair was not
 // written by this call and holds whatever an earlier one left there, so the row it names is
 // looked up again: only the row that really holds the pair counts. (Clearing the map first was
 // a launch of its own.)
 __device__ __forceinline__ int32_t row_of_pair(const int32_t* __restrict__ inverse, const int32_t* __restrict__ ids,
                                                int64_t pair, int64_t pairs) {
-  const int32_t row = __ldg(inverse + pair);
-  return (row >= 0 && row < pairs && __ldg(ids + row) == pair) ? row : -1;
+  return check_row(__ldg(inverse + pair), ids, pair, pairs);
 }
 
 // permute_quant_kernel the other way round, for large problems: a token is read and quantized
@@ -389,14 +393,31 @@ unpermute_vec8_kernel(T* __restrict__ out, const T* __restrict__ permuted, const
     float acc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    for (int k = 0; k < top_k; ++k) {
-      const int32_t prow = row_of_pair(inverse, ids, token * top_k + k, tokens * top_k);
-      if (prow < 0) continue;
-      const float w = __ldg(weights + token * top_k + k);
-      const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(permuted + static_cast<int64_t>(prow) * hidden) + c);
-      const T* x = reinterpret_cast<const T*>(&raw);
+    // four slots at a time: their index loads, then their rows, are in flight together (one slot
+    // after the other is a chain of three loads per slot)
+    for (int k0 = 0; k0 < top_k; k0 += 4) {
+      int32_t prow[4];
+      float w[4];
+      uint4 raw[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] = fmaf(to_f32<T>(x[j]), w, acc[j]);
+      for (int j = 0; j < 4; ++j) {
+        const bool in = k0 + j < top_k;
+        prow[j] = in ? __ldg(inverse + token * top_k + k0 + j) : -1;
+        w[j] = in ? __ldg(weights + token * top_k + k0 + j) : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) prow[j] = check_row(prow[j], ids, token * top_k + k0 + j, tokens * top_k);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (prow[j] >= 0)
+          raw[j] = __ldcs(reinterpret_cast<const uint4*>(permuted + static_cast<int64_t>(prow[j]) * hidden) + c);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (prow[j] < 0) continue;
+        const T* x = reinterpret_cast<const T*>(&raw[j]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = fmaf(to_f32<T>(x[i]), w[j], acc[i]);
+      }
     }
     uint4 o;
     T* y = reinterpret_cast<T*>(&o);
