@@ -179,3 +179,30 @@ def test_status_codes_on_device(ks, cuda):
     assert ks.device_count() >= 1
     props = ks.runtime.get_device_properties(0)
     assert props["compute_major"] == 10 and props["multiprocessor_count"] > 0
+
+
+@pytest.mark.parametrize("rows,cols,dtype,fp8", [
+    (259, 2464, torch.float16, "e4m3"),     # last group of 32
+    (7, 16, torch.bfloat16, "e4m3"),        # one segment: narrower than a group
+    (33, 240, torch.float32, "e5m2"),       # last group of 112
+    (1, 1040, torch.bfloat16, "e4m3"),
+    (129, 144, torch.float16, "e5m2"),
+])
+def test_quantizer_rows_of_whole_segments(ks, cuda, rows, cols, dtype, fp8):
+    """Widths that are a multiple of 16 but not of the group, against the oracle, and with infinities and NaN
+    against the general kernel (which an input off the 16-byte grid takes)."""
+    x = (torch.randn(rows, cols, generator=gen(rows + cols)) * 3.0).to(dtype)
+    x[0, :16] = 0
+    q_ref, s_ref = orc.quantize_fp8_group(x, 128, fp8)
+    q, s = run_quant(ks, x, 128, fp8, cuda)
+    assert torch.equal(s, s_ref)
+    assert torch.equal(q.view(torch.uint8), q_ref.view(torch.uint8))
+    x[0, 3], x[rows - 1, cols - 1], x[rows // 2, cols // 2] = float("inf"), float("nan"), float("-inf")
+    x = x.to(cuda)
+    off = torch.empty(rows * cols + 1, dtype=dtype, device=cuda)[1:].view(rows, cols)
+    off.copy_(x)
+    kw = dict(fp8_dtype=ks.DType.F8E5M2 if fp8 == "e5m2" else ks.DType.F8E4M3)
+    q, s = ks.dispatch.per_token_group_quant(x, **kw)
+    q2, s2 = ks.dispatch.per_token_group_quant(off, **kw)
+    assert torch.equal(q.view(torch.uint8), q2.view(torch.uint8))
+    assert torch.equal(s.view(torch.int32), s2.view(torch.int32))
