@@ -145,11 +145,19 @@ compute_permutation_kernel(int32_t* __restrict__ sorted_ids, int32_t* __restrict
   __shared__ int warp_sums[kPermWarps];
   __shared__ int routed_pairs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < kPermWarps * experts; i += kPermThreads) cnt[i] = 0;
-  for (int i = threadIdx.x; i < 2 * experts; i += kPermThreads) before[i] = 0;
-  __syncthreads();
   const int64_t c_begin = static_cast<int64_t>(blockIdx.x) * chunk;
   const int64_t c_end = c_begin + chunk < pairs ? c_begin + chunk : pairs;
+  // this CTA's pairs: a piece of chunk / 32 (a multiple of 32) per warp, in the first `warps` warps
+  const int64_t piece = chunk / kPermWarps;
+  const int64_t begin = c_begin + warp * piece;
+  const int64_t end = begin + piece < c_end ? begin + piece : c_end;
+  const int warps = static_cast<int>((c_end - c_begin + piece - 1) / piece);
+  // the ids of a warp's first step stay in registers: with up to 1024 pairs a CTA that is all of them
+  const int e_first = begin + lane < end ? __ldg(topk_idx + begin + lane) : -1;
+  const int rows = gridDim.x == 1 ? warps : kPermWarps;   // of `cnt` in use
+  for (int i = threadIdx.x; i < rows * experts; i += kPermThreads) cnt[i] = 0;
+  for (int i = threadIdx.x; i < 2 * experts; i += kPermThreads) before[i] = 0;
+  __syncthreads();
   int* mine = cnt + warp * experts;
   if (c_begin > 0) {
     count_pairs(mine, topk_idx, 0, c_begin, experts);
@@ -159,13 +167,9 @@ compute_permutation_kernel(int32_t* __restrict__ sorted_ids, int32_t* __restrict
     count_pairs(mine, topk_idx, c_end, pairs, experts);
     fold_counts(cnt, total, experts);
   }
-  // this CTA's pairs: a piece of chunk / 32 (a multiple of 32) per warp
-  const int64_t piece = chunk / kPermWarps;
-  const int64_t begin = c_begin + warp * piece;
-  const int64_t end = begin + piece < c_end ? begin + piece : c_end;
   for (int64_t base = begin; base < end; base += 32) {
     const int64_t i = base + lane;
-    const int e = i < end ? __ldg(topk_idx + i) : -1;
+    const int e = base == begin ? e_first : (i < end ? __ldg(topk_idx + i) : -1);
     const bool valid = e >= 0 && e < experts;
     const unsigned mask = __match_any_sync(0xffffffffu, valid ? e : experts + lane);
     if (valid && lane == __ffs(mask) - 1) mine[e] += __popc(mask);
@@ -176,7 +180,7 @@ compute_permutation_kernel(int32_t* __restrict__ sorted_ids, int32_t* __restrict
   for (int e = threadIdx.x; e < experts; e += kPermThreads) {
     int run = before[e];
 #pragma unroll 8
-    for (int w = 0; w < kPermWarps; ++w) {
+    for (int w = 0; w < warps; ++w) {
       const int c = cnt[w * experts + e];
       cnt[w * experts + e] = run;
       run += c;
@@ -219,7 +223,7 @@ compute_permutation_kernel(int32_t* __restrict__ sorted_ids, int32_t* __restrict
   __syncthreads();
   for (int64_t base = begin; base < end; base += 32) {
     const int64_t i = base + lane;
-    const int e = i < end ? __ldg(topk_idx + i) : -1;
+    const int e = base == begin ? e_first : (i < end ? __ldg(topk_idx + i) : -1);
     const bool valid = e >= 0 && e < experts;
     const unsigned mask = __match_any_sync(0xffffffffu, valid ? e : experts + lane);
     if (valid) sorted_ids[total[e] + mine[e] + __popc(mask & ((1u << lane) - 1u))] = static_cast<int32_t>(i);

@@ -242,11 +242,11 @@ __global__ void __launch_bounds__(kThreads, (Cfg<MG, FINE>::kCtasPerSm)) w4a16_d
   const size_t x_row16 = static_cast<size_t>(16) * p.k * 2;        // 16 tokens further down
   const uint8_t* const a_bytes = static_cast<const uint8_t*>(p.a);
   // (FINE: warps 2r and 2r + 1 copy the unit's row r)
-  const bool sz_zeros = (warp & 1) != 0;
-  const int sz_row = warp >> 1;
+  const bool sz_zeros = FINE ? (warp & 1) != 0 : warp != 0;
+  const int sz_row = FINE ? warp >> 1 : 0;
   const uint8_t* const sz_base = static_cast<const uint8_t*>(sz_zeros ? p.zeros : p.scales);
-  const bool sz_active = sz_row < (FINE ? p.sz_rows : 1) && (!sz_zeros || p.has_zeros);
-  const uint32_t sz_dst = kWBytes + C::kXBytes + sz_row * C::kSZRow + (sz_zeros ? kTileN * 2 : 0) + (lane << 4);
+  const bool sz_active = FINE ? sz_row < p.sz_rows && (!sz_zeros || p.has_zeros) : warp == 0 || (warp == 1 && p.has_zeros);
+  const uint32_t sz_dst = kWBytes + C::kXBytes + sz_row * C::kSZRow + ((FINE ? sz_zeros : warp == 1) ? kTileN * 2 : 0) + (lane << 4);
   // tokens this thread stages: ld_r0 + 16 i; rows at or beyond M are written as zeros
   uint32_t x_bytes[kXChunks];
 #pragma unroll
