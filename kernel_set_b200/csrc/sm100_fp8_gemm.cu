@@ -886,6 +886,19 @@ bool fp8_blockwise_eligible(const Fp8GemmArgs& a) {
   return tma_available();
 }
 
+namespace {
+
+// Parts that each of the `rem` tiles of a partial round is cut into along K: as many as the grid has
+// CTAs for, at most eight (each part is one more partial to add up), and four K-blocks a part at least.
+int64_t split_parts(int64_t grid, int64_t rem, int64_t nkb) {
+  int64_t s = grid / rem;
+  if (s > 8) s = 8;
+  while (s > 1 && nkb / s < 4) --s;
+  return s;
+}
+
+}  // namespace
+
 ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   const bool grouped = a.offsets != nullptr || a.masked_m != nullptr;
   const int experts = grouped ? a.num_experts : 1;
@@ -909,17 +922,36 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   int bn = (a.force_bn == 128 || a.force_bn == 256) ? a.force_bn : (cost256 <= cost128 ? 256 : 128);
 
   // Fewer tiles than SMs (dense block-scaled problems): cut every tile along K over a cluster of
-  // S CTAs. Same unit of cost; sharing a tile adds two cluster barriers and the exchange
-  // of the partials (~3000 cycles). At least two K-blocks per CTA.
+  // S CTAs. Same unit of cost, and never less than the weight takes from HBM (~3500 bytes a cycle). Sharing
+  // a tile costs ~9000 cycles by the shapes above and in the header: two cluster barriers, the
+  // exchange of the partials, and a pipeline fill that fewer K-blocks pay for (M=94, N=11632, K=7040 is
+  // better left to 91 unshared tiles of 128 columns). At least two K-blocks per CTA.
   int cluster_s = 1;
   if (!grouped && a.mode == 0 && a.force_split != 0 && a.num_out_parts == 0) {
     const int64_t nkb = (a.k + kBK - 1) / kBK;
+    const int64_t hbm = a.n * a.k / 3500;
     int64_t best = INT64_MAX;
     for (int w = 256; w >= 128; w -= 128) {
       if ((a.force_bn == 128 || a.force_bn == 256) && a.force_bn != w) continue;
       const int64_t tiles = w == 256 ? tiles256 : tiles128;
       const int64_t per_kb = w == 256 ? 850 : 550;
-      const int64_t whole = (tiles + sms - 1) / sms * nkb * per_kb;
+      // full rounds of tiles, then the partial round: a whole round, or (see below) its tiles cut
+      // along K over the idle SMs, plus the partials' way through memory and the reducing kernel:
+      // 10000 to 16000 cycles by shapes where one width needs it and the other does not. Without
+      // the second form 160 tiles of 256 columns counted as two rounds and lost to 320 of 128:
+      // M=2500, N=2000, K=4096 42.0 -> 37.9 us; M=426, N=10528, K=15616 107.5 -> 91.1.
+      const int64_t rem = tiles % sms;
+      int64_t part = nkb;
+      int64_t extra = 0;
+      if (rem > 0 && tiles > sms) {
+        const int64_t s = split_parts(sms, rem, nkb);
+        if (s >= 2) {
+          part = (nkb + s - 1) / s;
+          extra = 14000;
+        }
+      }
+      const int64_t chain = (tiles / sms * nkb + (rem > 0 ? part : 0)) * per_kb;
+      const int64_t whole = (chain > hbm ? chain : hbm) + extra;
       if (whole < best) {
         best = whole;
         bn = w;
@@ -927,7 +959,8 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
       }
       for (int s = 2; s <= kMaxClusterSplit && tiles * s <= sms && nkb >= 2 * s; ++s) {
         if (cluster_capacity(s) < tiles) break;   // all clusters run at once
-        const int64_t cost = (nkb + s - 1) / s * per_kb + 3000;
+        const int64_t shared = (nkb + s - 1) / s * per_kb;
+        const int64_t cost = (shared > hbm ? shared : hbm) + 9000;
         if (cost < best) {
           best = cost;
           bn = w;
@@ -1023,9 +1056,7 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
     p.split_s = cluster_s;
   } else if (!grouped && a.mode == 0 && a.force_split != 0 && a.num_out_parts == 0 && tiles > grid) {
     const int rem = static_cast<int>(tiles % grid);
-    int s = rem > 0 ? grid / rem : 1;
-    if (s > 8) s = 8;
-    while (s > 1 && p.nkb / s < 4) --s;
+    const int s = rem > 0 ? static_cast<int>(split_parts(grid, rem, p.nkb)) : 1;
     if (rem > 0 && s >= 2) {
       const size_t slot_bytes = static_cast<size_t>(rem) * s * kBM * bn * sizeof(float);
       float4* slots = static_cast<float4*>(stream_scratch(stream, slot_bytes, 2));

@@ -676,3 +676,46 @@ def test_w4a16_decode_kernel_fine_groups(ks, cuda, m, k, n, gs, dtype, zeros, bi
     with w4_path("general"):
         gen_out = ks.dispatch.w4a16(*args, **kw)
     assert orc.rel_frobenius(out.cpu().float(), gen_out.cpu().float()) < 2e-3
+
+
+@pytest.mark.parametrize("m,n,k,layout,bn_tile,out_dtype", [
+    (1, 256, 2048, "nk", 256, torch.float32),      # one row, one tile over a full cluster of eight
+    (16, 1024, 7168, "nk", 256, torch.bfloat16),
+    (129, 272, 4096, "kn", 128, torch.float16),    # a second row tile of one row, a ragged column tile
+    (40, 101, 1040, "nk", 128, torch.float32),     # rows off the 16-byte grid, ragged K
+    (6, 624, 3712, "kn", None, torch.bfloat16),    # tile width left to the rule
+    (300, 1040, 512, "nk", None, torch.float32),   # four K-blocks: at most two parts
+])
+def test_fp8_tiles_shared_by_a_cluster(ks, cuda, m, n, k, layout, bn_tile, out_dtype):
+    """Problems with fewer tiles than SMs, whose tiles a cluster cuts along K, against the oracle, the unsplit
+    kernel (same products, sums in another order) and a second run (bit for bit)."""
+    a8, a_s, b8, b_s = fp8_inputs(m, n, k, seed=m * 7 + n + k)
+    ref32, noise = fp8_reference(a8, a_s, b8, b_s)
+    with fp8_path("tcgen05", bn_tile):
+        out = run_fp8(ks, cuda, a8, a_s, b8, b_s, layout, out_dtype)
+        again = run_fp8(ks, cuda, a8, a_s, b8, b_s, layout, out_dtype)
+        os.environ["KS_B200_FP8_SPLIT"] = "0"
+        try:
+            whole = run_fp8(ks, cuda, a8, a_s, b8, b_s, layout, out_dtype)
+        finally:
+            os.environ.pop("KS_B200_FP8_SPLIT", None)
+    check_gemm(out, ref32, noise, f"cluster {m}x{n}x{k} {layout}")
+    assert torch.equal(out, again), "not reproducible run to run"
+    assert orc.rel_frobenius(out.float(), whole.float()) < (1e-5 if out_dtype == torch.float32 else 2e-3)
+
+
+def test_grouped_tiles_in_column_panels(ks, cuda):
+    """Experts with no, one, two and five row tiles over seven column tiles of 256 (a full and a partial panel),
+    every row against a dense product with its expert's weight."""
+    sizes, k, n = [0, 128, 1, 600, 0, 130, 256], 512, 1680
+    g = gen(9)
+    off = torch.tensor([0] + torch.tensor(sizes).cumsum(0).tolist(), dtype=torch.int32)
+    a = torch.randn(int(off[-1]), k, generator=g).to(torch.bfloat16)
+    w = (torch.randn(len(sizes), k, n, generator=g) * 0.05).to(torch.bfloat16)
+    out = ks.dispatch.moe(a.to(cuda), w.to(cuda), off.to(cuda), num_experts=len(sizes), n=n, k=k).cpu().float()
+    for e in range(len(sizes)):
+        lo, hi = int(off[e]), int(off[e + 1])
+        if hi > lo:
+            ref = a[lo:hi].double() @ w[e].double()
+            # bf16 outputs: half an ulp each, 2^-9 relative
+            assert orc.rel_frobenius(out[lo:hi], ref.float()) < 2.0 ** -8
