@@ -41,7 +41,7 @@
 // scale fetches ~10 %; barriers alone 58 us. The two sides are equally long and the two
 // accumulator buffers couple them instead of letting them overlap fully. Measured and not
 // better: handing the accumulator over in two 128-column halves (eight N=128 MMAs per
-// K-block read A twice: 232 us), wider loads, more loads in flight, sixteen narrower epilogue
+// K-block read A twice: 232 us), more loads in flight, sixteen narrower epilogue
 // warps, 224-wide tiles, scalar FMAs, paced MMA issue, sleeping or spinning waits.
 // Problems with fewer tiles than SMs (decode: M = 16, N = 7168 is 28 tiles of 256 columns) are
 // cut along K as well, over the S <= 8 CTAs of a cluster: each leaves its fp32 partial tile in
