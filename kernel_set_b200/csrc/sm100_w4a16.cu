@@ -9,7 +9,7 @@
 //
 // The GEMM is transposed onto the tensor core: the weight's N dimension is the
 // UMMA M dimension (128 TMEM lanes), the tokens are the UMMA N dimension
-// (16..256 columns), so a CTA streams 128 weight columns x 128 k per step ("unit").
+// (16..192 columns), so a CTA streams 128 weight columns x 128 k per step ("unit").
 //   warp 0        weight producer (TMA): boxes of two K-steps, [128 byte-rows x 128
 //                 columns] = 16 KB straight from HBM. (A warp keeps only
 //                 about three TMA loads in flight whatever their size; 8 KB boxes cap a
@@ -17,7 +17,7 @@
 //   warp 2        activation producer (TMA): [tokens x 64 or 128 k] from L2
 //   warps 4-19    dequantisation (see there): shared memory -> tensor memory, where the MMA
 //                 reads the weights as its A operand
-//   warps 1, 3    MMA issuers on alternate units (one at 256 tokens)
+//   warps 1, 3    MMA issuers on alternate units (above 128 tokens: on the two 64-k halves of every unit)
 //   the rest      epilogue: tensor memory -> registers -> C, or an fp32 partial
 // Work is dealt out in one of three ways, chosen by estimated time (geometry_of): a tile's
 // K range over a cluster of CTAs that add their partial sums over distributed shared memory; equal
@@ -27,11 +27,10 @@
 // What bounds it, from work-skipping builds at K=8192, N=18944 (one tile of 64 units per CTA, 82 MB:
 // 12.6 us at the HBM rate). 16 tokens: 42 us, without the dequantisation arithmetic 26, without the
 // arithmetic and seven of eight MMAs 22: the integer pipe (half rate) and instruction issue of
-// sixteen warps. 256 tokens: 62 us, without arithmetic 51, without MMAs 47, with neither 41: the 72 KB
-// per unit that every SM reads from L2, the MMAs' own 1024 cycles per unit and the arithmetic
-// overlap only partly. (The loop has since lost a third of its integer instructions: 34.6 and 58.9 us.)
-// Measured, start of this design -> now: K=4096 N=28672 M=2048 628 -> 442 us (1.1 PFLOP/s; the weights used
-// to go through shared memory in 128-row tiles), M=192 92 -> 54 us; M=100 N=11008 group 64 730 -> 22.5 us
+// sixteen warps. Wide tiles: the stream from L2 (8 KB of weight and 256 bytes per token a unit), the MMAs (4
+// cycles per token and unit) and the arithmetic overlap only partly.
+// Measured, 128-row tiles with the weights through shared memory -> this design: K=4096 N=28672
+// M=2048 545 -> 416 us (1.16 PFLOP/s), M=192 92 -> 49 us; M=100 N=11008 group 64 730 -> 22.5 us
 // (narrow groups ran on the SIMT kernel); K=N=4096 M=1 12.3 -> 9.4 us.
 //
 // Roofline: HBM-bound for M <= 64; algorithmic bytes per launch
@@ -63,7 +62,6 @@ constexpr int kGroups = 2;
 constexpr int kDeqGroupWarps = 8;
 constexpr int kDeqWarps = kGroups * kDeqGroupWarps;
 constexpr int kDeqStages = 4;      // operand stages in tensor memory
-constexpr int kDeqTmemCols = kStepK / 2;   // 64 columns of two k each
 constexpr int kAtomK = 64;         // k per 128-byte swizzle atom of the activations
 
 // Everything that depends on the width of the token tile. The numbers of operand stages and
@@ -74,10 +72,17 @@ constexpr int kAtomK = 64;         // k per 128-byte swizzle atom of the activat
 // protocol model under tests/.)
 template <int MTMAX>
 struct Cfg {
-  // Issuing a tcgen05.mma costs its thread ~55 cycles. Up to 64 token columns the tensor core
-  // needs less than that, at 128 about as much; two issuers take alternate units into accumulators
-  // of their own. 256 columns are bound by the tensor core (128 cycles per instruction).
-  static constexpr int kIssuers = MTMAX <= 128 ? 2 : 1;
+  // Issuing a tcgen05.mma costs its thread ~55 cycles: up to 64 token columns the tensor core needs
+  // less than that, at 128 about as much. Two issuers, with accumulators of their own, take alternate
+  // units, or above 128 rows the two 64-k halves of every unit (kHalfStages): the operand ring's 128
+  // columns are then four stages of 64 k, each filled by four warps. (One issuer for both halves: K=4096
+  // N=28672 M=2048 445 us instead of 416.)
+  // Two sums also halve the error. tcgen05.mma truncates what it adds up, so a sum's error grows with its
+  // instructions: at K=14336, f16, positive operands, 256-row tiles, which leave room for one accumulator, had
+  // 10.2 % of the results an ulp off, the tile of 192 rows 5.4 %. (256 rows take 370 us. Parking the sums
+  // of the first half of K in L2, 128 KB a tile, made that 460.)
+  static constexpr int kIssuers = 2;
+  static constexpr bool kHalfStages = MTMAX > 128;
   // Consecutive instructions into one accumulator wait for one another; with 32 columns that
   // latency would set the pace, so an issuer alternates between two.
   static constexpr int kAccsPerIssuer = MTMAX <= 32 ? 2 : 1;
@@ -88,17 +93,20 @@ struct Cfg {
   static constexpr int kAccBufs = MTMAX <= 64 ? 2 : 1;
   static constexpr int kAccCols = kAccBufs * kAccs * MTMAX;
   static constexpr int kOperandCol0 = kAccCols;
+  static constexpr int kDeqPerUnit = kHalfStages ? 2 : 1;            // operand stages per unit
+  static constexpr int kDeqTmemCols = kStepK / 2 / kDeqPerUnit;      // of two k each
   static constexpr int kTmemCols = 512;
   static_assert(kAccCols + kDeqStages * kDeqTmemCols <= 512, "TMEM holds 512 columns");
-  // Activations: a stage is a whole unit (both 64-k atoms), or one atom at 256 tokens, where
-  // a whole unit (64 KB) would leave room for two stages only.
-  static constexpr int kActAtoms = MTMAX <= 128 ? 2 : 1;      // atoms per stage
+  // Activations: a stage is a whole unit (both 64-k atoms), or one atom with half stages, which the
+  // commit that frees the operand stage frees too.
+  static constexpr int kActAtoms = kHalfStages ? 1 : 2;       // atoms per stage
   static constexpr int kActPerUnit = 2 / kActAtoms;           // stages per unit
   static constexpr int kActStage = MTMAX * kAtomK * 2 * kActAtoms;
   static constexpr int kActStages = MTMAX <= 32 ? 8 : (MTMAX <= 64 ? 6 : 4);
   static constexpr int kRawStages = MTMAX <= 32 ? 8 : (MTMAX <= 64 ? 7 : 5);
-  static_assert(kDeqStages % kIssuers == 0 && kActStages % (kIssuers * kActPerUnit) == 0, "see above");
-  static constexpr int kEpiWarps = MTMAX <= 128 ? 4 : 8;      // 256 tokens: two warps share a lane quarter
+  static_assert(kDeqStages % kIssuers == 0 && kActStages % kIssuers == 0, "see above");
+  static_assert(!kHalfStages || kActStages == kDeqStages, "one barrier frees a stage of either");
+  static constexpr int kEpiWarps = MTMAX <= 128 ? 4 : 8;      // 192 tokens: two warps share a lane quarter
   static constexpr int kEpiThreads = kEpiWarps * 32;
   static constexpr int kThreads = 128 + kDeqWarps * 32 + kEpiThreads;
   static constexpr int kRing = kActStages * kActStage + kRawStages * kRawStageBytes;
@@ -261,10 +269,10 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     }
     for (int s = 0; s < C::kActStages; ++s) {
       mbar_init(bar_act_full + 8 * s, 1);
-      mbar_init(bar_act_empty + 8 * s, 1);   // the issuer that owns the unit
+      mbar_init(bar_act_empty + 8 * s, 1);   // the issuer that owns the unit (half stages: not used)
     }
     for (int s = 0; s < kDeqStages; ++s) {
-      mbar_init(bar_deq_full + 8 * s, kDeqGroupWarps);
+      mbar_init(bar_deq_full + 8 * s, kDeqGroupWarps / C::kDeqPerUnit);
       mbar_init(bar_deq_empty + 8 * s, 1);
     }
     for (int b = 0; b < C::kAccBufs; ++b) {
@@ -346,7 +354,10 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 #pragma unroll
       for (int h = 0; h < C::kActPerUnit; ++h, ++ita) {
         const uint32_t sa = ita % C::kActStages, pa = (ita / C::kActStages) & 1u;
-        if (!mbar_wait(wctx, bar_act_empty + 8 * sa, pa ^ 1u, 0x180u + sa)) { ok = false; break; }
+        if (!mbar_wait(wctx, (C::kHalfStages ? bar_deq_empty : bar_act_empty) + 8 * sa, pa ^ 1u, 0x180u + sa)) {
+          ok = false;
+          break;
+        }
         const uint32_t full = bar_act_full + 8 * sa;
         mbar_arrive_expect_tx_elect(full, act_tx);
         // the map views A as [K/64][M][64]
@@ -357,9 +368,9 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         if (++mtile == p.m_tiles) mtile = 0;
       }
     }
-  } else if (warp == 1 || (warp == 3 && C::kIssuers == 2)) {
+  } else if (warp == 1 || warp == 3) {
     // ------------------------------ MMA issuers ------------------------------
-    // The issuers take the units in turn (unit it -> issuer it % kIssuers): per unit an
+    // The issuers take the units in turn (unit it -> issuer it % kIssuers; half stages: the halves): per unit an
     // issuer pays its barrier tests (~100 cycles each), eight MMAs and the commits; sharing
     // every unit between all issuers made each of them pay the fixed part for every unit. An
     // issuer owns its accumulator(s) of the segment buffer and tells the epilogue "done" after
@@ -369,50 +380,37 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     uint32_t it = 0, seg = 0;
     int step = static_cast<int>(u_begin % p.k_steps);
     uint32_t n_in_seg = 0;
-    bool ok = true;
-    for (long long u = u_begin; ok && u < u_end; ++u, ++it, step = (step + 1 == p.k_steps) ? 0 : step + 1) {
+    for (long long u = u_begin; u < u_end; ++u, ++it, step = (step + 1 == p.k_steps) ? 0 : step + 1) {
       const bool seg_first = (u == u_begin) || (step == 0);
       const bool seg_last = (u + 1 == u_end) || (step == p.k_steps - 1);
       // last unit of this segment: end of the tile or of this CTA's run
       const long long tile_last = u - step + p.k_steps - 1;
       const long long seg_last_u = tile_last < u_end - 1 ? tile_last : u_end - 1;
-      const bool mine = static_cast<int>(it % C::kIssuers) == me;
-      const bool my_last = u + C::kIssuers > seg_last_u;   // no later unit of mine in this segment
-      const uint32_t sd = it % kDeqStages, pd = (it / kDeqStages) & 1u;
+      const bool mine = C::kHalfStages || static_cast<int>(it % C::kIssuers) == me;
+      const bool my_last = u + (C::kHalfStages ? 1 : C::kIssuers) > seg_last_u;   // no later unit of mine in this segment
       const uint32_t buf = seg % C::kAccBufs, pacc = (seg / C::kAccBufs) & 1u;
       if (seg_first) n_in_seg = 0;
       if (mine) {
         if (n_in_seg == 0 && !mbar_wait(wctx, bar_acc_empty + 8 * buf, pacc ^ 1u, 0x200u + buf)) break;
         const uint32_t d_tmem = tmem_base + buf * (C::kAccs * MTMAX);
-        const uint32_t w_stage = tmem_base + C::kOperandCol0 + sd * kDeqTmemCols;
+        const uint32_t its = C::kHalfStages ? it * 2 + me : it;   // stage in order of use
+        const uint32_t sd = its % kDeqStages, pd = (its / kDeqStages) & 1u;
+        const uint32_t sa = its % C::kActStages, pa = (its / C::kActStages) & 1u;
+        if (!mbar_wait_both(wctx, bar_deq_full + 8 * sd, pd, 0x280u + sd, bar_act_full + 8 * sa, pa, 0x300u + sa)) break;
+        tc_fence_after_sync();
+        const uint32_t a_src = act_base + sa * C::kActStage;
+        const uint32_t w_stage = tmem_base + C::kOperandCol0 + sd * C::kDeqTmemCols;
 #pragma unroll
-        for (int h = 0; h < C::kActPerUnit; ++h) {
-          const uint32_t ita = it * C::kActPerUnit + h;
-          const uint32_t sa = ita % C::kActStages, pa = (ita / C::kActStages) & 1u;
-          if (h == 0) {
-            if (!mbar_wait_both(wctx, bar_deq_full + 8 * sd, pd, 0x280u + sd, bar_act_full + 8 * sa, pa, 0x300u + sa)) {
-              ok = false;
-              break;
-            }
-          } else {
-            if (!mbar_wait(wctx, bar_act_full + 8 * sa, pa, 0x300u + sa)) { ok = false; break; }
-          }
-          tc_fence_after_sync();
-          const uint32_t a_src = act_base + sa * C::kActStage;
-#pragma unroll
-          for (int k4 = 0; k4 < 4 * C::kActAtoms; ++k4) {
-            // tokens: K-major, 64-k atoms of mt rows, 32 B per instruction inside an atom;
-            // weights: 16 k = 8 columns of the operand stage in tensor memory
-            const int kk = h * 4 + k4;
-            const uint64_t a_desc = umma_smem_desc_sw128(a_src + (k4 >> 2) * (p.mt * 128) + (k4 & 3) * 32, 16, 1024);
-            const uint32_t d_acc = d_tmem + (me * C::kAccsPerIssuer + (kk % C::kAccsPerIssuer)) * MTMAX;
-            umma_f16_tmem_a_elect(d_acc, w_stage + kk * 8, a_desc, p.idesc,
-                                  (n_in_seg == 0 && kk < C::kAccsPerIssuer) ? 0u : 1u);
-          }
-          if (h == C::kActPerUnit - 1) tc_commit_elect(bar_deq_empty + 8 * sd);
-          tc_commit_elect(bar_act_empty + 8 * sa);
+        for (int kk = 0; kk < 4 * C::kActAtoms; ++kk) {
+          // tokens: K-major, 64-k atoms of mt rows, 32 B per instruction inside an atom;
+          // weights: 16 k = 8 columns of the operand stage in tensor memory
+          const uint64_t a_desc = umma_smem_desc_sw128(a_src + (kk >> 2) * (p.mt * 128) + (kk & 3) * 32, 16, 1024);
+          const uint32_t d_acc = d_tmem + (me * C::kAccsPerIssuer + (kk % C::kAccsPerIssuer)) * MTMAX;
+          umma_f16_tmem_a_elect(d_acc, w_stage + kk * 8, a_desc, p.idesc,
+                                (n_in_seg == 0 && kk < C::kAccsPerIssuer) ? 0u : 1u);
         }
-        if (!ok) break;
+        tc_commit_elect(bar_deq_empty + 8 * sd);
+        if constexpr (!C::kHalfStages) tc_commit_elect(bar_act_empty + 8 * sa);
         ++n_in_seg;
         if (my_last) tc_commit_elect(bar_acc_full + 8 * buf);   // my last unit of the segment
       } else if (seg_last && n_in_seg == 0) {
@@ -508,7 +506,8 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     const uint32_t lane_off =
         static_cast<uint32_t>(half * kRawBytes + khalf * (32 * 128) + ((lane >> 4) * 8 + (lane & 7)) * 128 +
                               (((quarter * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
-    const uint32_t lane_dst = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::kOperandCol0 + khalf * 32;
+    const uint32_t lane_dst = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::kOperandCol0 +
+                              (C::kHalfStages ? 0 : khalf * 32);
     uint32_t sr = 0, pr = 0;
     for (int b = 0; b < n_boxes; ++b, it += kGroups, sr = sr + 1 == C::kRawStages ? (pr ^= 1u, 0u) : sr + 1) {
       if (it < 0 || it >= n_units) {
@@ -517,7 +516,8 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         if (lane == 0) mbar_arrive(bar_raw_empty + 8 * sr);
         continue;
       }
-      const uint32_t sd = it & (kDeqStages - 1), pd = (static_cast<uint32_t>(it) / kDeqStages) & 1u;
+      const uint32_t its = C::kHalfStages ? it * 2 + khalf : it;
+      const uint32_t sd = its & (kDeqStages - 1), pd = (its / kDeqStages) & 1u;
       static_assert((kDeqStages & (kDeqStages - 1)) == 0, "a power of two");
       // constants of the unit: columns 2g, 2g + 1 of the first block of 16, then of the second
       V2 sd2[kSz][2], zd2[kSz][2];     // scale * kDown, -zero / kDown
@@ -542,7 +542,12 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         fetch_advance();
         fetch();
       }
-      if (!mbar_wait_both(wctx, bar_raw_full + 8 * sr, pr, 0x400u + sr, bar_deq_empty + 8 * sd, pd ^ 1u, 0x480u + sd)) break;
+      if constexpr (C::kHalfStages) {   // (the stage is waited for where the first store needs it)
+        if (!mbar_wait(wctx, bar_raw_full + 8 * sr, pr, 0x400u + sr)) break;
+      } else {
+        if (!mbar_wait_both(wctx, bar_raw_full + 8 * sr, pr, 0x400u + sr, bar_deq_empty + 8 * sd, pd ^ 1u, 0x480u + sd)) break;
+      }
+      bool ok = true;
       const uint32_t src = rawst_base + sr * kRawStageBytes + lane_off;
       uint32_t w[2][4];                // [32-k part][8-row block, block of 16 columns]
       ldmatrix_x4_trans(src, w[0]);
@@ -586,8 +591,10 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             }
           }
         }
-        tmem_st_16x256b(lane_dst + sd * kDeqTmemCols + (static_cast<uint32_t>(16 * cb) << 16), cells);
+        if (C::kHalfStages && cb == 0) ok = mbar_wait(wctx, bar_deq_empty + 8 * sd, pd ^ 1u, 0x480u + sd);
+        if (ok) tmem_st_16x256b(lane_dst + sd * C::kDeqTmemCols + (static_cast<uint32_t>(16 * cb) << 16), cells);
       }
+      if (!ok) break;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_raw_empty + 8 * sr);   // every byte of the packed stage has been read
       tmem_wait_st();
@@ -619,15 +626,15 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       const long long tile_end = tile_begin + p.k_steps;
       const long long seg_end = tile_end < u_end ? tile_end : u_end;
       const bool whole = (u == tile_begin) && (seg_end == tile_end);
-      // the MMA issuers take alternate units of the CTA's run; in a one-unit segment only one
-      // of them has written its accumulators
+      // the MMA issuers take alternate units of the CTA's run (or a half of every unit); in a one-unit
+      // segment only one of them has written its accumulators
       bool issuer_has_units[C::kIssuers];
 #pragma unroll
       for (int i = 0; i < C::kIssuers; ++i) {
         // units of the segment are it0 .. it0 + len - 1; issuer i owns those with it % kIssuers == i
         const long long it0 = u - u_begin, len = seg_end - u;
         const long long first = it0 + ((i - it0 % C::kIssuers) + C::kIssuers) % C::kIssuers;
-        issuer_has_units[i] = first < it0 + len;
+        issuer_has_units[i] = C::kHalfStages || first < it0 + len;
       }
       const uint32_t buf = seg % C::kAccBufs, pacc = (seg / C::kAccBufs) & 1u;
       ++seg;
@@ -811,7 +818,7 @@ ks_status_t launch_mt(int mtmax, const CUtensorMap& tm_w, const CUtensorMap& tm_
     case 32: return launch_t<T, 32, FINE>(tm_w, tm_a, p, grid, stream);
     case 64: return launch_t<T, 64, FINE>(tm_w, tm_a, p, grid, stream);
     case 128: return launch_t<T, 128, FINE>(tm_w, tm_a, p, grid, stream);
-    default: return launch_t<T, 256, FINE>(tm_w, tm_a, p, grid, stream);
+    default: return launch_t<T, 192, FINE>(tm_w, tm_a, p, grid, stream);
   }
 }
 
@@ -851,7 +858,7 @@ double unit_ns(int mt, bool fine) {
 //   whole      runs of whole tiles: the last round may leave SMs idle
 //   even runs  no SM idles, but a tile's last CTA reads the other parts from L2: ~2.5 us for the
 //              hand-over and ~0.25 us per part and 16 token rows (two warps share that work in
-//              256-row tiles). K = N = 4096, 16 rows: 12.5 us against 10.5 with clusters
+//              192-row tiles). K = N = 4096, 16 rows: 12.5 us against 10.5 with clusters
 // Fewer token tiles mean fewer dequantisations of a weight; more of them, more tiles to deal out.
 Geometry geometry_of(const W4A16Args& a) {
   Geometry g;
@@ -870,7 +877,7 @@ Geometry geometry_of(const W4A16Args& a) {
     g.cluster_s = cluster_s;
     g.split = split;
   };
-  const int lo = static_cast<int>((a.m + 255) / 256), hi = static_cast<int>((a.m + 31) / 32);
+  const int lo = static_cast<int>((a.m + 191) / 192), hi = static_cast<int>((a.m + 31) / 32);
   for (int want = lo; want <= hi && want < lo + 24; ++want) {
     const int mt = static_cast<int>(((a.m + want - 1) / want + 15) & ~int64_t(15));
     const int m_tiles = static_cast<int>((a.m + mt - 1) / mt);
@@ -887,7 +894,7 @@ Geometry geometry_of(const W4A16Args& a) {
     const int chunks = mt <= 128 ? mt / 16 : (mt + 31) / 32;
     offer(per_cta * unit + 2 * drain + 2500.0 + 250.0 * chunks * parts, mt, m_tiles, 1, true);
   }
-  g.mtmax = g.mt <= 32 ? 32 : (g.mt <= 64 ? 64 : (g.mt <= 128 ? 128 : 256));
+  g.mtmax = g.mt <= 32 ? 32 : (g.mt <= 64 ? 64 : (g.mt <= 128 ? 128 : 192));
   const long long tiles = static_cast<long long>(g.n_tiles) * g.m_tiles;
   const long long work = g.split ? tiles * g.k_steps : tiles;
   g.grid = g.cluster_s > 1 ? static_cast<int>(tiles * g.cluster_s) : static_cast<int>(work < sms ? work : sms);

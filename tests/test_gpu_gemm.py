@@ -719,3 +719,22 @@ def test_grouped_tiles_in_column_panels(ks, cuda):
             ref = a[lo:hi].double() @ w[e].double()
             # bf16 outputs: half an ulp each, 2^-9 relative
             assert orc.rel_frobenius(out[lo:hi], ref.float()) < 2.0 ** -8
+
+
+def test_w4a16_sums_of_wide_token_tiles(ks, cuda):
+    """tcgen05.mma truncates what it adds up, so a sum's error grows with its number of instructions. Token tiles
+    above 128 rows must sum K in two accumulators like narrower ones: with K=14336 and positive operands
+    5-6 % of the f16 results are an ulp off then (448 instructions a sum), 10-13 % with one accumulator."""
+    m, k, n = 2048, 14336, 2048
+    g = torch.Generator(device=cuda).manual_seed(5)
+    x = torch.randn(m, k, generator=g, device=cuda).abs().to(torch.float16)
+    codes = torch.randint(0, 256, (k // 2, n), generator=g, device=cuda, dtype=torch.uint8)
+    scales = (torch.randn(k // 128, n, generator=g, device=cuda).mul(0.02).abs() + 1e-3).div(16).to(torch.float16)
+    zeros = torch.zeros_like(scales)
+    out = ks.dispatch.w4a16(x, codes, scales, zeros, group_size=128)
+    q = torch.stack([codes & 15, codes >> 4], 1).reshape(k // 128, 128, n)
+    w = (q.float() * scales.float()[:, None]).view(k, n).to(torch.float16)
+    rows = slice(0, m, 8)
+    exact = x[rows].double() @ w.double()
+    assert float((out[rows] != exact.to(torch.float16)).double().mean()) < 0.08
+    assert float(((out[rows].double() - exact) / exact).mean().abs()) < 5.5e-5   # measured 3.7e-5; 7-9e-5 with one

@@ -23,8 +23,9 @@ class Bar:
     def done(s, parity): return (s.phase & 1) != parity
 def run_start(units, ctas, c): return (units*c)//ctas
 def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1):
-    # AB: accumulator (segment) buffers; AP: activation stages per unit
-    raw_full=[Bar(1) for _ in range(RS)]; raw_empty=[Bar(2) for _ in range(RS)]
+    # AB: accumulator (segment) buffers; AP: stages per unit. AP == 2 (token tiles of 192 rows): operand and
+    # activation stages of half a unit, each half with an issuer and half a group of its own, freed together
+    raw_full=[Bar(1) for _ in range(RS)]; raw_empty=[Bar(2*AP) for _ in range(RS)]
     act_full=[Bar(1) for _ in range(AS)]; act_empty=[Bar(1) for _ in range(AS)]
     deq_full=[Bar(1) for _ in range(DS)]; deq_empty=[Bar(1) for _ in range(DS)]
     acc_full=[Bar(K) for _ in range(AB)]; acc_empty=[Bar(1) for _ in range(AB)]
@@ -41,7 +42,7 @@ def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1)
         for u in range(ub,ue):
             for _ in range(AP):
                 sa=it%AS; pa=(it//AS)&1
-                yield ('wait', act_empty[sa], pa^1, it//AS, 'aprod act_empty')
+                yield ('wait', (deq_empty if AP==2 else act_empty)[sa], pa^1, it//AS, 'aprod act_empty')
                 act_full[sa].arrive()
                 it+=1
     def issuer(i):
@@ -51,19 +52,18 @@ def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1)
             seg_last=(u+1==ue) or step==k_steps-1
             tile_last=u-step+k_steps-1
             seg_last_u=min(tile_last,ue-1)
-            mine=(it%K)==i
-            my_last=u+K>seg_last_u
-            sd=it%DS; pd=(it//DS)&1
+            mine=AP==2 or (it%K)==i
+            my_last=u+(1 if AP==2 else K)>seg_last_u
+            its=2*it+i if AP==2 else it
+            sd=its%DS; pd=(its//DS)&1; sa=its%AS; pa=(its//AS)&1
             buf=seg%AB; pacc=(seg//AB)&1
             if seg_first: n_in_seg=0
             if mine:
                 if n_in_seg==0: yield ('wait', acc_empty[buf], pacc^1, seg//AB, f'issuer{i} acc_empty u={u}')
-                yield ('wait', deq_full[sd], pd, it//DS+1, f'issuer{i} deq_full u={u}')
-                for h in range(AP):
-                    ita=it*AP+h; sa=ita%AS; pa=(ita//AS)&1
-                    yield ('wait', act_full[sa], pa, ita//AS+1, f'issuer{i} act_full u={u}')
-                    if h==AP-1: deq_empty[sd].arrive()
-                    act_empty[sa].arrive()
+                yield ('wait', deq_full[sd], pd, its//DS+1, f'issuer{i} deq_full u={u}')
+                yield ('wait', act_full[sa], pa, its//AS+1, f'issuer{i} act_full u={u}')
+                deq_empty[sd].arrive()
+                if AP==1: act_empty[sa].arrive()
                 n_in_seg+=1
                 if my_last: acc_full[buf].arrive()
             elif seg_last and n_in_seg==0:
@@ -71,7 +71,7 @@ def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1)
                 acc_full[buf].arrive()
             if seg_last: seg+=1
             it+=1; step=0 if step+1==k_steps else step+1
-    def group(g):
+    def group(g, khalf=0):
         stride=G//2; half=g&1
         b=b_begin
         while (b%stride)!=(g>>1): b+=1
@@ -80,9 +80,9 @@ def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1)
             u=2*b+half
             if u<ub or u>=ue:
                 raw_empty[sr].arrive(); b+=stride; continue
-            it=u-ub; sd=it%DS; pd=(it//DS)&1
+            it=u-ub; its=AP*it+khalf; sd=its%DS; pd=(its//DS)&1
             yield ('wait', raw_full[sr], pr, itb//RS+1, f'group{g} raw_full u={u}')
-            yield ('wait', deq_empty[sd], pd^1, it//DS, f'group{g} deq_empty u={u}')
+            yield ('wait', deq_empty[sd], pd^1, its//DS, f'group{g} deq_empty u={u}')
             raw_empty[sr].arrive()
             deq_full[sd].arrive()
             b+=stride
@@ -98,7 +98,8 @@ def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1)
             acc_empty[buf].arrive()
     procs={'wprod':wprod(),'aprod':aprod(),'epi':epilogue()}
     for i in range(K): procs[f'iss{i}']=issuer(i)
-    for g in range(G): procs[f'grp{g}']=group(g)
+    for g in range(G):
+        for h in range(AP): procs[f'grp{g}.{h}']=group(g, h)
     blocked={}
     alive=list(procs)
     if order is not None:
@@ -199,7 +200,7 @@ def test_three_issuers_are_detected_as_broken():
     dict(K=2, G=2, RS=8, AS=8, AB=2),          # token tiles of up to 32 rows
     dict(K=2, G=2, RS=7, AS=6, AB=2),          # 64
     dict(K=2, G=2, RS=5, AS=4, AB=1),          # 128
-    dict(K=1, G=2, RS=5, AS=4, AB=1, AP=2),    # 256: one issuer, two activation stages per unit
+    dict(K=2, G=2, RS=5, AS=4, AB=1, AP=2),    # 192: stages of half a unit
 ])
 def test_protocol_of_every_token_tile(n_tiles, k_steps, config):
     assert deadlocked_ctas(n_tiles, k_steps, **config) == []
