@@ -53,14 +53,7 @@ constexpr int kTileN = 128;    // weight columns per tile = UMMA M
 constexpr int kStepK = 128;    // k per pipeline step ("unit" = 128 columns x 128 k)
 constexpr int kRawBytes = (kStepK / 2) * kTileN;      // 8192
 constexpr int kRawStageBytes = 2 * kRawBytes;         // one TMA box: two K-steps
-// Dequantisation: two groups of eight warps on alternate units; a warp takes one TMEM lane quarter
-// (32 columns) and one 64-k half of its group's unit. With four operand stages each group then has
-// two of its own, and fills one while the MMAs read the other. (Four groups of four warps
-// are each tied to one stage: a group's next unit waits for the MMAs of its last, and the two
-// times add up.)
-constexpr int kGroups = 2;
-constexpr int kDeqGroupWarps = 8;
-constexpr int kDeqWarps = kGroups * kDeqGroupWarps;
+constexpr int kDeqWarps = 16;      // dequantising warps, in two or four groups (see Cfg)
 constexpr int kDeqStages = 4;      // operand stages in tensor memory
 constexpr int kAtomK = 64;         // k per 128-byte swizzle atom of the activations
 
@@ -70,8 +63,19 @@ constexpr int kAtomK = 64;         // k per 128-byte swizzle atom of the activat
 // issuer consumed that use. (Three issuers with four stages let an issuer pass a fresh barrier
 // one phase early: intermittent bounded-wait timeouts on the GPU, and a deadlock in the
 // protocol model under tests/.)
-template <int MTMAX>
+template <int MTMAX, bool FINE>
 struct Cfg {
+  // Dequantisation: a warp takes one TMEM lane quarter (32 columns) of its group's unit. Above 32
+  // tokens two groups of eight warps take alternate units, a warp one 64-k half: with four
+  // operand stages a group has two of its own and fills one while the MMAs read the other. (Four groups of
+  // four are each tied to one stage: a group's next unit waits for the MMAs of its last, and the
+  // two times add up.) Up to 32 tokens the MMAs are short, and what counts is the work per warp and
+  // unit outside the cells (waits, scales, their tests: ~100 of 230 instructions): four groups, a warp
+  // takes both halves. K=14336 N=28672 M=24: 92.9 us with two groups, 78.7 with four; K=14336 N=4096 M=1 19.8
+  // and 17.6. Scale groups of 32 and 64 (FINE) need two constants per half, gain 1-2 % or lose it, and stay.
+  static constexpr int kGroups = MTMAX <= 32 && !FINE ? 4 : 2;
+  static constexpr int kDeqGroupWarps = kDeqWarps / kGroups;
+  static constexpr int kKHalves = kGroups / 2;   // 64-k halves of a unit that a warp takes
   // Issuing a tcgen05.mma costs its thread ~55 cycles: up to 64 token columns the tensor core needs
   // less than that, at 128 about as much. Two issuers, with accumulators of their own, take alternate
   // units, or above 128 rows the two 64-k halves of every unit (kHalfStages): the operand ring's 128
@@ -231,10 +235,10 @@ __device__ __forceinline__ void store_tokens16(T* c, int ld, const float (&v)[16
 
 // FINE: scale groups of 32 or 64 k (several per K-step); otherwise multiples of 128.
 template <typename T, int MTMAX, bool FINE>
-__global__ void __launch_bounds__((Cfg<MTMAX>::kThreads), 1)
+__global__ void __launch_bounds__((Cfg<MTMAX, FINE>::kThreads), 1)
 w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a,
                   const Params p) {
-  using C = Cfg<MTMAX>;
+  using C = Cfg<MTMAX, FINE>;
   using P16 = Pack16<T>;
   using V2 = typename P16::V2;
   extern __shared__ uint8_t smem_raw[];
@@ -265,14 +269,14 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kRawStages; ++s) {
       mbar_init(bar_raw_full + 8 * s, 1);
-      mbar_init(bar_raw_empty + 8 * s, 2 * kDeqGroupWarps);   // both halves of a box
+      mbar_init(bar_raw_empty + 8 * s, 2 * C::kDeqGroupWarps);   // both halves of a box
     }
     for (int s = 0; s < C::kActStages; ++s) {
       mbar_init(bar_act_full + 8 * s, 1);
       mbar_init(bar_act_empty + 8 * s, 1);   // the issuer that owns the unit (half stages: not used)
     }
     for (int s = 0; s < kDeqStages; ++s) {
-      mbar_init(bar_deq_full + 8 * s, kDeqGroupWarps / C::kDeqPerUnit);
+      mbar_init(bar_deq_full + 8 * s, C::kDeqGroupWarps / C::kDeqPerUnit);
       mbar_init(bar_deq_empty + 8 * s, 1);
     }
     for (int b = 0; b < C::kAccBufs; ++b) {
@@ -441,22 +445,26 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     // everything outside the cells counts: 32-bit counters relative to the CTA's run, ring
     // positions that advance instead of divisions, addresses of the scale rows that advance, and
     // zero-points tested two columns at a time.
-    const int half = (warp - 4) >> 3;           // group = K-step half of every box = parity of its units
-    const int khalf = ((warp - 4) >> 2) & 1;    // 64-k half of the unit
+    constexpr int kGroups = C::kGroups, kBoxStep = kGroups / 2;
+    const int group = (warp - 4) / C::kDeqGroupWarps;
+    const int half = group & 1;                 // K-step half of the group's boxes = parity of its units
+    const int box0 = group >> 1;                // first box: of four groups, two take every other box
+    const int khalf = C::kKHalves == 2 ? 0 : ((warp - 4) >> 2) & 1;   // (first) 64-k half of the unit
     static_assert(P16::kUnit * P16::kUp * P16::kDown == 1.0f, "the three factors cancel");
     const V2 up2 = P16::splat(P16::kUp), down2 = P16::splat(P16::kDown), neg_inv_down2 = P16::splat(-1.0f / P16::kDown);
     const V2 max_zero2 = P16::splat(P16::kMaxZero), zero2 = P16::from_bits(0u);
     const V2 max_scale2 = P16::splat(P16::kUp);
     const V2 whole2 = P16::splat(P16::kMaxZero + 1.0f);   // adding it rounds to whole numbers
     const int quarter = warp & 3;
-    constexpr int kSz = FINE ? 2 : 1;           // scale rows of this warp's 64 k: one per 32 k, or one
+    constexpr int kSz = FINE ? 2 : 1;           // scale rows of this warp's k: one per 32 k (FINE: 64 k), or one
+    static_assert(!FINE || C::kKHalves == 1, "see above");
     const int col0 = quarter * 32 + 2 * (lane >> 2);   // this lane's columns: col0, col0 + 1, col0 + 16, col0 + 17
     const int n_units = static_cast<int>(u_end - u_begin);
     const int odd0 = static_cast<int>(u_begin & 1);
     const int n_boxes = (n_units + odd0 + 1) >> 1;
     // Scales and zero-points come straight from global memory, fetched one unit of the group
     // ahead (k_steps and kGroups are even, so the parity of step is fixed).
-    int it = half - odd0;                       // unit of box 0, relative to the run; -1: a neighbour's
+    int it = 2 * box0 + half - odd0;            // unit of the first box, relative to the run; -1: a neighbour's
     const long long u_first = u_begin + (it < 0 ? it + kGroups : it);
     const long long f_t0 = u_first / p.k_steps;
     int f_step = static_cast<int>(u_first - f_t0 * p.k_steps);
@@ -487,8 +495,10 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     auto fetch_advance = [&]() {
       f_step += kGroups;
       if (f_step >= p.k_steps) {
-        f_step -= p.k_steps;
-        if (++f_mtile == p.m_tiles) { f_mtile = 0; ++f_ntile; }
+        do {   // (a tile may have fewer K-steps than there are groups)
+          f_step -= p.k_steps;
+          if (++f_mtile == p.m_tiles) { f_mtile = 0; ++f_ntile; }
+        } while (f_step >= p.k_steps);
         if constexpr (!FINE) {
           f_row = 0;
           f_in_row = f_step;
@@ -508,8 +518,12 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                               (((quarter * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
     const uint32_t lane_dst = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + C::kOperandCol0 +
                               (C::kHalfStages ? 0 : khalf * 32);
-    uint32_t sr = 0, pr = 0;
-    for (int b = 0; b < n_boxes; ++b, it += kGroups, sr = sr + 1 == C::kRawStages ? (pr ^= 1u, 0u) : sr + 1) {
+    static_assert(C::kRawStages % kBoxStep == 0, "a group keeps to its raw stages");
+    uint32_t stage = box0, phase = 0;
+    for (int b = box0; b < n_boxes; b += kBoxStep, it += kGroups) {
+      const uint32_t sr = stage, pr = phase;
+      stage += kBoxStep;
+      if (stage >= C::kRawStages) { stage -= C::kRawStages; phase ^= 1u; }
       if (it < 0 || it >= n_units) {
         // this half of the box belongs to a neighbouring CTA's run
         __syncwarp();
@@ -549,50 +563,53 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       }
       bool ok = true;
       const uint32_t src = rawst_base + sr * kRawStageBytes + lane_off;
-      uint32_t w[2][4];                // [32-k part][8-row block, block of 16 columns]
-      ldmatrix_x4_trans(src, w[0]);
-      ldmatrix_x4_trans(src + 16 * 128, w[1]);
 #pragma unroll
-      for (int cb = 0; cb < 2; ++cb) {
-        uint32_t cells[16];            // 64 k = 32 operand columns of this block's 16 weight columns
-        if (simple) {
-          const int r1 = FINE ? 1 : 0;
-          const V2 s_lo[2] = {P16::low(sd2[0][cb]), P16::low(sd2[r1][cb])}, s_hi[2] = {P16::high(sd2[0][cb]), P16::high(sd2[r1][cb])};
-          const V2 z_lo[2] = {P16::low(zd2[0][cb]), P16::low(zd2[r1][cb])}, z_hi[2] = {P16::high(zd2[0][cb]), P16::high(zd2[r1][cb])};
+      for (int kh = 0; kh < C::kKHalves; ++kh) {
+        uint32_t w[2][4];                // [32-k part][8-row block, block of 16 columns]
+        ldmatrix_x4_trans(src + kh * (32 * 128), w[0]);
+        ldmatrix_x4_trans(src + kh * (32 * 128) + 16 * 128, w[1]);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint32_t w0 = w[q >> 1][2 * (q & 1) + cb];
-            const uint32_t lo4 = w0 & 0x0F0F0F0Fu, hi4 = (w0 >> 4) & 0x0F0F0F0Fu;
+        for (int cb = 0; cb < 2; ++cb) {
+          uint32_t cells[16];            // 64 k = 32 operand columns of this block's 16 weight columns
+          if (simple) {
+            const int r1 = FINE ? 1 : 0;
+            const V2 s_lo[2] = {P16::low(sd2[0][cb]), P16::low(sd2[r1][cb])}, s_hi[2] = {P16::high(sd2[0][cb]), P16::high(sd2[r1][cb])};
+            const V2 z_lo[2] = {P16::low(zd2[0][cb]), P16::low(zd2[r1][cb])}, z_hi[2] = {P16::high(zd2[0][cb]), P16::high(zd2[r1][cb])};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              // byte i: column 2g + (i & 1), row 2s + (i >> 1); selector 8 + j replicates the sign of
-              // byte j, which is zero
-              const uint32_t sel = i | ((8 + i) << 4) | ((4 + i) << 8) | ((12 + i) << 12);
-              const V2 x = P16::from_bits(byte_perm_sign(lo4, hi4, sel));
-              const V2 z = (i & 1) ? z_hi[q >> 1] : z_lo[q >> 1], sx = (i & 1) ? s_hi[q >> 1] : s_lo[q >> 1];
-              cells[4 * q + 2 * (i & 1) + (i >> 1)] = P16::bits(__hmul2(__hfma2(x, up2, z), sx));
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t w0 = w[q >> 1][2 * (q & 1) + cb];
+              const uint32_t lo4 = w0 & 0x0F0F0F0Fu, hi4 = (w0 >> 4) & 0x0F0F0F0Fu;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                // byte i: column 2g + (i & 1), row 2s + (i >> 1); selector 8 + j replicates the sign of
+                // byte j, which is zero
+                const uint32_t sel = i | ((8 + i) << 4) | ((4 + i) << 8) | ((12 + i) << 12);
+                const V2 x = P16::from_bits(byte_perm_sign(lo4, hi4, sel));
+                const V2 z = (i & 1) ? z_hi[q >> 1] : z_lo[q >> 1], sx = (i & 1) ? s_hi[q >> 1] : s_lo[q >> 1];
+                cells[4 * q + 2 * (i & 1) + (i >> 1)] = P16::bits(__hmul2(__hfma2(x, up2, z), sx));
+              }
+            }
+          } else {
+            // zero-points that are not small integers: the fp32 statement, verbatim
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t w0 = w[q >> 1][2 * (q & 1) + cb];
+              const int r = FINE ? q >> 1 : 0;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const uint32_t b8 = (w0 >> (8 * i)) & 0xFFu;
+                const V2 sv = P16::from_bits(s_cur[r][cb]), zv = P16::from_bits(z_cur[r][cb]);
+                const float z0 = (i & 1) ? P16::hi(zv) : P16::lo(zv);
+                const float s0 = (i & 1) ? P16::hi(sv) : P16::lo(sv);
+                cells[4 * q + 2 * (i & 1) + (i >> 1)] =
+                    P16::bits(P16::make(__fmul_rn(__fsub_rn(static_cast<float>(b8 & 15u), z0), s0),
+                                        __fmul_rn(__fsub_rn(static_cast<float>(b8 >> 4), z0), s0)));
+              }
             }
           }
-        } else {
-          // zero-points that are not small integers: the fp32 statement, verbatim
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint32_t w0 = w[q >> 1][2 * (q & 1) + cb];
-            const int r = FINE ? q >> 1 : 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const uint32_t b8 = (w0 >> (8 * i)) & 0xFFu;
-              const V2 sv = P16::from_bits(s_cur[r][cb]), zv = P16::from_bits(z_cur[r][cb]);
-              const float z0 = (i & 1) ? P16::hi(zv) : P16::lo(zv);
-              const float s0 = (i & 1) ? P16::hi(sv) : P16::lo(sv);
-              cells[4 * q + 2 * (i & 1) + (i >> 1)] =
-                  P16::bits(P16::make(__fmul_rn(__fsub_rn(static_cast<float>(b8 & 15u), z0), s0),
-                                      __fmul_rn(__fsub_rn(static_cast<float>(b8 >> 4), z0), s0)));
-            }
-          }
+          if (C::kHalfStages && cb == 0) ok = mbar_wait(wctx, bar_deq_empty + 8 * sd, pd ^ 1u, 0x480u + sd);
+          if (ok) tmem_st_16x256b(lane_dst + kh * 32 + sd * C::kDeqTmemCols + (static_cast<uint32_t>(16 * cb) << 16), cells);
         }
-        if (C::kHalfStages && cb == 0) ok = mbar_wait(wctx, bar_deq_empty + 8 * sd, pd ^ 1u, 0x480u + sd);
-        if (ok) tmem_st_16x256b(lane_dst + sd * C::kDeqTmemCols + (static_cast<uint32_t>(16 * cb) << 16), cells);
       }
       if (!ok) break;
       __syncwarp();
@@ -792,7 +809,7 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 template <typename T, int MTMAX, bool FINE>
 ks_status_t launch_t(const CUtensorMap& tm_w, const CUtensorMap& tm_a, const Params& p, int grid,
                      cudaStream_t stream) {
-  using C = Cfg<MTMAX>;
+  using C = Cfg<MTMAX, FINE>;
   auto kernel = w4a16_umma_kernel<T, MTMAX, FINE>;
   static std::mutex mu;
   static bool attr_done[64] = {};

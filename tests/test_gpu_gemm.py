@@ -738,3 +738,29 @@ def test_w4a16_sums_of_wide_token_tiles(ks, cuda):
     exact = x[rows].double() @ w.double()
     assert float((out[rows] != exact.to(torch.float16)).double().mean()) < 0.08
     assert float(((out[rows].double() - exact) / exact).mean().abs()) < 5.5e-5   # measured 3.7e-5; 7-9e-5 with one
+
+
+@pytest.mark.parametrize("m,k,n,gs", [
+    (24, 128, 28688, 128),    # two K-steps (one padded) a tile: a group's next unit is two tiles on
+    (32, 256, 28688, 256),
+    (17, 384, 28688, 128),
+    (8, 1408, 9232, 128),     # runs that begin in the middle of a box and of a tile
+    (1, 1152, 2064, 384),     # three K-steps per scale row, four units between a group's fetches
+])
+def test_w4a16_narrow_tiles_four_groups(ks, cuda, m, k, n, gs):
+    """Token tiles of up to 32 rows: four dequantising groups, of which two take every other box."""
+    g = gen(m + k + n)
+    a = torch.randn(m, k, generator=g).to(torch.float16)
+    b_packed = torch.randint(0, 256, (k // 2, n), generator=g, dtype=torch.uint8)
+    scales = (torch.randn(k // gs, n, generator=g).mul(0.02).abs() + 1e-3).to(torch.float16)
+    zeros = torch.randint(0, 16, (k // gs, n), generator=g).to(torch.float16)
+    ref32 = orc.w4a16(a, b_packed, scales, zeros, gs, None, out_dtype=None)
+    noise = accumulation_noise(a.float().abs(), orc.w4a16_weight(b_packed, scales, zeros, gs).float().abs(), k)
+    dev = [t.to(cuda) for t in (a, b_packed, scales, zeros)]
+    with w4_path("tcgen05"):
+        out = ks.dispatch.w4a16(*dev, group_size=gs)
+        again = ks.dispatch.w4a16(*dev, group_size=gs)
+        torch.cuda.synchronize()
+        ks.runtime.stream_synchronize(0)
+    check_gemm(out.cpu(), ref32, noise, f"w4a16 {m}x{n}x{k} group {gs}")
+    assert torch.equal(out, again), "not reproducible run to run"

@@ -22,9 +22,10 @@ class Bar:
         if s.pending==0: s.phase+=1; s.pending=s.count
     def done(s, parity): return (s.phase & 1) != parity
 def run_start(units, ctas, c): return (units*c)//ctas
-def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1):
+def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1, REL=False):
     # AB: accumulator (segment) buffers; AP: stages per unit. AP == 2 (token tiles of 192 rows): operand and
-    # activation stages of half a unit, each half with an issuer and half a group of its own, freed together
+    # activation stages of half a unit, each half with an issuer and half a group of its own, freed together.
+    # REL: of four groups, two begin with the first box of the run (else: with even box numbers)
     raw_full=[Bar(1) for _ in range(RS)]; raw_empty=[Bar(2*AP) for _ in range(RS)]
     act_full=[Bar(1) for _ in range(AS)]; act_empty=[Bar(1) for _ in range(AS)]
     deq_full=[Bar(1) for _ in range(DS)]; deq_empty=[Bar(1) for _ in range(DS)]
@@ -74,7 +75,7 @@ def sim_cta(ub, ue, k_steps, K=2, G=4, RS=8, AS=8, DS=4, order=None, AB=2, AP=1)
     def group(g, khalf=0):
         stride=G//2; half=g&1
         b=b_begin
-        while (b%stride)!=(g>>1): b+=1
+        while ((b-b_begin if REL else b)%stride)!=(g>>1): b+=1
         while b<b_end:
             itb=b-b_begin; sr=itb%RS; pr=(itb//RS)&1
             u=2*b+half
@@ -197,7 +198,8 @@ def test_three_issuers_are_detected_as_broken():
 
 @pytest.mark.parametrize("n_tiles,k_steps", [(224, 32), (32, 112), (28, 32), (2, 8), (5, 2), (1, 2), (3, 6), (37, 4)])
 @pytest.mark.parametrize("config", [
-    dict(K=2, G=2, RS=8, AS=8, AB=2),          # token tiles of up to 32 rows
+    dict(K=2, G=4, RS=8, AS=8, AB=2, REL=True),          # token tiles of up to 32 rows
+    dict(K=2, G=2, RS=8, AS=8, AB=2),          # ... scale groups of 32 and 64
     dict(K=2, G=2, RS=7, AS=6, AB=2),          # 64
     dict(K=2, G=2, RS=5, AS=4, AB=1),          # 128
     dict(K=2, G=2, RS=5, AS=4, AB=1, AP=2),    # 192: stages of half a unit
