@@ -760,8 +760,10 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     const int part = static_cast<int>(blockIdx.x) % p.cluster_s;
     const int tile = static_cast<int>(blockIdx.x) / p.cluster_s;
     const int ntile = tile / p.m_tiles, m0 = (tile - ntile * p.m_tiles) * p.mt;
+    // Block by block from CTA to CTA. (A CTA's warps first left all reading to the first CTA or two:
+    // K=2048 N=1024 M=128 with eight parts 14.6 us, now 10.6.)
     constexpr int kWarps = C::kThreads / 32;
-    for (int i = part * kWarps + warp; i < p.mt / 4; i += p.cluster_s * kWarps) {
+    for (int i = warp * p.cluster_s + part; i < p.mt / 4; i += p.cluster_s * kWarps) {
       const int cc = (i >> 2) * 16, quarter = i & 3;
       if (m0 + cc >= p.m) continue;
       const int n_local = quarter * 32 + column_of_lane(lane), n = ntile * kTileN + n_local;
@@ -861,21 +863,20 @@ struct Geometry {
   size_t counter_bytes = 0, slot_bytes = 0;
 };
 
-// Time of one unit (128 columns x 128 k) of a token tile of `mt` rows in a long run, in ns:
-// measured as the slope of time against K (2048 to 8192) with one whole tile per CTA, group 128:
-// 420 at 16 rows, 480 at 64, 490 at 128, 710 at 192, 830 at 256; groups of 32 about a fifth more.
-double unit_ns(int mt, bool fine) {
-  const double t = mt <= 128 ? 420.0 + mt * 0.55 : 490.0 + (mt - 128) * 2.7;
-  return fine ? t * 1.2 : t;
-}
+// Estimated times, in ns, fitted to 1091 shapes (N 1024..28672, K 1024..14336, 1 to 2048 rows, scale groups of
+// 128, 64 and 32), each with every way below and up to five tile widths; the choice by them takes 1.3-1.5 % more
+// than the best of those on average (with the constants that 8 units per CTA had given: 3.2-3.6 %).
+// One unit (128 columns x 128 k) of a token tile of `mt` rows in a long run:
+double unit_ns(int mt, bool fine) { return mt <= 32 && !fine ? 385.0 + 0.95 * mt : 430.0 + 1.15 * mt; }
 
 // Token tiles, and how the units go to the CTAs: whichever finishes first by this estimate.
 //   cluster    a tile's K range over S CTAs, which exchange partial sums through shared memory
-//              (~1.5 us); needs all clusters resident at once
+//              (3 us with the second pipeline fill); needs all clusters resident at once
 //   whole      runs of whole tiles: the last round may leave SMs idle
-//   even runs  no SM idles, but a tile's last CTA reads the other parts from L2: ~2.5 us for the
-//              hand-over and ~0.25 us per part and 16 token rows (two warps share that work in
-//              192-row tiles). K = N = 4096, 16 rows: 12.5 us against 10.5 with clusters
+//   even runs  no SM idles, but a tile's last CTA reads the other parts from L2: 5 us for the
+//              hand-over and 0.27 us per part and 16 token rows (two warps share that work in
+//              192-row tiles). K=4096 N=4096 M=16: 11.8 us against 10.1 with clusters; K=14336 N=6144
+//              M=16: 23.3 against 25.3
 // Fewer token tiles mean fewer dequantisations of a weight; more of them, more tiles to deal out.
 Geometry geometry_of(const W4A16Args& a) {
   Geometry g;
@@ -900,16 +901,16 @@ Geometry geometry_of(const W4A16Args& a) {
     const int m_tiles = static_cast<int>((a.m + mt - 1) / mt);
     const long long tiles = static_cast<long long>(g.n_tiles) * m_tiles;
     const double unit = unit_ns(mt, fine);
-    const double drain = mt * 8.0;   // accumulators to C
+    const double drain = mt * 19.0;   // a tile's accumulators to C
     offer(static_cast<double>((tiles + sms - 1) / sms) * (g.k_steps * unit + drain), mt, m_tiles, 1, false);
     for (int s = 2; s <= kMaxClusterSplit && 2 * s <= g.k_steps && tiles * s <= sms; ++s) {
       if (capacity[s] < tiles) break;
-      offer(2.0 * ((g.k_steps / 2 + s - 1) / s) * unit + drain + 1500.0, mt, m_tiles, s, false);
+      offer(2.0 * ((g.k_steps / 2 + s - 1) / s) * unit + drain + 3000.0, mt, m_tiles, s, false);
     }
     const double per_cta = static_cast<double>(tiles) * g.k_steps / (tiles * g.k_steps < sms ? tiles * g.k_steps : sms);
     const double parts = g.k_steps / per_cta + 1.0;
     const int chunks = mt <= 128 ? mt / 16 : (mt + 31) / 32;
-    offer(per_cta * unit + 2 * drain + 2500.0 + 250.0 * chunks * parts, mt, m_tiles, 1, true);
+    offer(per_cta * unit + (per_cta / g.k_steps + 1.0) * drain + 5000.0 + 270.0 * chunks * parts, mt, m_tiles, 1, true);
   }
   g.mtmax = g.mt <= 32 ? 32 : (g.mt <= 64 ? 64 : (g.mt <= 128 ? 128 : 192));
   const long long tiles = static_cast<long long>(g.n_tiles) * g.m_tiles;
@@ -918,20 +919,6 @@ Geometry geometry_of(const W4A16Args& a) {
   g.slot_bytes = g.split ? static_cast<size_t>(g.grid) * 2 * g.mt * kTileN * sizeof(float) : 0;
   g.counter_bytes = (static_cast<size_t>(g.grid) * sizeof(unsigned int) + 255) & ~size_t(255);
   return g;
-}
-
-// What the fixed scratch array is held against: counters and slots per (column tile, part) of equal
-// runs with one token tile of up to 128 rows. The shapes that entry point takes do not depend on
-// how a launch is dealt out.
-size_t per_tile_scratch(const W4A16Args& a) {
-  const int sms = sm_count();
-  const long long mt = (a.m + 15) & ~int64_t(15);
-  const long long n_tiles = (a.n + kTileN - 1) / kTileN, k_steps = a.k / kStepK;
-  const long long units = n_tiles * k_steps;
-  const long long per_cta = units / (units < sms ? units : sms);   // shortest run
-  const long long max_parts = (k_steps + per_cta - 1) / per_cta + 1;
-  return static_cast<size_t>(n_tiles * max_parts * mt * kTileN) * sizeof(float) +
-         ((static_cast<size_t>(n_tiles) * sizeof(unsigned int) + 255) & ~size_t(255));
 }
 
 // Encodes the tensor maps and enqueues the kernel on scratch memory the caller of this
@@ -996,18 +983,24 @@ ks_status_t enqueue_w4a16(const W4A16Args& a, const Geometry& g, unsigned int* c
 }  // namespace
 
 // Which fast kernel. The register-operand decode kernel feeds legacy mma.sync, whose rate on
-// this part is about a tenth of tcgen05's (measured: ~100 bf16 FMA per clock and SM
-// sub-partition): up to 8 tokens (one MMA per 16 x 16 weight block) it is well ahead of the
-// tcgen05 kernel on wide weights (K=4096, N=28672, queued launches: 24.6 us against 29.7), at
-// 16 tokens slightly (29.0 against 30.4), beyond that it is MMA-bound (32 tokens: 41 us
-// against 33). On problems with few units per CTA (K=14336, N=4096: 6 per CTA) its pipeline
-// fill and the split-K fix-up of every CTA cost what they save (19.8 us against 19.1).
-// Chosen: at most 16 tokens and at least 10 units per CTA; the caller can pin either kernel.
+// this part is about a tenth of tcgen05's. Up to 8 rows (one MMA per 16 x 16 weight block) its cheaper
+// arithmetic wins on long runs of units (256 columns x 128 k): from about 9 per SM, with scale groups of 32 or
+// 64, where the other kernel's arithmetic costs more, from 5. Its split-K fix-up grows with the parts per
+// tile, 2 per SM and tile: with fewer than one tile per 8 SMs (N < 4864) it loses what it gains.
+// From 9 rows it is ahead only with narrow groups on wide weights. us, decode kernel | tcgen05:
+//   M=8  group 128  N=28672 K=4096 24.7 | 28.3   N=11008 K=4096 15.3 | 16.5   N=6144 K=8192 16.0 | 17.1
+//                   N=11008 K=2048 12.6 | 10.0   N=4096 K=14336 20.0 | 18.4
+//   M=8  group 64   N=11008 K=4096 16.5 | 19.0   N=4096 K=8192 13.7 | 15.7    N=11008 K=2048 13.3 | 12.1
+//   M=16 group 128  N=28672 K=4096 30.0 | 28.3   N=11008 K=8192 26.6 | 23.5
+//   M=16 group 64   N=28672 K=4096 32.0 | 35.4   N=11008 K=8192 28.1 | 29.1   N=4096 K=14336 27.2 | 22.6
+// The caller can pin either kernel.
 bool use_decode_kernel(const W4A16Args& a) {
   if (a.kernel == 1 || !decode::eligible(a)) return false;
   if (a.kernel == 2 || !w4a16_eligible(a)) return true;
-  const long long units = ((a.n + 255) / 256) * (a.k / 128);
-  return a.m <= 16 && units >= 20ll * sm_count();
+  const long long sms = sm_count(), tiles = (a.n + 255) / 256, units = tiles * (a.k / 128);
+  const bool fine = a.group_size % kStepK != 0;
+  if (a.m <= 8) return fine ? units >= 5 * sms : units >= 9 * sms && 8 * tiles >= sms;
+  return fine && a.m <= 16 && units >= 12 * sms && 4 * tiles >= sms;
 }
 
 ks_status_t launch_w4a16(const W4A16Args& a, cudaStream_t stream) {
@@ -1082,39 +1075,54 @@ ks_status_t static_scratch_address(uint8_t** out) {
 
 }  // namespace
 
+// What the fixed array is held against. Which shapes the entry point takes is part of its contract and
+// must not change with the choice of kernel or deal, so this is not what a launch uses, but a bound
+// of its own: partial sums per (column tile, part of K in equal runs), tiles of all rows. Where the
+// kernel or deal chosen needs more than the array holds, one that fits takes its place: whole tiles
+// need nothing.
+size_t nominal_scratch(const W4A16Args& a) {
+  if (a.m > 128 || a.group_size % kStepK != 0) return 0;
+  const long long sms = sm_count();
+  if (decode::eligible(a) && (a.kernel == 2 || (a.kernel == 0 && a.m <= 16 && (a.n + 255) / 256 * (a.k / 128) >= 20 * sms))) {
+    const decode::Geometry d = decode::geometry_of(a);
+    return d.counter_bytes + d.slot_bytes;
+  }
+  const long long mt = (a.m + 15) & ~int64_t(15);
+  const long long n_tiles = (a.n + kTileN - 1) / kTileN, k_steps = a.k / kStepK;
+  const long long units = n_tiles * k_steps;
+  const long long per_cta = units / (units < sms ? units : sms);   // shortest run
+  const long long max_parts = (k_steps + per_cta - 1) / per_cta + 1;
+  return static_cast<size_t>(n_tiles * max_parts * mt * kTileN) * sizeof(float) +
+         ((static_cast<size_t>(n_tiles) * sizeof(unsigned int) + 255) & ~size_t(255));
+}
+
 size_t w4a16_static_scratch_capacity() { return kStaticScratchBytes; }
 
 ks_status_t launch_w4a16_static(const W4A16Args& a, cudaStream_t stream) {
   bool dec = use_decode_kernel(a);
-  if (dec && a.group_size % kStepK != 0 && a.kernel == 0) {
-    // scale groups of 32 or 64 are taken at any size
-    const decode::Geometry d = decode::geometry_of(a);
-    dec = d.counter_bytes + d.slot_bytes <= kStaticScratchBytes;
-  }
-  Geometry g = dec ? Geometry{} : geometry_of(a);
   const decode::Geometry gd = dec ? decode::geometry_of(a) : decode::Geometry{};
-  const size_t counter_bytes = dec ? gd.counter_bytes : g.counter_bytes;
-  size_t need = gd.counter_bytes + gd.slot_bytes;
-  if (!dec) {
-    // more than 128 rows, and scale groups of 32 or 64, are taken at any size
-    const bool any_size = a.m > 128 || a.group_size % kStepK != 0;
-    need = any_size ? 0 : per_tile_scratch(a);
-    if (g.split && g.counter_bytes + g.slot_bytes > kStaticScratchBytes) {
-      // whole tiles per CTA need no slots
-      g.split = false;
-      const long long tiles = static_cast<long long>(g.n_tiles) * g.m_tiles;
-      g.grid = static_cast<int>(tiles < sm_count() ? tiles : sm_count());
-      g.slot_bytes = 0;
-    }
+  size_t need = nominal_scratch(a);
+  if (dec && gd.counter_bytes + gd.slot_bytes > kStaticScratchBytes) {
+    if (a.kernel == 0 && w4a16_eligible(a)) dec = false;
+    else need = gd.counter_bytes + gd.slot_bytes;
   }
   if (need > kStaticScratchBytes) {
     char msg[224];
     snprintf(msg, sizeof(msg),
-             "ks_gemm_w4a16_static_scratch: this shape needs %zu bytes of split-K scratch, the built-in array "
+             "ks_gemm_w4a16_static_scratch: this shape counts as %zu bytes of split-K scratch, the built-in array "
              "holds %zu; use ks_gemm_w4a16 or fewer rows per call",
              need, kStaticScratchBytes);
     KSB_FAIL(KS_ERROR_UNSUPPORTED_SHAPE, msg);
   }
+  Geometry g = dec ? Geometry{} : geometry_of(a);
+  if (g.split && g.counter_bytes + g.slot_bytes > kStaticScratchBytes) {
+    // whole tiles per CTA need no slots
+    g.split = false;
+    const long long tiles = static_cast<long long>(g.n_tiles) * g.m_tiles;
+    g.grid = static_cast<int>(tiles < sm_count() ? tiles : sm_count());
+    g.slot_bytes = 0;
+  }
+  const size_t counter_bytes = dec ? gd.counter_bytes : g.counter_bytes;
   uint8_t* scratch = nullptr;
   ks_status_t st = static_scratch_address(&scratch);
   if (st != KS_SUCCESS) return st;

@@ -764,3 +764,31 @@ def test_w4a16_narrow_tiles_four_groups(ks, cuda, m, k, n, gs):
         ks.runtime.stream_synchronize(0)
     check_gemm(out.cpu(), ref32, noise, f"w4a16 {m}x{n}x{k} group {gs}")
     assert torch.equal(out, again), "not reproducible run to run"
+
+
+@pytest.mark.parametrize("m,k,n,gs", [
+    (8, 9088, 4864, 128),     # 19 tiles of 256 columns, 9 units per SM: the decode kernel
+    (8, 9088, 4608, 128),     # 18 tiles: tcgen05
+    (9, 9088, 4864, 128),     # 9 rows
+    (8, 4992, 4864, 64),      # narrow groups: the decode kernel from 5 units per SM
+    (8, 4864, 4864, 32),
+    (16, 6144, 9472, 64),     # 9 to 16 rows, narrow groups: 37 tiles, 12 units per SM
+    (16, 6144, 9216, 64),
+    (128, 2048, 1040, 128),   # a cluster of many parts: blocks of the exchange go round its CTAs
+])
+def test_w4a16_either_side_of_the_kernel_choice(ks, cuda, m, k, n, gs):
+    """Shapes next to the lines of the default choice, through both entry points."""
+    g = gen(m + k + n)
+    a = torch.randn(m, k, generator=g).to(torch.bfloat16)
+    b_packed = torch.randint(0, 256, (k // 2, n), generator=g, dtype=torch.uint8)
+    scales = (torch.randn(k // gs, n, generator=g).mul(0.02).abs() + 1e-3).to(torch.bfloat16)
+    zeros = torch.randint(0, 16, (k // gs, n), generator=g).to(torch.bfloat16)
+    ref32 = orc.w4a16(a, b_packed, scales, zeros, gs, None, out_dtype=None)
+    noise = accumulation_noise(a.float().abs(), orc.w4a16_weight(b_packed, scales, zeros, gs).float().abs(), k)
+    dev = [t.to(cuda) for t in (a, b_packed, scales, zeros)]
+    out = ks.dispatch.w4a16(*dev, group_size=gs)
+    fixed = ks.gemm.gemm_w4a16_static_scratch(torch.empty_like(out), *dev, m, n, k, gs)
+    torch.cuda.synchronize()
+    ks.runtime.stream_synchronize(0)
+    check_gemm(out.cpu(), ref32, noise, f"w4a16 {m}x{n}x{k} group {gs}")
+    assert torch.equal(out, fixed), "the entry points share kernel and deal"
