@@ -301,3 +301,26 @@ def test_permute_quant_of_large_problems_takes_any_ids(ks, cuda, top_k, dtype):
     ks.moe.permute(p, x, ids, tokens, top_k, hidden)
     q2, s2 = ks.dispatch.per_token_group_quant(p)
     assert torch.equal(q.view(torch.uint8), q2.view(torch.uint8)) and torch.equal(s, s2)
+
+
+@pytest.mark.parametrize("hidden,dtype", [(64, torch.bfloat16), (33, torch.float16), (64, torch.float32)])
+def test_unpermute_does_not_see_an_earlier_permutation(ks, cuda, hidden, dtype):
+    """The inverse map outlives a call. A permutation that names every pair, then one on the same stream that drops
+    most of them (ids -1 and out of range): the dropped pairs add nothing, whatever row the map still has for them."""
+    tokens, top_k = 300, 4
+    pairs = tokens * top_k
+    g = gen(8)
+    w = torch.rand(tokens, top_k, generator=g).to(cuda)
+    for drop in (0.0, 0.7, 0.0, 1.0):
+        ids = torch.randperm(pairs, generator=g).to(torch.int32)
+        cut = torch.rand(pairs, generator=g) < drop
+        ids[cut] = torch.where(torch.rand(int(cut.sum()), generator=g) < 0.5, -1, pairs + 3).to(torch.int32)
+        y = torch.randint(-8, 9, (pairs, hidden), generator=g).to(dtype)
+        out = torch.full((tokens, hidden), float("nan"), dtype=dtype, device=cuda)
+        ks.moe.unpermute(out, y.to(cuda), ids.to(cuda), w, tokens, top_k, hidden)
+        ref = torch.zeros(pairs, hidden, dtype=torch.float64)
+        ref[ids[~cut].long()] = y[~cut].double()
+        ref = (ref.view(tokens, top_k, hidden) * w.cpu().double()[:, :, None]).sum(1)
+        # four fp32 additions and one rounding to the output type
+        eps = {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -22}[dtype]
+        assert torch.allclose(out.cpu().double(), ref, rtol=2 * eps, atol=32 * 2.0 ** -22), drop
