@@ -323,20 +323,32 @@ __device__ __forceinline__ int32_t row_of_pair(const int32_t* __restrict__ inver
 // again: 145 instructions per 512 elements, top_k times, made that the bound: 141 us for 4096
 // tokens x 7168 x top 8, where writing the 242 MB takes ~40.) Blocks from `token_blocks` on walk the rows and
 // do those that no token's inverse entry names: ids out of range (a row of zeros) and
-// repeated ids, which the row-by-row kernel takes as they come.
+// repeated ids, which the row-by-row kernel takes as they come. With experts on other ranks most ids are
+// out of range, so such rows have a warp each and are written without the quantizer's arithmetic:
+// the shape above with 7/8 dropped 106 us row by row, 285 with 32 rows to a warp and the arithmetic, 68 now.
+// With two or three pairs a token it also pays to look whether the token has a row at all before it is read
+// (`look_first`): 16384 tokens x 4096, top 2, all dropped 55 us row by row, 75 without, 45 with; f32 with none
+// dropped 106 us row by row, 79 without, 85 with.
 template <typename T, bool E5M2>
 __global__ void __launch_bounds__(256)
 permute_quant_tokens_kernel(uint8_t* __restrict__ out, float* __restrict__ scale, const T* __restrict__ in,
                             const int32_t* __restrict__ ids, const int32_t* __restrict__ inverse, int64_t tokens,
-                            int top_k, int64_t hidden, unsigned token_blocks, float qmax) {
+                            int top_k, int64_t hidden, unsigned token_blocks, bool look_first, float qmax) {
   const int64_t segs_per_row = hidden / 16;
   const int64_t pairs = tokens * top_k;
   float v[16];
   if (blockIdx.x < token_blocks) {
     const int64_t seg = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t token = seg / segs_per_row;
-    const bool live = token < tokens;
     const int64_t c = seg - token * segs_per_row;
+    bool live = token < tokens;
+    if (look_first) {
+      // a token without rows, all its experts elsewhere, is not even read
+      bool named = false;
+      for (int k = 0; k < top_k && !named && live; ++k) named = row_of_pair(inverse, ids, token * top_k + k, pairs) >= 0;
+      live = named;
+      if (!__any_sync(0xffffffffu, live)) return;
+    }
     if (live) {
       quantmath::Vec16<T>::load(in + token * hidden + c * 16, v);
     } else {
@@ -356,30 +368,28 @@ permute_quant_tokens_kernel(uint8_t* __restrict__ out, float* __restrict__ scale
     return;
   }
   const int lane = threadIdx.x & 31;
-  const int64_t warp = (static_cast<int64_t>(blockIdx.x - token_blocks) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t mine = warp * 32 + lane;
-  bool left = false;
-  if (mine < pairs) {
-    const int32_t pair = __ldg(ids + mine);
-    left = !(pair >= 0 && pair < pairs && __ldg(inverse + pair) == mine);
-  }
-  unsigned todo = __ballot_sync(0xffffffffu, left);
-  while (todo != 0u) {
-    const int64_t r = warp * 32 + __ffs(todo) - 1;
-    todo &= todo - 1;
-    const int32_t pair = __ldg(ids + r);
-    const bool have = pair >= 0 && pair < pairs;
-    for (int64_t c0 = 0; c0 < segs_per_row; c0 += 32) {   // (segs_per_row is a multiple of 8)
-      const int64_t c = c0 + lane;
-      const bool live = c < segs_per_row;
-      if (have && live) {
-        quantmath::Vec16<T>::load(in + static_cast<int64_t>(pair / top_k) * hidden + c * 16, v);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = 0.f;
-      }
-      quantmath::quant_segment<T, E5M2>(out, scale, v, r * segs_per_row + c, live, qmax);
+  const int64_t r = (static_cast<int64_t>(blockIdx.x - token_blocks) * blockDim.x + threadIdx.x) >> 5;   // this warp's row
+  if (r >= pairs) return;
+  const int32_t pair = __ldg(ids + r);
+  if (pair < 0 || pair >= pairs) {   // what the quantizer makes of a row of zeros
+    for (int64_t c = lane; c < segs_per_row; c += 32) {
+      const int64_t dst = r * segs_per_row + c;
+      if ((c & 7) == 0) scale[dst >> 3] = quantmath::kScaleFloor;
+      __stcs(reinterpret_cast<uint4*>(out + dst * 16), make_uint4(0u, 0u, 0u, 0u));
     }
+    return;
+  }
+  if (__ldg(inverse + pair) == r) return;
+  for (int64_t c0 = 0; c0 < segs_per_row; c0 += 32) {   // (segs_per_row is a multiple of 8)
+    const int64_t c = c0 + lane;
+    const bool live = c < segs_per_row;
+    if (live) {
+      quantmath::Vec16<T>::load(in + static_cast<int64_t>(pair / top_k) * hidden + c * 16, v);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = 0.f;
+    }
+    quantmath::quant_segment<T, E5M2>(out, scale, v, r * segs_per_row + c, live, qmax);
   }
 }
 
@@ -706,10 +716,15 @@ ks_status_t ks_moe_permute_quant_fp8(void* out_fp8, float* out_scale, const void
   const unsigned blocks = static_cast<unsigned>((segs + 255) / 256);
   const bool e5 = fp8_dtype == KS_DTYPE_F8E5M2;
   uint8_t* o = static_cast<uint8_t*>(out_fp8);
-  // Token by token where the quantizing outweighs the extra launch (the inverse map, ~2.5 us): from
-  // about 16 M elements, with at least two pairs per token. The map lives in stream scratch; a
-  // stream under capture, where scratch may not grow, keeps to rows.
-  if (top_k >= 2 && pairs * hidden >= (int64_t(16) << 20)) {
+  // Token by token where the quantizing that it saves outweighs the extra launch (the inverse map,
+  // ~2.5 us), also with most pairs dropped, where row by row has little to do: from 24 M elements with six
+  // pairs a token, 32 M with four, 64 M with two. us, row by row | token by token, none and all dropped:
+  //   1024 x 6 x 4096 16.5 | 14.0, 12.4 | 12.4    512 x 8 x 4096 12.4 | 11.4, 10.3 | 11.2 (stays row by row)
+  //   4096 x 4 x 4096 41.0 | 23.2, 28.8 | 25.4    2400 x 4 x 2048 14.4 | 12.0, 10.4 | 12.4 (stays)
+  //   16384 x 2 x 4096 88 | 68, 55 | 45           4096 x 2 x 7168 38.8 | 33.4, half dropped 30.9 | 34.1 (stays)
+  // The map lives in stream scratch; a stream under capture, where scratch may not grow, keeps to rows.
+  const int64_t token_route_from = int64_t(top_k >= 6 ? 24 : top_k >= 4 ? 32 : 64) << 20;
+  if (top_k >= 2 && pairs * hidden >= token_route_from) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) {
       cudaGetLastError();
@@ -721,11 +736,11 @@ ks_status_t ks_moe_permute_quant_fp8(void* out_fp8, float* out_scale, const void
     if (inverse != nullptr) {
       inverse_permutation_kernel<<<static_cast<unsigned>((pairs + 255) / 256), 256, 0, s>>>(inverse, sorted_token_ids, pairs);
       const unsigned token_blocks = static_cast<unsigned>((num_tokens * (hidden / 16) + 255) / 256);
-      const unsigned total_blocks = token_blocks + static_cast<unsigned>((pairs + 255) / 256);
+      const unsigned total_blocks = token_blocks + static_cast<unsigned>((pairs + 7) / 8);
 #define KSB_PT(T, E5, QMAX)                                                                                      \
   permute_quant_tokens_kernel<T, E5><<<total_blocks, 256, 0, s>>>(o, out_scale, static_cast<const T*>(input),    \
                                                                   sorted_token_ids, inverse, num_tokens, top_k,  \
-                                                                  hidden, token_blocks, QMAX)
+                                                                  hidden, token_blocks, top_k < 4, QMAX)
       if (in_dtype == KS_DTYPE_F32) { if (e5) KSB_PT(float, true, 57344.0f); else KSB_PT(float, false, 448.0f); }
       else if (in_dtype == KS_DTYPE_F16) { if (e5) KSB_PT(__half, true, 57344.0f); else KSB_PT(__half, false, 448.0f); }
       else { if (e5) KSB_PT(__nv_bfloat16, true, 57344.0f); else KSB_PT(__nv_bfloat16, false, 448.0f); }

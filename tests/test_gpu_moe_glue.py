@@ -283,9 +283,9 @@ def test_peer_dispatch_and_combine_on_one_device(ks, cuda):
 
 @pytest.mark.parametrize("top_k,dtype", [(2, torch.bfloat16), (4, torch.float32)])
 def test_permute_quant_of_large_problems_takes_any_ids(ks, cuda, top_k, dtype):
-    """From 16 M elements on, tokens are quantized once and written to all their rows; ids out of range and
+    """From 64 M elements on (32 M with four pairs a token), tokens are quantized once and written to all their rows; ids out of range and
     repeated ids are rows that no token writes. Bit for bit what gather + quantizer give."""
-    tokens, hidden = (16 << 20) // 4096 // top_k + 3, 4096
+    tokens, hidden = ((64 if top_k < 4 else 32) << 20) // 4096 // top_k + 3, 4096
     pairs = tokens * top_k
     g = gen(31)
     ids = torch.randperm(pairs, generator=g).to(torch.int32)
@@ -300,6 +300,31 @@ def test_permute_quant_of_large_problems_takes_any_ids(ks, cuda, top_k, dtype):
     p = torch.empty(pairs, hidden, dtype=dtype, device=cuda)
     ks.moe.permute(p, x, ids, tokens, top_k, hidden)
     q2, s2 = ks.dispatch.per_token_group_quant(p)
+    assert torch.equal(q.view(torch.uint8), q2.view(torch.uint8)) and torch.equal(s, s2)
+
+
+@pytest.mark.parametrize("top_k,hidden,fp8", [(2, 4096, "e4m3"), (3, 1152, "e5m2"), (4, 4096, "e4m3"), (6, 640, "e4m3"), (8, 2048, "e5m2")])
+@pytest.mark.parametrize("drop", [0.6, 1.0])
+def test_permute_quant_of_large_problems_drops_tokens(ks, cuda, top_k, hidden, fp8, drop):
+    """Just above the sizes from which tokens are quantized once, with whole tokens dropped (hidden widths
+    where a warp holds segments of two tokens among them): bit for bit what gather + quantizer give."""
+    from_m = 24 if top_k >= 6 else 32 if top_k >= 4 else 64
+    tokens = (from_m << 20) // (hidden * top_k) + 5
+    pairs = tokens * top_k
+    g = torch.Generator(device=cuda).manual_seed(top_k)
+    ids = torch.randperm(pairs, generator=g, device=cuda).to(torch.int32)
+    gone = torch.rand(tokens, generator=g, device=cuda) < drop
+    ids[gone[(ids // top_k).long()]] = -1
+    ids[::7] = torch.where(ids[::7] % 5 == 0, -1, ids[::7])
+    x = torch.randn(tokens, hidden, generator=g, device=cuda).to(torch.bfloat16)
+    dt = {"e4m3": torch.float8_e4m3fn, "e5m2": torch.float8_e5m2}[fp8]
+    kw = dict(fp8_dtype=ks.DType.F8E5M2 if fp8 == "e5m2" else ks.DType.F8E4M3)
+    q = torch.full((pairs, hidden), 7, dtype=torch.uint8, device=cuda).view(dt)
+    s = torch.full((pairs, hidden // 128), float("nan"), dtype=torch.float32, device=cuda)
+    ks.moe.permute_quant_fp8(q, s, x, ids, tokens, top_k, hidden, **kw)
+    p = torch.empty(pairs, hidden, dtype=torch.bfloat16, device=cuda)
+    ks.moe.permute(p, x, ids, tokens, top_k, hidden)
+    q2, s2 = ks.dispatch.per_token_group_quant(p, **kw)
     assert torch.equal(q.view(torch.uint8), q2.view(torch.uint8)) and torch.equal(s, s2)
 
 
