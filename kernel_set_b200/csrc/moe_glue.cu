@@ -20,6 +20,8 @@
 #include <cstdio>
 #include <type_traits>
 
+#include <mutex>
+
 #include "common.cuh"
 #include "kernel_set/activation.h"
 #include "kernel_set/moe.h"
@@ -636,14 +638,20 @@ ks_status_t ks_moe_compute_permutation(int32_t* sorted_token_ids, int32_t* exper
   const int64_t per_thread = (per_cta + kPermThreads - 1) / kPermThreads;
   const int64_t chunk = (per_thread > 0 ? per_thread : 1) * kPermThreads;
   const unsigned ctas = pairs > 0 ? static_cast<unsigned>((pairs + chunk - 1) / chunk) : 1u;
+  // once per device and always: the kernel's static shared memory counts towards the 48 KB that need no
+  // opt-in, so a test of the dynamic part alone left out 361 experts (49096 + 132 bytes)
+  static std::mutex mu;
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (smem > 48 * 1024 && dev >= 0 && dev < 64 && !attr_done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(compute_permutation_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>((kPermWarps + 2) * kMaxExperts * sizeof(int)));
-    if (e != cudaSuccess) return cuda_status(e, where);
-    attr_done[dev] = true;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev >= 0 && dev < 64 && !attr_done[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(compute_permutation_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           static_cast<int>((kPermWarps + 2) * kMaxExperts * sizeof(int)));
+      if (e != cudaSuccess) return cuda_status(e, where);
+      attr_done[dev] = true;
+    }
   }
   compute_permutation_kernel<<<ctas, kPermThreads, smem, s>>>(sorted_token_ids, expert_offsets, topk_indices, pairs,
                                                               num_experts, chunk);

@@ -6,6 +6,10 @@ through the C ABI against the oracle's restatement of the reference's torch chec
 Bars: indices, permutations, gathered rows and every fp8 code / scale of the fused
 forms bit-exact; routing weights within 2e-6 relative; sums and activations within one
 rounding of the output type of the fp32 value."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -349,3 +353,43 @@ def test_unpermute_does_not_see_an_earlier_permutation(ks, cuda, hidden, dtype):
         # four fp32 additions and one rounding to the output type
         eps = {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -22}[dtype]
         assert torch.allclose(out.cpu().double(), ref, rtol=2 * eps, atol=32 * 2.0 ** -22), drop
+
+
+@pytest.mark.parametrize("experts", [360, 361, 362, 372])
+def test_compute_permutation_around_48_kb(ks, cuda, experts):
+    """34 counters an expert are 48 KB of dynamic shared memory at 361 experts, with the static part just over it. In
+    a process of its own: a call with more experts before it would have raised the limit for the rest."""
+    code = f"""
+import torch, kernel_set_b200 as ks
+ids = torch.randint(0, {experts}, (50, 4), dtype=torch.int32, device="cuda")
+so = torch.empty(200, dtype=torch.int32, device="cuda"); off = torch.empty({experts} + 1, dtype=torch.int32, device="cuda")
+ks.moe.compute_permutation(so, off, ids, 50, {experts}, 4)
+assert torch.equal(so.long(), torch.sort(ids.view(-1), stable=True).indices)
+assert int(off[-1]) == 200
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=root, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("tokens,experts,top_k", [
+    (25000, 64, 8),        # 200000 pairs, more than a pair per thread of 148 CTAs: a warp's piece has several steps
+    (50001, 7, 3),         # ... 150003 pairs, not a multiple of 32
+    (4001, 40, 5),         # several CTAs of one step, the last one partial
+])
+def test_compute_permutation_of_many_pairs_with_dropped_ones(ks, cuda, tokens, experts, top_k):
+    """Many CTAs, running counters carried from step to step, ids out of range in every CTA."""
+    g = gen(tokens)
+    ids = torch.randint(0, experts, (tokens, top_k), generator=g).to(torch.int32)
+    ids[torch.rand(tokens, top_k, generator=g) < 0.1] = -1
+    ids[torch.rand(tokens, top_k, generator=g) < 0.05] = experts + 2
+    pairs = tokens * top_k
+    sorted_ids = torch.full((pairs,), -7, dtype=torch.int32, device=cuda)
+    offsets = torch.full((experts + 1,), -7, dtype=torch.int32, device=cuda)
+    ks.moe.compute_permutation(sorted_ids, offsets, ids.to(cuda), tokens, experts, top_k)
+    flat = ids.view(-1).long()
+    valid = ((flat >= 0) & (flat < experts)).nonzero().view(-1)
+    order = valid[torch.sort(flat[valid], stable=True).indices]
+    assert torch.equal(sorted_ids.cpu()[:order.numel()].long(), order)
+    assert bool((sorted_ids.cpu()[order.numel():] == -1).all())
+    assert torch.equal(offsets.cpu().long()[1:], torch.bincount(flat[valid], minlength=experts).cumsum(0)) and int(offsets[0]) == 0
