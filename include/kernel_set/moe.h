@@ -72,7 +72,8 @@ KS_API ks_status_t ks_moe_permute(void* permuted, const void* input,
  * ks_moe_permute fused with ks_quantize_fp8_group(group_size = 128): row r of
  * the output holds the fp8 codes and the 1 x 128 scales of input row
  * sorted_token_ids[r] / top_k, bit-identical to running the two calls one
- * after the other, without the 16-bit intermediate.
+ * after the other, without the 16-bit intermediate. Large problems (from 24 M
+ * elements) use the inverse map of ks_moe_unpermute, outside stream capture.
  *   out_fp8 [num_tokens*top_k, hidden], out_scale [num_tokens*top_k, hidden/128]
  * hidden must be a multiple of 128. No counterpart in the reference.
  */
@@ -91,7 +92,8 @@ KS_API ks_status_t ks_moe_permute_quant_fp8(void* out_fp8, float* out_scale,
  *   permuted [num_tokens*top_k, hidden], out [num_tokens, hidden], f32/f16/bf16
  *   routing_weights [num_tokens, top_k] fp32
  * The inverse permutation lives in a library-owned, stream-ordered buffer
- * (first use of a stream allocates it; do that before any stream capture); the
+ * (first use of a stream allocates it; do that before any stream capture), which
+ * several host threads may use through one stream; the
  * reference allocates, synchronises and frees per call
  * (moe_permute.cu:317-375). Same contract otherwise: moe.h:49-56.
  */

@@ -738,9 +738,10 @@ ks_status_t ks_moe_permute_quant_fp8(void* out_fp8, float* out_scale, const void
       cudaGetLastError();
       capturing = cudaStreamCaptureStatusActive;
     }
+    sm100::StreamScratch scratch(s);   // (until both kernels are enqueued)
     int32_t* inverse = capturing != cudaStreamCaptureStatusNone
                            ? nullptr
-                           : static_cast<int32_t*>(sm100::stream_scratch(s, static_cast<size_t>(pairs) * sizeof(int32_t), 4));
+                           : static_cast<int32_t*>(scratch.get(static_cast<size_t>(pairs) * sizeof(int32_t), 4));
     if (inverse != nullptr) {
       inverse_permutation_kernel<<<static_cast<unsigned>((pairs + 255) / 256), 256, 0, s>>>(inverse, sorted_token_ids, pairs);
       const unsigned token_blocks = static_cast<unsigned>((num_tokens * (hidden / 16) + 255) / 256);
@@ -792,7 +793,8 @@ ks_status_t ks_moe_unpermute(void* out, const void* permuted, const int32_t* sor
   // inverse[pair] = row of the pair after the sort (not written for dropped pairs). Stream-ordered
   // library workspace: allocated when the stream first needs it (or needs more), never freed
   // or synchronised per call.
-  int32_t* inverse = static_cast<int32_t*>(sm100::stream_scratch(s, static_cast<size_t>(pairs) * sizeof(int32_t), 4));
+  sm100::StreamScratch scratch(s);   // (until both kernels are enqueued)
+  int32_t* inverse = static_cast<int32_t*>(scratch.get(static_cast<size_t>(pairs) * sizeof(int32_t), 4));
   if (inverse == nullptr) KSB_FAIL(KS_ERROR_OUT_OF_MEMORY, "ks_moe_unpermute: workspace allocation failed");
   const bool vec = dtype != KS_DTYPE_F32 && hidden % 8 == 0 && aligned16(out) && aligned16(permuted);
   if (!vec) {

@@ -56,6 +56,7 @@
 // Roofline: tensor-bound for M >= ~1024 (2*M*N*K flop over 4.5 PFLOP/s dense
 // FP8); bytes per launch M*K + N*K + M*N*sizeof(out) + scales.
 #include <mutex>
+#include <optional>
 #include <type_traits>
 
 #include "common.cuh"
@@ -1037,6 +1038,7 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   p.split_items = 0;
   p.split_s = 1;
   p.split_slots = nullptr;
+  std::optional<StreamScratch> scratch;
   p.cluster_s = cluster_s;
   if (cluster_s > 1) {
     p.split_from = 0;
@@ -1047,7 +1049,8 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
     const int s = rem > 0 ? static_cast<int>(split_parts(grid, rem, p.nkb)) : 1;
     if (rem > 0 && s >= 2) {
       const size_t slot_bytes = static_cast<size_t>(rem) * s * kBM * bn * sizeof(float);
-      float4* slots = static_cast<float4*>(stream_scratch(stream, slot_bytes, 2));
+      scratch.emplace(stream);   // (until both kernels are enqueued)
+      float4* slots = static_cast<float4*>(scratch->get(slot_bytes, 2));
       if (slots != nullptr) {
         p.split_from = static_cast<int>(tiles) - rem;
         p.split_items = rem * s;

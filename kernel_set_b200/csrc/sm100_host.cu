@@ -60,9 +60,22 @@ bool tma_encode(CUtensorMap* map, CUtensorMapDataType dtype, int rank, const voi
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-void* stream_scratch(cudaStream_t stream, size_t bytes, int kind) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+StreamScratch::StreamScratch(cudaStream_t stream) : stream_(stream) {
+  if (cudaGetDevice(&dev_) != cudaSuccess) {
+    dev_ = -1;
+    return;
+  }
+  // a lock per (device, stream), out of a fixed set: streams that share one wait for each other's
+  // launches, a few microseconds of host time
+  static std::mutex locks[64];
+  const uintptr_t h = reinterpret_cast<uintptr_t>(stream) / 16 + static_cast<uintptr_t>(dev_) * 7;
+  lock_ = std::unique_lock<std::mutex>(locks[(h ^ (h >> 6) ^ (h >> 12)) % 64]);
+}
+
+void* StreamScratch::get(size_t bytes, int kind) {
+  if (dev_ < 0) return nullptr;
+  const int dev = dev_;
+  const cudaStream_t stream = stream_;
   std::lock_guard<std::mutex> lock(g_scratch_mutex);
   Scratch& s = g_scratch[std::make_pair(std::make_pair(dev, stream), kind)];
   if (s.bytes >= bytes && s.ptr != nullptr) return s.ptr;

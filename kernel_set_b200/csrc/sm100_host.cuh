@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 namespace ksb {
 namespace sm100 {
 
@@ -20,14 +22,26 @@ bool tma_available();
 bool tma_encode(CUtensorMap* map, CUtensorMapDataType dtype, int rank, const void* base, const uint64_t* dims,
                 const uint64_t* strides_bytes, const uint32_t* box, CUtensorMapSwizzle swizzle);
 
-// Library-owned scratch memory for the current device, the given stream and the given
-// purpose (`kind`: buffers of different kinds never share memory), at least `bytes` large
-// and zero-filled when (re)allocated. The pointer stays valid until a later call asks for
-// more of the same kind on the same (device, stream); growth is stream-ordered
-// (cudaMallocAsync / cudaFreeAsync), so work already queued on the stream keeps its buffer.
-// Returns NULL when the allocation fails.
-void* stream_scratch(cudaStream_t stream, size_t bytes, int kind = 0);
-// Size of that buffer (0 when none exists).
+// Library-owned scratch memory of the current device and one stream, for the host thread that holds
+// this object: what it gets and what it enqueues on it before the object goes is one step, with no other
+// thread's calls on that stream in between. (Without that another thread's launches could overwrite
+// a map between the launch that writes and the one that reads it, or free a buffer by growing it.)
+class StreamScratch {
+ public:
+  explicit StreamScratch(cudaStream_t stream);
+  StreamScratch(const StreamScratch&) = delete;
+  StreamScratch& operator=(const StreamScratch&) = delete;
+  // At least `bytes` bytes for one purpose (`kind`: buffers of different kinds never share memory), zero-
+  // filled when (re)allocated. Growth is stream-ordered (cudaMallocAsync / cudaFreeAsync), so work
+  // already queued on the stream keeps its buffer. NULL when the allocation fails.
+  void* get(size_t bytes, int kind);
+
+ private:
+  cudaStream_t stream_;
+  int dev_ = -1;
+  std::unique_lock<std::mutex> lock_;
+};
+// Size of a stream's buffer (0 when none exists).
 size_t stream_scratch_bytes(cudaStream_t stream, int kind);
 // Marks every buffer of `kind` on the current device as possibly modified by a kernel
 // that stopped half-way; stream_scratch_take_dirty() reports and clears the mark of one

@@ -1016,8 +1016,9 @@ ks_status_t launch_w4a16(const W4A16Args& a, cudaStream_t stream) {
   const size_t counter_bytes = dec ? gd.counter_bytes : g.counter_bytes;
   // Whole tiles and clusters share nothing through memory.
   if (!dec && !g.split) return enqueue_w4a16(a, g, nullptr, nullptr, kernel_fault_word(), stream);
-  float* slots = static_cast<float*>(stream_scratch(stream, slot_bytes, 0));
-  unsigned int* counters = static_cast<unsigned int*>(stream_scratch(stream, counter_bytes, 1));
+  StreamScratch scratch(stream);
+  float* slots = static_cast<float*>(scratch.get(slot_bytes, 0));
+  unsigned int* counters = static_cast<unsigned int*>(scratch.get(counter_bytes, 1));
   if (slots == nullptr || counters == nullptr)
     KSB_FAIL(KS_ERROR_OUT_OF_MEMORY, "ks_gemm_w4a16: workspace allocation failed");
   if (std::getenv("KS_B200_ENV_RELOAD") != nullptr && std::getenv("KS_B200_TEST_DIRTY_COUNTERS") != nullptr) {
@@ -1130,6 +1131,9 @@ ks_status_t launch_w4a16_static(const W4A16Args& a, cudaStream_t stream) {
   // arrival counters to be zero on entry (a clean run leaves them so, an aborted
   // one may not, and another shape lays them out differently); the slots are
   // fully overwritten before being read.
+  // (one step with the launch: another thread's call on the stream may put slots where these counters are)
+  static std::mutex enqueue_mutex;
+  std::lock_guard<std::mutex> hold(enqueue_mutex);
   cudaError_t e = cudaMemsetAsync(scratch, 0, counter_bytes, stream);
   if (e != cudaSuccess) return cuda_status(e, "ks_gemm_w4a16_static_scratch: cudaMemsetAsync");
   unsigned int* counters = reinterpret_cast<unsigned int*>(scratch);

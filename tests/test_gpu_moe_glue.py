@@ -9,6 +9,7 @@ rounding of the output type of the fp32 value."""
 import os
 import subprocess
 import sys
+import threading
 
 import pytest
 import torch
@@ -393,3 +394,47 @@ def test_compute_permutation_of_many_pairs_with_dropped_ones(ks, cuda, tokens, e
     assert torch.equal(sorted_ids.cpu()[:order.numel()].long(), order)
     assert bool((sorted_ids.cpu()[order.numel():] == -1).all())
     assert torch.equal(offsets.cpu().long()[1:], torch.bincount(flat[valid], minlength=experts).cumsum(0)) and int(offsets[0]) == 0
+
+
+def test_host_threads_share_a_stream(ks, cuda):
+    """Two host threads on one stream, each with problems of its own and growing sizes: the inverse map that a call
+    writes is the one that it reads. (Values are small integers and weights powers of two: sums are exact.)"""
+    stream = torch.cuda.Stream(cuda)
+    hidden, top_k, calls = 64, 4, 60
+
+    def problem(seed, tokens):
+        g = gen(seed)
+        pairs = tokens * top_k
+        ids = torch.randperm(pairs, generator=g).to(torch.int32)
+        ids[torch.rand(pairs, generator=g) < 0.3] = -1
+        y = torch.randint(-8, 9, (pairs, hidden), generator=g)
+        ref = torch.zeros(pairs, hidden, dtype=torch.int64)
+        keep = ids >= 0
+        ref[ids[keep].long()] = y[keep]
+        return ids.to(cuda), y.to(torch.float32).to(cuda), ref.view(tokens, top_k, hidden).sum(1), tokens
+
+    problems = [[problem(100 * t + i, 50 + (7 + 3 * t) * i * i) for i in range(calls)] for t in range(2)]
+    weights = torch.ones(max(p[3] for ps in problems for p in ps), top_k, device=cuda)
+    outs = [[torch.empty(p[3], hidden, dtype=torch.bfloat16 if i % 2 else torch.float32, device=cuda)
+             for i, p in enumerate(ps)] for ps in problems]
+    ys = [[p[1].to(o.dtype) for p, o in zip(ps, os_)] for ps, os_ in zip(problems, outs)]
+    torch.cuda.synchronize()
+    errors = []
+
+    def run(t):
+        try:
+            for p, y, o in zip(problems[t], ys[t], outs[t]):
+                ks.moe.unpermute(o, y, p[0], weights, p[3], top_k, hidden, stream=stream)
+        except Exception as e:   # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=run, args=(t,)) for t in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    stream.synchronize()
+    assert not errors
+    for t in range(2):
+        for i, (p, o) in enumerate(zip(problems[t], outs[t])):
+            assert torch.equal(o.cpu().long(), p[2]), (t, i)
