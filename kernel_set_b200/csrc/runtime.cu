@@ -76,6 +76,9 @@ unsigned int* kernel_fault_word() {
   if (!d->fault_tried) {
     d->fault_tried = true;
     void* h = nullptr;
+    // (a process's first call may come while a stream is being captured, which pinning memory must not end)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     if (cudaHostAlloc(&h, 64, cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
       *static_cast<volatile unsigned int*>(h) = 0u;
       void* dp = nullptr;
@@ -86,6 +89,7 @@ unsigned int* kernel_fault_word() {
         cudaFreeHost(h);
       }
     }
+    cudaThreadExchangeStreamCaptureMode(&mode);
     cudaGetLastError();
   }
   return d->fault_dev;

@@ -5,6 +5,7 @@
 #include <map>
 #include <mutex>
 #include <utility>
+#include <vector>
 
 namespace ksb {
 namespace sm100 {
@@ -32,6 +33,8 @@ struct Scratch {
   void* ptr = nullptr;
   size_t bytes = 0;
   bool dirty = false;
+  bool in_graph = false;         // a captured graph holds the address
+  std::vector<void*> retired;    // buffers that graphs hold and that have been outgrown
 };
 __global__ void __launch_bounds__(256) full_sm_kernel() {}   // only asked about, never launched
 
@@ -70,31 +73,74 @@ StreamScratch::StreamScratch(cudaStream_t stream) : stream_(stream) {
   static std::mutex locks[64];
   const uintptr_t h = reinterpret_cast<uintptr_t>(stream) / 16 + static_cast<uintptr_t>(dev_) * 7;
   lock_ = std::unique_lock<std::mutex>(locks[(h ^ (h >> 6) ^ (h >> 12)) % 64]);
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+    cudaGetLastError();
+    status = cudaStreamCaptureStatusActive;
+  }
+  capturing_ = status != cudaStreamCaptureStatusNone;
 }
 
-void* StreamScratch::get(size_t bytes, int kind) {
-  if (dev_ < 0) return nullptr;
-  const int dev = dev_;
-  const cudaStream_t stream = stream_;
-  std::lock_guard<std::mutex> lock(g_scratch_mutex);
-  Scratch& s = g_scratch[std::make_pair(std::make_pair(dev, stream), kind)];
-  if (s.bytes >= bytes && s.ptr != nullptr) return s.ptr;
-  const size_t floor_bytes = kind == 0 ? (size_t(1) << 20) : (size_t(64) << 10);
-  size_t want = bytes < floor_bytes ? floor_bytes : bytes;
-  want = (want + 0xFFFF) & ~size_t(0xFFFF);
+StreamScratch::~StreamScratch() {
+  for (int i = 0; i < owned_count_; ++i)
+    if (cudaFreeAsync(owned_[i], stream_) != cudaSuccess) cudaGetLastError();
+}
+
+bool StreamScratch::cold_capture(size_t bytes, int kind) const {
+  return capturing_ && stream_scratch_bytes(stream_, kind) < bytes;
+}
+
+namespace {
+
+void* zeroed(size_t bytes, cudaStream_t stream) {
   void* fresh = nullptr;
-  if (cudaMallocAsync(&fresh, want, stream) != cudaSuccess) {
+  if (cudaMallocAsync(&fresh, bytes, stream) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (cudaMemsetAsync(fresh, 0, want, stream) != cudaSuccess) {
+  if (cudaMemsetAsync(fresh, 0, bytes, stream) != cudaSuccess) {
     cudaGetLastError();
     cudaFreeAsync(fresh, stream);
     return nullptr;
   }
-  if (s.ptr != nullptr) cudaFreeAsync(s.ptr, stream);
+  return fresh;
+}
+
+}  // namespace
+
+void* StreamScratch::get(size_t bytes, int kind) {
+  if (dev_ < 0) return nullptr;
+  const size_t floor_bytes = kind == 0 ? (size_t(1) << 20) : (size_t(64) << 10);
+  size_t want = bytes < floor_bytes ? floor_bytes : bytes;
+  want = (want + 0xFFFF) & ~size_t(0xFFFF);
+  std::lock_guard<std::mutex> lock(g_scratch_mutex);
+  Scratch& s = g_scratch[std::make_pair(std::make_pair(dev_, stream_), kind)];
+  if (s.bytes >= bytes && s.ptr != nullptr) {
+    if (s.dirty) {
+      if (cudaMemsetAsync(s.ptr, 0, s.bytes, stream_) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+      s.dirty = capturing_;   // a captured clearing has not happened yet
+    }
+    s.in_graph = s.in_graph || capturing_;
+    return s.ptr;
+  }
+  if (capturing_) {
+    void* fresh = owned_count_ < 4 ? zeroed(want, stream_) : nullptr;
+    if (fresh != nullptr) owned_[owned_count_++] = fresh;
+    return fresh;
+  }
+  if (s.in_graph && want < 2 * s.bytes) want = 2 * s.bytes;   // what is retired stays below what is in use
+  void* fresh = zeroed(want, stream_);
+  if (fresh == nullptr) return nullptr;
+  if (s.ptr != nullptr) {
+    if (s.in_graph) s.retired.push_back(s.ptr);
+    else cudaFreeAsync(s.ptr, stream_);
+  }
   s.ptr = fresh;
   s.bytes = want;
+  s.dirty = s.in_graph = false;
   return fresh;
 }
 
@@ -114,16 +160,6 @@ void stream_scratch_mark_dirty(int kind) {
     if (kv.first.first.first == dev && kv.first.second == kind) kv.second.dirty = true;
 }
 
-bool stream_scratch_take_dirty(cudaStream_t stream, int kind) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  std::lock_guard<std::mutex> lock(g_scratch_mutex);
-  auto it = g_scratch.find(std::make_pair(std::make_pair(dev, stream), kind));
-  if (it == g_scratch.end() || !it->second.dirty) return false;
-  it->second.dirty = false;
-  return true;
-}
-
 void stream_scratch_release(cudaStream_t stream) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return;
@@ -131,6 +167,7 @@ void stream_scratch_release(cudaStream_t stream) {
   for (auto it = g_scratch.begin(); it != g_scratch.end();) {
     if (it->first.first.first == dev && it->first.first.second == stream) {
       if (it->second.ptr != nullptr) cudaFreeAsync(it->second.ptr, stream);
+      for (void* p : it->second.retired) cudaFreeAsync(p, stream);
       it = g_scratch.erase(it);
     } else {
       ++it;

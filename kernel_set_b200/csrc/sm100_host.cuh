@@ -29,25 +29,33 @@ bool tma_encode(CUtensorMap* map, CUtensorMapDataType dtype, int rank, const voi
 class StreamScratch {
  public:
   explicit StreamScratch(cudaStream_t stream);
+  ~StreamScratch();
   StreamScratch(const StreamScratch&) = delete;
   StreamScratch& operator=(const StreamScratch&) = delete;
   // At least `bytes` bytes for one purpose (`kind`: buffers of different kinds never share memory), zero-
-  // filled when (re)allocated. Growth is stream-ordered (cudaMallocAsync / cudaFreeAsync), so work
-  // already queued on the stream keeps its buffer. NULL when the allocation fails.
+  // filled when (re)allocated or marked dirty. Growth is stream-ordered (cudaMallocAsync / cudaFreeAsync),
+  // so work already queued on the stream keeps its buffer. NULL when the allocation fails.
+  // Under stream capture the stream's buffer serves if it is large enough, and from then on outlives its
+  // growth, since a graph holds its address; otherwise the graph gets memory of its own, from here to the
+  // end of this object (an allocation and a free node), and nothing is kept. (A buffer first allocated
+  // under capture is the graph's: kept for later calls, its address would be used while no graph runs.)
   void* get(size_t bytes, int kind);
+  // Under capture, and the stream has no buffer that would serve.
+  bool cold_capture(size_t bytes, int kind) const;
 
  private:
   cudaStream_t stream_;
   int dev_ = -1;
+  bool capturing_ = false;
+  int owned_count_ = 0;
+  void* owned_[4];   // the graph's own memory
   std::unique_lock<std::mutex> lock_;
 };
 // Size of a stream's buffer (0 when none exists).
 size_t stream_scratch_bytes(cudaStream_t stream, int kind);
 // Marks every buffer of `kind` on the current device as possibly modified by a kernel
-// that stopped half-way; stream_scratch_take_dirty() reports and clears the mark of one
-// (device, stream) buffer, whose owner then restores the buffer's invariant.
+// that stopped half-way: it is cleared before its next use.
 void stream_scratch_mark_dirty(int kind);
-bool stream_scratch_take_dirty(cudaStream_t stream, int kind);
 // Frees (stream-ordered) every buffer of the current device that belongs to `stream`;
 // called when the stream is destroyed, so that a recycled handle starts clean.
 void stream_scratch_release(cudaStream_t stream);

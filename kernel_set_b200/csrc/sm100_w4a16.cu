@@ -921,6 +921,16 @@ Geometry geometry_of(const W4A16Args& a) {
   return g;
 }
 
+// The same token tiles dealt out whole, which takes no slots.
+Geometry in_whole_tiles(Geometry g) {
+  if (!g.split) return g;
+  g.split = false;
+  const long long tiles = static_cast<long long>(g.n_tiles) * g.m_tiles;
+  g.grid = static_cast<int>(tiles < sm_count() ? tiles : sm_count());
+  g.slot_bytes = 0;
+  return g;
+}
+
 // Encodes the tensor maps and enqueues the kernel on scratch memory the caller of this
 // function has already obtained: the arrival counters (all zero on entry; the
 // kernel leaves them zero) and the fp32 partial slots.
@@ -1008,7 +1018,7 @@ ks_status_t launch_w4a16(const W4A16Args& a, cudaStream_t stream) {
   // kernel is running, and a region that another shape used for partial sums is not.
   // The tcgen05 kernels can give up on a bounded wait and leave counters non-zero; when
   // the fault poll has reported such a launch on this device, every stream's counters are
-  // cleared before their next use (stream_scratch_dirty).
+  // cleared before their next use (stream_scratch_mark_dirty).
   const bool dec = use_decode_kernel(a);
   const Geometry g = dec ? Geometry{} : geometry_of(a);
   const decode::Geometry gd = dec ? decode::geometry_of(a) : decode::Geometry{};
@@ -1017,8 +1027,17 @@ ks_status_t launch_w4a16(const W4A16Args& a, cudaStream_t stream) {
   // Whole tiles and clusters share nothing through memory.
   if (!dec && !g.split) return enqueue_w4a16(a, g, nullptr, nullptr, kernel_fault_word(), stream);
   StreamScratch scratch(stream);
-  float* slots = static_cast<float*>(scratch.get(slot_bytes, 0));
-  unsigned int* counters = static_cast<unsigned int*>(scratch.get(counter_bytes, 1));
+  // More than 128 rows, and scale groups of 32 or 64, run without scratch memory where there is none: a graph
+  // that is captured on a stream without it, a device without room.
+  const bool can_do_without = w4a16_eligible(a) && a.kernel != 2 && (a.m > 128 || a.group_size % kStepK != 0);
+  float* slots = nullptr;
+  unsigned int* counters = nullptr;
+  if (!(can_do_without && (scratch.cold_capture(slot_bytes, 0) || scratch.cold_capture(counter_bytes, 1)))) {
+    slots = static_cast<float*>(scratch.get(slot_bytes, 0));
+    counters = static_cast<unsigned int*>(scratch.get(counter_bytes, 1));
+  }
+  if (can_do_without && (slots == nullptr || counters == nullptr))
+    return enqueue_w4a16(a, in_whole_tiles(geometry_of(a)), nullptr, nullptr, kernel_fault_word(), stream);
   if (slots == nullptr || counters == nullptr)
     KSB_FAIL(KS_ERROR_OUT_OF_MEMORY, "ks_gemm_w4a16: workspace allocation failed");
   if (std::getenv("KS_B200_ENV_RELOAD") != nullptr && std::getenv("KS_B200_TEST_DIRTY_COUNTERS") != nullptr) {
@@ -1026,10 +1045,8 @@ ks_status_t launch_w4a16(const W4A16Args& a, cudaStream_t stream) {
     // garbage in the counters and the mark that the fault poll would have set
     cudaMemsetAsync(counters, 0xFF, stream_scratch_bytes(stream, 1), stream);
     stream_scratch_mark_dirty(1);
-  }
-  if (stream_scratch_take_dirty(stream, 1)) {
-    cudaError_t e = cudaMemsetAsync(counters, 0, stream_scratch_bytes(stream, 1), stream);
-    if (e != cudaSuccess) return cuda_status(e, "ks_gemm_w4a16: clearing the split-K counters");
+    counters = static_cast<unsigned int*>(scratch.get(counter_bytes, 1));
+    if (counters == nullptr) KSB_FAIL(KS_ERROR_INTERNAL, "ks_gemm_w4a16: clearing the split-K counters");
   }
   if (dec) return decode::enqueue(a, gd, counters, slots, stream);
   return enqueue_w4a16(a, g, counters, slots, kernel_fault_word(), stream);
@@ -1116,13 +1133,7 @@ ks_status_t launch_w4a16_static(const W4A16Args& a, cudaStream_t stream) {
     KSB_FAIL(KS_ERROR_UNSUPPORTED_SHAPE, msg);
   }
   Geometry g = dec ? Geometry{} : geometry_of(a);
-  if (g.split && g.counter_bytes + g.slot_bytes > kStaticScratchBytes) {
-    // whole tiles per CTA need no slots
-    g.split = false;
-    const long long tiles = static_cast<long long>(g.n_tiles) * g.m_tiles;
-    g.grid = static_cast<int>(tiles < sm_count() ? tiles : sm_count());
-    g.slot_bytes = 0;
-  }
+  if (g.split && g.counter_bytes + g.slot_bytes > kStaticScratchBytes) g = in_whole_tiles(g);
   const size_t counter_bytes = dec ? gd.counter_bytes : g.counter_bytes;
   uint8_t* scratch = nullptr;
   ks_status_t st = static_scratch_address(&scratch);
