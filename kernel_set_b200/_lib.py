@@ -14,7 +14,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import POINTER, c_char_p, c_float, c_int, c_int64, c_size_t, c_void_p
+from ctypes import POINTER, c_char_p, c_float, c_int, c_int32, c_int64, c_size_t, c_void_p
 from typing import Optional
 
 KS_SUCCESS = 0
@@ -115,6 +115,18 @@ _VP = c_void_p
 _MISSING: list[str] = []
 
 
+class _ByAddress:
+    """The same functions for the package's own wrappers, with every data pointer taken as a plain
+    address: the wrappers have checked their arguments, and building a ctypes pointer object for each
+    typed one costs about 1 us a call. Direct callers use ``lib``, whose prototypes check the types."""
+
+    def __getattr__(self, name):   # symbols without a prototype
+        return getattr(lib, name)
+
+
+by_address = _ByAddress()
+
+
 def _decl(name: str, argtypes, restype=c_int) -> None:
     try:
         fn = getattr(lib, name)
@@ -123,6 +135,10 @@ def _decl(name: str, argtypes, restype=c_int) -> None:
         return
     fn.argtypes = argtypes
     fn.restype = restype
+    own = lib[name]   # a function object of its own, where getattr gives the one above
+    own.argtypes = [_VP if t in (POINTER(c_float), POINTER(c_int32)) else t for t in argtypes]
+    own.restype = restype
+    setattr(by_address, name, own)
 
 
 class DeviceProperties(ctypes.Structure):
@@ -159,22 +175,22 @@ _decl("ks_memset_device", [_VP, c_int, c_size_t, _VP])
 _W4A16 = [_VP, _VP, _VP, _VP, _VP, _VP, c_int64, c_int64, c_int64, c_int, c_int, _VP]
 _decl("ks_gemm_w4a16", _W4A16)
 _decl("ks_gemm_w4a16_static_scratch", _W4A16)
-_FP8_BW = [_VP, _VP, _VP, _VP, _VP, c_int64, c_int64, c_int64,
+_FP8_BW = [_VP, _VP, _VP, POINTER(c_float), POINTER(c_float), c_int64, c_int64, c_int64,
            c_int, c_int, c_int, c_int, _VP]
-_SCALED = [_VP, _VP, _VP, _VP, _VP]
+_SCALED = [_VP, _VP, _VP, POINTER(c_float), POINTER(c_float)]
 _decl("ks_gemm_fp8", _SCALED + [c_int64, c_int64, c_int64, c_int, c_int, c_int, c_int, _VP])
 _decl("ks_gemm_w8a8", _SCALED + [_VP, c_int64, c_int64, c_int64, c_int, c_int, c_int, _VP])
-_decl("ks_gemm_fp8_blockwise_colscale", [_VP, _VP, _VP, _VP, c_int64, _VP, c_int64, c_int64,
+_decl("ks_gemm_fp8_blockwise_colscale", [_VP, _VP, _VP, POINTER(c_float), c_int64, POINTER(c_float), c_int64, c_int64,
                                         c_int64, c_int, c_int, c_int, _VP])
-_decl("ks_gemm_fp8_blockwise_scatter", [POINTER(_VP), c_int, c_int64, _VP, _VP, _VP, _VP,
+_decl("ks_gemm_fp8_blockwise_scatter", [POINTER(_VP), c_int, c_int64, _VP, _VP, POINTER(c_float), POINTER(c_float),
                                        c_int64, c_int64, c_int64, c_int, c_int, c_int, _VP])
 _decl("ks_sum_parts", [POINTER(_VP), c_int, _VP, c_int, c_int64, c_int64, c_int, c_int, _VP])
 _decl("ks_gemm_fp8_blockwise", _FP8_BW)
 _decl("ks_gemm_fp8_blockwise_nt", _FP8_BW)
 
 # quant.h
-_decl("ks_quantize_fp8_group", [_VP, _VP, _VP, c_int64, c_int64, c_int, c_int, c_int, _VP])
-_decl("ks_quantize_fp8_group_colscale", [_VP, _VP, c_int64, _VP, c_int64, c_int64, c_int, c_int, _VP])
+_decl("ks_quantize_fp8_group", [_VP, POINTER(c_float), _VP, c_int64, c_int64, c_int, c_int, c_int, _VP])
+_decl("ks_quantize_fp8_group_colscale", [_VP, POINTER(c_float), c_int64, _VP, c_int64, c_int64, c_int, c_int, _VP])
 _decl("ks_dequantize_int4", [_VP, _VP, _VP, _VP, c_int64, c_int64, c_int, c_int, _VP])
 _decl("ks_repack_int4", [_VP, _VP, _VP, c_int64, c_int64, c_int, _VP])
 _decl("ks_int4_import_weight", [_VP, _VP, _VP, c_int64, c_int64, c_int, c_int, _VP])
@@ -182,32 +198,32 @@ _decl("ks_int4_import_zeros", [_VP, _VP, c_int64, c_int64, c_int, c_int, c_int, 
 _decl("ks_gather_columns", [_VP, _VP, _VP, c_int64, c_int64, c_int, _VP])
 
 # moe.h
-_decl("ks_moe_gate_softmax_topk", [_VP, _VP, _VP, c_int64, c_int, c_int, c_int, c_int, _VP])
-_decl("ks_moe_compute_permutation", [_VP, _VP, _VP, c_int64, c_int, c_int, _VP])
-_decl("ks_moe_permute", [_VP, _VP, _VP, c_int64, c_int, c_int64, c_int, _VP])
-_decl("ks_moe_permute_quant_fp8", [_VP, _VP, _VP, _VP, c_int64, c_int, c_int64, c_int, c_int, _VP])
-_decl("ks_moe_unpermute", [_VP, _VP, _VP, _VP, c_int64, c_int, c_int64, c_int, _VP])
-_decl("ks_moe_dispatch_plan", [_VP, _VP, _VP, _VP, _VP,
+_decl("ks_moe_gate_softmax_topk", [POINTER(c_float), POINTER(c_int32), _VP, c_int64, c_int, c_int, c_int, c_int, _VP])
+_decl("ks_moe_compute_permutation", [POINTER(c_int32), POINTER(c_int32), POINTER(c_int32), c_int64, c_int, c_int, _VP])
+_decl("ks_moe_permute", [_VP, _VP, POINTER(c_int32), c_int64, c_int, c_int64, c_int, _VP])
+_decl("ks_moe_permute_quant_fp8", [_VP, POINTER(c_float), _VP, POINTER(c_int32), c_int64, c_int, c_int64, c_int, c_int, _VP])
+_decl("ks_moe_unpermute", [_VP, _VP, POINTER(c_int32), POINTER(c_float), c_int64, c_int, c_int64, c_int, _VP])
+_decl("ks_moe_dispatch_plan", [POINTER(c_int32), POINTER(c_int32), POINTER(c_int32), POINTER(c_int32), POINTER(c_int32),
                               c_int, c_int, c_int, _VP])
-_decl("ks_moe_permute_quant_fp8_scatter", [POINTER(_VP), POINTER(_VP), c_int, c_int64, _VP, _VP,
-                                          c_int, c_int, _VP, _VP, c_int64, c_int, c_int64, c_int, c_int, _VP])
-_decl("ks_moe_scatter_rows", [POINTER(_VP), c_int, c_int64, _VP, c_int64, _VP, _VP, c_int, c_int64,
+_decl("ks_moe_permute_quant_fp8_scatter", [POINTER(_VP), POINTER(_VP), c_int, c_int64, POINTER(c_int32), POINTER(c_int32),
+                                          c_int, c_int, _VP, POINTER(c_int32), c_int64, c_int, c_int64, c_int, c_int, _VP])
+_decl("ks_moe_scatter_rows", [POINTER(_VP), c_int, c_int64, _VP, c_int64, POINTER(c_int32), POINTER(c_int32), c_int, c_int64,
                              c_int, _VP])
-_decl("ks_moe_grouped_gemm", [_VP, _VP, _VP, _VP, c_int, c_int64, c_int64, c_int64, c_int, _VP])
+_decl("ks_moe_grouped_gemm", [_VP, _VP, _VP, POINTER(c_int32), c_int, c_int64, c_int64, c_int64, c_int, _VP])
 _decl("ks_moe_grouped_gemm_fp8_blockwise",
-      [_VP, _VP, _VP, _VP, _VP, _VP, c_int, c_int64, c_int64, c_int64,
+      [_VP, _VP, _VP, POINTER(c_float), POINTER(c_float), POINTER(c_int32), c_int, c_int64, c_int64, c_int64,
        c_int, c_int, c_int, c_int, c_int, _VP])
 
 # norm.h
 _decl("ks_rms_norm", [_VP, _VP, _VP, c_int64, c_int64, c_float, c_int, _VP])
-_decl("ks_rms_norm_quant_fp8", [_VP, _VP, _VP, _VP, c_int64, c_int64, c_float, c_int, c_int, _VP])
+_decl("ks_rms_norm_quant_fp8", [_VP, POINTER(c_float), _VP, _VP, c_int64, c_int64, c_float, c_int, c_int, _VP])
 
 # activation.h
 _decl("ks_swiglu", [_VP, _VP, _VP, c_int64, c_int64, c_int, _VP])
 _decl("ks_swiglu_packed", [_VP, _VP, c_int64, c_int64, c_int, _VP])
-_decl("ks_swiglu_packed_quant_fp8", [_VP, _VP, _VP, c_int64, c_int64, c_int, c_int, _VP])
+_decl("ks_swiglu_packed_quant_fp8", [_VP, POINTER(c_float), _VP, c_int64, c_int64, c_int, c_int, _VP])
 _decl("ks_moe_grouped_gemm_fp8_blockwise_masked",
-      [_VP, _VP, _VP, _VP, _VP, _VP, c_int, c_int64, c_int64, c_int64,
+      [_VP, _VP, _VP, POINTER(c_float), POINTER(c_float), POINTER(c_int32), c_int, c_int64, c_int64, c_int64,
        c_int, c_int, c_int, c_int, c_int, _VP])
 
 

@@ -23,7 +23,7 @@ from typing import Optional
 import torch
 
 from . import gemm as _gemm
-from ._lib import check, lib
+from ._lib import by_address as lib, check
 from ._tensor import TensorLike, default_stream, dtype_to_ks, infer_dtype, ptr
 from .enums import Int4Packing, Int4Source
 

@@ -9,7 +9,7 @@ from typing import Optional
 
 import torch
 
-from ._lib import check, lib
+from ._lib import by_address as lib, check
 from ._tensor import TensorLike, default_stream, dtype_to_ks, f32_ptr, i32_ptr, infer_dtype, ptr
 
 

@@ -8,7 +8,7 @@ from typing import Optional
 
 import torch
 
-from ._lib import check, lib
+from ._lib import by_address as lib, check
 from ._tensor import TensorLike, default_stream, f32_ptr, infer_dtype, ptr
 
 

@@ -6,7 +6,7 @@ from __future__ import annotations
 
 from typing import Optional
 
-from ._lib import check, lib
+from ._lib import by_address as lib, check
 from ._tensor import TensorLike, default_stream, f32_ptr, infer_dtype, ptr
 from .enums import DType
 

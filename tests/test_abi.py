@@ -223,3 +223,25 @@ def test_python_marshalling_rejects_host_tensors(ks):
     assert ks.dispatch.per_token_group_quant_fp8 is ks.dispatch.per_token_group_quant
     e = ks.KernelSetError(3, "KS_ERROR_UNSUPPORTED_SHAPE", "msg", "ks_x")
     assert e.status == 3 and "ks_x failed" in str(e)
+
+
+def test_direct_callers_keep_the_pointer_checks(ks):
+    """The prototypes on ``lib`` take float and int32 pointers as such: an integer, bytes or a pointer to something
+    else in their place is refused before it reaches the library. (Nothing here gets that far.)"""
+    import ctypes
+    lib = ks._lib.lib
+    F, I, V = ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_int32), ctypes.c_void_p
+    f, i = ctypes.cast(16, F), ctypes.cast(16, I)
+    assert list(lib.ks_gemm_fp8_blockwise.argtypes)[3:5] == [F, F]
+    assert list(lib.ks_moe_compute_permutation.argtypes)[:3] == [I, I, I]
+    assert list(lib.ks_moe_unpermute.argtypes)[:4] == [V, V, I, F]
+    for bad in (4096, b"1234", ctypes.c_void_p(4096), i):
+        with pytest.raises(ctypes.ArgumentError):
+            lib.ks_quantize_fp8_group(V(16), bad, V(16), 1, 128, 128, 1, 3, None)
+    for bad in (4096, b"1234", f):
+        with pytest.raises(ctypes.ArgumentError):
+            lib.ks_moe_compute_permutation(i, i, bad, 1, 1, 1, None)
+    # the package's own wrappers pass addresses, through functions of their own
+    own = ks._lib.by_address
+    assert all(t is V for t in list(own.ks_moe_compute_permutation.argtypes)[:3])
+    assert own.ks_version() == lib.ks_version()
