@@ -359,17 +359,15 @@ def test_w4a16_baseline_shapes(ks, cuda, k, n):
             check_gemm(out[:, w], ref32, noise, f"w4a16 M={m} K={k} N={n} columns {w.start}..{w.stop}")
 
 
-@pytest.mark.parametrize("operand", ["smem", "tmem"])
 @pytest.mark.parametrize("m,k,n,gs,dtype,zeros", [
     (8, 1024, 512, 128, torch.bfloat16, "random"),
     (32, 512, 208, 256, torch.float16, "eight"),      # ragged last column tile, two K-steps per group
     (3, 768, 128, 128, torch.bfloat16, "fraction"),   # K = 6 steps, fp32 fallback for the zero-points
     (17, 256, 384, 128, torch.bfloat16, None),
 ])
-def test_w4a16_operand_paths(ks, cuda, operand, m, k, n, gs, dtype, zeros):
-    """Decode shapes through both ways of feeding the tensor core (shared-memory operand,
-    tensor-memory operand); both multiply the same rounded weights and differ by the
-    order of the fp32 sums only."""
+def test_w4a16_tcgen05_decode_shapes(ks, cuda, m, k, n, gs, dtype, zeros):
+    """Decode shapes through the tcgen05 kernel, against the oracle and the general kernel, which multiplies the
+    same rounded weights: order of the fp32 sums only."""
     g = gen(m * 3 + k + n)
     a = torch.randn(m, k, generator=g).to(dtype)
     codes = torch.randint(0, 16, (k, n), generator=g).to(torch.int32)
@@ -381,23 +379,15 @@ def test_w4a16_operand_paths(ks, cuda, operand, m, k, n, gs, dtype, zeros):
     b_packed = orc.pack_int4_bytes(codes)
     ref32 = orc.w4a16(a, b_packed, scales, zp, gs, None, out_dtype=None)
     noise = accumulation_noise(a.float().abs(), orc.w4a16_weight(b_packed, scales, zp, gs).float().abs(), k)
-    old = os.environ.get("KS_B200_W4A16_OPERAND")
+    dev = (a.to(cuda), b_packed.to(cuda), scales.to(cuda), zp.to(cuda) if zp is not None else None)
     outs = {}
-    try:
-        for path in ("smem", "tmem"):
-            os.environ["KS_B200_W4A16_OPERAND"] = path
-            with w4_path("tcgen05"):
-                outs[path] = ks.dispatch.w4a16(a.to(cuda), b_packed.to(cuda), scales.to(cuda),
-                                               zp.to(cuda) if zp is not None else None, group_size=gs).cpu()
-            torch.cuda.synchronize()
-            ks.runtime.stream_synchronize(0)
-    finally:
-        if old is None:
-            os.environ.pop("KS_B200_W4A16_OPERAND", None)
-        else:
-            os.environ["KS_B200_W4A16_OPERAND"] = old
-    check_gemm(outs[operand], ref32, noise, f"w4a16 {operand} operand {m}x{n}x{k}")
-    assert orc.rel_frobenius(outs["smem"].float(), outs["tmem"].float()) < 2e-3
+    for path in ("tcgen05", "general"):
+        with w4_path(path):
+            outs[path] = ks.dispatch.w4a16(*dev, group_size=gs).cpu()
+        torch.cuda.synchronize()
+        ks.runtime.stream_synchronize(0)
+    check_gemm(outs["tcgen05"], ref32, noise, f"w4a16 tcgen05 {m}x{n}x{k}")
+    assert orc.rel_frobenius(outs["tcgen05"].float(), outs["general"].float()) < 2e-3
 
 
 def test_w4a16_scratch_survives_shape_changes(ks, cuda):
@@ -611,8 +601,8 @@ def test_grouped_gemm_fp8_256_experts(ks, cuda, n, k):
 ])
 def test_w4a16_tcgen05_token_tiles_and_fine_groups(ks, cuda, m, k, n, gs, dtype, zeros, bias):
     """Every token-tile width, scale groups narrower than a K-step, odd numbers of K-steps, and each
-    way of dealing the work out (the fixed-scratch entry point never shares tiles through scratch above
-    128 rows), against the general kernel, which multiplies the same rounded weights: summation order only."""
+    way of dealing the work out, through both entry points, against the general kernel, which multiplies
+    the same rounded weights: summation order only."""
     g = gen(m + k + n)
     a = torch.randn(m, k, generator=g).to(dtype).to(cuda)
     b_packed = torch.randint(0, 256, (k // 2, n), generator=g, dtype=torch.uint8).to(cuda)
@@ -792,3 +782,28 @@ def test_w4a16_either_side_of_the_kernel_choice(ks, cuda, m, k, n, gs):
     ks.runtime.stream_synchronize(0)
     check_gemm(out.cpu(), ref32, noise, f"w4a16 {m}x{n}x{k} group {gs}")
     assert torch.equal(out, fixed), "the entry points share kernel and deal"
+
+
+@pytest.mark.parametrize("gs", [128, 32])
+@pytest.mark.parametrize("dtype,scale_set,zero_set", [
+    # f16: the short form needs scale * 2^9 <= 2^15, and integer zero-points up to 1023
+    (torch.float16, [2.0 ** -24, 3 * 2.0 ** -24, 2.0 ** -15, 0.013, -0.02, 1.0, 63.97, 64.0, 64.06, 128.0, 0.0],
+     [-0.0, 0.0, 7.0, 8.0, 15.0, 16.0, 100.0, 255.0, 0.5, -3.0]),
+    (torch.float16, [2.0 ** -24, 5 * 2.0 ** -20, 0.5, -0.25], [512.0, 1000.0, 1023.0, 1024.0, 1025.0, 2000.0]),
+    # bf16: scale * 2^6 <= 2^127, zero-points up to 127
+    (torch.bfloat16, [2.0 ** -120, 0.013, -0.02, 1.0, 2.0 ** 118, 0.0], [-0.0, 0.0, 8.0, 15.0, 16.0, 100.0, 127.0, 128.0, 129.0, 0.5, -3.0]),
+])
+def test_w4a16_dequantised_weights_to_the_bit(ks, cuda, dtype, scale_set, zero_set, gs):
+    """One-hot activations read the dequantised weights back, one per result: every code with scales and zero-points
+    on either side of what the short form of the dequantisation takes, against the oracle's rounding."""
+    k, n = 128, 272
+    g = gen(gs + len(scale_set))
+    a = torch.eye(k).to(dtype)
+    b_packed = torch.randint(0, 256, (k // 2, n), generator=g, dtype=torch.uint8)
+    pick = lambda values: torch.tensor(values)[torch.randint(0, len(values), (k // gs, n), generator=g)].to(dtype)   # noqa: E731
+    scales, zeros = pick(scale_set), pick(zero_set)
+    ref = orc.w4a16_weight(b_packed, scales, zeros, gs).to(dtype)
+    assert bool(torch.isfinite(ref.float()).all())
+    with w4_path("tcgen05"):
+        out = ks.dispatch.w4a16(a.to(cuda), b_packed.to(cuda), scales.to(cuda), zeros.to(cuda), group_size=gs).cpu()
+    assert torch.equal(out.float(), ref.float())
