@@ -33,10 +33,10 @@
 // tile inside the GEMM kernel measured 3-4 % gain instead of the 10 % the idle round costs:
 // one CTA then reads S x 128 KB behind a fence and four dependent atomics while its tensor
 // core waits.)
-// Measured on B200 with work-skipping builds of this kernel (M=4096, N=K=7168; the full kernel
-// 201-204 us): MMAs and operand loads without any epilogue work 152 us (TMA writes 48 KB and
+// Measured on B200 with work-skipping builds of this kernel before its promotion loop was rolled (M=4096,
+// N=K=7168; the full kernel 201-204 us then, 187-198 now): MMAs and operand loads without any epilogue work 152 us (TMA writes 48 KB and
 // the MMAs read 48 KB of shared memory per K-block; MMAs alone, from resident shared memory,
-// 125 us); the epilogue alone 155 us, of which the eight TMEM loads per K-block are nearly
+// 125 us); the epilogue alone 155 us, of which the TMEM loads (eight of 16 columns per K-block then) were nearly
 // free and the 128 FMAs per thread cost ~540 cycles (two epilogue warps per scheduler), the
 // scale fetches ~10 %; barriers alone 58 us. The two sides are equally long and the two
 // accumulator buffers couple them instead of letting them overlap fully. Measured and not
