@@ -183,7 +183,7 @@ KS_API ks_status_t ks_gemm_fp8_blockwise_colscale(void* out, const void* a_fp8,
  * are written to out_parts[b], a [rows_per_part, n] matrix of `out_dtype` that may
  * live in another GPU's memory (a peer-mapped address, e.g. rank b's buffer of a
  * symmetric allocation, offset to the slot of the calling rank). The finished
- * tiles leave by TMA stores, so the transfer over NVLink runs under the tiles
+ * tiles are stored there at once, so the transfer over NVLink runs under the tiles
  * still being computed; ks_sum_parts on the owning rank then adds the ranks'
  * slots. `out_parts` is a HOST array of num_parts (1..8) device pointers.
  * rows_per_part a multiple of 128, m = num_parts * rows_per_part, rows 16-byte

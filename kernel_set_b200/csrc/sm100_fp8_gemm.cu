@@ -14,16 +14,15 @@
 //               accumulator buffers (two of 256 columns, four of 128); ONE
 //               tcgen05.commit per K-block both releases the stage to the producer
 //               and tells the epilogue that the partial product is complete
-//   warps 2,3   idle (they complete warpgroup 0 so that register budgets can be
-//               moved between warpgroups with setmaxnreg)
+//   warps 2,3   schedule: walk the tiles ahead of the epilogue and hand it every K-block's
+//               a_scale * b_scale products and every tile's place through shared memory
 //   warps 4-11  epilogue: warp w reads TMEM lanes 32*(w%4).. and BN/2 columns in
-//               32-column loads, double-buffered so that one load is in flight
+//               16-column loads, double-buffered so that one load is in flight
 //               while the previous one is folded in:
 //               acc = fma(partial, a_scale[row,kb] * b_scale[kb,nb], acc) in
 //               registers (packed two-wide), frees the TMEM buffer, and after
-//               the last K-block rounds once to the output type. Dense problems
-//               stage the tile in swizzled shared memory and leave by TMA store;
-//               grouped and unaligned ones store row segments from registers.
+//               the last K-block rounds once to the output type; the tile is turned
+//               round in shared memory and stored in whole row segments.
 // Last partial round of a dense problem: when T tiles leave T mod #CTAs tiles for a final
 // round that would keep most SMs idle (896 tiles on 148 SMs: 8 tiles, 140 idle SMs for a
 // whole tile time), those tiles are cut along K into S parts (S <= 8, parts x tiles <=
@@ -33,15 +32,17 @@
 // tile inside the GEMM kernel measured 3-4 % gain instead of the 10 % the idle round costs:
 // one CTA then reads S x 128 KB behind a fence and four dependent atomics while its tensor
 // core waits.)
-// Measured on B200 with work-skipping builds of this kernel before its promotion loop was rolled (M=4096,
-// N=K=7168; the full kernel 201-204 us then, 187-198 now): MMAs and operand loads without any epilogue work 152 us (TMA writes 48 KB and
-// the MMAs read 48 KB of shared memory per K-block; MMAs alone, from resident shared memory,
-// 125 us); the epilogue alone 155 us, of which the TMEM loads (eight of 16 columns per K-block then) were nearly
-// free and the 128 FMAs per thread cost ~540 cycles (two epilogue warps per scheduler), the
-// scale fetches ~10 %; barriers alone 58 us. The two sides are equally long and the two
-// accumulator buffers couple them instead of letting them overlap fully. Measured and not
-// better: handing the accumulator over in two 128-column halves (eight N=128 MMAs per
-// K-block read A twice: 232 us), more loads in flight, sixteen narrower epilogue
+// What bounds it: the epilogue warps' chain per K-block (wait, TMEM loads, 64 two-wide FMAs, release) and, back to
+// back, the card's power limit. Per K-block of 128 x 256 x 128 the MMAs need 512 cycles; the loop took 872 while the
+// epilogue warps loaded scales from global memory (a load over 32 lines per warp), looked for their next tile
+// and stored by TMA piece by piece, 727 since warps 2 and 3 do the first two (M=4096, N=K=7168; with 28
+// K-blocks a tile and f32 results 994 -> 881, 4096 tokens over 256 experts, N=7168, K=2048, 1340 -> 985).
+// In time: M=4096, N=K=7168 alone 169 us (193 before), back to back 186 (200); SM clock 1.6 -> 1.5 GHz, the
+// rest is power. The register budget decides: nothing of the K loop may be spilled (with one spilled value and 16-column
+// loads 197 us, with two 200, with copies of the accumulators 240), so every address comes
+// from one base, the tile's place is read again behind the loop, and no other wait stands in it.
+// Measured and not better: 32-column loads (187), accumulators as 64-bit integers (240), handing the accumulator over
+// in two 128-column halves (eight N=128 MMAs per K-block read A twice: 232), sixteen narrower epilogue
 // warps, 224-wide tiles, scalar FMAs, paced MMA issue, sleeping or spinning waits.
 // Problems with fewer tiles than SMs (decode: M = 16, N = 7168 is 28 tiles of 256 columns) are
 // cut along K as well, over the S <= 8 CTAs of a cluster: each leaves its fp32 partial tile in
@@ -82,6 +83,7 @@ namespace {
 constexpr int kBM = 128;
 constexpr int kBK = 128;
 constexpr int kMaxExperts = 1024;
+constexpr int kMaxOutParts = 8;
 
 template <int BN>
 struct Cfg {
@@ -110,13 +112,22 @@ struct Cfg {
   // whose MMAs are short, need more buffers in flight to keep the tensor core fed.
   static constexpr int kAccBufs = BN == 256 ? 2 : KSB_FP8_ACC_BUFS_128;
   static constexpr int kTmemCols = 512;
-  // Dense problems stage the finished tile for TMA stores: 32 rows x 128 B per epilogue warp.
-  static constexpr int kStoreStageBytes = 32 * 128;
-  // ring + 1024 B alignment slack + barriers/flags, then either the store staging
-  // (dense) or the tile prefix, first rows and end rows of the experts (grouped)
+  // The finished tile is turned round in shared memory, 32 rows x 64 B per epilogue warp at a time.
+  static constexpr int kPieceBytes = 64;
+  static constexpr int kStagingBytes = kEpiWarps * 32 * kPieceBytes;
+  static constexpr int kCtrlBytes = 512;   // barriers and flags
+  // Slots of the schedule (see warps 2 and 3): a_scale * b_scale for the K-block's 128 rows and two column
+  // slices. The tiles lie beside them: the schedule is at most kSlots tiles ahead of the one being stored.
+  static constexpr int kSlots = 4;
+  static constexpr int kSlotBytes = 2 * kBM * 4;
+  static constexpr int kTileSlots = 8;
+  static constexpr int kTileBytes = 32;
+  static constexpr int kSchedBytes = kSlots * kSlotBytes + kTileSlots * kTileBytes;
+  // ring + 1024 B alignment slack + store staging + barriers + slots, then the tile prefix, first rows
+  // and end rows of the experts (grouped)
   static constexpr int smem_bytes(bool grouped) {
-    return kStages * kStageBytes + 1024 + 256 +
-           (grouped ? 3 * 4 * (kMaxExperts + 1) : kEpiWarps * kStoreStageBytes);
+    return kStages * kStageBytes + 1024 + kStagingBytes + kCtrlBytes + kSchedBytes +
+           (grouped ? 3 * 4 * (kMaxExperts + 1) : 0);
   }
 };
 
@@ -134,7 +145,6 @@ struct Params {
   int tiles_m;  // dense only
   uint32_t idesc;
   int vec_store;  // 16-byte output stores are legal
-  int tma_store;  // dense problems: finished tiles leave through shared memory and TMA stores
   // K-split of the last partial round (dense only): work items [0, split_from) are whole
   // tiles; item split_from + r is part r % split_s of tile split_from + r / split_s.
   int split_from;
@@ -150,15 +160,10 @@ struct Params {
   // grouped, masked layout: expert e owns rows [e * max_m, e * max_m + masked_m[e])
   const int32_t* masked_m;
   int max_m;
-  // scattered output (dense, TMA-store epilogue only): rows [b * rows_per_part, (b + 1) *
-  // rows_per_part) leave through output tensor map b, as rows 0.. of that map; 0 = one output
+  // scattered output (dense, 16-byte stores only): rows [b * rows_per_part, (b + 1) *
+  // rows_per_part) are rows 0.. of out_parts[b]; 0 = one output
   int rows_per_part;
-};
-
-// Output tensor maps: one, or one per destination of a scattered output.
-constexpr int kMaxOutParts = 8;
-struct OutMaps {
-  CUtensorMap m[kMaxOutParts];
+  void* out_parts[kMaxOutParts];
 };
 
 struct TileCoord {
@@ -182,7 +187,7 @@ __device__ __forceinline__ void place_in_panels(int t, int tiles_m, int tiles_n,
 }
 
 template <int BN, bool GROUPED>
-__device__ __forceinline__ bool locate_tile(const Params& p, const int* prefix, const int* offs, int t,
+__device__ __forceinline__ bool locate_tile(const Params& p, uint32_t tables, int t,
                                             TileCoord* tc) {
   if constexpr (!GROUPED) {
     tc->kb0 = 0;
@@ -210,22 +215,25 @@ __device__ __forceinline__ bool locate_tile(const Params& p, const int* prefix, 
     tc->kb1 = p.nkb;
     tc->part = -1;
     tc->tail = 0;
-    const int total_mt = prefix[p.num_experts];
+    // tables: row tiles before an expert | its first row | its end row
+    const auto prefix = [&](int e) { return ld_shared_s32(tables + 4 * e); };
+    const int total_mt = prefix(p.num_experts);
     if (t >= total_mt * p.tiles_n) return false;
     const int mt = t / p.tiles_n;
     int lo = 0, hi = p.num_experts - 1;  // last e with prefix[e] <= mt
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if (prefix[mid] <= mt) lo = mid; else hi = mid - 1;
+      if (prefix(mid) <= mt) lo = mid; else hi = mid - 1;
     }
     // The expert's tiles in panels, like a dense problem's: with all columns of one row tile before
     // the next row tile, the second row tile of an expert found its weights gone from L2 where the
     // expert's weight is larger (K=4096, N=28672 in 16 bits: 235 MB) and read them from HBM again.
+    const int first = prefix(lo);
     int em, en;
-    place_in_panels(t - prefix[lo] * p.tiles_n, prefix[lo + 1] - prefix[lo], p.tiles_n, &em, &en);
+    place_in_panels(t - first * p.tiles_n, prefix(lo + 1) - first, p.tiles_n, &em, &en);
     tc->expert = lo;
-    tc->row0 = offs[lo] + em * kBM;
-    tc->row_end = offs[kMaxExperts + 1 + lo];   // ends[lo]
+    tc->row0 = ld_shared_s32(tables + 4 * (kMaxExperts + 1 + lo)) + em * kBM;
+    tc->row_end = ld_shared_s32(tables + 4 * (2 * (kMaxExperts + 1) + lo));
     tc->n0 = en * BN;
     return true;
   }
@@ -238,12 +246,12 @@ struct ItemWalk {
   __device__ explicit ItemWalk(const Params& p)
       : n((p.split_s > 1 && static_cast<int>(blockIdx.x) < p.split_items) ? -1 : 0) {}
   template <int BN, bool GROUPED>
-  __device__ __forceinline__ bool next(const Params& p, const int* prefix, const int* offs, TileCoord* tc) {
+  __device__ __forceinline__ bool next(const Params& p, uint32_t tables, TileCoord* tc) {
     const int t = n < 0 ? p.split_from + static_cast<int>(blockIdx.x)
                         : static_cast<int>(blockIdx.x) + n * static_cast<int>(gridDim.x);
     if (n >= 0 && t >= p.split_from) return false;
     ++n;
-    return locate_tile<BN, GROUPED>(p, prefix, offs, t, tc);
+    return locate_tile<BN, GROUPED>(p, tables, t, tc);
   }
 };
 
@@ -283,44 +291,58 @@ __device__ __forceinline__ void store_4(OutT* dst, const float4& v, bool vec_ok,
 template <int BN, bool NT, bool GROUPED, typename OutT, int MODE = 0>
 __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1)
 fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-                          const __grid_constant__ OutMaps tm_cs, const Params p) {
+                          const __grid_constant__ Params p) {
   using C = Cfg<BN>;
   extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw_addr = smem_u32(smem_raw);
-  const uint32_t ring = (raw_addr + 1023u) & ~1023u;  // 1024-byte aligned for the 128 B swizzle
-  // dense: [ring | store staging | control]; grouped: [ring | control | prefix, offsets]
-  constexpr int kStagingBytes = GROUPED ? 0 : C::kEpiWarps * C::kStoreStageBytes;
-  const uint32_t staging = ring + C::kStages * C::kStageBytes;
-  uint8_t* ctrl = smem_raw + (ring - raw_addr) + C::kStages * C::kStageBytes + kStagingBytes;
-  const uint32_t ctrl_addr = staging + kStagingBytes;
-  // control block: full[S] | empty[S] | tmem_empty[B] | tmem slot | abort flag
-  const uint32_t bar_full = ctrl_addr;
-  const uint32_t bar_empty = ctrl_addr + 8 * C::kStages;
-  const uint32_t bar_tempty = ctrl_addr + 16 * C::kStages;
-  const uint32_t bar_accfull = bar_tempty + 8 * C::kAccBufs;   // MODE 1 / 2: a tile's accumulator is complete
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(ctrl + 16 * C::kStages + 16 * C::kAccBufs);
+  // Shared memory, from a 1024-byte boundary (for the 128 B swizzle): ring | store staging | full[S] | empty[S] |
+  // tmem_empty[B] | acc_full[B] | slot_empty[] | tmem slot | abort flag | slots | tiles | grouped: tables.
+  // Every role starts from a base of its own (base_of) and adds these: addresses that all roles share would
+  // each take a register through all of them.
+  constexpr uint32_t kStaging = C::kStages * C::kStageBytes;
+  constexpr uint32_t kBarFull = kStaging + C::kStagingBytes;
+  constexpr uint32_t kBarEmpty = kBarFull + 8 * C::kStages;
+  constexpr uint32_t kBarTempty = kBarEmpty + 8 * C::kStages;
+  constexpr uint32_t kBarAcc = kBarTempty + 8 * C::kAccBufs;   // MODE 1 / 2 / 3: a tile's accumulator is complete
+  constexpr uint32_t kBarSempty = kBarAcc + 8 * C::kAccBufs;
+  constexpr uint32_t kTmemSlot = kBarSempty + 8 * C::kSlots;
+  constexpr uint32_t kSlotsAt = kBarFull + C::kCtrlBytes;
+  constexpr uint32_t kTilesAt = kSlotsAt + C::kSlots * C::kSlotBytes;
+  constexpr uint32_t kTables = kSlotsAt + C::kSchedBytes;
+  static_assert(kTmemSlot + 8 <= kSlotsAt, "control block");
+  // The barrier on which the epilogue waits also counts the arrival of the schedule's warp, whose lead, the
+  // slots in use, is therefore no more than that barrier's turns: stages in MODE 0, accumulators otherwise.
+  constexpr uint32_t kSlots = MODE == 0 ? C::kSlots : C::kAccBufs;
+  static_assert(C::kSlots <= C::kStages && C::kAccBufs <= C::kSlots, "lead of the schedule");
+  const auto base_of = [&]() {
+    uint32_t b = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    asm volatile("" : "+r"(b));
+    return b;
+  };
+  const auto wait_ctx = [&](uint32_t sm) { return WaitCtx{sm + kTmemSlot + 4, p.fault_word}; };
+  uint8_t* const smem = smem_raw + (((smem_u32(smem_raw) + 1023u) & ~1023u) - smem_u32(smem_raw));
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kTmemSlot);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  int* prefix = reinterpret_cast<int*>(ctrl + 256);
-  int* offs = prefix + (kMaxExperts + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const WaitCtx wctx{abort_flag, p.fault_word};
 
   if (threadIdx.x == 0) {
+    const uint32_t sm = base_of();
     for (int s = 0; s < C::kStages; ++s) {
-      mbar_init(bar_full + 8 * s, 1);
-      mbar_init(bar_empty + 8 * s, 1);
+      mbar_init(sm + kBarFull + 8 * s, 1);
+      mbar_init(sm + kBarEmpty + 8 * s, MODE == 0 ? 2 : 1);   // commit; MODE 0: and the K-block's scales
     }
     for (int b = 0; b < C::kAccBufs; ++b) {
-      mbar_init(bar_tempty + 8 * b, C::kEpiWarps);
-      mbar_init(bar_accfull + 8 * b, 1);
+      mbar_init(sm + kBarTempty + 8 * b, C::kEpiWarps);
+      mbar_init(sm + kBarAcc + 8 * b, 2);   // commit and the tile's place
+    }
+    for (int q = 0; q < C::kSlots; ++q) {
+      mbar_init(sm + kBarSempty + 8 * q, C::kEpiWarps);
     }
     *abort_flag = 0u;
     fence_barrier_init();
     prefetch_tensormap(&tm_a);
     prefetch_tensormap(&tm_b);
-    if (!GROUPED && p.tma_store) prefetch_tensormap(&tm_cs.m[0]);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), C::kTmemCols);
@@ -329,6 +351,8 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
   if constexpr (GROUPED) {
     // offs[e] = first row of expert e; with the masked layout the rows of an expert end at
     // offs[e] + masked_m[e] instead of at offs[e + 1] (ends[] holds either)
+    int* prefix = reinterpret_cast<int*>(smem + kTables);
+    int* offs = prefix + (kMaxExperts + 1);
     int* ends = offs + (kMaxExperts + 1);
     for (int e = threadIdx.x; e <= p.num_experts; e += blockDim.x) {
       if (p.masked_m != nullptr) {
@@ -370,17 +394,18 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if constexpr (C::kRebalanceRegs) setmaxnreg_dec<C::kRegsIssue>();
+    const uint32_t sm = base_of();
     uint32_t it = 0;
     bool ok = true;
     TileCoord tc;
-    for (ItemWalk walk(p); ok && walk.template next<BN, GROUPED>(p, prefix, offs, &tc);) {
+    for (ItemWalk walk(p); ok && walk.template next<BN, GROUPED>(p, sm + kTables, &tc);) {
       for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
         const uint32_t s = it % C::kStages;
         const uint32_t ph = (it / C::kStages) & 1u;
-        if (!mbar_wait(wctx, bar_empty + 8 * s, ph ^ 1u, 0x100u + s)) { ok = false; break; }
+        if (!mbar_wait(wait_ctx(sm), sm + kBarEmpty + 8 * s, ph ^ 1u, 0x100u + s)) { ok = false; break; }
         {
-          const uint32_t full = bar_full + 8 * s;
-          const uint32_t a_dst = ring + s * C::kStageBytes;
+          const uint32_t full = sm + kBarFull + 8 * s;
+          const uint32_t a_dst = sm + s * C::kStageBytes;
           const uint32_t b_dst = a_dst + C::kABytes;
           mbar_arrive_expect_tx_elect(full, C::kStageBytes);
           tma_load_2d_elect(a_dst, &tm_a, full, kb * kBK, tc.row0);
@@ -402,50 +427,66 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -------------------------------
     if constexpr (C::kRebalanceRegs) setmaxnreg_dec<C::kRegsIssue>();
+    const uint32_t sm = base_of();
     uint32_t it = 0;
     uint32_t tile_n = 0;   // MODE 1 / 2: tiles so far (one accumulator buffer per tile)
     bool ok = true;
-    TileCoord tc;
-    for (ItemWalk walk(p); ok && walk.template next<BN, GROUPED>(p, prefix, offs, &tc);) {
+    // what it needs of the walk is the number of K-blocks: a part of a split tile first, then whole tiles
+    int items = GROUPED ? ld_shared_s32(sm + kTables + 4 * p.num_experts) * p.tiles_n : p.split_from;
+    items = (items - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+    int nk = p.nkb;
+    if (!GROUPED && p.split_s > 1 && static_cast<int>(blockIdx.x) < p.split_items) {
+      const int part = static_cast<int>(blockIdx.x) % p.split_s;
+      nk = ((part + 1) * p.nkb) / p.split_s - (part * p.nkb) / p.split_s;
+      ++items;
+    }
+    for (; ok && items > 0; --items, nk = p.nkb) {
       if constexpr (MODE != 0) {
         const uint32_t tbuf = tile_n % C::kAccBufs, tph = (tile_n / C::kAccBufs) & 1u;
-        if (!mbar_wait(wctx, bar_tempty + 8 * tbuf, tph ^ 1u, 0x200u + tbuf)) { ok = false; break; }
+        if (!mbar_wait(wait_ctx(sm), sm + kBarTempty + 8 * tbuf, tph ^ 1u, 0x200u + tbuf)) { ok = false; break; }
       }
-      for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
+      for (int kb = 0; kb < nk; ++kb, ++it) {
         const uint32_t s = it % C::kStages;
         const uint32_t ph = (it / C::kStages) & 1u;
         const uint32_t buf = MODE != 0 ? tile_n % C::kAccBufs : it % C::kAccBufs;
+        // A and (NT) B are K-major: 8-row groups 1024 B apart, a K step of 32
+        // elements is 32 B inside the swizzle atom. B stored [K,N] is MN-major:
+        // 128-column atoms 16 KB apart, 8-k groups 1024 B apart, a K step of 32
+        // rows is 32 * 128 B.
+        // (16-bit operands, MODE 3: the same bytes per instruction, 16 elements; an MN-major
+        // atom is 64 columns x 64 k-rows = 8 KB and a K step of 16 rows is 16 * 128 B)
+        const uint32_t a_src = sm + s * C::kStageBytes;
+        const uint32_t b_src = a_src + C::kABytes;
+        const uint32_t d_tmem = tmem_base + buf * BN;
+        uint64_t a_desc[kBK / 32], b_desc[kBK / 32];
+#pragma unroll
+        for (int kk = 0; kk < kBK / 32; ++kk) {
+          a_desc[kk] = umma_smem_desc_sw128(a_src + kk * 32, 16, 1024);
+          b_desc[kk] = NT ? umma_smem_desc_sw128(b_src + kk * 32, 16, 1024)
+                     : MODE == 3 ? umma_smem_desc_sw128(b_src + kk * 16 * 128, 64 * 128, 1024)
+                                 : umma_smem_desc_sw128(b_src + kk * 32 * 128, 128 * kBK, 1024);
+        }
+        // The operands are tested first: they are there long before the accumulator buffer is handed
+        // back, and even a test that succeeds takes ~100 cycles, which in the other order lay between the
+        // release of the buffer and the MMAs that it lets start.
+        if (!mbar_wait(wait_ctx(sm), sm + kBarFull + 8 * s, ph, 0x300u + s)) { ok = false; break; }
         if constexpr (MODE == 0) {
           const uint32_t aph = (it / C::kAccBufs) & 1u;
-          if (!mbar_wait(wctx, bar_tempty + 8 * buf, aph ^ 1u, 0x200u + buf)) { ok = false; break; }
+          if (!mbar_wait(wait_ctx(sm), sm + kBarTempty + 8 * buf, aph ^ 1u, 0x200u + buf)) { ok = false; break; }
         }
-        if (!mbar_wait(wctx, bar_full + 8 * s, ph, 0x300u + s)) { ok = false; break; }
         tc_fence_after_sync();
         {
           // all 32 lanes run this code; each instruction elects its one issuing lane
-          const uint32_t a_src = ring + s * C::kStageBytes;
-          const uint32_t b_src = a_src + C::kABytes;
-          const uint32_t d_tmem = tmem_base + buf * BN;
 #pragma unroll
           for (int kk = 0; kk < kBK / 32; ++kk) {
-            // A and (NT) B are K-major: 8-row groups 1024 B apart, a K step of 32
-            // elements is 32 B inside the swizzle atom. B stored [K,N] is MN-major:
-            // 128-column atoms 16 KB apart, 8-k groups 1024 B apart, a K step of 32
-            // rows is 32 * 128 B.
-            const uint64_t a_desc = umma_smem_desc_sw128(a_src + kk * 32, 16, 1024);
-            // (16-bit operands, MODE 3: the same bytes per instruction, 16 elements; an MN-major
-            // atom is 64 columns x 64 k-rows = 8 KB and a K step of 16 rows is 16 * 128 B)
-            const uint64_t b_desc = NT ? umma_smem_desc_sw128(b_src + kk * 32, 16, 1024)
-                                    : MODE == 3 ? umma_smem_desc_sw128(b_src + kk * 16 * 128, 64 * 128, 1024)
-                                                : umma_smem_desc_sw128(b_src + kk * 32 * 128, 128 * kBK, 1024);
-            const uint32_t accumulate = (kk > 0 || (MODE != 0 && kb > tc.kb0)) ? 1u : 0u;
-            if constexpr (MODE == 2) umma_i8_elect(d_tmem, a_desc, b_desc, p.idesc, accumulate);
-            else if constexpr (MODE == 3) umma_f16_elect(d_tmem, a_desc, b_desc, p.idesc, accumulate);
-            else umma_f8f6f4_elect(d_tmem, a_desc, b_desc, p.idesc, accumulate);
+            const uint32_t accumulate = (kk > 0 || (MODE != 0 && kb > 0)) ? 1u : 0u;
+            if constexpr (MODE == 2) umma_i8_elect(d_tmem, a_desc[kk], b_desc[kk], p.idesc, accumulate);
+            else if constexpr (MODE == 3) umma_f16_elect(d_tmem, a_desc[kk], b_desc[kk], p.idesc, accumulate);
+            else umma_f8f6f4_elect(d_tmem, a_desc[kk], b_desc[kk], p.idesc, accumulate);
           }
-          tc_commit_elect(bar_empty + 8 * s);
+          tc_commit_elect(sm + kBarEmpty + 8 * s);
           if constexpr (MODE != 0) {
-            if (kb == tc.kb1 - 1) tc_commit_elect(bar_accfull + 8 * buf);
+            if (kb == nk - 1) tc_commit_elect(sm + kBarAcc + 8 * buf);
           }
         }
       }
@@ -459,21 +500,23 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     constexpr int EC = C::kEpiCols;
     const int row_in_tile = quarter * 32 + lane;
     OutT* out = static_cast<OutT*>(p.out);
-    uint32_t it = 0;
-    uint32_t tile_n = 0;   // MODE 1 / 2: tiles so far
+    uint32_t it = 0;       // slots read so far: K-blocks in MODE 0, tiles otherwise
+    uint32_t tile_n = 0;
     bool ok = true;
-    TileCoord tc;
-    for (ItemWalk walk(p); ok && walk.template next<BN, GROUPED>(p, prefix, offs, &tc);) {
-      const int row = tc.row0 + row_in_tile;
-      const bool row_ok = row < tc.row_end;
-      const int col0 = tc.n0 + slice * EC;
-      int nb = col0 >> 7;
-      if (nb > p.nnb - 1) nb = p.nnb - 1;
-      const float* as_ptr = MODE == 3 ? nullptr : p.a_scale + static_cast<size_t>(row_ok ? row : 0) * p.as_row_stride;
-      const float* bs_ptr = MODE == 3 ? nullptr
-                                      : p.b_scale + static_cast<size_t>(tc.expert) * p.nkb * p.nnb +
-                                            (NT ? static_cast<size_t>(nb) * p.nkb : static_cast<size_t>(nb));
-      const size_t bs_step = NT ? 1 : static_cast<size_t>(p.nnb);
+    const uint32_t my_scale = (slice * kBM + row_in_tile) * 4;   // within a slot
+    while (true) {
+      const uint32_t sm = base_of();
+      // the tile's first K-block, or (MODE 1, 2, 3) all of it, and its place
+      const uint32_t turns = MODE == 0 ? C::kStages : C::kAccBufs;
+      const uint32_t done = (MODE == 0 ? sm + kBarEmpty : sm + kBarAcc) + 8 * (it % turns);
+      if (!(MODE == 0 ? mbar_wait_hinted(wait_ctx(sm), done, (it / turns) & 1u, 0x400u + it % turns, 50u)
+                      : mbar_wait_long(wait_ctx(sm), done, (it / turns) & 1u, 0x400u + it % turns))) {
+        ok = false;
+        break;
+      }
+      const uint32_t tile_at = sm + kTilesAt + (tile_n++ % C::kTileSlots) * C::kTileBytes;
+      const int nk = ld_shared_s32(tile_at);
+      if (nk == 0) break;   // no more work
 
       float2 acc[EC / 2];
 #pragma unroll
@@ -483,10 +526,11 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
         // the tile's accumulator is complete: scale by a_scale[row] * b_scale[col] (and add
         // the bias) on the way out of tensor memory, as kernels/src/gemm/gemm_fp8.cu:147-153
         // and gemm_w8a8.cu:134-141 of the reference do
-        const uint32_t tbuf = tile_n % C::kAccBufs, tph = (tile_n / C::kAccBufs) & 1u;
-        ++tile_n;
-        if (!mbar_wait_long(wctx, bar_accfull + 8 * tbuf, tph, 0x400u + tbuf)) { ok = false; break; }
+        const uint32_t tbuf = it % C::kAccBufs;
         tc_fence_after_sync();
+        const int row = ld_shared_s32(tile_at + 4) + row_in_tile;
+        const bool row_ok = row < ld_shared_s32(tile_at + 8);
+        const int col0 = ld_shared_s32(tile_at + 12) + slice * EC;
         float a_sc = 1.f, b_one = 1.f;
         if constexpr (MODE != 3) {
           a_sc = (p.a_per_row && row_ok) ? __ldg(p.a_scale + row) : __ldg(p.a_scale);
@@ -502,8 +546,12 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
           if (c == EC / 16 - 1) {
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_tempty + 8 * tbuf);
+            if (lane == 0) {
+              mbar_arrive(sm + kBarTempty + 8 * tbuf);
+              mbar_arrive(sm + kBarSempty + 8 * (it % kSlots));
+            }
           }
+          float v2[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int col = col0 + c * 16 + j;
@@ -515,48 +563,30 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
               v = __fmul_rn(__fmul_rn(raw, a_sc), b_sc);
               if (bias != nullptr && col_ok) v = __fadd_rn(v, to_f32<OutT>(bias[col]));
             }
-            if (j & 1) acc[c * 8 + (j >> 1)].y = v; else acc[c * 8 + (j >> 1)].x = v;
+            v2[j] = v;
           }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[c * 8 + j] = make_float2(v2[2 * j], v2[2 * j + 1]);
         }
+        ++it;
       }
 
-      // The promotion: one K-block per pass of a rolled loop. (Two K-blocks per pass, with an exit between
-      // them, spent ~275 cycles per K-block behind the release of the buffer, for 16 columns' FMAs and
-      // the next scales.) The scales of the next K-block are fetched while this one is folded in;
-      // 32 of them share a cache line. M=4096, N=K=7168 191.4 -> 187.4 us, 4096 tokens over 256
-      // experts, N=4096, K=7168 1620 -> 1584 us; with 16-column loads 191.4 and 1674.
+      // The promotion: one K-block per pass of a rolled loop, its scale one shared-memory load.
       if constexpr (MODE == 0) {
-        constexpr int CW = 32;   // TMEM columns per load
-        const float* as_p = as_ptr + tc.kb0 * p.as_kb_stride;
-        const float* bs_p = bs_ptr + static_cast<size_t>(tc.kb0) * bs_step;
-        float as_nxt = row_ok ? __ldg(as_p) : 0.f;
-        float bs_nxt = __ldg(bs_p);
+        constexpr int CW = 16;   // TMEM columns per load
         const uint32_t tquarter = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + slice * EC;
+        int kb = nk;
 #pragma unroll 1
-        for (int kb = tc.kb0; kb < tc.kb1; ++kb) {
-          const float sc = as_nxt * bs_nxt;
-          const float2 scale2 = make_float2(sc, sc);
-          as_p += p.as_kb_stride;
-          bs_p += bs_step;
-          if (kb + 1 < tc.kb1) {
-            as_nxt = row_ok ? __ldg(as_p) : 0.f;
-            bs_nxt = __ldg(bs_p);
-          }
-          const uint32_t buf = it % C::kAccBufs;
-          // One tcgen05.commit per K-block serves both consumers: the barrier that hands the
-          // shared-memory stage back to the producer also tells the epilogue that the
-          // accumulator is complete (each extra commit costs the tensor core ~50 idle cycles).
-          // short suspend hint: these warps are the critical path of every K-block, and a
-          // waiter parked for the default period is resumed later than one that re-polls
-          if (!mbar_wait_hinted(wctx, bar_empty + 8 * (it % C::kStages), (it / C::kStages) & 1u, 0x400u + buf, 50u)) {
-            ok = false;
-            break;
-          }
-          ++it;
+        while (true) {
+          // (every address from one base: kept apart they would take registers that the accumulators need)
+          const uint32_t sm = base_of();
           tc_fence_after_sync();
+          const uint32_t buf = it % C::kAccBufs, slot = it % kSlots;
           const uint32_t taddr = tquarter + buf * BN;
           uint32_t r0[CW], r1[CW];
           tmem_ld(taddr, r0);
+          const float sc = ld_shared_f32(sm + kSlotsAt + slot * C::kSlotBytes + my_scale);
+          const float2 scale2 = make_float2(sc, sc);
 #pragma unroll
           for (int c = 0; c < EC / CW; ++c) {
             if (c & 1) tmem_wait_ld(r1);
@@ -568,7 +598,10 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
               // every column of this warp's slice is in registers: hand the buffer back
               tc_fence_before_sync();
               __syncwarp();
-              if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
+              if (lane == 0) {
+                mbar_arrive(sm + kBarTempty + 8 * buf);
+                mbar_arrive(sm + kBarSempty + 8 * slot);
+              }
             }
 #pragma unroll
             for (int j = 0; j < CW / 2; ++j) {
@@ -577,15 +610,39 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
               ffma2(acc[c * (CW / 2) + j], lo, hi, scale2);
             }
           }
+          ++it;
+          if (--kb == 0) break;
+          // One tcgen05.commit per K-block serves both consumers: the barrier that hands the
+          // shared-memory stage back to the producer also tells the epilogue that the
+          // accumulator is complete (each extra commit costs the tensor core ~50 idle cycles).
+          // short suspend hint: these warps are the critical path of every K-block, and a
+          // waiter parked for the default period is resumed later than one that re-polls
+          if (!mbar_wait_hinted(wait_ctx(sm), sm + kBarEmpty + 8 * (it % C::kStages), (it / C::kStages) & 1u,
+                                0x400u + it % C::kStages, 50u)) {
+            ok = false;
+            break;
+          }
         }
       }
+      // (the rest of the tile's place is not held in registers over the K loop)
+      const uint4 t0 = ld_shared_v4(tile_at);
+      const uint4 t1 = ld_shared_v4(tile_at + 16);
+      struct { int row0, row_end, n0, part, tail; } tc;
+      tc.row0 = static_cast<int>(t0.y);
+      tc.row_end = static_cast<int>(t0.z);
+      tc.n0 = static_cast<int>(t0.w);
+      tc.part = static_cast<int>(t1.x);
+      tc.tail = static_cast<int>(t1.y);
+      const int row = tc.row0 + row_in_tile;
+      const bool row_ok = row < tc.row_end;
+      const int col0 = tc.n0 + slice * EC;
       bool stored = false;
       if constexpr (!GROUPED) {
         if (ok && tc.part >= 0 && p.cluster_s > 1) {
           // One K-part of a tile that the cluster shares: rows of BN + 4 floats (the padding
           // keeps the 16-byte stores of eight neighbouring lanes on different banks).
           if (row_ok) {
-            const uint32_t dst = ring + (row_in_tile * (BN + 4) + slice * EC) * 4;
+            const uint32_t dst = sm + (row_in_tile * (BN + 4) + slice * EC) * 4;
 #pragma unroll
             for (int c4 = 0; c4 < EC / 4; ++c4)
               st_shared_v4(dst + c4 * 16, __float_as_uint(acc[2 * c4].x), __float_as_uint(acc[2 * c4].y),
@@ -605,39 +662,56 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
             __stcg(mine + c4 * 32, make_float4(acc[2 * c4].x, acc[2 * c4].y, acc[2 * c4 + 1].x, acc[2 * c4 + 1].y));
           stored = true;
         }
-        if (ok && !stored && p.tma_store) {
-          // The warp's 32 x EC block leaves in pieces of 32 rows x 128 bytes: written
-          // to shared memory in the 128-byte swizzle (conflict-free: lanes 0-7 hit eight
-          // different 16-byte columns), then one TMA store, which clips rows and columns
-          // outside the matrix. The next tile's K loop starts while the store drains.
-          constexpr int kPieceCols = 128 / static_cast<int>(sizeof(OutT));
-          constexpr int kChunkCols = 16 / static_cast<int>(sizeof(OutT));
-          const uint32_t my_stage = staging + (warp - 4) * C::kStoreStageBytes;
-          const int store_row = tc.row0 + quarter * 32;
-          // a tile lies inside one part: rows_per_part is a multiple of the tile height
-          const int part_of_tile = p.rows_per_part > 0 ? tc.row0 / p.rows_per_part : 0;
-          const int part_row = store_row - part_of_tile * p.rows_per_part;
-          const CUtensorMap* out_map = &tm_cs.m[part_of_tile];
-#pragma unroll
-          for (int pc = 0; pc < EC / kPieceCols; ++pc) {
-            const int pcol = col0 + pc * kPieceCols;
-            if (pcol >= p.n || store_row >= p.m) break;   // warp-uniform
-            if (lane == 0) bulk_wait_group_read_all();     // the previous piece has left the buffer
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const uint4 w = pack_16_bytes<OutT>(acc, pc * kPieceCols + j * kChunkCols);
-              st_shared_v4(my_stage + lane * 128 + ((j ^ (lane & 7)) << 4), w.x, w.y, w.z, w.w);
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(out_map, my_stage, pcol, part_row);
-              bulk_commit_group();
-            }
+      }
+      if (ok && !stored && p.vec_store) {
+        // The warp's 32 x EC block leaves in pieces of 32 rows x 64 bytes: a lane writes its row to
+        // shared memory (16-byte chunks swizzled so that neighbouring lanes hit different banks), then
+        // four lanes read a row and store it. (By TMA store every piece waited for the one before to be
+        // read; from the lanes' own rows, as grouped problems had it, every 16-byte store touched 32 lines.)
+        constexpr int kPieceCols = C::kPieceBytes / static_cast<int>(sizeof(OutT));
+        constexpr int kChunkCols = 16 / static_cast<int>(sizeof(OutT));
+        constexpr int kChunks = C::kPieceBytes / 16;
+        constexpr int kRows = 32 / kChunks;   // rows that the warp reads at a time
+        static_assert(kChunks == 4, "the swizzle");
+        // (the compiler is kept from working out the addresses below once for all tiles: they would take the K
+        // loop's registers)
+        int ln = lane;
+        asm volatile("" : "+r"(ln));
+        const uint32_t my_stage = sm + kStaging + (warp - 4) * (32 * C::kPieceBytes);   // aligned to its size
+        // chunk j of row r lies at r * 64 + 16 * (j ^ ((r >> 1) & 3))
+        const uint32_t w_base = my_stage + ln * C::kPieceBytes + (((ln >> 1) & 3) << 4);
+        const int r0 = ln / kChunks, cj = ln % kChunks;   // this lane reads chunk cj of rows r0, r0 + 8, ...
+        const uint32_t r_base = my_stage + r0 * C::kPieceBytes + ((cj ^ ((r0 >> 1) & 3)) << 4);
+        OutT* dst = out;
+        int dst_row = tc.row0 + quarter * 32;
+        if constexpr (!GROUPED) {
+          if (p.rows_per_part > 0) {   // a tile lies inside one part: rows_per_part is a multiple of its height
+            const int part = tc.row0 / p.rows_per_part;
+            dst = static_cast<OutT*>(p.out_parts[part]);
+            dst_row -= part * p.rows_per_part;
           }
-          stored = true;
         }
+        const int rows = tc.row_end - (tc.row0 + quarter * 32);   // of this warp's 32 that exist
+        dst += static_cast<size_t>(dst_row + r0) * p.n + col0 + cj * kChunkCols;
+#pragma unroll
+        for (int pc = 0; pc < EC / kPieceCols; ++pc) {
+          if (col0 + pc * kPieceCols >= p.n || rows <= 0) break;   // warp-uniform
+          __syncwarp();   // the piece before has been read
+#pragma unroll
+          for (int j = 0; j < kChunks; ++j) {
+            const uint4 w = pack_16_bytes<OutT>(acc, pc * kPieceCols + j * kChunkCols);
+            st_shared_v4(w_base ^ (j << 4), w.x, w.y, w.z, w.w);
+          }
+          __syncwarp();
+          const bool col_ok = col0 + pc * kPieceCols + cj * kChunkCols < p.n;   // rows are whole chunks here
+#pragma unroll
+          for (int i = 0; i < kChunks; ++i) {
+            const uint4 w = ld_shared_v4(r_base + i * kRows * C::kPieceBytes);
+            if (col_ok && i * kRows + r0 < rows)
+              *reinterpret_cast<uint4*>(dst + static_cast<size_t>(i * kRows) * p.n + pc * kPieceCols) = w;
+          }
+        }
+        stored = true;
       }
       if (ok && row_ok && !stored) {
         OutT* dst = out + static_cast<size_t>(row) * p.n + col0;
@@ -653,11 +727,81 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
           if (valid > 0) store_16<OutT>(dst + c * 16, v, p.vec_store != 0, valid);
         }
       }
+      if (!ok) break;
     }
-    if (lane == 0) bulk_wait_group_all();   // shared memory must outlive the stores that read it
   } else {
-    // warps 2 and 3 only complete warpgroup 0
+    // -------------------------- schedule and scales ---------------------------
+    // Warps 2 and 3 walk the tiles ahead of the epilogue and hand it, K-block by K-block in turn, a slot
+    // with the scales of the block's 128 rows and of the two column slices, and the tile (MODE 1, 2, 3: one
+    // slot per tile, no scales). The epilogue warps then neither divide nor search for their next tile, nor
+    // wait for a load from L2 or HBM between two tiles, and read a scale with one shared-memory load where
+    // each of them had a load over 32 cache lines per K-block.
     if constexpr (C::kRebalanceRegs) setmaxnreg_dec<C::kRegsIssue>();
+    const uint32_t sm = base_of();
+    const uint32_t mine = static_cast<uint32_t>(warp - 2);
+    uint32_t it = 0, tile_n = 0;
+    bool ok = true;
+    TileCoord tc;
+    for (ItemWalk walk(p); ok && walk.template next<BN, GROUPED>(p, sm + kTables, &tc);) {
+      const int nk = MODE == 0 ? tc.kb1 - tc.kb0 : 1;
+      const int first = static_cast<int>((it ^ mine) & 1u);   // this warp's first K-block of the tile
+      const float* ap = nullptr;   // row 0 of the tile, and the other rows' distance from there
+      int off[4] = {};
+      const float* bp = nullptr;
+      if constexpr (MODE == 0) {
+        const int64_t kb = tc.kb0 + first;
+        ap = p.a_scale + tc.row0 * p.as_row_stride + kb * p.as_kb_stride;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = i * 32 + lane, last = tc.row_end - 1 - tc.row0;
+          off[i] = (r < last ? r : last) * static_cast<int>(p.as_row_stride);
+        }
+        int nb = (tc.n0 + ((lane >> 4) & 1) * C::kEpiCols) >> 7;   // lanes 0-15 the first slice, 16-31 the second
+        if (nb > p.nnb - 1) nb = p.nnb - 1;
+        bp = p.b_scale + static_cast<int64_t>(tc.expert) * p.nkb * p.nnb + (NT ? nb * static_cast<int64_t>(p.nkb) + kb : kb * p.nnb + nb);
+      }
+      for (int kb = first; kb < nk; kb += 2) {
+        const uint32_t n = it + static_cast<uint32_t>(kb);
+        const uint32_t slot = n % kSlots;
+        const uint32_t base = sm + kSlotsAt + slot * C::kSlotBytes;
+        float a[4], b = 0.f;
+        if constexpr (MODE == 0) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) a[i] = ld_global_nc_f32(ap + off[i]);
+          ap += 2 * p.as_kb_stride;
+          b = ld_global_nc_f32(bp);
+          bp += NT ? 2 : 2 * static_cast<int64_t>(p.nnb);
+        }
+        if (!mbar_wait(wait_ctx(sm), sm + kBarSempty + 8 * slot, ((n / kSlots) & 1u) ^ 1u, 0x600u + slot)) { ok = false; break; }
+        if constexpr (MODE == 0) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            st_shared_f32(base + (i * 32 + lane) * 4, a[i] * __shfl_sync(0xffffffffu, b, 0));
+            st_shared_f32(base + (kBM + i * 32 + lane) * 4, a[i] * __shfl_sync(0xffffffffu, b, 16));
+          }
+        }
+        if (kb == 0 && lane == 2) {
+          const uint32_t at = sm + kTilesAt + (tile_n % C::kTileSlots) * C::kTileBytes;
+          st_shared_v4(at, nk, tc.row0, tc.row_end, tc.n0);
+          st_shared_v4(at + 16, tc.part, tc.tail, 0, 0);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(MODE == 0 ? sm + kBarEmpty + 8 * (n % C::kStages) : sm + kBarAcc + 8 * (n % C::kAccBufs));
+      }
+      it += static_cast<uint32_t>(nk);
+      ++tile_n;
+    }
+    if (ok && ((it ^ mine) & 1u) == 0u) {   // the last slot says that there is no more
+      const uint32_t slot = it % kSlots;
+      if (mbar_wait(wait_ctx(sm), sm + kBarSempty + 8 * slot, ((it / kSlots) & 1u) ^ 1u, 0x600u + slot)) {
+        if (lane == 0) {
+          st_shared_v4(sm + kTilesAt + (tile_n % C::kTileSlots) * C::kTileBytes, 0, 0, 0, 0);
+          const uint32_t bar = MODE == 0 ? sm + kBarEmpty + 8 * (it % C::kStages) : sm + kBarAcc + 8 * (it % C::kAccBufs);
+          mbar_arrive(bar);   // twice: there is no commit
+          mbar_arrive(bar);
+        }
+      }
+    }
   }
 
   if constexpr (!GROUPED && MODE == 0) {
@@ -666,16 +810,17 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
       __syncwarp();
       cluster_sync();   // every CTA's partial is in its shared memory
       if (warp >= 4) {
+        const uint32_t sm = base_of();
         // this CTA's share of the tile, in units of four columns
         TileCoord tc;
-        locate_tile<BN, GROUPED>(p, prefix, offs, static_cast<int>(blockIdx.x), &tc);
+        locate_tile<BN, GROUPED>(p, sm + kTables, static_cast<int>(blockIdx.x), &tc);
         const int rows = tc.row_end - tc.row0 < kBM ? tc.row_end - tc.row0 : kBM;
         const int total = rows * (BN / 4);
         const int begin = (tc.part * total) / p.cluster_s, end = ((tc.part + 1) * total) / p.cluster_s;
         for (int i = begin + static_cast<int>(threadIdx.x) - 128; i < end; i += C::kEpiWarps * 32) {
           const int r = i / (BN / 4), col = tc.n0 + (i % (BN / 4)) * 4;
           if (col >= p.n) continue;
-          const uint32_t src = ring + (r * (BN + 4) + (i % (BN / 4)) * 4) * 4;
+          const uint32_t src = sm + (r * (BN + 4) + (i % (BN / 4)) * 4) * 4;
           float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
           for (int q = 0; q < p.cluster_s; ++q) {
             const float4 v = ld_shared_cluster_f4(cluster_map_shared(src, q));
@@ -763,35 +908,7 @@ ks_status_t launch_one(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUte
       attr_done[dev] = true;
     }
   }
-  // Output tensor map for the TMA-store epilogue (dense problems whose rows keep
-  // 16-byte alignment); otherwise the kernel stores from registers.
-  OutMaps tm_cs;
-  for (int i = 0; i < kMaxOutParts; ++i) tm_cs.m[i] = tm_a;
-  p.tma_store = 0;
-  p.rows_per_part = 0;
-  if (!GROUPED && p.vec_store) {
-    const CUtensorMapDataType dt = std::is_same<OutT, float>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                                   : std::is_same<OutT, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                                                       : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    const uint64_t str[1] = {static_cast<uint64_t>(a.n) * sizeof(OutT)};
-    const uint32_t box[2] = {static_cast<uint32_t>(128 / sizeof(OutT)), 32u};
-    if (a.num_out_parts > 0) {
-      // every part is a [rows_per_part, n] matrix of its own (possibly in another GPU's memory)
-      bool ok = true;
-      for (int i = 0; i < a.num_out_parts && ok; ++i) {
-        const uint64_t dims[2] = {static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.rows_per_part)};
-        ok = tma_encode(&tm_cs.m[i], dt, 2, a.out_parts[i], dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
-      }
-      if (ok) {
-        p.tma_store = 1;
-        p.rows_per_part = static_cast<int>(a.rows_per_part);
-      }
-    } else {
-      const uint64_t dims[2] = {static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.m)};
-      if (tma_encode(&tm_cs.m[0], dt, 2, a.out, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) p.tma_store = 1;
-    }
-  }
-  if (a.num_out_parts > 0 && !p.tma_store)
+  if (a.num_out_parts > 0 && !p.vec_store)
     KSB_FAIL(KS_ERROR_UNSUPPORTED_SHAPE, std::string(a.where) + ": the scattered output needs 16-byte aligned rows and parts");
   // (Programmatic dependent launch was measured on the quantizer -> GEMM -> reducer chain and
   // lost 1 % there: these kernels have no input-independent prologue worth overlapping, and
@@ -809,9 +926,9 @@ ks_status_t launch_one(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUte
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, tm_a, tm_b, tm_cs, p), a.where);
+    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, tm_a, tm_b, p), a.where);
   }
-  kernel<<<grid, C::kThreads, C::smem_bytes(GROUPED), stream>>>(tm_a, tm_b, tm_cs, p);
+  kernel<<<grid, C::kThreads, C::smem_bytes(GROUPED), stream>>>(tm_a, tm_b, p);
   if constexpr (!GROUPED) {
     if (p.split_s > 1) {
       const int tails = p.split_items / p.split_s;
@@ -1003,6 +1120,8 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   p.masked_m = a.masked_m;
   p.max_m = static_cast<int>(a.max_m);
   p.bias = a.bias;
+  p.rows_per_part = a.num_out_parts > 0 ? static_cast<int>(a.rows_per_part) : 0;
+  for (int i = 0; i < kMaxOutParts; ++i) p.out_parts[i] = i < a.num_out_parts ? a.out_parts[i] : nullptr;
   p.a_per_row = a.a_per_row ? 1 : 0;
   p.b_per_col = a.b_per_col ? 1 : 0;
   p.fault_word = kernel_fault_word();

@@ -41,7 +41,7 @@ struct Fp8GemmArgs {
   // Scattered output (dense, mode 0): rows [b * rows_per_part, (b + 1) * rows_per_part) of the
   // product are written to out_parts[b] as a [rows_per_part, n] matrix; `out` is not used.
   // rows_per_part is a multiple of 128 and m = num_out_parts * rows_per_part. The parts may
-  // live in other GPUs' memory (peer-mapped addresses): the tiles leave by TMA stores.
+  // live in other GPUs' memory (peer-mapped addresses): every row segment is stored there.
   void* const* out_parts = nullptr;
   int num_out_parts = 0;
   int64_t rows_per_part = 0;

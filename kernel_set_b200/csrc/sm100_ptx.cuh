@@ -50,9 +50,6 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -93,8 +90,21 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity
 
 // Shared state of a CTA's bounded waits.
 struct WaitCtx {
-  volatile uint32_t* abort_flag;  // shared memory, zero while healthy
-  unsigned int* fault_word;       // host-mapped, may be NULL
+  uint32_t abort_at;         // shared address of the CTA's abort flag, zero while healthy
+  unsigned int* fault_word;  // host-mapped, may be NULL
+
+  __device__ __forceinline__ bool raised() const {
+    uint32_t v;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(abort_at) : "memory");
+    return v != 0u;
+  }
+  __device__ __forceinline__ void give_up(uint32_t code) const {
+    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_at), "r"(1u) : "memory");
+    if (fault_word != nullptr) {
+      *reinterpret_cast<volatile unsigned int*>(fault_word) = 0x80000000u | code;
+      __threadfence_system();
+    }
+  }
 };
 
 // Waits for the phase with the given parity to complete. Returns false when
@@ -111,13 +121,9 @@ __device__ __forceinline__ bool mbar_wait_long(const WaitCtx& ctx, uint32_t bar,
 #pragma unroll 1
     for (int i = 0; i < 64; ++i)
       if (mbar_try_wait_hint(bar, parity, 20000u)) return true;
-    if (*ctx.abort_flag != 0u) return false;
+    if (ctx.raised()) return false;
     if (global_ns() - t0 > kWaitLimitNs) {
-      *ctx.abort_flag = 1u;
-      if (ctx.fault_word != nullptr) {
-        *reinterpret_cast<volatile unsigned int*>(ctx.fault_word) = 0x80000000u | code;
-        __threadfence_system();
-      }
+      ctx.give_up(code);
       return false;
     }
   }
@@ -147,13 +153,9 @@ __device__ __forceinline__ bool mbar_wait_hinted(const WaitCtx& ctx, uint32_t ba
 #pragma unroll 1
     for (int i = 0; i < 256; ++i)
       if (mbar_try_wait_hint(bar, parity, hint_ns)) return true;
-    if (*ctx.abort_flag != 0u) return false;
+    if (ctx.raised()) return false;
     if (global_ns() - t0 > kWaitLimitNs) {
-      *ctx.abort_flag = 1u;
-      if (ctx.fault_word != nullptr) {
-        *reinterpret_cast<volatile unsigned int*>(ctx.fault_word) = 0x80000000u | code;
-        __threadfence_system();
-      }
+      ctx.give_up(code);
       return false;
     }
   }
@@ -173,13 +175,9 @@ __device__ __forceinline__ bool mbar_wait(const WaitCtx& ctx, uint32_t bar, uint
 #pragma unroll 1
     for (int i = 0; i < 256; ++i)
       if (mbar_try_wait(bar, parity)) return true;
-    if (*ctx.abort_flag != 0u) return false;
+    if (ctx.raised()) return false;
     if (global_ns() - t0 > kWaitLimitNs) {
-      *ctx.abort_flag = 1u;
-      if (ctx.fault_word != nullptr) {
-        *reinterpret_cast<volatile unsigned int*>(ctx.fault_word) = 0x80000000u | code;
-        __threadfence_system();
-      }
+      ctx.give_up(code);
       return false;
     }
   }
@@ -489,23 +487,36 @@ __device__ __forceinline__ void tma_load_3d_elect(uint32_t smem_dst, const CUten
                : "memory");
 }
 
-// ---- TMA stores (shared -> global), tracked in per-thread bulk groups ---------------------
-// x (innermost coordinate) times the element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, uint32_t smem_src, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                   reinterpret_cast<uint64_t>(m)),
-               "r"(smem_src), "r"(x), "r"(y)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Returns once the bulk groups of this thread have finished READING shared memory.
-__device__ __forceinline__ void bulk_wait_group_read_all() {
-  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-// Returns once the bulk groups of this thread are complete.
-__device__ __forceinline__ void bulk_wait_group_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// A read-only load that stays where it is written: the compiler moves __ldg down to its use when registers
+// are short, which puts the load's latency back on the path it was issued early for.
+__device__ __forceinline__ float ld_global_nc_f32(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void st_shared_f32(uint32_t addr, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_shared_s32(uint32_t addr) {
+  int v;
+  asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
 }
 
 }  // namespace sm100

@@ -264,7 +264,7 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const WaitCtx wctx{abort_flag, p.fault_word};
+  const WaitCtx wctx{smem_u32(const_cast<uint32_t*>(abort_flag)), p.fault_word};
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kRawStages; ++s) {

@@ -201,7 +201,7 @@ class FusedRowParallel:
     peer memory, instead of as a collective behind the GEMM.
 
     Rank ``r`` owns the output rows ``[r * m / g, (r + 1) * m / g)``. Every rank's GEMM writes
-    its partial product of row block ``b`` straight into rank ``b``'s memory (TMA stores of
+    its partial product of row block ``b`` straight into rank ``b``'s memory (stores of
     the finished tiles, ``ks_gemm_fp8_blockwise_scatter``), so the reduce-scatter's traffic
     crosses NVLink while later tiles are still being computed. After a barrier each rank adds
     the ``g`` slots of its rows in rank order in fp32 (``ks_sum_parts``: the same bits on

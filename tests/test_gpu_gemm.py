@@ -107,6 +107,26 @@ def test_fp8_tcgen05_kernel(ks, cuda, m, n, k, layout, bn_tile, out_dtype, fp8):
 
 
 
+@pytest.mark.parametrize("k", [128, 256, 384, 640, 1152])   # 1 to 9 K-blocks a tile: the rings of 4 to 8 slots go round
+@pytest.mark.parametrize("m,n,layout,bn_tile,out_dtype", [
+    (2600, 4360, "nk", 256, torch.bfloat16),   # 2.5 tiles a CTA, the last piece of a row partly outside
+    (1290, 2100, "nk", 128, torch.float32),    # narrow tiles; rows of no whole 64-byte pieces
+    (2600, 4352, "kn", 256, torch.float16),
+    (1300, 2051, "nk", 256, torch.bfloat16),   # rows not 16-byte aligned: stored from registers
+])
+def test_fp8_scales_and_tiles_handed_over_ahead(ks, cuda, m, n, k, layout, bn_tile, out_dtype):
+    a8, a_s, b8, b_s = fp8_inputs(m, n, k, seed=m + n + k)
+    ref32, noise = fp8_reference(a8, a_s, b8, b_s)
+    with fp8_path("tcgen05", bn_tile):
+        out = run_fp8(ks, cuda, a8, a_s, b8, b_s, layout, out_dtype)
+        check_gemm(out, ref32, noise, f"{m}x{n}x{k} {layout}")
+        if layout == "nk":   # column-major activation scales
+            t = torch.empty(m, n, dtype=out_dtype, device=cuda)
+            ks.gemm.gemm_fp8_blockwise_colscale(t, a8.to(cuda), b8.t().contiguous().to(cuda), a_s.t().contiguous().to(cuda),
+                                                b_s.t().contiguous().to(cuda), m, n, k, a_scale_ld=m, b_layout="nk")
+            assert torch.equal(t.cpu(), out)
+
+
 def _headline_inputs(m, n, k, dev, seed):
     """Operands of a BASELINE-sized dense problem, made on the device (weights ~N(0, 0.02)
     block-quantized 128 x 128, activations ~N(0,1) quantized 1 x 128), [N,K] layout."""
