@@ -290,7 +290,8 @@ __device__ __forceinline__ void store_4(OutT* dst, const float4& v, bool vec_ok,
 //         bytes per row), B stored [K,N] is loaded in 64-column atoms. The unscaled grouped GEMM.
 template <int BN, bool NT, bool GROUPED, typename OutT, int MODE = 0>
 __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1)
-fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
+fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_a32,
+                          const __grid_constant__ CUtensorMap tm_b,
                           const __grid_constant__ Params p) {
   using C = Cfg<BN>;
   extern __shared__ uint8_t smem_raw[];
@@ -342,6 +343,7 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     *abort_flag = 0u;
     fence_barrier_init();
     prefetch_tensormap(&tm_a);
+    prefetch_tensormap(&tm_a32);
     prefetch_tensormap(&tm_b);
   }
   if (warp == 1) {
@@ -399,6 +401,12 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     bool ok = true;
     TileCoord tc;
     for (ItemWalk walk(p); ok && walk.template next<BN, GROUPED>(p, sm + kTables, &tc);) {
+      // A tile of up to 32 rows takes a box of 32: the rows behind its end (of no matrix, or of the next
+      // expert) stay away, and what the MMAs read there goes into rows that are not stored. M=16, N=14336:
+      // K=7168 33.7 -> 25.4 us, K=4096 19.8 -> 17.2 (64 rows took 25.6 and 17.2 already); decode of 48 tokens
+      // over 64 experts 251 -> 242. Up to three such boxes for 33 to 96 rows were slower than one of 128
+      // (8 experts, K=14336, N=4096, 16 bits 204 -> 211 us), so more rows keep that.
+      const bool few = tc.row_end - tc.row0 <= 32;
       for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
         const uint32_t s = it % C::kStages;
         const uint32_t ph = (it / C::kStages) & 1u;
@@ -407,8 +415,13 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
           const uint32_t full = sm + kBarFull + 8 * s;
           const uint32_t a_dst = sm + s * C::kStageBytes;
           const uint32_t b_dst = a_dst + C::kABytes;
-          mbar_arrive_expect_tx_elect(full, C::kStageBytes);
-          tma_load_2d_elect(a_dst, &tm_a, full, kb * kBK, tc.row0);
+          if (few) {
+            mbar_arrive_expect_tx_elect(full, C::kBBytes + 32 * kBK);
+            tma_load_2d_elect(a_dst, &tm_a32, full, kb * kBK, tc.row0);
+          } else {
+            mbar_arrive_expect_tx_elect(full, C::kStageBytes);
+            tma_load_2d_elect(a_dst, &tm_a, full, kb * kBK, tc.row0);
+          }
           if constexpr (NT) {
             tma_load_3d_elect(b_dst, &tm_b, full, kb * kBK, tc.n0, tc.expert);
           } else if constexpr (MODE == 3) {
@@ -891,7 +904,7 @@ bool encode_u8(CUtensorMap* map, const void* base, int rank, const uint64_t* dim
 }
 
 template <int BN, bool NT, bool GROUPED, typename OutT, int MODE = 0>
-ks_status_t launch_one(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUtensorMap& tm_b, Params p,
+ks_status_t launch_one(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUtensorMap& tm_a32, const CUtensorMap& tm_b, Params p,
                        int grid, cudaStream_t stream) {
   using C = Cfg<BN>;
   auto kernel = fp8_blockwise_umma_kernel<BN, NT, GROUPED, OutT, MODE>;
@@ -926,9 +939,9 @@ ks_status_t launch_one(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUte
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, tm_a, tm_b, p), a.where);
+    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, tm_a, tm_a32, tm_b, p), a.where);
   }
-  kernel<<<grid, C::kThreads, C::smem_bytes(GROUPED), stream>>>(tm_a, tm_b, p);
+  kernel<<<grid, C::kThreads, C::smem_bytes(GROUPED), stream>>>(tm_a, tm_a32, tm_b, p);
   if constexpr (!GROUPED) {
     if (p.split_s > 1) {
       const int tails = p.split_items / p.split_s;
@@ -942,34 +955,34 @@ ks_status_t launch_one(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUte
 }
 
 template <int BN, bool NT, bool GROUPED, int MODE = 0>
-ks_status_t launch_out(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p,
+ks_status_t launch_out(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUtensorMap& tm_a32, const CUtensorMap& tm_b, const Params& p,
                        int grid, cudaStream_t stream) {
   switch (a.out_dtype) {
-    case KS_DTYPE_F32: return launch_one<BN, NT, GROUPED, float, MODE>(a, tm_a, tm_b, p, grid, stream);
-    case KS_DTYPE_F16: return launch_one<BN, NT, GROUPED, __half, MODE>(a, tm_a, tm_b, p, grid, stream);
-    default: return launch_one<BN, NT, GROUPED, __nv_bfloat16, MODE>(a, tm_a, tm_b, p, grid, stream);
+    case KS_DTYPE_F32: return launch_one<BN, NT, GROUPED, float, MODE>(a, tm_a, tm_a32, tm_b, p, grid, stream);
+    case KS_DTYPE_F16: return launch_one<BN, NT, GROUPED, __half, MODE>(a, tm_a, tm_a32, tm_b, p, grid, stream);
+    default: return launch_one<BN, NT, GROUPED, __nv_bfloat16, MODE>(a, tm_a, tm_a32, tm_b, p, grid, stream);
   }
 }
 
 template <int BN>
-ks_status_t launch_bn(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUtensorMap& tm_b, const Params& p,
+ks_status_t launch_bn(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUtensorMap& tm_a32, const CUtensorMap& tm_b, const Params& p,
                       int grid, cudaStream_t stream) {
   const bool grouped = a.offsets != nullptr || a.masked_m != nullptr;
   // the per-row / per-column scaled kernels exist for the reference's layout (B stored [K,N]), dense
-  if (a.mode == 1) return launch_out<BN, false, false, 1>(a, tm_a, tm_b, p, grid, stream);
-  if (a.mode == 2) return launch_out<BN, false, false, 2>(a, tm_a, tm_b, p, grid, stream);
+  if (a.mode == 1) return launch_out<BN, false, false, 1>(a, tm_a, tm_a32, tm_b, p, grid, stream);
+  if (a.mode == 2) return launch_out<BN, false, false, 2>(a, tm_a, tm_a32, tm_b, p, grid, stream);
   // 16-bit operands, B stored [K,N]: the output has the operands' type
   if (a.mode == 3) {
     if (a.out_dtype == KS_DTYPE_F16)
-      return grouped ? launch_one<BN, false, true, __half, 3>(a, tm_a, tm_b, p, grid, stream)
-                     : launch_one<BN, false, false, __half, 3>(a, tm_a, tm_b, p, grid, stream);
-    return grouped ? launch_one<BN, false, true, __nv_bfloat16, 3>(a, tm_a, tm_b, p, grid, stream)
-                   : launch_one<BN, false, false, __nv_bfloat16, 3>(a, tm_a, tm_b, p, grid, stream);
+      return grouped ? launch_one<BN, false, true, __half, 3>(a, tm_a, tm_a32, tm_b, p, grid, stream)
+                     : launch_one<BN, false, false, __half, 3>(a, tm_a, tm_a32, tm_b, p, grid, stream);
+    return grouped ? launch_one<BN, false, true, __nv_bfloat16, 3>(a, tm_a, tm_a32, tm_b, p, grid, stream)
+                   : launch_one<BN, false, false, __nv_bfloat16, 3>(a, tm_a, tm_a32, tm_b, p, grid, stream);
   }
-  if (a.nt) return grouped ? launch_out<BN, true, true>(a, tm_a, tm_b, p, grid, stream)
-                           : launch_out<BN, true, false>(a, tm_a, tm_b, p, grid, stream);
-  return grouped ? launch_out<BN, false, true>(a, tm_a, tm_b, p, grid, stream)
-                 : launch_out<BN, false, false>(a, tm_a, tm_b, p, grid, stream);
+  if (a.nt) return grouped ? launch_out<BN, true, true>(a, tm_a, tm_a32, tm_b, p, grid, stream)
+                           : launch_out<BN, true, false>(a, tm_a, tm_a32, tm_b, p, grid, stream);
+  return grouped ? launch_out<BN, false, true>(a, tm_a, tm_a32, tm_b, p, grid, stream)
+                 : launch_out<BN, false, false>(a, tm_a, tm_a32, tm_b, p, grid, stream);
 }
 
 }  // namespace
@@ -1073,14 +1086,15 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
     }
   }
 
-  CUtensorMap tm_a, tm_b;
+  CUtensorMap tm_a, tm_a32, tm_b;
   // 16-bit operands (mode 3) are described to TMA as bytes: a row of A is 2K bytes, of B 2N
   const int64_t k_bytes = a.mode == 3 ? 2 * a.k : a.k;
   if (a.mode == 3) {
     const uint64_t dims[2] = {static_cast<uint64_t>(k_bytes), static_cast<uint64_t>(a.m)};
     const uint64_t str[1] = {static_cast<uint64_t>(k_bytes)};
     const uint32_t box[2] = {static_cast<uint32_t>(kBK), static_cast<uint32_t>(kBM)};
-    if (!encode_u8(&tm_a, a.a, 2, dims, str, box))
+    const uint32_t box32[2] = {static_cast<uint32_t>(kBK), 32u};
+    if (!encode_u8(&tm_a, a.a, 2, dims, str, box) || !encode_u8(&tm_a32, a.a, 2, dims, str, box32))
       KSB_FAIL(KS_ERROR_INTERNAL, std::string(a.where) + ": tensor map for A rejected");
     const uint64_t bdims[3] = {static_cast<uint64_t>(2 * a.n), static_cast<uint64_t>(a.k), static_cast<uint64_t>(experts)};
     const uint64_t bstr[2] = {static_cast<uint64_t>(2 * a.n), static_cast<uint64_t>(2 * a.n) * static_cast<uint64_t>(a.k)};
@@ -1092,7 +1106,8 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
     const uint64_t dims[2] = {static_cast<uint64_t>(a.k), static_cast<uint64_t>(a.m)};
     const uint64_t str[1] = {static_cast<uint64_t>(a.k)};
     const uint32_t box[2] = {static_cast<uint32_t>(kBK), static_cast<uint32_t>(kBM)};
-    if (!encode_u8(&tm_a, a.a, 2, dims, str, box))
+    const uint32_t box32[2] = {static_cast<uint32_t>(kBK), 32u};
+    if (!encode_u8(&tm_a, a.a, 2, dims, str, box) || !encode_u8(&tm_a32, a.a, 2, dims, str, box32))
       KSB_FAIL(KS_ERROR_INTERNAL, std::string(a.where) + ": tensor map for A rejected");
   }
   if (a.nt) {
@@ -1175,7 +1190,7 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
       }
     }
   }
-  return bn == 256 ? launch_bn<256>(a, tm_a, tm_b, p, grid, stream) : launch_bn<128>(a, tm_a, tm_b, p, grid, stream);
+  return bn == 256 ? launch_bn<256>(a, tm_a, tm_a32, tm_b, p, grid, stream) : launch_bn<128>(a, tm_a, tm_a32, tm_b, p, grid, stream);
 }
 
 }  // namespace sm100

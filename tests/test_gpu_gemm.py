@@ -827,3 +827,36 @@ def test_w4a16_dequantised_weights_to_the_bit(ks, cuda, dtype, scale_set, zero_s
     with w4_path("tcgen05"):
         out = ks.dispatch.w4a16(a.to(cuda), b_packed.to(cuda), scales.to(cuda), zeros.to(cuda), group_size=gs).cpu()
     assert torch.equal(out.float(), ref.float())
+
+
+@pytest.mark.parametrize("mode", ["dense", "grouped", "grouped16"])
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 128 + 1, 128 + 32, 128 + 33])
+def test_tiles_of_few_rows_take_a_small_box(ks, cuda, mode, rows):
+    """Up to 32 rows of a tile are loaded without the rows behind them, in whose place the MMAs then read what the
+    tile before left in shared memory: NaN, from the call before."""
+    n, k = 1296, 1280
+    a8, a_s, b8, b_s = fp8_inputs(2 * rows + 40, n, k, seed=rows)
+    b, bs = b8.t().contiguous(), b_s.t().contiguous()
+    nan8 = torch.full((512, k), 0x7f, dtype=torch.uint8, device=cuda).view(torch.float8_e4m3fn)
+    with fp8_path("tcgen05", 256):
+        ks.dispatch.fp8_gemm_blockwise(nan8, b.repeat(8, 1).to(cuda), torch.ones(512, k // 128, device=cuda),
+                                       torch.ones(-(-8 * n // 128), k // 128, device=cuda), b_layout="nk")
+        if mode == "dense":
+            out = run_fp8(ks, cuda, a8[:rows], a_s[:rows], b8, b_s, "nk")
+            ref32, noise = fp8_reference(a8[:rows], a_s[:rows], b8, b_s)
+            check_gemm(out, ref32, noise, f"{rows} rows")
+            return
+        counts = [rows, 0, 40, rows]   # rows of the next expert follow at once
+        off = torch.tensor([0, rows, rows, rows + 40, 2 * rows + 40], dtype=torch.int32)
+        if mode == "grouped":
+            out = ks.dispatch.moe(a8.to(cuda), b.expand(4, n, k).contiguous().to(cuda), off.to(cuda), n=n, k=k,
+                                  a_scale=a_s.to(cuda), b_scale=bs.expand(4, -1, -1).contiguous().to(cuda), b_layout="nk")
+            ref32, noise = fp8_reference(a8, a_s, b8, b_s)
+        else:
+            a = orc.dequantize_a(a8, a_s).to(torch.bfloat16)
+            w = orc.dequantize_b(b8, b_s).to(torch.bfloat16)
+            out = ks.dispatch.moe(a.to(cuda), w.expand(4, k, n).contiguous().to(cuda), off.to(cuda), num_experts=4, n=n, k=k)
+            ref32 = a.float() @ w.float()
+            noise = accumulation_noise(a.float().abs(), w.float().abs(), k)
+        torch.cuda.synchronize()
+        check_gemm(out.cpu(), ref32, noise, f"{mode} {counts}")
