@@ -31,6 +31,8 @@
 
 #include "common.cuh"
 #include "kernel_set/quant.h"
+#include "sm100_host.cuh"
+#include "sm100_ptx.cuh"
 
 namespace ksb {
 namespace {
@@ -217,6 +219,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 gather_columns_kernel(T* __restrict__ out, const T* __restrict__ in, const int32_t* __restrict__ perm,
                       int64_t cols) {
+  sm100::grid_dependency_wait();
   const int64_t row = blockIdx.y;
   for (int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < cols;
        j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -393,11 +396,14 @@ ks_status_t ks_gather_columns(void* out, const void* input, const int32_t* perm,
   cudaStream_t s = as_stream(stream);
   const dim3 grid(static_cast<unsigned>(std::min<int64_t>((cols + 255) / 256, 64)), static_cast<unsigned>(rows));
   if (dtype == KS_DTYPE_F32)
-    gather_columns_kernel<float><<<grid, 256, 0, s>>>(static_cast<float*>(out), static_cast<const float*>(input), perm, cols);
+    sm100::launch_programmatic(gather_columns_kernel<float>, grid, 256, 0, s,
+        static_cast<float*>(out), static_cast<const float*>(input), perm, cols);
   else if (dtype == KS_DTYPE_F16)
-    gather_columns_kernel<__half><<<grid, 256, 0, s>>>(static_cast<__half*>(out), static_cast<const __half*>(input), perm, cols);
+    sm100::launch_programmatic(gather_columns_kernel<__half>, grid, 256, 0, s,
+        static_cast<__half*>(out), static_cast<const __half*>(input), perm, cols);
   else
-    gather_columns_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(input), perm, cols);
+    sm100::launch_programmatic(gather_columns_kernel<__nv_bfloat16>, grid, 256, 0, s,
+        static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(input), perm, cols);
   KSB_CHECK_LAUNCH("ks_gather_columns");
   return KS_SUCCESS;
 }

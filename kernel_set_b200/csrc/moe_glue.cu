@@ -27,6 +27,7 @@
 #include "kernel_set/moe.h"
 #include "quant_math.cuh"
 #include "sm100_host.cuh"
+#include "sm100_ptx.cuh"
 
 namespace ksb {
 namespace {
@@ -41,6 +42,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 gate_softmax_topk_kernel(float* __restrict__ out_w, int32_t* __restrict__ out_i, const T* __restrict__ logits,
                          int64_t tokens, int experts, int top_k, int renorm) {
+  sm100::grid_start();
   extern __shared__ float gate_smem[];   // [warps][experts]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t token = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
@@ -140,6 +142,7 @@ __device__ __forceinline__ void fold_counts(int* cnt, int* sum, int experts) {
 __global__ void __launch_bounds__(kPermThreads)
 compute_permutation_kernel(int32_t* __restrict__ sorted_ids, int32_t* __restrict__ offsets,
                            const int32_t* __restrict__ topk_idx, int64_t pairs, int experts, int64_t chunk) {
+  sm100::grid_start();
   extern __shared__ int perm_smem[];       // [warps][experts] counters, then two [experts] rows
   int* cnt = perm_smem;
   int* before = perm_smem + kPermWarps * experts;   // pairs of an expert in the chunks before this one
@@ -245,6 +248,7 @@ compute_permutation_kernel(int32_t* __restrict__ sorted_ids, int32_t* __restrict
 __global__ void __launch_bounds__(256)
 permute_rows16_kernel(uint4* __restrict__ out, const uint4* __restrict__ in, const int32_t* __restrict__ ids,
                       int64_t pairs, int top_k, int64_t row_vec) {
+  sm100::grid_dependency_wait();
   const int64_t total = pairs * row_vec;
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -260,6 +264,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 permute_rows_any_kernel(T* __restrict__ out, const T* __restrict__ in, const int32_t* __restrict__ ids,
                         int64_t pairs, int top_k, int64_t hidden) {
+  sm100::grid_dependency_wait();
   const int64_t total = pairs * hidden;
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -275,6 +280,7 @@ template <typename T, bool E5M2>
 __global__ void __launch_bounds__(256)
 permute_quant_kernel(uint8_t* __restrict__ out, float* __restrict__ scale, const T* __restrict__ in,
                      const int32_t* __restrict__ ids, int64_t pairs, int top_k, int64_t hidden, float qmax) {
+  sm100::grid_start();
   const int64_t segs_per_row = hidden / 16;
   const int64_t seg = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t r = seg / segs_per_row;
@@ -300,6 +306,7 @@ permute_quant_kernel(uint8_t* __restrict__ out, float* __restrict__ scale, const
 // ---------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 inverse_permutation_kernel(int32_t* __restrict__ inverse, const int32_t* __restrict__ ids, int64_t pairs) {
+  sm100::grid_start();
   const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (r >= pairs) return;
   const int32_t pair = ids[r];
@@ -336,6 +343,7 @@ __global__ void __launch_bounds__(256)
 permute_quant_tokens_kernel(uint8_t* __restrict__ out, float* __restrict__ scale, const T* __restrict__ in,
                             const int32_t* __restrict__ ids, const int32_t* __restrict__ inverse, int64_t tokens,
                             int top_k, int64_t hidden, unsigned token_blocks, bool look_first, float qmax) {
+  sm100::grid_start();
   const int64_t segs_per_row = hidden / 16;
   const int64_t pairs = tokens * top_k;
   float v[16];
@@ -402,6 +410,7 @@ __global__ void __launch_bounds__(256)
 unpermute_vec8_kernel(T* __restrict__ out, const T* __restrict__ permuted, const int32_t* __restrict__ inverse,
                       const int32_t* __restrict__ ids,
                       const float* __restrict__ weights, int64_t tokens, int top_k, int64_t hidden) {
+  sm100::grid_dependency_wait();
   const int64_t row_vec = hidden / 8;
   const int64_t total = tokens * row_vec;
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
@@ -451,6 +460,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 unpermute_any_kernel(T* __restrict__ out, const T* __restrict__ permuted, const int32_t* __restrict__ inverse,
                      const float* __restrict__ weights, int64_t tokens, int top_k, int64_t hidden) {
+  sm100::grid_dependency_wait();
   const int64_t total = tokens * hidden;
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -476,6 +486,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 swiglu_kernel(T* __restrict__ out, const T* __restrict__ gate0, const T* __restrict__ up0, int64_t rows,
               int64_t inter, int64_t in_stride) {
+  sm100::grid_dependency_wait();
   const int64_t total = rows * inter;
   for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total;
        t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -488,6 +499,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 swiglu_vec16_kernel(T* __restrict__ out, const T* __restrict__ gate0, const T* __restrict__ up0, int64_t rows,
                     int64_t inter, int64_t in_stride) {
+  sm100::grid_dependency_wait();
   const int64_t segs_per_row = inter / 16;
   const int64_t seg = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t r = seg / segs_per_row;
@@ -511,6 +523,7 @@ template <typename T, bool E5M2>
 __global__ void __launch_bounds__(256)
 swiglu_quant_kernel(uint8_t* __restrict__ out, float* __restrict__ scale, const T* __restrict__ in, int64_t rows,
                     int64_t inter, float qmax) {
+  sm100::grid_start();
   const int64_t segs_per_row = inter / 16;
   const int64_t seg = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t r = seg / segs_per_row;
@@ -556,10 +569,11 @@ void launch_swiglu(void* out, const void* gate, const void* up, int64_t rows, in
                    aligned16(gate) && aligned16(up);
   if (vec) {
     const int64_t segs = rows * (inter / 16);
-    swiglu_vec16_kernel<T><<<static_cast<unsigned>((segs + 255) / 256), 256, 0, s>>>(
+    sm100::launch_programmatic(swiglu_vec16_kernel<T>, static_cast<unsigned>((segs + 255) / 256), 256, 0, s,
         static_cast<T*>(out), static_cast<const T*>(gate), static_cast<const T*>(up), rows, inter, stride);
   } else {
-    swiglu_kernel<T><<<grid_for(rows * inter), 256, 0, s>>>(static_cast<T*>(out), static_cast<const T*>(gate),
+    sm100::launch_programmatic(swiglu_kernel<T>, grid_for(rows * inter), 256, 0, s,
+        static_cast<T*>(out), static_cast<const T*>(gate),
                                                             static_cast<const T*>(up), rows, inter, stride);
   }
 }
@@ -604,7 +618,8 @@ ks_status_t ks_moe_gate_softmax_topk(float* out_weights, int32_t* out_indices, c
   const unsigned blocks = static_cast<unsigned>((num_tokens + warps - 1) / warps);
   const size_t smem = static_cast<size_t>(warps) * num_experts * sizeof(float);
 #define KSB_GATE(T)                                                                                          \
-  gate_softmax_topk_kernel<T><<<blocks, warps * 32, smem, s>>>(out_weights, out_indices,                     \
+  sm100::launch_programmatic(gate_softmax_topk_kernel<T>, blocks, warps * 32, smem, s, \
+      out_weights, out_indices, \
                                                                static_cast<const T*>(logits), num_tokens,   \
                                                                num_experts, top_k, renormalize)
   if (dtype == KS_DTYPE_F32) KSB_GATE(float);
@@ -653,7 +668,8 @@ ks_status_t ks_moe_compute_permutation(int32_t* sorted_token_ids, int32_t* exper
       attr_done[dev] = true;
     }
   }
-  compute_permutation_kernel<<<ctas, kPermThreads, smem, s>>>(sorted_token_ids, expert_offsets, topk_indices, pairs,
+  sm100::launch_programmatic(compute_permutation_kernel, ctas, kPermThreads, smem, s,
+      sorted_token_ids, expert_offsets, topk_indices, pairs,
                                                               num_experts, chunk);
   KSB_CHECK_LAUNCH(where);
   return KS_SUCCESS;
@@ -678,16 +694,16 @@ ks_status_t ks_moe_permute(void* permuted, const void* input, const int32_t* sor
   const int64_t row_bytes = hidden * elt;
   if (row_bytes % 16 == 0 && aligned16(permuted) && aligned16(input)) {
     const int64_t row_vec = row_bytes / 16;
-    permute_rows16_kernel<<<grid_for(pairs * row_vec), 256, 0, s>>>(
+    sm100::launch_programmatic(permute_rows16_kernel, grid_for(pairs * row_vec), 256, 0, s,
         static_cast<uint4*>(permuted), static_cast<const uint4*>(input), sorted_token_ids, pairs, top_k, row_vec);
   } else if (elt == 4) {
-    permute_rows_any_kernel<float><<<grid_for(pairs * hidden), 256, 0, s>>>(
+    sm100::launch_programmatic(permute_rows_any_kernel<float>, grid_for(pairs * hidden), 256, 0, s,
         static_cast<float*>(permuted), static_cast<const float*>(input), sorted_token_ids, pairs, top_k, hidden);
   } else if (elt == 2) {
-    permute_rows_any_kernel<__half><<<grid_for(pairs * hidden), 256, 0, s>>>(
+    sm100::launch_programmatic(permute_rows_any_kernel<__half>, grid_for(pairs * hidden), 256, 0, s,
         static_cast<__half*>(permuted), static_cast<const __half*>(input), sorted_token_ids, pairs, top_k, hidden);
   } else {
-    permute_rows_any_kernel<__nv_fp8_e4m3><<<grid_for(pairs * hidden), 256, 0, s>>>(
+    sm100::launch_programmatic(permute_rows_any_kernel<__nv_fp8_e4m3>, grid_for(pairs * hidden), 256, 0, s,
         static_cast<__nv_fp8_e4m3*>(permuted), static_cast<const __nv_fp8_e4m3*>(input), sorted_token_ids, pairs,
         top_k, hidden);
   }
@@ -743,11 +759,13 @@ ks_status_t ks_moe_permute_quant_fp8(void* out_fp8, float* out_scale, const void
                            ? nullptr
                            : static_cast<int32_t*>(scratch.get(static_cast<size_t>(pairs) * sizeof(int32_t), 4));
     if (inverse != nullptr) {
-      inverse_permutation_kernel<<<static_cast<unsigned>((pairs + 255) / 256), 256, 0, s>>>(inverse, sorted_token_ids, pairs);
+      sm100::launch_programmatic(inverse_permutation_kernel, static_cast<unsigned>((pairs + 255) / 256), 256, 0, s,
+          inverse, sorted_token_ids, pairs);
       const unsigned token_blocks = static_cast<unsigned>((num_tokens * (hidden / 16) + 255) / 256);
       const unsigned total_blocks = token_blocks + static_cast<unsigned>((pairs + 7) / 8);
 #define KSB_PT(T, E5, QMAX)                                                                                      \
-  permute_quant_tokens_kernel<T, E5><<<total_blocks, 256, 0, s>>>(o, out_scale, static_cast<const T*>(input),    \
+  sm100::launch_programmatic(permute_quant_tokens_kernel<T, E5>, total_blocks, 256, 0, s, \
+      o, out_scale, static_cast<const T*>(input), \
                                                                   sorted_token_ids, inverse, num_tokens, top_k,  \
                                                                   hidden, token_blocks, top_k < 4, QMAX)
       if (in_dtype == KS_DTYPE_F32) { if (e5) KSB_PT(float, true, 57344.0f); else KSB_PT(float, false, 448.0f); }
@@ -760,9 +778,11 @@ ks_status_t ks_moe_permute_quant_fp8(void* out_fp8, float* out_scale, const void
   }
 #define KSB_PQ(T)                                                                                               \
   do {                                                                                                          \
-    if (e5) permute_quant_kernel<T, true><<<blocks, 256, 0, s>>>(o, out_scale, static_cast<const T*>(input),   \
+    if (e5) sm100::launch_programmatic(permute_quant_kernel<T, true>, blocks, 256, 0, s, \
+        o, out_scale, static_cast<const T*>(input), \
                                                                  sorted_token_ids, pairs, top_k, hidden, 57344.0f); \
-    else permute_quant_kernel<T, false><<<blocks, 256, 0, s>>>(o, out_scale, static_cast<const T*>(input),     \
+    else sm100::launch_programmatic(permute_quant_kernel<T, false>, blocks, 256, 0, s, \
+        o, out_scale, static_cast<const T*>(input), \
                                                                sorted_token_ids, pairs, top_k, hidden, 448.0f); \
   } while (0)
   if (in_dtype == KS_DTYPE_F32) KSB_PQ(float);
@@ -801,17 +821,20 @@ ks_status_t ks_moe_unpermute(void* out, const void* permuted, const int32_t* sor
     const cudaError_t e = cudaMemsetAsync(inverse, 0xFF, static_cast<size_t>(pairs) * sizeof(int32_t), s);
     if (e != cudaSuccess) return cuda_status(e, where);
   }
-  inverse_permutation_kernel<<<static_cast<unsigned>((pairs + 255) / 256), 256, 0, s>>>(inverse, sorted_token_ids, pairs);
+  sm100::launch_programmatic(inverse_permutation_kernel, static_cast<unsigned>((pairs + 255) / 256), 256, 0, s,
+      inverse, sorted_token_ids, pairs);
 #define KSB_UNPERMUTE(T)                                                                                           \
   do {                                                                                                             \
     T* o = static_cast<T*>(out);                                                                                   \
     const T* x = static_cast<const T*>(permuted);                                                                  \
-    if (vec) unpermute_vec8_kernel<T><<<grid_for(num_tokens * (hidden / 8)), 256, 0, s>>>(                         \
+    if (vec) sm100::launch_programmatic(unpermute_vec8_kernel<T>, grid_for(num_tokens * (hidden / 8)), 256, 0, s, \
         o, x, inverse, sorted_token_ids, routing_weights, num_tokens, top_k, hidden);                              \
-    else unpermute_any_kernel<T><<<grid_for(num_tokens * hidden), 256, 0, s>>>(o, x, inverse, routing_weights,     \
+    else sm100::launch_programmatic(unpermute_any_kernel<T>, grid_for(num_tokens * hidden), 256, 0, s, \
+        o, x, inverse, routing_weights, \
                                                                                num_tokens, top_k, hidden);         \
   } while (0)
-  if (dtype == KS_DTYPE_F32) unpermute_any_kernel<float><<<grid_for(num_tokens * hidden), 256, 0, s>>>(
+  if (dtype == KS_DTYPE_F32) sm100::launch_programmatic(unpermute_any_kernel<float>,
+      grid_for(num_tokens * hidden), 256, 0, s,
       static_cast<float*>(out), static_cast<const float*>(permuted), inverse, routing_weights, num_tokens, top_k, hidden);
   else if (dtype == KS_DTYPE_F16) KSB_UNPERMUTE(__half);
   else KSB_UNPERMUTE(__nv_bfloat16);
@@ -864,9 +887,11 @@ ks_status_t ks_swiglu_packed_quant_fp8(void* out_fp8, float* out_scale, const vo
   uint8_t* o = static_cast<uint8_t*>(out_fp8);
 #define KSB_SQ(T)                                                                                                    \
   do {                                                                                                               \
-    if (e5) swiglu_quant_kernel<T, true><<<blocks, 256, 0, s>>>(o, out_scale, static_cast<const T*>(input), rows,   \
+    if (e5) sm100::launch_programmatic(swiglu_quant_kernel<T, true>, blocks, 256, 0, s, \
+        o, out_scale, static_cast<const T*>(input), rows, \
                                                                 inter, 57344.0f);                                    \
-    else swiglu_quant_kernel<T, false><<<blocks, 256, 0, s>>>(o, out_scale, static_cast<const T*>(input), rows,     \
+    else sm100::launch_programmatic(swiglu_quant_kernel<T, false>, blocks, 256, 0, s, \
+        o, out_scale, static_cast<const T*>(input), rows, \
                                                               inter, 448.0f);                                        \
   } while (0)
   if (in_dtype == KS_DTYPE_F16) KSB_SQ(__half);

@@ -19,6 +19,8 @@
 #include "common.cuh"
 #include "kernel_set/norm.h"
 #include "quant_math.cuh"
+#include "sm100_host.cuh"
+#include "sm100_ptx.cuh"
 
 namespace ksb {
 namespace {
@@ -42,6 +44,8 @@ template <typename T, bool QUANT, bool E5M2>
 __global__ void __launch_bounds__(kNormThreads)
 rms_norm_rows_kernel(void* __restrict__ out, float* __restrict__ scale, const T* __restrict__ in,
                      const T* __restrict__ weight, int64_t cols, float eps, float qmax) {
+  if constexpr (QUANT) sm100::grid_launch_dependents();
+  sm100::grid_dependency_wait();
   const int64_t row = blockIdx.x;
   const int segs = static_cast<int>(cols / 16);
   const T* x = in + row * cols;
@@ -101,6 +105,7 @@ template <typename T>
 __global__ void __launch_bounds__(kNormThreads)
 rms_norm_any_kernel(T* __restrict__ out, const T* __restrict__ in, const T* __restrict__ weight, int64_t cols,
                     float eps) {
+  sm100::grid_dependency_wait();
   const int64_t row = blockIdx.x;
   const T* x = in + row * cols;
   float sumsq = 0.f;
@@ -141,9 +146,10 @@ extern "C" ks_status_t ks_rms_norm(void* out, const void* input, const void* wei
   const bool fast = rows_kernel_fits(cols, out, input, weight);
 #define KSB_RN(T)                                                                                               \
   do {                                                                                                          \
-    if (fast) rms_norm_rows_kernel<T, false, false><<<grid, kNormThreads, 0, s>>>(                              \
+    if (fast) sm100::launch_programmatic(rms_norm_rows_kernel<T, false, false>, grid, kNormThreads, 0, s, \
         out, nullptr, static_cast<const T*>(input), static_cast<const T*>(weight), cols, eps, 0.f);             \
-    else rms_norm_any_kernel<T><<<grid, kNormThreads, 0, s>>>(static_cast<T*>(out), static_cast<const T*>(input), \
+    else sm100::launch_programmatic(rms_norm_any_kernel<T>, grid, kNormThreads, 0, s, \
+        static_cast<T*>(out), static_cast<const T*>(input), \
                                                               static_cast<const T*>(weight), cols, eps);        \
   } while (0)
   if (dtype == KS_DTYPE_F32) KSB_RN(float);
@@ -178,9 +184,9 @@ extern "C" ks_status_t ks_rms_norm_quant_fp8(void* out_fp8, float* out_scale, co
   const bool e5 = fp8_dtype == KS_DTYPE_F8E5M2;
 #define KSB_RQ(T)                                                                                                 \
   do {                                                                                                            \
-    if (e5) rms_norm_rows_kernel<T, true, true><<<grid, kNormThreads, 0, s>>>(                                    \
+    if (e5) sm100::launch_programmatic(rms_norm_rows_kernel<T, true, true>, grid, kNormThreads, 0, s, \
         out_fp8, out_scale, static_cast<const T*>(input), static_cast<const T*>(weight), cols, eps, 57344.0f);    \
-    else rms_norm_rows_kernel<T, true, false><<<grid, kNormThreads, 0, s>>>(                                      \
+    else sm100::launch_programmatic(rms_norm_rows_kernel<T, true, false>, grid, kNormThreads, 0, s, \
         out_fp8, out_scale, static_cast<const T*>(input), static_cast<const T*>(weight), cols, eps, 448.0f);      \
   } while (0)
   if (in_dtype == KS_DTYPE_F16) KSB_RQ(__half);

@@ -20,6 +20,8 @@
 #include "common.cuh"
 #include "kernel_set/quant.h"
 #include "quant_math.cuh"
+#include "sm100_host.cuh"
+#include "sm100_ptx.cuh"
 
 #ifndef KSB_QUANT_SEGS
 #define KSB_QUANT_SEGS 1
@@ -39,6 +41,7 @@ template <typename T, bool E5M2>
 __global__ void __launch_bounds__(256)
 quant_group128_colscale_kernel(uint8_t* __restrict__ out, float* __restrict__ scale_t, int64_t ld,
                                const T* __restrict__ in, int64_t total_groups, int groups_per_row, float qmax) {
+  sm100::grid_start();
   const int64_t seg = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool live = (seg >> 3) < total_groups;
   float v[16];
@@ -63,6 +66,7 @@ template <typename T, bool E5M2, int kSegs>
 __global__ void __launch_bounds__(256)
 quant_group128_kernel(uint8_t* __restrict__ out, float* __restrict__ scale,
                       const T* __restrict__ in, int64_t total_groups, float qmax) {
+  sm100::grid_start();
   // a block owns kSegs consecutive runs of 256 segments (contiguous in memory)
   const int64_t stride = blockDim.x;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x * kSegs + threadIdx.x;
@@ -91,6 +95,7 @@ template <typename T, bool E5M2>
 __global__ void __launch_bounds__(256)
 quant_group128_ragged_kernel(uint8_t* __restrict__ out, float* __restrict__ scale, const T* __restrict__ in,
                              int64_t rows, int64_t cols, int64_t segs_per_row, float qmax) {
+  sm100::grid_start();
   const int64_t seg = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t row = seg / segs_per_row;
   const int64_t c = (seg - row * segs_per_row) * 16;
@@ -115,6 +120,7 @@ __global__ void __launch_bounds__(256)
 quant_group_any_kernel(uint8_t* __restrict__ out, float* __restrict__ scale,
                        const T* __restrict__ in, int64_t rows, int64_t cols, int group_size,
                        int64_t groups_per_row, float qmax) {
+  sm100::grid_start();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   if (warp >= rows * groups_per_row) return;  // whole warp leaves together
@@ -147,16 +153,18 @@ void launch(uint8_t* out, float* scale, const T* in, int64_t rows, int64_t cols,
     // shared-memory ring, ~190 KB in flight per SM: 5.4 TB/s on [16384, 7168] where this kernel
     // reaches 5.6, and slower on [4096, 7168]. At that size a fixed ~5 us of launch, ramp and
     // tail is what separates the kernel from its steady-state rate.)
-    quant_group128_kernel<T, E5M2, kSegs><<<static_cast<unsigned>(blocks), 256, 0, s>>>(out, scale, in, total_groups, qmax);
+    sm100::launch_programmatic(quant_group128_kernel<T, E5M2, kSegs>, static_cast<unsigned>(blocks), 256, 0, s,
+        out, scale, in, total_groups, qmax);
   } else if (gs == 128 && cols % 16 == 0 && aligned16(in) && aligned16(out)) {
     const int64_t segs_per_row = groups_per_row * 8;
     const int64_t blocks = (rows * segs_per_row + 255) / 256;
-    quant_group128_ragged_kernel<T, E5M2><<<static_cast<unsigned>(blocks), 256, 0, s>>>(out, scale, in, rows, cols,
+    sm100::launch_programmatic(quant_group128_ragged_kernel<T, E5M2>, static_cast<unsigned>(blocks), 256, 0, s,
+        out, scale, in, rows, cols,
                                                                                         segs_per_row, qmax);
   } else {
     const int64_t warps = rows * groups_per_row;
     const int64_t blocks = (warps + 7) / 8;
-    quant_group_any_kernel<T, E5M2><<<static_cast<unsigned>(blocks), 256, 0, s>>>(
+    sm100::launch_programmatic(quant_group_any_kernel<T, E5M2>, static_cast<unsigned>(blocks), 256, 0, s,
         out, scale, in, rows, cols, gs, groups_per_row, qmax);
   }
 }
@@ -229,9 +237,11 @@ extern "C" ks_status_t ks_quantize_fp8_group_colscale(void* out, float* scale_t,
   const bool e5 = fp8_dtype == KS_DTYPE_F8E5M2;
 #define KSB_QC(T)                                                                                                   \
   do {                                                                                                              \
-    if (e5) quant_group128_colscale_kernel<T, true><<<blocks, 256, 0, s>>>(o, scale_t, scale_ld, static_cast<const T*>(input), \
+    if (e5) sm100::launch_programmatic(quant_group128_colscale_kernel<T, true>, blocks, 256, 0, s, \
+        o, scale_t, scale_ld, static_cast<const T*>(input), \
                                                                            total_groups, static_cast<int>(groups_per_row), 57344.0f); \
-    else quant_group128_colscale_kernel<T, false><<<blocks, 256, 0, s>>>(o, scale_t, scale_ld, static_cast<const T*>(input),  \
+    else sm100::launch_programmatic(quant_group128_colscale_kernel<T, false>, blocks, 256, 0, s, \
+        o, scale_t, scale_ld, static_cast<const T*>(input), \
                                                                          total_groups, static_cast<int>(groups_per_row), 448.0f);  \
   } while (0)
   if (in_dtype == KS_DTYPE_F32) KSB_QC(float);

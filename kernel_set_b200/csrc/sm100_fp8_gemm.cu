@@ -350,6 +350,7 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), C::kTmemCols);
     tmem_relinquish();
   }
+  grid_dependency_wait();   // nothing before this touches memory that the kernel before may still write or read
   if constexpr (GROUPED) {
     // offs[e] = first row of expert e; with the masked layout the rows of an expert end at
     // offs[e] + masked_m[e] instead of at offs[e + 1] (ends[] holds either)
@@ -870,6 +871,7 @@ __global__ void __launch_bounds__(256)
 split_reduce_kernel(OutT* __restrict__ out, const float4* __restrict__ slots, int split_from, int split_s, int tails,
                     int tiles_m, int tiles_n, int m, int n, int vec_ok) {
   using C = Cfg<BN>;
+  grid_start();
   constexpr int EC = C::kEpiCols;
   constexpr int kChunks = EC / 4;
   constexpr int kPerTile = C::kEpiWarps * kChunks * 32;   // float4 per (tile, part)
@@ -923,30 +925,21 @@ ks_status_t launch_one(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUte
   }
   if (a.num_out_parts > 0 && !p.vec_store)
     KSB_FAIL(KS_ERROR_UNSUPPORTED_SHAPE, std::string(a.where) + ": the scattered output needs 16-byte aligned rows and parts");
-  // (Programmatic dependent launch was measured on the quantizer -> GEMM -> reducer chain and
-  // lost 1 % there: these kernels have no input-independent prologue worth overlapping, and
-  // the dependency wait costs more than an ordinary kernel boundary.)
-  if (p.cluster_s > 1) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(C::kThreads);
-    cfg.dynamicSmemBytes = C::smem_bytes(GROUPED);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = p.cluster_s;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, tm_a, tm_a32, tm_b, p), a.where);
-  }
-  kernel<<<grid, C::kThreads, C::smem_bytes(GROUPED), stream>>>(tm_a, tm_a32, tm_b, p);
+  // A short problem is set up under the tail of the kernel before it (the quantizer, a gather), which saves 2-3 us:
+  // M=2500, N=2000, K=4096 behind the quantizer 44.0 -> 40.8 us, 48 tokens over 64 experts 249 -> 240, M=4096,
+  // N=K=7168 behind the norm 248 -> 245 (339 K-blocks per CTA). A long one loses 1 % that way (M=16384, N=8192, K=3584,
+  // 775 K-blocks: 600 -> 609), so from 512 on it is launched the ordinary way. The GEMM does not let
+  // its own successor begin early: with that the same four took 42.7, 245, 252 and 614.
+  const int64_t tiles = p.tiles_n * (GROUPED ? (a.m + kBM - 1) / kBM + p.num_experts : static_cast<int64_t>(p.tiles_m));
+  const bool is_short = tiles * p.nkb <= 512 * static_cast<int64_t>(sm_count());
+  const cudaError_t e = launch_programmatic_cluster(kernel, grid, p.cluster_s, is_short, C::kThreads,
+                                                    C::smem_bytes(GROUPED), stream, tm_a, tm_a32, tm_b, p);
+  if (e != cudaSuccess) return cuda_status(e, a.where);
   if constexpr (!GROUPED) {
-    if (p.split_s > 1) {
+    if (p.split_s > 1 && p.cluster_s == 1) {   // (a cluster adds its parts up itself and has no slots)
       const int tails = p.split_items / p.split_s;
       const int work = tails * C::kEpiWarps * (C::kEpiCols / 4) * 32;
-      split_reduce_kernel<BN, OutT><<<(work + 255) / 256, 256, 0, stream>>>(
+      launch_programmatic(split_reduce_kernel<BN, OutT>, (work + 255) / 256, 256, 0, stream,
           static_cast<OutT*>(p.out), p.split_slots, p.split_from, p.split_s, tails, p.tiles_m, p.tiles_n, p.m, p.n,
           p.vec_store);
     }

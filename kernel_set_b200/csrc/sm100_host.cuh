@@ -70,10 +70,10 @@ void stream_scratch_release(cudaStream_t stream);
 bool programmatic_launch_enabled();
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_programmatic(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
+inline cudaError_t launch_programmatic(void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t smem,
                                        cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -85,9 +85,9 @@ inline cudaError_t launch_programmatic(void (*kernel)(KArgs...), unsigned grid, 
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// The same with the grid cut into clusters of `cluster` CTAs (1: no clusters).
+// The same with the grid cut into clusters of `cluster` CTAs (1: no clusters), and the ordinary way unless `programmatic`.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_programmatic_cluster(void (*kernel)(KArgs...), unsigned grid, unsigned cluster,
+inline cudaError_t launch_programmatic_cluster(void (*kernel)(KArgs...), unsigned grid, unsigned cluster, bool programmatic,
                                                unsigned block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
@@ -103,7 +103,7 @@ inline cudaError_t launch_programmatic_cluster(void (*kernel)(KArgs...), unsigne
     attr[n].val.clusterDim.z = 1;
     ++n;
   }
-  if (programmatic_launch_enabled()) {
+  if (programmatic && programmatic_launch_enabled()) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n].val.programmaticStreamSerializationAllowed = 1;
     ++n;

@@ -825,7 +825,7 @@ ks_status_t launch_t(const CUtensorMap& tm_w, const CUtensorMap& tm_a, const Par
       attr_done[dev] = true;
     }
   }
-  return cuda_status(launch_programmatic_cluster(kernel, static_cast<unsigned>(grid), static_cast<unsigned>(p.cluster_s),
+  return cuda_status(launch_programmatic_cluster(kernel, static_cast<unsigned>(grid), static_cast<unsigned>(p.cluster_s), true,
                                                  C::kThreads, C::kSmemBytes, stream, tm_w, tm_a, p),
                      "ks_gemm_w4a16");
 }

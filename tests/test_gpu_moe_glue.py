@@ -438,3 +438,60 @@ def test_host_threads_share_a_stream(ks, cuda):
     for t in range(2):
         for i, (p, o) in enumerate(zip(problems[t], outs[t])):
             assert torch.equal(o.cpu().long(), p[2]), (t, i)
+
+
+@pytest.mark.parametrize("tokens", [1, 40, 700])
+def test_kernels_that_begin_early_wait_for_each_other(ks, cuda, tokens):
+    """A layer's steps on buffers that every pass overwrites, queued back to back, against the same steps with the
+    device drained after each: a kernel that read or wrote before the one before it was done would show."""
+    hidden, inter, experts, top_k = 1024, 512, 16, 4
+    rows = tokens * top_k
+    g = torch.Generator(device=cuda).manual_seed(tokens)
+    e = lambda *shape, **kw: torch.empty(*shape, device=cuda, **kw)
+    w1 = torch.randint(0, 120, (experts, 2 * inter, hidden), generator=g, device=cuda, dtype=torch.uint8).view(torch.float8_e4m3fn)
+    w2 = torch.randint(0, 120, (experts, hidden, inter), generator=g, device=cuda, dtype=torch.uint8).view(torch.float8_e4m3fn)
+    s1 = torch.rand(experts, 2 * inter // 128, hidden // 128, generator=g, device=cuda) * 1e-3
+    s2 = torch.rand(experts, hidden // 128, inter // 128, generator=g, device=cuda) * 1e-3
+    codes = torch.randint(0, 256, (hidden // 2, hidden), generator=g, device=cuda, dtype=torch.uint8)
+    scales = (torch.rand(hidden // 128, hidden, generator=g, device=cuda) * 0.02).bfloat16()
+    perm = torch.randperm(hidden, generator=g, device=cuda).to(torch.int32)
+    gamma = torch.ones(hidden, device=cuda, dtype=torch.bfloat16)
+    inputs = [(torch.randn(tokens, hidden, generator=g, device=cuda).bfloat16(),
+               torch.randn(tokens, experts, generator=g, device=cuda)) for _ in range(6)]
+    x8, xs = e(tokens, hidden, dtype=torch.float8_e4m3fn), e(tokens, hidden // 128)
+    wts, ids = e(tokens, top_k), e(tokens, top_k, dtype=torch.int32)
+    order, off = e(rows, dtype=torch.int32), e(experts + 1, dtype=torch.int32)
+    p8, ps = e(rows, hidden, dtype=torch.float8_e4m3fn), e(rows, hidden // 128)
+    h, y = e(rows, 2 * inter, dtype=torch.bfloat16), e(rows, hidden, dtype=torch.bfloat16)
+    a8, as_ = e(rows, inter, dtype=torch.float8_e4m3fn), e(rows, inter // 128)
+    z, gx, o = (e(tokens, hidden, dtype=torch.bfloat16) for _ in range(3))
+
+    def layer(x, logits, after):
+        outs = []
+        steps = [
+            lambda: ks.int4.gather_columns(gx, x, perm, tokens, hidden),
+            lambda: ks.gemm.gemm_w4a16(z, gx, codes, scales, None, tokens, hidden, hidden, group_size=128),
+            lambda: ks.norm.rms_norm_quant_fp8(x8, xs, z, gamma),
+            lambda: ks.gemm.gemm_fp8_blockwise(z, x8, w1[0, :, :].view(2 * inter, hidden), xs, s1[0], tokens, 2 * inter, hidden,
+                                               b_layout="nk"),
+            lambda: ks.moe.gate_softmax_topk(wts, ids, logits, tokens, experts, top_k),
+            lambda: ks.moe.compute_permutation(order, off, ids, tokens, experts, top_k),
+            lambda: ks.moe.permute_quant_fp8(p8, ps, z, order, tokens, top_k, hidden),
+            lambda: ks.moe.grouped_gemm_fp8_blockwise(h, p8, w1, ps, s1, off, experts, rows, 2 * inter, hidden),
+            lambda: ks.activation.swiglu_packed_quant_fp8(a8, as_, h, rows, inter),
+            lambda: ks.moe.grouped_gemm_fp8_blockwise(y, a8, w2, as_, s2, off, experts, rows, hidden, inter),
+            lambda: ks.moe.unpermute(o, y, order, wts, tokens, top_k, hidden),
+        ]
+        for step in steps:
+            step()
+            after()
+        outs.append(o.clone())
+        return outs
+
+    drained = [layer(x, lg, torch.cuda.synchronize)[0] for x, lg in inputs]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        queued = [layer(x, lg, lambda: None)[0] for x, lg in inputs]
+        torch.cuda.synchronize()
+        for a, b in zip(queued, drained):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))
