@@ -11,9 +11,12 @@
 // scales are bit-identical to the two calls run one after the other, without the 16-bit
 // intermediate ever reaching memory (the row is read once and kept in registers).
 //
-// One CTA of 128 threads per row; a thread owns the 16-element segments t, t + 128, ... of the
-// row (up to four: rows of at most 8192 elements), so eight consecutive lanes hold the eight
-// segments of a quantisation group, the arrangement quant_segment_codes expects.
+// A CTA per row, a thread owns one or two 16-element segments of it (rows of at most 8192 elements), so eight
+// consecutive lanes hold the eight segments of a quantisation group, the arrangement quant_segment_codes
+// expects. Issue-bound rather than memory-bound, so the work is laid out to leave no lane idle (7168 elements
+// are 224 threads x 2; with 128 threads x 4 an eighth of the lanes worked on nothing) and the
+// products with the weight are taken two to an instruction: the normalised values and the weight are 16-bit,
+// their product is exact in fp32, so the packed multiplication rounds once, as the scalar one did.
 #include <string>
 
 #include "common.cuh"
@@ -27,21 +30,55 @@ namespace {
 
 using namespace quantmath;
 
-constexpr int kNormThreads = 128;
-constexpr int kMaxSegsPerThread = 4;
+constexpr int kNormThreads = 128;      // of the kernel for any width
+constexpr int kMaxRowThreads = 256;
+constexpr int kMaxSegs = 2;            // per thread
 
-__device__ __forceinline__ float block_sum_128(float v) {
-  __shared__ float red[kNormThreads / 32];
+__device__ __forceinline__ float block_sum(float v) {
+  __shared__ float red[kMaxRowThreads / 32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  return (red[0] + red[1]) + (red[2] + red[3]);
+  float sum = 0.f;
+  for (unsigned w = 0; w < blockDim.x / 32; ++w) sum += red[w];
+  return sum;
+}
+
+// y = (v * inv).to(T) * w, rounded to T: 16 elements. f32 needs no rounding in between.
+__device__ __forceinline__ void scale_row(float (&v)[16], float inv, const Raw16<float>& w, uint4 (&y)[4]) {
+  float g[16];
+  w.unpack(g);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = (v[j] * inv) * g[j];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    y[q] = make_uint4(__float_as_uint(v[4 * q]), __float_as_uint(v[4 * q + 1]), __float_as_uint(v[4 * q + 2]),
+                      __float_as_uint(v[4 * q + 3]));
+}
+template <typename T>
+__device__ __forceinline__ void scale_row(float (&v)[16], float inv, const Raw16<T>& w, uint4 (&y)[2]) {
+  const uint32_t g[8] = {w.a.x, w.a.y, w.a.z, w.a.w, w.b.x, w.b.y, w.b.z, w.b.w};
+  uint32_t o[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if constexpr (__is_same(T, __half)) {
+      const __half2 n = __floats2half2_rn(v[2 * j] * inv, v[2 * j + 1] * inv);
+      const __half2 p = __hmul2_rn(n, *reinterpret_cast<const __half2*>(&g[j]));
+      o[j] = *reinterpret_cast<const uint32_t*>(&p);
+    } else {
+      const __nv_bfloat162 n = __floats2bfloat162_rn(v[2 * j] * inv, v[2 * j + 1] * inv);
+      const __nv_bfloat162 p = __hmul2_rn(n, *reinterpret_cast<const __nv_bfloat162*>(&g[j]));
+      o[j] = *reinterpret_cast<const uint32_t*>(&p);
+    }
+  }
+  y[0] = make_uint4(o[0], o[1], o[2], o[3]);
+  y[1] = make_uint4(o[4], o[5], o[6], o[7]);
 }
 
 // QUANT == false: out is T [rows, cols]. QUANT == true: out is fp8 [rows, cols], scale [rows, cols / 128].
 template <typename T, bool QUANT, bool E5M2>
-__global__ void __launch_bounds__(kNormThreads)
+__global__ void __launch_bounds__(kMaxRowThreads)
 rms_norm_rows_kernel(void* __restrict__ out, float* __restrict__ scale, const T* __restrict__ in,
                      const T* __restrict__ weight, int64_t cols, float eps, float qmax) {
   if constexpr (QUANT) sm100::grid_launch_dependents();
@@ -49,42 +86,36 @@ rms_norm_rows_kernel(void* __restrict__ out, float* __restrict__ scale, const T*
   const int64_t row = blockIdx.x;
   const int segs = static_cast<int>(cols / 16);
   const T* x = in + row * cols;
-  Raw16<T> raw[kMaxSegsPerThread];
+  Raw16<T> raw[kMaxSegs];
   float sumsq = 0.f;
 #pragma unroll
-  for (int i = 0; i < kMaxSegsPerThread; ++i) {
-    const int seg = threadIdx.x + i * kNormThreads;
-    if (seg < segs) {
-      raw[i] = Raw16<T>::load(x + seg * 16);
-      float v[16];
-      raw[i].unpack(v);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) sumsq = fmaf(v[j], v[j], sumsq);
-    } else {
-      raw[i] = Raw16<T>::zero();
-    }
+  for (int i = 0; i < kMaxSegs; ++i) {
+    const int seg = threadIdx.x + i * blockDim.x;
+    raw[i] = seg < segs ? Raw16<T>::load(x + seg * 16) : Raw16<T>::zero();
   }
-  sumsq = block_sum_128(sumsq);
+#pragma unroll
+  for (int i = 0; i < kMaxSegs; ++i) {
+    float v[16];
+    raw[i].unpack(v);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) sumsq = fmaf(v[j], v[j], sumsq);
+  }
+  sumsq = block_sum(sumsq);
   const float inv_rms = rsqrtf(sumsq / static_cast<float>(cols) + eps);
 #pragma unroll
-  for (int i = 0; i < kMaxSegsPerThread; ++i) {
-    if (i * kNormThreads >= segs) break;   // uniform over the CTA
-    const int seg = threadIdx.x + i * kNormThreads;
+  for (int i = 0; i < kMaxSegs; ++i) {
+    const int seg = threadIdx.x + i * blockDim.x;
     const bool live = seg < segs;
-    float v[16], w[16];
+    if (!__any_sync(0xffffffffu, live)) break;
+    float v[16];
     raw[i].unpack(v);
-    if (live) {
-      Raw16<T>::load(weight + seg * 16).unpack(w);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) w[j] = 0.f;
-    }
-    T y[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) y[j] = from_f32<T>(to_f32<T>(from_f32<T>(v[j] * inv_rms)) * w[j]);
+    uint4 y[sizeof(T)];
+    scale_row(v, inv_rms, live ? Raw16<T>::load(weight + seg * 16) : Raw16<T>::zero(), y);
     if constexpr (QUANT) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = to_f32<T>(y[j]);
+      Raw16<T> r;
+      r.a = y[0];
+      r.b = y[1];
+      r.unpack(v);
       float sc;
       const uint4 codes = quant_segment_codes<E5M2>(v, qmax, &sc);
       if (live) {
@@ -93,9 +124,8 @@ rms_norm_rows_kernel(void* __restrict__ out, float* __restrict__ scale, const T*
       }
     } else if (live) {
       uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(out) + row * cols + seg * 16);
-      const uint4* src = reinterpret_cast<const uint4*>(y);
 #pragma unroll
-      for (int q = 0; q < static_cast<int>(sizeof(T)) * 16 / 16; ++q) dst[q] = src[q];
+      for (int q = 0; q < static_cast<int>(sizeof(T)); ++q) dst[q] = y[q];
     }
   }
 }
@@ -113,14 +143,17 @@ rms_norm_any_kernel(T* __restrict__ out, const T* __restrict__ in, const T* __re
     const float v = to_f32<T>(x[c]);
     sumsq = fmaf(v, v, sumsq);
   }
-  sumsq = block_sum_128(sumsq);
+  sumsq = block_sum(sumsq);
   const float inv_rms = rsqrtf(sumsq / static_cast<float>(cols) + eps);
   for (int64_t c = threadIdx.x; c < cols; c += kNormThreads)
     out[row * cols + c] = from_f32<T>(to_f32<T>(from_f32<T>(to_f32<T>(x[c]) * inv_rms)) * to_f32<T>(weight[c]));
 }
 
+// Threads for a row: two segments to a thread, in whole warps.
+unsigned row_threads(int64_t cols) { return static_cast<unsigned>((cols / 16 + 63) / 64 * 32); }
+
 bool rows_kernel_fits(int64_t cols, const void* a, const void* b, const void* c) {
-  return cols % 128 == 0 && cols <= 16 * kNormThreads * kMaxSegsPerThread && aligned16(a) && aligned16(b) &&
+  return cols % 128 == 0 && cols <= 16 * kMaxRowThreads * kMaxSegs && aligned16(a) && aligned16(b) &&
          aligned16(c);
 }
 
@@ -146,7 +179,7 @@ extern "C" ks_status_t ks_rms_norm(void* out, const void* input, const void* wei
   const bool fast = rows_kernel_fits(cols, out, input, weight);
 #define KSB_RN(T)                                                                                               \
   do {                                                                                                          \
-    if (fast) sm100::launch_programmatic(rms_norm_rows_kernel<T, false, false>, grid, kNormThreads, 0, s, \
+    if (fast) sm100::launch_programmatic(rms_norm_rows_kernel<T, false, false>, grid, row_threads(cols), 0, s, \
         out, nullptr, static_cast<const T*>(input), static_cast<const T*>(weight), cols, eps, 0.f);             \
     else sm100::launch_programmatic(rms_norm_any_kernel<T>, grid, kNormThreads, 0, s, \
         static_cast<T*>(out), static_cast<const T*>(input), \
@@ -184,9 +217,9 @@ extern "C" ks_status_t ks_rms_norm_quant_fp8(void* out_fp8, float* out_scale, co
   const bool e5 = fp8_dtype == KS_DTYPE_F8E5M2;
 #define KSB_RQ(T)                                                                                                 \
   do {                                                                                                            \
-    if (e5) sm100::launch_programmatic(rms_norm_rows_kernel<T, true, true>, grid, kNormThreads, 0, s, \
+    if (e5) sm100::launch_programmatic(rms_norm_rows_kernel<T, true, true>, grid, row_threads(cols), 0, s, \
         out_fp8, out_scale, static_cast<const T*>(input), static_cast<const T*>(weight), cols, eps, 57344.0f);    \
-    else sm100::launch_programmatic(rms_norm_rows_kernel<T, true, false>, grid, kNormThreads, 0, s, \
+    else sm100::launch_programmatic(rms_norm_rows_kernel<T, true, false>, grid, row_threads(cols), 0, s, \
         out_fp8, out_scale, static_cast<const T*>(input), static_cast<const T*>(weight), cols, eps, 448.0f);      \
   } while (0)
   if (in_dtype == KS_DTYPE_F16) KSB_RQ(__half);

@@ -100,3 +100,11 @@ def test_gemm_with_column_major_scales_equals_row_major(ks, cuda, m, n, k, layou
     torch.cuda.synchronize()
     ks.runtime.stream_synchronize(0)
     assert torch.equal(out_row, out_col)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("cols", [128, 640, 1024, 1152, 2176, 8064])   # threads of a row: 32 to 256, the last with one segment or none
+def test_rms_norm_rows_that_do_not_fill_their_threads(ks, cuda, cols, dtype):
+    test_rms_norm(ks, cuda, 9, cols, dtype)
+    if dtype != torch.float32:
+        test_rms_norm_quant_equals_norm_then_quantize(ks, cuda, 64, cols, dtype)
