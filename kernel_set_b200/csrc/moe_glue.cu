@@ -480,6 +480,73 @@ unpermute_any_kernel(T* __restrict__ out, const T* __restrict__ permuted, const 
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ float silu(float x) { return __fdiv_rn(x, 1.0f + expf(-x)); }
 
+// Two 16-bit values in a word: as fp32, and from fp32.
+template <typename T>
+__device__ __forceinline__ float2 unpack_pair(uint32_t w) {
+  if constexpr (__is_same(T, __half)) return __half22float2(*reinterpret_cast<const __half2*>(&w));
+  else return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+template <typename T>
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
+  if constexpr (__is_same(T, __half)) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  } else {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+// |both| < 64 (false with a NaN).
+template <typename T>
+__device__ __forceinline__ bool below_64(uint32_t w) {
+  constexpr uint32_t k64 = __is_same(T, __half) ? 0x5400u : 0x4280u;
+  return (w & 0x7fffu) < k64 && ((w >> 16) & 0x7fffu) < k64;
+}
+
+// y = silu(g) * u, rounded to T, for 16 elements in words of two; g is replaced. These kernels are bound by
+// their instructions, most of which the IEEE division took (with its test for operands that need scaling):
+// for |g| < 64 the divisor lies in [1, 7e27] and the quotient is far from overflow, so the
+// approximate reciprocal and one correction step (Markstein: q0 = g * r, q = q0 + (g - q0 * d) * r, the residual
+// exact in an FMA) do, two to an instruction, within an ulp of fp32 of the quotient. Anything else, infinities
+// and NaN with it, is divided.
+template <typename T>
+__device__ __forceinline__ void silu_mul_16(uint32_t (&g)[8], const uint32_t (&u)[8]) {
+  using namespace quantmath;
+  bool small = true;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) small = small && below_64<T>(g[i]);
+  if (small) {
+    const F2 one = pack2(1.f, 1.f), neg1 = pack2(-1.f, -1.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 gf = unpack_pair<T>(g[i]), uf = unpack_pair<T>(u[i]);
+      const F2 x = pack2(gf.x, gf.y);
+      const F2 d = fma2(pack2(expf(-gf.x), expf(-gf.y)), one, one);
+      float d0, d1, r0, r1, y0, y1;
+      unpack2(d, &d0, &d1);
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d0));
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d1));
+      const F2 r = pack2(r0, r1);
+      const F2 q0 = mul2(x, r);
+      const F2 e = fma2(q0, d, mul2(x, neg1));   // q0 * d - x
+      unpack2(mul2(fma2(e, mul2(r, neg1), q0), pack2(uf.x, uf.y)), &y0, &y1);
+      g[i] = pack_pair<T>(y0, y1);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 gf = unpack_pair<T>(g[i]), uf = unpack_pair<T>(u[i]);
+      g[i] = pack_pair<T>(silu(gf.x) * uf.x, silu(gf.y) * uf.y);
+    }
+  }
+}
+template <typename T>
+__device__ __forceinline__ void load_words(const T* p, uint32_t (&w)[8]) {
+  const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+  w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+  w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+}
+
 // out[r, c] = silu(gate[r, c]) * up[r, c]; gate and up are rows of `in_stride` elements
 // starting at gate0 / up0 (packed: gate0 = in, up0 = in + inter, stride 2 * inter).
 template <typename T>
@@ -505,16 +572,13 @@ swiglu_vec16_kernel(T* __restrict__ out, const T* __restrict__ gate0, const T* _
   const int64_t r = seg / segs_per_row;
   if (r >= rows) return;
   const int64_t c = (seg - r * segs_per_row) * 16;
-  float g[16], u[16];
-  quantmath::Vec16<T>::load(gate0 + r * in_stride + c, g);
-  quantmath::Vec16<T>::load(up0 + r * in_stride + c, u);
-  T y[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) y[i] = from_f32<T>(silu(g[i]) * u[i]);
+  uint32_t g[8], u[8];
+  load_words(gate0 + r * in_stride + c, g);
+  load_words(up0 + r * in_stride + c, u);
+  silu_mul_16<T>(g, u);
   uint4* dst = reinterpret_cast<uint4*>(out + r * inter + c);
-  const uint4* src = reinterpret_cast<const uint4*>(y);
-#pragma unroll
-  for (int i = 0; i < static_cast<int>(sizeof(T)); ++i) dst[i] = src[i];
+  dst[0] = make_uint4(g[0], g[1], g[2], g[3]);
+  dst[1] = make_uint4(g[4], g[5], g[6], g[7]);
 }
 
 // Packed SwiGLU fused with the 1 x 128 quantizer: the activation is rounded to T exactly
@@ -531,11 +595,16 @@ swiglu_quant_kernel(uint8_t* __restrict__ out, float* __restrict__ scale, const 
   float v[16];
   if (live) {
     const int64_t c = (seg - r * segs_per_row) * 16;
-    float g[16], u[16];
-    quantmath::Vec16<T>::load(in + r * 2 * inter + c, g);
-    quantmath::Vec16<T>::load(in + r * 2 * inter + inter + c, u);
+    uint32_t g[8], u[8];
+    load_words(in + r * 2 * inter + c, g);
+    load_words(in + r * 2 * inter + inter + c, u);
+    silu_mul_16<T>(g, u);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = to_f32<T>(from_f32<T>(silu(g[i]) * u[i]));
+    for (int i = 0; i < 8; ++i) {
+      const float2 f = unpack_pair<T>(g[i]);
+      v[2 * i] = f.x;
+      v[2 * i + 1] = f.y;
+    }
   } else {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = 0.f;

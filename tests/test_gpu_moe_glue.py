@@ -495,3 +495,37 @@ def test_kernels_that_begin_early_wait_for_each_other(ks, cuda, tokens):
         torch.cuda.synchronize()
         for a, b in zip(queued, drained):
             assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("up", [1.0, -3.25])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_quotient_over_every_gate(ks, cuda, dtype, up):
+    """Every bit pattern as the gate: the kernel that corrects an approximate reciprocal against the one that divides
+    (rows at an odd address). The two quotients differ by at most an ulp of fp32, 2^-23, so where they do not round
+    alike the exact value lies that close to a tie of the 16-bit type: the results are then neighbours,
+    and of 65536 values a share of 2^-23 * 2^8 (bf16) or 2^-23 * 2^11 (f16) may be such, 2 or 16."""
+    gate = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(dtype).view(256, 256)
+    x = torch.cat([gate, torch.full_like(gate, up)], 1).to(cuda)
+    out = torch.empty(256, 256, dtype=dtype, device=cuda)
+    ks.activation.swiglu_packed(out, x)
+    odd = torch.empty(256 * 512 + 1, dtype=dtype, device=cuda)[1:].view(256, 512).copy_(x)
+    ref = torch.empty(256 * 256 + 1, dtype=dtype, device=cuda)[1:].view(256, 256)
+    ks.activation.swiglu_packed(ref, odd)
+    a, b = out.cpu().flatten(), ref.cpu().flatten()
+    nan = torch.isnan(b)
+    assert torch.equal(torch.isnan(a), nan)
+    ia, ib = a.view(torch.int16).int()[~nan], b.view(torch.int16).int()[~nan]
+    assert (ia - ib).abs().max() <= 1
+    assert (ia != ib).sum() <= (2 if dtype == torch.bfloat16 else 16)
+    # mixed rows: one value beyond the range sends its neighbours through the division too
+    mixed = torch.randn(64, 256, generator=gen(1)).to(dtype)
+    mixed[::3, 5] = 100.0
+    mixed[1::3, 77] = float("inf")
+    mixed[2::3, 130] = float("nan")
+    m = torch.cat([mixed, torch.full_like(mixed, up)], 1).to(cuda)
+    om = torch.empty(64, 256, dtype=dtype, device=cuda)
+    ks.activation.swiglu_packed(om, m)
+    want = orc.swiglu_packed(m.cpu())
+    ok = ~torch.isnan(want)
+    assert torch.equal(torch.isnan(om.cpu()), ~ok)
+    assert (om.cpu().view(torch.int16).int() - want.view(torch.int16).int())[ok].abs().max() <= 1
