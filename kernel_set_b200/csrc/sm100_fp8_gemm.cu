@@ -145,12 +145,14 @@ struct Params {
   int tiles_m;  // dense only
   uint32_t idesc;
   int vec_store;  // 16-byte output stores are legal
-  // K-split of the last partial round (dense only): work items [0, split_from) are whole
-  // tiles; item split_from + r is part r % split_s of tile split_from + r / split_s.
+  // K-split of the last partial round: work items [0, split_from) are whole tiles; item split_from + r is
+  // part r % split_s of tile split_from + r / split_s. Grouped problems work the three numbers out on the
+  // device (where there are slots).
   int split_from;
   int split_items;        // number of K-part items (tail tiles x split_s), at most the grid size
   int split_s;            // 1 = no split
   float4* split_slots;    // [tail tile][part][epilogue warp][16-byte column chunk][lane]
+  unsigned int* split_count;   // grouped: parts that have arrived, [tail tile][epilogue warp]; zero between launches
   int cluster_s;          // > 1: every tile is split (split_from = 0) over the CTAs of a cluster
   // MODE 1 / 2 (one scale per row and per column, the whole K range accumulated in TMEM)
   int64_t as_row_stride, as_kb_stride;   // a_scale[row * as_row_stride + kb * as_kb_stride]
@@ -186,22 +188,37 @@ __device__ __forceinline__ void place_in_panels(int t, int tiles_m, int tiles_n,
   *nt = panel * kPanel + (r - *mt * width);
 }
 
+// The K-split that a CTA goes by: Params' of a dense problem, worked out at kernel start of a grouped one.
+struct Split {
+  int from, items, s;
+};
+// Cycles. Marginal cases lose: 32 experts of 125 rows, N=K=2048 in 16 bits 55.5 us whole, 59.2 in two parts.
+constexpr int kSplitFixed = 8000, kSplitPerPart = 3000;
+
+// Parts that each of the `rem` tiles of a partial round is cut into along K: as many as the grid has
+// CTAs for, at most eight (each part is one more partial to add up), and four K-blocks a part at least.
+__host__ __device__ inline int split_parts(int grid, int rem, int nkb) {
+  int s = grid / rem;
+  if (s > 8) s = 8;
+  while (s > 1 && nkb / s < 4) --s;
+  return s;
+}
+
 template <int BN, bool GROUPED>
-__device__ __forceinline__ bool locate_tile(const Params& p, uint32_t tables, int t,
-                                            TileCoord* tc) {
+__device__ __forceinline__ bool locate_tile(const Params& p, const Split& sp, uint32_t tables, int t, TileCoord* tc) {
+  tc->kb0 = 0;
+  tc->kb1 = p.nkb;
+  tc->part = -1;
+  tc->tail = 0;
+  if (t >= sp.from) {
+    const int r = t - sp.from;
+    tc->tail = r / sp.s;
+    tc->part = r - tc->tail * sp.s;
+    tc->kb0 = (tc->part * p.nkb) / sp.s;
+    tc->kb1 = ((tc->part + 1) * p.nkb) / sp.s;
+    t = sp.from + tc->tail;
+  }
   if constexpr (!GROUPED) {
-    tc->kb0 = 0;
-    tc->kb1 = p.nkb;
-    tc->part = -1;
-    tc->tail = 0;
-    if (t >= p.split_from) {
-      const int r = t - p.split_from;
-      tc->tail = r / p.split_s;
-      tc->part = r - tc->tail * p.split_s;
-      tc->kb0 = (tc->part * p.nkb) / p.split_s;
-      tc->kb1 = ((tc->part + 1) * p.nkb) / p.split_s;
-      t = p.split_from + tc->tail;
-    }
     if (t >= p.tiles_m * p.tiles_n) return false;
     int mt, nt;
     place_in_panels(t, p.tiles_m, p.tiles_n, &mt, &nt);
@@ -211,10 +228,6 @@ __device__ __forceinline__ bool locate_tile(const Params& p, uint32_t tables, in
     tc->n0 = nt * BN;
     return true;
   } else {
-    tc->kb0 = 0;
-    tc->kb1 = p.nkb;
-    tc->part = -1;
-    tc->tail = 0;
     // tables: row tiles before an expert | its first row | its end row
     const auto prefix = [&](int e) { return ld_shared_s32(tables + 4 * e); };
     const int total_mt = prefix(p.num_experts);
@@ -243,15 +256,15 @@ __device__ __forceinline__ bool locate_tile(const Params& p, uint32_t tables, in
 // it has one), then whole tiles blockIdx.x, blockIdx.x + gridDim.x, ...
 struct ItemWalk {
   int n;
-  __device__ explicit ItemWalk(const Params& p)
-      : n((p.split_s > 1 && static_cast<int>(blockIdx.x) < p.split_items) ? -1 : 0) {}
+  __device__ explicit ItemWalk(const Split& sp)
+      : n((sp.s > 1 && static_cast<int>(blockIdx.x) < sp.items) ? -1 : 0) {}
   template <int BN, bool GROUPED>
-  __device__ __forceinline__ bool next(const Params& p, uint32_t tables, TileCoord* tc) {
-    const int t = n < 0 ? p.split_from + static_cast<int>(blockIdx.x)
+  __device__ __forceinline__ bool next(const Params& p, const Split& sp, uint32_t tables, TileCoord* tc) {
+    const int t = n < 0 ? sp.from + static_cast<int>(blockIdx.x)
                         : static_cast<int>(blockIdx.x) + n * static_cast<int>(gridDim.x);
-    if (n >= 0 && t >= p.split_from) return false;
+    if (n >= 0 && t >= sp.from) return false;
     ++n;
-    return locate_tile<BN, GROUPED>(p, tables, t, tc);
+    return locate_tile<BN, GROUPED>(p, sp, tables, t, tc);
   }
 };
 
@@ -318,6 +331,12 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     uint32_t b = (smem_u32(smem_raw) + 1023u) & ~1023u;
     asm volatile("" : "+r"(b));
     return b;
+  };
+  constexpr uint32_t kSplitAt = kTmemSlot + 16;   // grouped: the Split
+  static_assert(kSplitAt + 12 <= kSlotsAt, "control block");
+  const auto split_of = [&](uint32_t sm) {
+    return GROUPED ? Split{ld_shared_s32(sm + kSplitAt), ld_shared_s32(sm + kSplitAt + 4), ld_shared_s32(sm + kSplitAt + 8)}
+                   : Split{p.split_from, p.split_items, p.split_s};
   };
   const auto wait_ctx = [&](uint32_t sm) { return WaitCtx{sm + kTmemSlot + 4, p.fault_word}; };
   uint8_t* const smem = smem_raw + (((smem_u32(smem_raw) + 1023u) & ~1023u) - smem_u32(smem_raw));
@@ -386,7 +405,26 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
         if (e < p.num_experts) prefix[e] = run + inc - tiles;
         run += __shfl_sync(0xffffffffu, inc, 31);
       }
-      if (lane == 0) prefix[p.num_experts] = run;
+      if (lane == 0) {
+        prefix[p.num_experts] = run;
+        const int total = run * p.tiles_n, grid = static_cast<int>(gridDim.x);
+        Split sp{total, 0, 1};
+        if (p.split_slots != nullptr) {
+          // parts by cycles: what the shorter round saves, at the measured cost of a K-block, less what a part
+          // costs, in the main its 128 x BN partial sums through the L2 port of the SM that adds them up
+          const int rem = total % grid;
+          int best = 0;
+          for (int parts = rem > 0 ? split_parts(grid, rem, p.nkb) : 1; parts >= 2; --parts) {
+            const int saved = (p.nkb - (p.nkb + parts - 1) / parts) * (MODE == 0 ? (BN == 256 ? 750 : 500) : (BN == 256 ? 512 : 300));
+            const int gain = saved - kSplitFixed - parts * (BN == 256 ? kSplitPerPart : kSplitPerPart / 2);
+            if (gain > best) {
+              best = gain;
+              sp = Split{total - rem, rem * parts, parts};
+            }
+          }
+        }
+        *reinterpret_cast<Split*>(smem + kSplitAt) = sp;
+      }
     }
   }
   tc_fence_before_sync();
@@ -401,7 +439,8 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     uint32_t it = 0;
     bool ok = true;
     TileCoord tc;
-    for (ItemWalk walk(p); ok && walk.template next<BN, GROUPED>(p, sm + kTables, &tc);) {
+    const Split sp = split_of(sm);
+    for (ItemWalk walk(sp); ok && walk.template next<BN, GROUPED>(p, sp, sm + kTables, &tc);) {
       // A tile of up to 32 rows takes a box of 32: the rows behind its end (of no matrix, or of the next
       // expert) stay away, and what the MMAs read there goes into rows that are not stored. M=16, N=14336:
       // K=7168 33.7 -> 25.4 us, K=4096 19.8 -> 17.2 (64 rows took 25.6 and 17.2 already); decode of 48 tokens
@@ -446,12 +485,13 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     uint32_t tile_n = 0;   // MODE 1 / 2: tiles so far (one accumulator buffer per tile)
     bool ok = true;
     // what it needs of the walk is the number of K-blocks: a part of a split tile first, then whole tiles
-    int items = GROUPED ? ld_shared_s32(sm + kTables + 4 * p.num_experts) * p.tiles_n : p.split_from;
+    const Split sp = split_of(sm);
+    int items = sp.from;
     items = (items - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
     int nk = p.nkb;
-    if (!GROUPED && p.split_s > 1 && static_cast<int>(blockIdx.x) < p.split_items) {
-      const int part = static_cast<int>(blockIdx.x) % p.split_s;
-      nk = ((part + 1) * p.nkb) / p.split_s - (part * p.nkb) / p.split_s;
+    if (sp.s > 1 && static_cast<int>(blockIdx.x) < sp.items) {
+      const int part = static_cast<int>(blockIdx.x) % sp.s;
+      nk = ((part + 1) * p.nkb) / sp.s - (part * p.nkb) / sp.s;
       ++items;
     }
     for (; ok && items > 0; --items, nk = p.nkb) {
@@ -641,12 +681,13 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
       // (the rest of the tile's place is not held in registers over the K loop)
       const uint4 t0 = ld_shared_v4(tile_at);
       const uint4 t1 = ld_shared_v4(tile_at + 16);
-      struct { int row0, row_end, n0, part, tail; } tc;
+      struct { int row0, row_end, n0, part, tail, parts; } tc;
       tc.row0 = static_cast<int>(t0.y);
       tc.row_end = static_cast<int>(t0.z);
       tc.n0 = static_cast<int>(t0.w);
       tc.part = static_cast<int>(t1.x);
       tc.tail = static_cast<int>(t1.y);
+      tc.parts = static_cast<int>(t1.z);
       const int row = tc.row0 + row_in_tile;
       const bool row_ok = row < tc.row_end;
       const int col0 = tc.n0 + slice * EC;
@@ -663,18 +704,73 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
                            __float_as_uint(acc[2 * c4 + 1].x), __float_as_uint(acc[2 * c4 + 1].y));
           }
           stored = true;
-        } else if (ok && tc.part >= 0) {
-          // One K-part of a split tile. The warp's 32 x EC partial goes to its slot (16 bytes
-          // per lane and column chunk, chunks 512 B apart: every store of the warp is one
-          // contiguous 512-byte piece); split_reduce_kernel adds the parts up afterwards.
+        }
+      }
+      if (ok && !stored && tc.part >= 0) {
+        // One K-part of a split tile. The warp's 32 x EC partial goes to its slot (16 bytes per lane and column
+        // chunk, chunks 512 B apart: every store of the warp is one contiguous 512-byte piece). With counters,
+        // in a grouped problem, the warp that finds all the others of its block there adds them up, in part order, and
+        // stores the sum: a part is a CTA's first work item, so this runs while the others are at their whole tiles,
+        // and a second kernel for the sums would cost ~5 us also when there is nothing to add. A dense problem,
+        // whose parts the host knows, leaves the sums to split_reduce_kernel and all SMs (M=2500, N=2000,
+        // K=4096 35.0 us, 44.0 with the sums in here). Rows that do not exist stay away, 32 at a time.
+        stored = true;
+        if (tc.row0 + quarter * 32 < tc.row_end) {
           constexpr int kChunks = EC / 4;      // float4 chunks per lane
-          const int ew = warp - 4;
-          const size_t warp_f4 = static_cast<size_t>(kChunks) * 32;
-          float4* mine = p.split_slots + ((static_cast<size_t>(tc.tail) * p.split_s + tc.part) * C::kEpiWarps + ew) * warp_f4 + lane;
+          constexpr size_t kWarpF4 = static_cast<size_t>(kChunks) * 32;
+          int ew = warp - 4;
+          asm volatile("" : "+r"(ew));   // (as below: nothing of this is to be worked out ahead)
+          float4* slot0 = p.split_slots + (static_cast<size_t>(tc.tail) * tc.parts * C::kEpiWarps + ew) * kWarpF4 + lane;
+          float4* mine = slot0 + static_cast<size_t>(tc.part) * C::kEpiWarps * kWarpF4;
 #pragma unroll
           for (int c4 = 0; c4 < kChunks; ++c4)
             __stcg(mine + c4 * 32, make_float4(acc[2 * c4].x, acc[2 * c4].y, acc[2 * c4 + 1].x, acc[2 * c4 + 1].y));
-          stored = true;
+          if (p.split_count != nullptr) {
+            __syncwarp();
+            int last = 0;
+            if (lane == 0) {
+              unsigned int* count = p.split_count + tc.tail * C::kEpiWarps + ew;
+              __threadfence();   // the warp's partial is visible before its arrival
+              last = atomicAdd(count, 1u) == static_cast<unsigned int>(tc.parts - 1);
+              if (last) *count = 0u;
+              __threadfence();   // the others' partials are read behind their arrivals
+            }
+            if (__shfl_sync(0xffffffffu, last, 0)) {
+#pragma unroll 1
+              for (int c0 = 0; c0 < kChunks; c0 += 4) {
+                float4 sum[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+                for (int q0 = 0; q0 < tc.parts; q0 += 4) {   // sixteen loads in flight
+                  float4 v[4][4];
+#pragma unroll
+                  for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                      v[q][j] = q0 + q < tc.parts
+                                    ? ld_global_cg_f4(slot0 + static_cast<size_t>(q0 + q) * C::kEpiWarps * kWarpF4 + (c0 + j) * 32)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                  for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                      sum[j].x += v[q][j].x;
+                      sum[j].y += v[q][j].y;
+                      sum[j].z += v[q][j].z;
+                      sum[j].w += v[q][j].w;
+                    }
+                }
+                if (row_ok) {
+#pragma unroll
+                  for (int j = 0; j < 4; ++j) {
+                    const int col = col0 + 4 * (c0 + j);
+                    if (col < p.n) store_4<OutT>(out + static_cast<size_t>(row) * p.n + col, sum[j], p.vec_store != 0, p.n - col);
+                  }
+                }
+              }
+            }
+          }
         }
       }
       if (ok && !stored && p.vec_store) {
@@ -756,7 +852,8 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     uint32_t it = 0, tile_n = 0;
     bool ok = true;
     TileCoord tc;
-    for (ItemWalk walk(p); ok && walk.template next<BN, GROUPED>(p, sm + kTables, &tc);) {
+    const Split sp = split_of(sm);
+    for (ItemWalk walk(sp); ok && walk.template next<BN, GROUPED>(p, sp, sm + kTables, &tc);) {
       const int nk = MODE == 0 ? tc.kb1 - tc.kb0 : 1;
       const int first = static_cast<int>((it ^ mine) & 1u);   // this warp's first K-block of the tile
       const float* ap = nullptr;   // row 0 of the tile, and the other rows' distance from there
@@ -797,7 +894,7 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
         if (kb == 0 && lane == 2) {
           const uint32_t at = sm + kTilesAt + (tile_n % C::kTileSlots) * C::kTileBytes;
           st_shared_v4(at, nk, tc.row0, tc.row_end, tc.n0);
-          st_shared_v4(at + 16, tc.part, tc.tail, 0, 0);
+          st_shared_v4(at + 16, tc.part, tc.tail, sp.s, 0);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(MODE == 0 ? sm + kBarEmpty + 8 * (n % C::kStages) : sm + kBarAcc + 8 * (n % C::kAccBufs));
@@ -827,7 +924,7 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
         const uint32_t sm = base_of();
         // this CTA's share of the tile, in units of four columns
         TileCoord tc;
-        locate_tile<BN, GROUPED>(p, sm + kTables, static_cast<int>(blockIdx.x), &tc);
+        locate_tile<BN, GROUPED>(p, split_of(sm), sm + kTables, static_cast<int>(blockIdx.x), &tc);
         const int rows = tc.row_end - tc.row0 < kBM ? tc.row_end - tc.row0 : kBM;
         const int total = rows * (BN / 4);
         const int begin = (tc.part * total) / p.cluster_s, end = ((tc.part + 1) * total) / p.cluster_s;
@@ -850,6 +947,9 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
   }
 
   // ------------------------------- teardown -------------------------------
+  // Parts of a dense problem: the next kernel is split_reduce_kernel, which waits, and lines up from here on
+  // (M=2500, N=2000, K=4096 37.3 -> 35.0 us).
+  if (!GROUPED && p.split_slots != nullptr) grid_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag != 0u) {
@@ -871,7 +971,7 @@ __global__ void __launch_bounds__(256)
 split_reduce_kernel(OutT* __restrict__ out, const float4* __restrict__ slots, int split_from, int split_s, int tails,
                     int tiles_m, int tiles_n, int m, int n, int vec_ok) {
   using C = Cfg<BN>;
-  grid_start();
+  grid_dependency_wait();
   constexpr int EC = C::kEpiCols;
   constexpr int kChunks = EC / 4;
   constexpr int kPerTile = C::kEpiWarps * kChunks * 32;   // float4 per (tile, part)
@@ -936,7 +1036,7 @@ ks_status_t launch_one(const Fp8GemmArgs& a, const CUtensorMap& tm_a, const CUte
                                                     C::smem_bytes(GROUPED), stream, tm_a, tm_a32, tm_b, p);
   if (e != cudaSuccess) return cuda_status(e, a.where);
   if constexpr (!GROUPED) {
-    if (p.split_s > 1 && p.cluster_s == 1) {   // (a cluster adds its parts up itself and has no slots)
+    if (p.split_slots != nullptr) {   // (a cluster adds its parts up itself)
       const int tails = p.split_items / p.split_s;
       const int work = tails * C::kEpiWarps * (C::kEpiCols / 4) * 32;
       launch_programmatic(split_reduce_kernel<BN, OutT>, (work + 255) / 256, 256, 0, stream,
@@ -998,19 +1098,6 @@ bool fp8_blockwise_eligible(const Fp8GemmArgs& a) {
   return tma_available();
 }
 
-namespace {
-
-// Parts that each of the `rem` tiles of a partial round is cut into along K: as many as the grid has
-// CTAs for, at most eight (each part is one more partial to add up), and four K-blocks a part at least.
-int64_t split_parts(int64_t grid, int64_t rem, int64_t nkb) {
-  int64_t s = grid / rem;
-  if (s > 8) s = 8;
-  while (s > 1 && nkb / s < 4) --s;
-  return s;
-}
-
-}  // namespace
-
 ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   const bool grouped = a.offsets != nullptr || a.masked_m != nullptr;
   const int experts = grouped ? a.num_experts : 1;
@@ -1053,7 +1140,7 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
       int64_t part = nkb;
       int64_t extra = 0;
       if (rem > 0 && tiles > sms) {
-        const int64_t s = split_parts(sms, rem, nkb);
+        const int64_t s = split_parts(sms, static_cast<int>(rem), static_cast<int>(nkb));
         if (s >= 2) {
           part = (nkb + s - 1) / s;
           extra = 14000;
@@ -1154,14 +1241,14 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   int64_t tiles = tiles_m_bound * p.tiles_n;
   const int grid = static_cast<int>(cluster_s > 1 ? tiles * cluster_s : (tiles < sms ? (tiles < 1 ? 1 : tiles) : sms));
 
-  // K-split of the last partial round (dense problems only). Worth it when the tiles left
+  // K-split of the last partial round. Worth it when the tiles left
   // over after the full rounds occupy at most half of the CTAs and every part keeps at least
-  // four K-blocks; the part count is capped at eight (each part costs the finishing warp one
-  // more partial to read).
+  // four K-blocks; the part count is capped at eight (each part is one more partial to read).
   p.split_from = static_cast<int>(tiles);
   p.split_items = 0;
   p.split_s = 1;
   p.split_slots = nullptr;
+  p.split_count = nullptr;
   std::optional<StreamScratch> scratch;
   p.cluster_s = cluster_s;
   if (cluster_s > 1) {
@@ -1170,7 +1257,7 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
     p.split_s = cluster_s;
   } else if (!grouped && a.mode == 0 && a.force_split != 0 && a.num_out_parts == 0 && tiles > grid) {
     const int rem = static_cast<int>(tiles % grid);
-    const int s = rem > 0 ? static_cast<int>(split_parts(grid, rem, p.nkb)) : 1;
+    const int s = rem > 0 ? split_parts(grid, rem, p.nkb) : 1;
     if (rem > 0 && s >= 2) {
       const size_t slot_bytes = static_cast<size_t>(rem) * s * kBM * bn * sizeof(float);
       scratch.emplace(stream);   // (until both kernels are enqueued)
@@ -1180,6 +1267,21 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
         p.split_items = rem * s;
         p.split_s = s;
         p.split_slots = slots;
+      }
+    }
+  } else if (grouped && (a.mode == 0 || a.mode == 3) && a.force_split != 0 && p.nkb >= 8) {
+    // A grouped problem's rounds are known on the device only: there may be a partial one worth cutting unless
+    // even the fewest row tiles give so many rounds that it hardly counts. Slots for every CTA's part, and
+    // the counters that the W4A16 kernels use as well (zero whenever no kernel runs, cleared
+    // after a launch that gave up).
+    const int64_t fewest = a.masked_m != nullptr ? 0 : (a.m + kBM - 1) / kBM * p.tiles_n;
+    if (fewest < 16 * static_cast<int64_t>(grid)) {
+      scratch.emplace(stream);   // (until the kernel is enqueued)
+      void* counts = scratch->get(static_cast<size_t>(grid) * Cfg<256>::kEpiWarps * sizeof(unsigned int), 1);
+      void* slots = counts != nullptr ? scratch->get(static_cast<size_t>(grid) * kBM * bn * sizeof(float), 2) : nullptr;
+      if (slots != nullptr) {
+        p.split_slots = static_cast<float4*>(slots);
+        p.split_count = static_cast<unsigned int*>(counts);
       }
     }
   }

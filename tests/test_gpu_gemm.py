@@ -860,3 +860,60 @@ def test_tiles_of_few_rows_take_a_small_box(ks, cuda, mode, rows):
             noise = accumulation_noise(a.float().abs(), w.float().abs(), k)
         torch.cuda.synchronize()
         check_gemm(out.cpu(), ref32, noise, f"{mode} {counts}")
+
+
+@pytest.mark.parametrize("kind,n,k", [
+    ("fp8", 1024, 7168),     # 44 tiles: fewer than CTAs, all of them cut
+    ("fp8", 1030, 7168),     # rows not 16-byte aligned
+    ("masked", 1024, 7168),
+    ("fp8", 14336, 7168),    # 616 tiles: four rounds on 148 CTAs and 24 tiles to cut
+    ("16", 1024, 8192),
+    ("16", 7168, 8192),      # 308 tiles: two rounds and 12
+])
+def test_grouped_last_round_cut_along_k(ks, cuda, kind, n, k):
+    """The tiles of a grouped problem's last partial round, whose parts the last arriving warps add up, against
+    64-bit products of the same operands (bf16 outputs: half an ulp each, 2^-9 relative), three calls with the same bits
+    (the arrival counters are zero again), and rows of 1, 17 and 44 in a tile of 128."""
+    sizes = [300, 0, 129, 17, 640]
+    e, rows = len(sizes), sum(sizes)
+    g = torch.Generator(device=cuda).manual_seed(n + k)
+    off = torch.tensor([0] + torch.tensor(sizes).cumsum(0).tolist(), dtype=torch.int32, device=cuda)
+    x = torch.randn(rows, k, generator=g, device=cuda).bfloat16()
+    np_ = -(-n // 128) * 128
+    if kind == "16":
+        w = torch.randn(e, k, n, generator=g, device=cuda).mul_(0.05).bfloat16()
+        call = lambda: ks.dispatch.moe(x, w, off, num_experts=e, n=n, k=k)
+        a, weight = x.double(), lambda i, c: w[i, :, c].double()
+    else:
+        q = [block_quant_nk_device(torch.randn(np_, k, generator=g, device=cuda).mul_(0.05)) for _ in range(e)]
+        w = torch.stack([t[0].view(torch.uint8)[:n] for t in q]).view(torch.float8_e4m3fn)
+        ws = torch.stack([t[1] for t in q])
+        x8, xs = ks.dispatch.per_token_group_quant(x)
+        a = (x8.float().view(rows, k // 128, 128) * xs[:, :, None]).view(rows, k).double()
+        weight = lambda i, c: (w[i, c].float() * ws[i].repeat_interleave(128, 0)[:n][c].repeat_interleave(128, 1)).double().t()
+        if kind == "masked":
+            top = max(sizes)
+            m8 = torch.zeros(e, top, k, dtype=torch.uint8, device=cuda)
+            ms = torch.ones(e, top, k // 128, device=cuda)
+            for i, s in enumerate(sizes):
+                m8[i, :s] = x8[off[i]:off[i] + s].view(torch.uint8)
+                ms[i, :s] = xs[off[i]:off[i] + s]
+            counts = torch.tensor(sizes, dtype=torch.int32, device=cuda)
+
+            def call():
+                o = torch.zeros(e, top, n, dtype=torch.bfloat16, device=cuda)
+                ks.moe.grouped_gemm_fp8_blockwise_masked(o, m8.view(torch.float8_e4m3fn), w, ms, ws, counts, e, top, n, k)
+                return torch.cat([o[i, :s] for i, s in enumerate(sizes)])
+        else:
+            call = lambda: ks.dispatch.moe(x8, w, off, n=n, k=k, a_scale=xs, b_scale=ws, b_layout="nk")
+    out = call()
+    for _ in range(2):
+        assert torch.equal(call(), out)
+    ks.runtime.stream_synchronize(0)
+    for i, s in enumerate(sizes):
+        for c in (slice(0, 300), slice(n - 700, n)):
+            if s:
+                r = slice(int(off[i]), int(off[i]) + s)
+                ref = a[r] @ weight(i, c)
+                assert orc.rel_frobenius(out[r, c].float().cpu(), ref.float().cpu()) < 2.0 ** -8
+                assert float(((out[r, c].double() - ref).norm(dim=1) / ref.norm(dim=1)).max()) < 2.0 ** -7   # no single row
