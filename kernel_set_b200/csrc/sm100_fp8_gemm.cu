@@ -145,14 +145,12 @@ struct Params {
   int tiles_m;  // dense only
   uint32_t idesc;
   int vec_store;  // 16-byte output stores are legal
-  // K-split of the last partial round: work items [0, split_from) are whole tiles; item split_from + r is
-  // part r % split_s of tile split_from + r / split_s. Grouped problems work the three numbers out on the
-  // device (where there are slots).
+  // K-split of the last partial round (dense only): work items [0, split_from) are whole
+  // tiles; item split_from + r is part r % split_s of tile split_from + r / split_s.
   int split_from;
   int split_items;        // number of K-part items (tail tiles x split_s), at most the grid size
   int split_s;            // 1 = no split
   float4* split_slots;    // [tail tile][part][epilogue warp][16-byte column chunk][lane]
-  unsigned int* split_count;   // grouped: parts that have arrived, [tail tile][epilogue warp]; zero between launches
   int cluster_s;          // > 1: every tile is split (split_from = 0) over the CTAs of a cluster
   // MODE 1 / 2 (one scale per row and per column, the whole K range accumulated in TMEM)
   int64_t as_row_stride, as_kb_stride;   // a_scale[row * as_row_stride + kb * as_kb_stride]
@@ -188,16 +186,15 @@ __device__ __forceinline__ void place_in_panels(int t, int tiles_m, int tiles_n,
   *nt = panel * kPanel + (r - *mt * width);
 }
 
-// The K-split that a CTA goes by: Params' of a dense problem, worked out at kernel start of a grouped one.
+// The K-split that a CTA goes by: Params' of a dense problem; a grouped one's tiles are whole, their number is
+// known on the device only.
 struct Split {
   int from, items, s;
 };
-// Cycles. Marginal cases lose: 32 experts of 125 rows, N=K=2048 in 16 bits 55.5 us whole, 59.2 in two parts.
-constexpr int kSplitFixed = 8000, kSplitPerPart = 3000;
 
 // Parts that each of the `rem` tiles of a partial round is cut into along K: as many as the grid has
 // CTAs for, at most eight (each part is one more partial to add up), and four K-blocks a part at least.
-__host__ __device__ inline int split_parts(int grid, int rem, int nkb) {
+inline int split_parts(int grid, int rem, int nkb) {
   int s = grid / rem;
   if (s > 8) s = 8;
   while (s > 1 && nkb / s < 4) --s;
@@ -210,7 +207,7 @@ __device__ __forceinline__ bool locate_tile(const Params& p, const Split& sp, ui
   tc->kb1 = p.nkb;
   tc->part = -1;
   tc->tail = 0;
-  if (t >= sp.from) {
+  if (!GROUPED && t >= sp.from) {
     const int r = t - sp.from;
     tc->tail = r / sp.s;
     tc->part = r - tc->tail * sp.s;
@@ -332,10 +329,10 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     asm volatile("" : "+r"(b));
     return b;
   };
-  constexpr uint32_t kSplitAt = kTmemSlot + 16;   // grouped: the Split
-  static_assert(kSplitAt + 12 <= kSlotsAt, "control block");
+  constexpr uint32_t kTilesTotal = kTmemSlot + 16;   // grouped: the number of tiles
+  static_assert(kTilesTotal + 4 <= kSlotsAt, "control block");
   const auto split_of = [&](uint32_t sm) {
-    return GROUPED ? Split{ld_shared_s32(sm + kSplitAt), ld_shared_s32(sm + kSplitAt + 4), ld_shared_s32(sm + kSplitAt + 8)}
+    return GROUPED ? Split{ld_shared_s32(sm + kTilesTotal), 0, 1}
                    : Split{p.split_from, p.split_items, p.split_s};
   };
   const auto wait_ctx = [&](uint32_t sm) { return WaitCtx{sm + kTmemSlot + 4, p.fault_word}; };
@@ -407,23 +404,8 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
       }
       if (lane == 0) {
         prefix[p.num_experts] = run;
-        const int total = run * p.tiles_n, grid = static_cast<int>(gridDim.x);
-        Split sp{total, 0, 1};
-        if (p.split_slots != nullptr) {
-          // parts by cycles: what the shorter round saves, at the measured cost of a K-block, less what a part
-          // costs, in the main its 128 x BN partial sums through the L2 port of the SM that adds them up
-          const int rem = total % grid;
-          int best = 0;
-          for (int parts = rem > 0 ? split_parts(grid, rem, p.nkb) : 1; parts >= 2; --parts) {
-            const int saved = (p.nkb - (p.nkb + parts - 1) / parts) * (MODE == 0 ? (BN == 256 ? 750 : 500) : (BN == 256 ? 512 : 300));
-            const int gain = saved - kSplitFixed - parts * (BN == 256 ? kSplitPerPart : kSplitPerPart / 2);
-            if (gain > best) {
-              best = gain;
-              sp = Split{total - rem, rem * parts, parts};
-            }
-          }
-        }
-        *reinterpret_cast<Split*>(smem + kSplitAt) = sp;
+        // (worked out by every role for itself, the product costs the 40-register warps spills)
+        *reinterpret_cast<int*>(smem + kTilesTotal) = run * p.tiles_n;
       }
     }
   }
@@ -706,70 +688,21 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
           stored = true;
         }
       }
-      if (ok && !stored && tc.part >= 0) {
-        // One K-part of a split tile. The warp's 32 x EC partial goes to its slot (16 bytes per lane and column
-        // chunk, chunks 512 B apart: every store of the warp is one contiguous 512-byte piece). With counters,
-        // in a grouped problem, the warp that finds all the others of its block there adds them up, in part order, and
-        // stores the sum: a part is a CTA's first work item, so this runs while the others are at their whole tiles,
-        // and a second kernel for the sums would cost ~5 us also when there is nothing to add. A dense problem,
-        // whose parts the host knows, leaves the sums to split_reduce_kernel and all SMs (M=2500, N=2000,
-        // K=4096 35.0 us, 44.0 with the sums in here). Rows that do not exist stay away, 32 at a time.
-        stored = true;
-        if (tc.row0 + quarter * 32 < tc.row_end) {
-          constexpr int kChunks = EC / 4;      // float4 chunks per lane
-          constexpr size_t kWarpF4 = static_cast<size_t>(kChunks) * 32;
-          int ew = warp - 4;
-          asm volatile("" : "+r"(ew));   // (as below: nothing of this is to be worked out ahead)
-          float4* slot0 = p.split_slots + (static_cast<size_t>(tc.tail) * tc.parts * C::kEpiWarps + ew) * kWarpF4 + lane;
-          float4* mine = slot0 + static_cast<size_t>(tc.part) * C::kEpiWarps * kWarpF4;
+      if constexpr (!GROUPED) {
+        if (ok && !stored && tc.part >= 0) {
+          // One K-part of a split tile. The warp's 32 x EC partial goes to its slot (16 bytes per lane and column
+          // chunk, chunks 512 B apart: every store of the warp is one contiguous 512-byte piece); split_reduce_kernel
+          // adds the parts up afterwards, on all SMs (M=2500, N=2000, K=4096 35.0 us, 44.0 with the sums in here).
+          // Rows that do not exist stay away, 32 at a time.
+          stored = true;
+          if (tc.row0 + quarter * 32 < tc.row_end) {
+            constexpr int kChunks = EC / 4;      // float4 chunks per lane
+            int ew = warp - 4;
+            asm volatile("" : "+r"(ew));   // (as below: nothing of this is to be worked out ahead)
+            float4* mine = p.split_slots + ((static_cast<size_t>(tc.tail) * tc.parts + tc.part) * C::kEpiWarps + ew) * (kChunks * 32) + lane;
 #pragma unroll
-          for (int c4 = 0; c4 < kChunks; ++c4)
-            __stcg(mine + c4 * 32, make_float4(acc[2 * c4].x, acc[2 * c4].y, acc[2 * c4 + 1].x, acc[2 * c4 + 1].y));
-          if (p.split_count != nullptr) {
-            __syncwarp();
-            int last = 0;
-            if (lane == 0) {
-              unsigned int* count = p.split_count + tc.tail * C::kEpiWarps + ew;
-              __threadfence();   // the warp's partial is visible before its arrival
-              last = atomicAdd(count, 1u) == static_cast<unsigned int>(tc.parts - 1);
-              if (last) *count = 0u;
-              __threadfence();   // the others' partials are read behind their arrivals
-            }
-            if (__shfl_sync(0xffffffffu, last, 0)) {
-#pragma unroll 1
-              for (int c0 = 0; c0 < kChunks; c0 += 4) {
-                float4 sum[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-                for (int q0 = 0; q0 < tc.parts; q0 += 4) {   // sixteen loads in flight
-                  float4 v[4][4];
-#pragma unroll
-                  for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                      v[q][j] = q0 + q < tc.parts
-                                    ? ld_global_cg_f4(slot0 + static_cast<size_t>(q0 + q) * C::kEpiWarps * kWarpF4 + (c0 + j) * 32)
-                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                  for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                      sum[j].x += v[q][j].x;
-                      sum[j].y += v[q][j].y;
-                      sum[j].z += v[q][j].z;
-                      sum[j].w += v[q][j].w;
-                    }
-                }
-                if (row_ok) {
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) {
-                    const int col = col0 + 4 * (c0 + j);
-                    if (col < p.n) store_4<OutT>(out + static_cast<size_t>(row) * p.n + col, sum[j], p.vec_store != 0, p.n - col);
-                  }
-                }
-              }
-            }
+            for (int c4 = 0; c4 < kChunks; ++c4)
+              __stcg(mine + c4 * 32, make_float4(acc[2 * c4].x, acc[2 * c4].y, acc[2 * c4 + 1].x, acc[2 * c4 + 1].y));
           }
         }
       }
@@ -947,7 +880,7 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
   }
 
   // ------------------------------- teardown -------------------------------
-  // Parts of a dense problem: the next kernel is split_reduce_kernel, which waits, and lines up from here on
+  // Parts of a split round: the next kernel is split_reduce_kernel, which waits, and lines up from here on
   // (M=2500, N=2000, K=4096 37.3 -> 35.0 us).
   if (!GROUPED && p.split_slots != nullptr) grid_launch_dependents();
   tc_fence_before_sync();
@@ -1241,14 +1174,13 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   int64_t tiles = tiles_m_bound * p.tiles_n;
   const int grid = static_cast<int>(cluster_s > 1 ? tiles * cluster_s : (tiles < sms ? (tiles < 1 ? 1 : tiles) : sms));
 
-  // K-split of the last partial round. Worth it when the tiles left
+  // K-split of the last partial round (dense problems only). Worth it when the tiles left
   // over after the full rounds occupy at most half of the CTAs and every part keeps at least
   // four K-blocks; the part count is capped at eight (each part is one more partial to read).
   p.split_from = static_cast<int>(tiles);
   p.split_items = 0;
   p.split_s = 1;
   p.split_slots = nullptr;
-  p.split_count = nullptr;
   std::optional<StreamScratch> scratch;
   p.cluster_s = cluster_s;
   if (cluster_s > 1) {
@@ -1267,21 +1199,6 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
         p.split_items = rem * s;
         p.split_s = s;
         p.split_slots = slots;
-      }
-    }
-  } else if (grouped && (a.mode == 0 || a.mode == 3) && a.force_split != 0 && p.nkb >= 8) {
-    // A grouped problem's rounds are known on the device only: there may be a partial one worth cutting unless
-    // even the fewest row tiles give so many rounds that it hardly counts. Slots for every CTA's part, and
-    // the counters that the W4A16 kernels use as well (zero whenever no kernel runs, cleared
-    // after a launch that gave up).
-    const int64_t fewest = a.masked_m != nullptr ? 0 : (a.m + kBM - 1) / kBM * p.tiles_n;
-    if (fewest < 16 * static_cast<int64_t>(grid)) {
-      scratch.emplace(stream);   // (until the kernel is enqueued)
-      void* counts = scratch->get(static_cast<size_t>(grid) * Cfg<256>::kEpiWarps * sizeof(unsigned int), 1);
-      void* slots = counts != nullptr ? scratch->get(static_cast<size_t>(grid) * kBM * bn * sizeof(float), 2) : nullptr;
-      if (slots != nullptr) {
-        p.split_slots = static_cast<float4*>(slots);
-        p.split_count = static_cast<unsigned int*>(counts);
       }
     }
   }

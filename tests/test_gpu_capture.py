@@ -1,5 +1,7 @@
 """GPU: calls that use the library's scratch memory, captured into CUDA graphs: on a stream that has no scratch yet, on
 one that has, and with calls on the same stream between replays that need more of it."""
+import ctypes
+
 import pytest
 import torch
 
@@ -48,6 +50,30 @@ def _fp8(ks, cuda, m, k, n):
     return a_s, out, lambda: ks.gemm.gemm_fp8_blockwise(out, a8, b8, a_s, b_s, m, n, k, b_layout="nk")
 
 
+def _grouped(ks, cuda, kind, sizes=(300, 0, 129, 17), n=1024, k=4096):
+    e, rows = len(sizes), sum(sizes)
+    off = torch.tensor([0] + torch.tensor(sizes).cumsum(0).tolist(), dtype=torch.int32, device=cuda)
+    g = torch.Generator(device=cuda).manual_seed(rows + n + k)
+    x = torch.randn(rows, k, generator=g, device=cuda).bfloat16()
+    out = torch.empty(rows, n, dtype=torch.bfloat16, device=cuda)
+    if kind == "16":
+        w = torch.randn(e, k, n, generator=g, device=cuda).mul_(0.05).bfloat16()
+        return x, out, lambda: ks.moe.grouped_gemm(out, x, w, off, e, rows, n, k)
+    x8, xs = ks.dispatch.per_token_group_quant(x)
+    w = torch.randint(0, 120, (e, n, k), generator=g, device=cuda, dtype=torch.uint8).view(torch.float8_e4m3fn)
+    ws = torch.rand(e, n // 128, k // 128, generator=g, device=cuda) * 1e-3
+    if kind == "fp8":
+        return xs, out, lambda: ks.moe.grouped_gemm_fp8_blockwise(out, x8, w, xs, ws, off, e, rows, n, k)
+    top = max(sizes)
+    m8 = torch.zeros(e, top, k, dtype=torch.uint8, device=cuda)
+    ms = torch.ones(e, top, k // 128, device=cuda)
+    for i, s in enumerate(sizes):
+        m8[i, :s], ms[i, :s] = x8.view(torch.uint8)[int(off[i]):int(off[i]) + s], xs[int(off[i]):int(off[i]) + s]
+    m8, out = m8.view(torch.float8_e4m3fn), torch.zeros(e, top, n, dtype=torch.bfloat16, device=cuda)
+    counts = torch.tensor(sizes, dtype=torch.int32, device=cuda)
+    return ms, out, lambda: ks.moe.grouped_gemm_fp8_blockwise_masked(out, m8, w, ms, ws, counts, e, top, n, k)
+
+
 CALLS = {
     "w4a16 equal runs": lambda ks, d: _w4a16(ks, d, 24, 8192, 28688, 128),
     "w4a16 decode kernel": lambda ks, d: _w4a16(ks, d, 8, 4096, 11008, 128),
@@ -58,6 +84,9 @@ CALLS = {
     "unpermute f32": lambda ks, d: _unpermute(ks, d, 500, 256, torch.float32),
     "permute + quantize": lambda ks, d: _permute_quant(ks, d, 800, 4096),
     "fp8 with a split last round": lambda ks, d: _fp8(ks, d, 2500, 4096, 2000),
+    "grouped fp8": lambda ks, d: _grouped(ks, d, "fp8"),
+    "grouped fp8, masked": lambda ks, d: _grouped(ks, d, "masked"),
+    "grouped 16-bit": lambda ks, d: _grouped(ks, d, "16"),
 }
 
 
@@ -98,7 +127,8 @@ def test_scratch_in_a_graph(ks, cuda, name, warm):
     stream.synchronize()
     assert torch.equal(out, eager[0])
     big = {"w4a16": lambda: _w4a16(ks, cuda, 128, 4096, 28672, 128)[2], "unpermute": lambda: _unpermute(ks, cuda, 70000, 64, torch.bfloat16)[2],
-           "permute": lambda: _unpermute(ks, cuda, 70000, 64, torch.float32)[2], "fp8": lambda: _fp8(ks, cuda, 5000, 4096, 4096)[2]}
+           "permute": lambda: _unpermute(ks, cuda, 70000, 64, torch.float32)[2], "fp8": lambda: _fp8(ks, cuda, 5000, 4096, 4096)[2],
+           "grouped": lambda: _fp8(ks, cuda, 5000, 4096, 4096)[2]}
     grow = big[name.split()[0]]()
     for turn in range(3):
         for what, factor in enumerate((1.0, 0.5)):
@@ -114,3 +144,31 @@ def test_scratch_in_a_graph(ks, cuda, name, warm):
             del filler
     torch.cuda.synchronize()
     ks.runtime.stream_synchronize(0)
+
+
+@pytest.mark.parametrize("kind", ["fp8", "masked", "16"])
+def test_grouped_call_is_one_kernel_in_a_graph(ks, cuda, kind):
+    """A grouped GEMM neither allocates nor clears nor shares scratch: captured on a stream that has none, it is one
+    kernel node and no other."""
+    driver = ctypes.CDLL("libcuda.so.1")
+    _, out, call = _grouped(ks, cuda, kind)
+    call()
+    torch.cuda.synchronize()
+    eager = out.clone()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream(cuda)):
+        call()
+    handle, count = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t()
+    assert driver.cuGraphGetNodes(handle, None, ctypes.byref(count)) == 0
+    nodes = (ctypes.c_void_p * count.value)()
+    assert driver.cuGraphGetNodes(handle, nodes, ctypes.byref(count)) == 0
+    kinds = []
+    for node in nodes:
+        t = ctypes.c_int(-1)
+        assert driver.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(t)) == 0
+        kinds.append(t.value)
+    assert kinds == [0], kinds     # CU_GRAPH_NODE_TYPE_KERNEL
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager)

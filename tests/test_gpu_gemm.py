@@ -863,17 +863,16 @@ def test_tiles_of_few_rows_take_a_small_box(ks, cuda, mode, rows):
 
 
 @pytest.mark.parametrize("kind,n,k", [
-    ("fp8", 1024, 7168),     # 44 tiles: fewer than CTAs, all of them cut
+    ("fp8", 1024, 7168),     # fewer tiles than CTAs
     ("fp8", 1030, 7168),     # rows not 16-byte aligned
     ("masked", 1024, 7168),
-    ("fp8", 14336, 7168),    # 616 tiles: four rounds on 148 CTAs and 24 tiles to cut
+    ("fp8", 14336, 7168),    # 616 tiles: four rounds on 148 CTAs and 24 tiles
     ("16", 1024, 8192),
     ("16", 7168, 8192),      # 308 tiles: two rounds and 12
 ])
-def test_grouped_last_round_cut_along_k(ks, cuda, kind, n, k):
-    """The tiles of a grouped problem's last partial round, whose parts the last arriving warps add up, against
-    64-bit products of the same operands (bf16 outputs: half an ulp each, 2^-9 relative), three calls with the same bits
-    (the arrival counters are zero again), and rows of 1, 17 and 44 in a tile of 128."""
+def test_grouped_partial_rounds(ks, cuda, kind, n, k):
+    """Grouped problems that end in a partial round of tiles, against 64-bit products of the same operands (bf16
+    outputs: half an ulp each, 2^-9 relative), three calls with the same bits, and rows of 1, 17 and 44 in a tile of 128."""
     sizes = [300, 0, 129, 17, 640]
     e, rows = len(sizes), sum(sizes)
     g = torch.Generator(device=cuda).manual_seed(n + k)
@@ -917,3 +916,40 @@ def test_grouped_last_round_cut_along_k(ks, cuda, kind, n, k):
                 ref = a[r] @ weight(i, c)
                 assert orc.rel_frobenius(out[r, c].float().cpu(), ref.float().cpu()) < 2.0 ** -8
                 assert float(((out[r, c].double() - ref).norm(dim=1) / ref.norm(dim=1)).max()) < 2.0 ** -7   # no single row
+
+
+@pytest.mark.parametrize("kind,k", [("fp8", 7168), ("masked", 7168), ("16", 4096)])
+@pytest.mark.parametrize("n", [2048, 1032])
+def test_grouped_rows_do_not_depend_on_the_call_around_them(ks, cuda, kind, n, k):
+    """The same rows of an expert in a call of a few tiles and in one of many rounds of tiles: the same bits (a row's sum
+    over K has one order, whatever the other rows are and however many CTAs find no tile)."""
+    g = torch.Generator(device=cuda).manual_seed(n + k)
+    small = [130, 0, 40]
+    rows = 300 * 128
+    x = torch.randn(rows, k, generator=g, device=cuda).bfloat16()
+    big = [rows - 40 - 256, 256, 40]       # the small call's rows: the first of the first expert, all of the last
+    take = torch.cat([torch.arange(130), torch.arange(rows - 40, rows)]).to(cuda)
+    ends = lambda sizes: torch.tensor([0] + torch.tensor(sizes).cumsum(0).tolist(), dtype=torch.int32, device=cuda)   # noqa: E731
+    if kind == "16":
+        w = torch.randn(3, k, n, generator=g, device=cuda).mul_(0.05).bfloat16()
+        whole = ks.dispatch.moe(x, w, ends(big), num_experts=3, n=n, k=k)[take]
+        part = ks.dispatch.moe(x[take], w, ends(small), num_experts=3, n=n, k=k)
+    else:
+        w = torch.randint(0, 120, (3, n, k), generator=g, device=cuda, dtype=torch.uint8).view(torch.float8_e4m3fn)
+        ws = torch.rand(3, -(-n // 128), k // 128, generator=g, device=cuda) * 1e-3
+        x8, xs = ks.dispatch.per_token_group_quant(x)
+        whole = ks.dispatch.moe(x8, w, ends(big), n=n, k=k, a_scale=xs, b_scale=ws, b_layout="nk")[take]
+        few8, fews = x8.view(torch.uint8)[take].view(torch.float8_e4m3fn), xs[take]
+        if kind == "fp8":
+            part = ks.dispatch.moe(few8, w, ends(small), n=n, k=k, a_scale=fews, b_scale=ws, b_layout="nk")
+        else:
+            m8 = torch.zeros(3, 130, k, dtype=torch.uint8, device=cuda)
+            ms = torch.ones(3, 130, k // 128, device=cuda)
+            m8[0], m8[2, :40] = few8[:130].view(torch.uint8), few8[130:].view(torch.uint8)
+            ms[0], ms[2, :40] = fews[:130], fews[130:]
+            out = torch.zeros(3, 130, n, dtype=torch.bfloat16, device=cuda)
+            ks.moe.grouped_gemm_fp8_blockwise_masked(out, m8.view(torch.float8_e4m3fn), w, ms, ws,
+                                                     torch.tensor(small, dtype=torch.int32, device=cuda), 3, 130, n, k)
+            part = torch.cat([out[0], out[2, :40]])
+    ks.runtime.stream_synchronize(0)
+    assert torch.equal(part, whole)
