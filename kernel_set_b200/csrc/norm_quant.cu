@@ -81,8 +81,8 @@ template <typename T, bool QUANT, bool E5M2>
 __global__ void __launch_bounds__(kMaxRowThreads)
 rms_norm_rows_kernel(void* __restrict__ out, float* __restrict__ scale, const T* __restrict__ in,
                      const T* __restrict__ weight, int64_t cols, float eps, float qmax) {
-  if constexpr (QUANT) sm100::grid_launch_dependents();
   sm100::grid_dependency_wait();
+  if constexpr (QUANT) sm100::grid_launch_dependents();
   const int64_t row = blockIdx.x;
   const int segs = static_cast<int>(cols / 16);
   const T* x = in + row * cols;

@@ -194,12 +194,14 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 // First statement of a kernel whose every access depends on the kernel before it: what is saved is the
 // gap between two kernels, 2.6-3.6 us from the end of one to the first instruction of the next.
-// Not for a kernel that writes 16-bit or 32-bit matrices: the W4A16 kernels read their weights, scales and
-// zero-points before they wait, and such an output may be one of those. It waits, but lets nothing
-// begin before its end.
+// It waits before it lets its successor begin: a W4A16 kernel behind it reads int4 codes, scales and zero-points ahead of
+// its own wait, and finds everything written before this kernel (by whatever kernels) complete. For the same reason
+// no kernel may start this way whose output can be such an operand: fp8 codes with f32 scales, f32 routing
+// weights and int32 maps cannot, a 16-bit matrix (norm, gather, permute, SwiGLU) or repacked codes can. Those wait
+// likewise, but let nothing begin before their end.
 __device__ __forceinline__ void grid_start() {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
 }
 
 // ---- thread-block clusters ------------------------------------------------------------

@@ -497,6 +497,37 @@ def test_kernels_that_begin_early_wait_for_each_other(ks, cuda, tokens):
             assert torch.equal(a.view(torch.int16), b.view(torch.int16))
 
 
+@pytest.mark.parametrize("tokens", [2, 24])     # the decode kernel and the tcgen05 kernel
+def test_w4a16_behind_a_quantizer_reads_scales_written_just_before(ks, cuda, tokens):
+    """New scales and zero-points by another library's kernels, a quantizer, then W4A16, queued back to back: W4A16 reads
+    them ahead of its own wait, so the quantizer must not have let it begin before they were there."""
+    k, n = 2048, 11008
+    g = torch.Generator(device=cuda).manual_seed(tokens)
+    x = torch.randn(tokens, k, generator=g, device=cuda).bfloat16()
+    codes = torch.randint(0, 256, (k // 2, n), generator=g, device=cuda, dtype=torch.uint8)
+    versions = [(torch.rand(k // 128, n, generator=g, device=cuda).mul(0.02).bfloat16(),
+                 torch.randint(0, 16, (k // 128, n), generator=g, device=cuda).bfloat16()) for _ in range(4)]
+    scales, zeros = torch.empty_like(versions[0][0]), torch.empty_like(versions[0][1])
+    x8 = torch.empty(tokens, k, dtype=torch.float8_e4m3fn, device=cuda)
+    xs = torch.empty(tokens, k // 128, device=cuda)
+
+    def layer(version, after):
+        out = torch.empty(tokens, n, dtype=torch.bfloat16, device=cuda)
+        for step in (lambda: scales.copy_(version[0]), lambda: zeros.copy_(version[1]),
+                     lambda: ks.quant.quantize_fp8_group(x8, xs, x, tokens, k),
+                     lambda: ks.gemm.gemm_w4a16(out, x, codes, scales, zeros, tokens, n, k, group_size=128)):
+            step()
+            after()
+        return out
+
+    drained = [layer(v, torch.cuda.synchronize) for v in versions]
+    for _ in range(10):
+        queued = [layer(v, lambda: None) for v in versions]
+        torch.cuda.synchronize()
+        for a, b in zip(queued, drained):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("up", [1.0, -3.25])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_swiglu_quotient_over_every_gate(ks, cuda, dtype, up):
