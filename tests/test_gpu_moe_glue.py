@@ -528,26 +528,31 @@ def test_w4a16_behind_a_quantizer_reads_scales_written_just_before(ks, cuda, tok
             assert torch.equal(a, b)
 
 
+def _swiglu_both_ways(ks, x, inter):
+    """SwiGLU of packed x by the kernel that corrects an approximate reciprocal, and by the one that divides (rows at
+    an odd address)."""
+    out = torch.empty(x.shape[0], inter, dtype=x.dtype, device=x.device)
+    ks.activation.swiglu_packed(out, x)
+    odd = torch.empty(x.numel() + 1, dtype=x.dtype, device=x.device)[1:].view(x.shape).copy_(x)
+    ref = torch.empty(out.numel() + 1, dtype=x.dtype, device=x.device)[1:].view(out.shape)
+    ks.activation.swiglu_packed(ref, odd)
+    return out, ref
+
+
 @pytest.mark.parametrize("up", [1.0, -3.25])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_swiglu_quotient_over_every_gate(ks, cuda, dtype, up):
-    """Every bit pattern as the gate: the kernel that corrects an approximate reciprocal against the one that divides
-    (rows at an odd address). The two quotients differ by at most an ulp of fp32, 2^-23, so where they do not round
-    alike the exact value lies that close to a tie of the 16-bit type: the results are then neighbours,
-    and of 65536 values a share of 2^-23 * 2^8 (bf16) or 2^-23 * 2^11 (f16) may be such, 2 or 16."""
-    gate = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(dtype).view(256, 256)
-    x = torch.cat([gate, torch.full_like(gate, up)], 1).to(cuda)
-    out = torch.empty(256, 256, dtype=dtype, device=cuda)
-    ks.activation.swiglu_packed(out, x)
-    odd = torch.empty(256 * 512 + 1, dtype=dtype, device=cuda)[1:].view(256, 512).copy_(x)
-    ref = torch.empty(256 * 256 + 1, dtype=dtype, device=cuda)[1:].view(256, 256)
-    ks.activation.swiglu_packed(ref, odd)
-    a, b = out.cpu().flatten(), ref.cpu().flatten()
+    """Every bit pattern as the gate times an up of every significand: the corrected quotient is the rounded one, so the two
+    kernels agree to the bit, and no result depends on its neighbours or on the address of its row."""
+    bits = 7 if dtype == torch.bfloat16 else 10
+    gate = torch.arange(-32768, 32768, dtype=torch.int32, device=cuda).to(torch.int16).view(dtype)
+    ups = (torch.arange(2 ** bits, device=cuda).float() / 2 ** bits + 1).mul(up).to(dtype)
+    x = torch.empty(2 ** bits, 2 * 65536, dtype=dtype, device=cuda)
+    x[:, :65536], x[:, 65536:] = gate, ups[:, None]
+    a, b = _swiglu_both_ways(ks, x, 65536)
     nan = torch.isnan(b)
     assert torch.equal(torch.isnan(a), nan)
-    ia, ib = a.view(torch.int16).int()[~nan], b.view(torch.int16).int()[~nan]
-    assert (ia - ib).abs().max() <= 1
-    assert (ia != ib).sum() <= (2 if dtype == torch.bfloat16 else 16)
+    assert torch.equal(a.view(torch.int16).masked_fill(nan, 0), b.view(torch.int16).masked_fill(nan, 0))
     # mixed rows: one value beyond the range sends its neighbours through the division too
     mixed = torch.randn(64, 256, generator=gen(1)).to(dtype)
     mixed[::3, 5] = 100.0
@@ -560,3 +565,5 @@ def test_swiglu_quotient_over_every_gate(ks, cuda, dtype, up):
     ok = ~torch.isnan(want)
     assert torch.equal(torch.isnan(om.cpu()), ~ok)
     assert (om.cpu().view(torch.int16).int() - want.view(torch.int16).int())[ok].abs().max() <= 1
+    divided = _swiglu_both_ways(ks, m, 256)[1].cpu()
+    assert torch.equal(om.cpu().view(torch.int16)[ok], divided.view(torch.int16)[ok])
