@@ -70,9 +70,6 @@ namespace ksb {
 namespace sm100 {
 namespace {
 
-#ifndef KSB_FP8_EPI_COLS
-#define KSB_FP8_EPI_COLS 128
-#endif
 #ifndef KSB_FP8_ACC_BUFS_128
 #define KSB_FP8_ACC_BUFS_128 4
 #endif
@@ -91,21 +88,18 @@ struct Cfg {
   static constexpr int kABytes = kBM * kBK;
   static constexpr int kBBytes = BN * kBK;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  // An epilogue warp owns 32 TMEM lanes x kEpiCols columns. Narrow slices keep
-  // the per-K-block chain (wait, TMEM loads, FMAs, release) short: with 64
-  // columns it is ~440 cycles, under the ~512 the MMAs of a K-block take.
-  static constexpr int kEpiCols = BN == 256 ? KSB_FP8_EPI_COLS : 64;
-  static constexpr int kEpiWarps = (BN / kEpiCols) * 4;
+  // An epilogue warp owns 32 TMEM lanes x one of two column slices (a slot of the schedule holds the scales of two).
+  static constexpr int kEpiCols = BN / 2;
+  static constexpr int kEpiWarps = 8;
   static constexpr int kThreads = 128 + kEpiWarps * 32;
   // Warpgroup 0 (TMA, MMA issue) hands registers to the epilogue warpgroups,
   // which hold the accumulators plus the TMEM values in flight. The budgets must add up to no more than
   // the CTA's launch-time pool (threads x launch registers): setmaxnreg.inc
   // blocks, without a time limit, until the pool can satisfy it.
   static constexpr bool kRebalanceRegs = (BN == 256);
-  // 64-column slices: 20 warps, 96 registers at launch -> 32 / 112.
-  // 128-column slices: 12 warps, 168 registers at launch -> 40 / 232.
-  static constexpr int kRegsIssue = kEpiCols == 64 ? 32 : 40;
-  static constexpr int kRegsEpi = kEpiCols == 64 ? 112 : 232;
+  // 12 warps, 168 registers at launch -> 40 / 232.
+  static constexpr int kRegsIssue = 40;
+  static constexpr int kRegsEpi = 232;
   // Accumulator buffers in TMEM (512 columns): the MMA warp runs this many K-blocks
   // ahead of the epilogue. A K-block's round trip (issue -> complete -> drained ->
   // handed back) is about 1400 cycles whatever the tile width, so narrow tiles,
