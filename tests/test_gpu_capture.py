@@ -172,3 +172,41 @@ def test_grouped_call_is_one_kernel_in_a_graph(ks, cuda, kind):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, eager)
+
+
+def test_forked_streams_in_a_graph(ks, cuda):
+    """Programmatic launches behind event waits: a quantizer forks into two streams, each runs a layer's GEMM on its codes,
+    and the kernel behind the join depends on both."""
+    m, k, n = 200, 1024, 1024
+    g = torch.Generator(device=cuda).manual_seed(2)
+    x = torch.randn(m, k, generator=g, device=cuda).bfloat16()
+    w = [torch.randint(0, 120, (n, k), generator=g, device=cuda, dtype=torch.uint8).view(torch.float8_e4m3fn) for _ in range(2)]
+    ws = [torch.rand(n // 128, k // 128, generator=g, device=cuda) * 1e-3 for _ in range(2)]
+    x8, xs = torch.empty(m, k, dtype=torch.float8_e4m3fn, device=cuda), torch.empty(m, k // 128, device=cuda)
+    gate_up = torch.empty(2, m, n, dtype=torch.bfloat16, device=cuda)
+    out = torch.empty(m, n, dtype=torch.bfloat16, device=cuda)
+    a, b = torch.cuda.Stream(cuda), torch.cuda.Stream(cuda)
+
+    def layer():
+        ks.quant.quantize_fp8_group(x8, xs, x, m, k)
+        b.wait_stream(a)
+        ks.gemm.gemm_fp8_blockwise(gate_up[0], x8, w[0], xs, ws[0], m, n, k, b_layout="nk")
+        with torch.cuda.stream(b):
+            ks.gemm.gemm_fp8_blockwise(gate_up[1], x8, w[1], xs, ws[1], m, n, k, b_layout="nk")
+        a.wait_stream(b)
+        ks.activation.swiglu(out, gate_up[0], gate_up[1], m, n)
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        layer()
+    torch.cuda.synchronize()
+    eager = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=a):
+        layer()
+    for _ in range(5):
+        out.zero_()
+        gate_up.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, eager)
