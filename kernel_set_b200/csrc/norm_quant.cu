@@ -13,10 +13,12 @@
 //
 // A CTA per row, a thread owns one or two 16-element segments of it (rows of at most 8192 elements), so eight
 // consecutive lanes hold the eight segments of a quantisation group, the arrangement quant_segment_codes
-// expects. Issue-bound rather than memory-bound, so the work is laid out to leave no lane idle (7168 elements
-// are 224 threads x 2; with 128 threads x 4 an eighth of the lanes worked on nothing) and the
+// expects. Issue-bound rather than memory-bound, so warps without segments are left out, and the
 // products with the weight are taken two to an instruction: the normalised values and the weight are 16-bit,
 // their product is exact in fp32, so the packed multiplication rounds once, as the scalar one did.
+// Cold, event to event, with the quantizer, bf16: [4096,7168] 29.2 us, [4096,4096] 19.1, [16384,2048] 29.3 (128 threads
+// with up to four segments and scalar products: 36.6, 23.0, 40.0).
+#include <algorithm>
 #include <string>
 
 #include "common.cuh"
@@ -33,16 +35,47 @@ using namespace quantmath;
 constexpr int kNormThreads = 128;      // of the kernel for any width
 constexpr int kMaxRowThreads = 256;
 constexpr int kMaxSegs = 2;            // per thread
+constexpr int kChains = 128;           // of a row's sum of squares
 
-__device__ __forceinline__ float block_sum(float v) {
-  __shared__ float red[kMaxRowThreads / 32];
+// A row's sum of squares has one order, whatever the number of threads, since a last place of it decides how some
+// values of the row round: 128 chains, of which chain c adds up elements in turn (the kernel for any width: c, c + 128, ...;
+// the other: segments c, c + 128, c + 256, c + 384), 32 chains to a warp, then the four warps' sums in pairs.
+__device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  return v;
+}
+
+// add(i, sum) adds a thread's i-th segment to a chain. With 128 threads and more the second segment continues the
+// first one's chain, with fewer it is a chain of its own.
+template <typename Add>
+__device__ __forceinline__ float row_sum(const Add& add) {
+  __shared__ float red[kChains / 32];
+  __shared__ float handed[kChains];
+  const int t = threadIdx.x, nt = blockDim.x, warp = t >> 5;
+  if (nt < kChains) {
+    const float a = warp_sum(add(0, 0.f)), b = warp_sum(add(1, 0.f));
+    if ((t & 31) == 0) {
+      red[warp] = a;
+      red[warp + nt / 32] = b;
+    }
+    __syncthreads();
+    return nt == 32 ? red[0] + red[1] : (red[0] + red[1]) + (red[2] + red[3]);
+  }
+  float v = 0.f;
+  if (t < kChains) v = add(1, add(0, 0.f));
+  if (nt > kChains) {
+    // chain c goes on in thread c + 128
+    if (t < kChains) handed[t] = v;
+    __syncthreads();
+    if (t >= kChains) v = add(1, add(0, handed[t - kChains]));
+  }
+  if (t >= kChains || t + kChains >= nt) {   // (whole warps)
+    v = warp_sum(v);
+    if ((t & 31) == 0) red[warp & 3] = v;
+  }
   __syncthreads();
-  float sum = 0.f;
-  for (unsigned w = 0; w < blockDim.x / 32; ++w) sum += red[w];
-  return sum;
+  return (red[0] + red[1]) + (red[2] + red[3]);
 }
 
 // y = (v * inv).to(T) * w, rounded to T: 16 elements. f32 needs no rounding in between.
@@ -86,25 +119,25 @@ rms_norm_rows_kernel(void* __restrict__ out, float* __restrict__ scale, const T*
   const int64_t row = blockIdx.x;
   const int segs = static_cast<int>(cols / 16);
   const T* x = in + row * cols;
+  // threads 0-127 own segments t and t + 128 (up to 64 threads: t and t + 64 or 32), the others those 256 further on
+  const int first = threadIdx.x + (threadIdx.x & kChains), step = blockDim.x < kChains ? blockDim.x : kChains;
   Raw16<T> raw[kMaxSegs];
-  float sumsq = 0.f;
 #pragma unroll
   for (int i = 0; i < kMaxSegs; ++i) {
-    const int seg = threadIdx.x + i * blockDim.x;
+    const int seg = first + i * step;
     raw[i] = seg < segs ? Raw16<T>::load(x + seg * 16) : Raw16<T>::zero();
   }
-#pragma unroll
-  for (int i = 0; i < kMaxSegs; ++i) {
+  const float sumsq = row_sum([&](int i, float sum) {
     float v[16];
     raw[i].unpack(v);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) sumsq = fmaf(v[j], v[j], sumsq);
-  }
-  sumsq = block_sum(sumsq);
+    for (int j = 0; j < 16; ++j) sum = fmaf(v[j], v[j], sum);
+    return sum;
+  });
   const float inv_rms = rsqrtf(sumsq / static_cast<float>(cols) + eps);
 #pragma unroll
   for (int i = 0; i < kMaxSegs; ++i) {
-    const int seg = threadIdx.x + i * blockDim.x;
+    const int seg = first + i * step;
     const bool live = seg < segs;
     if (!__any_sync(0xffffffffu, live)) break;
     float v[16];
@@ -138,19 +171,26 @@ rms_norm_any_kernel(T* __restrict__ out, const T* __restrict__ in, const T* __re
   sm100::grid_dependency_wait();
   const int64_t row = blockIdx.x;
   const T* x = in + row * cols;
-  float sumsq = 0.f;
-  for (int64_t c = threadIdx.x; c < cols; c += kNormThreads) {
-    const float v = to_f32<T>(x[c]);
-    sumsq = fmaf(v, v, sumsq);
-  }
-  sumsq = block_sum(sumsq);
+  const float sumsq = row_sum([&](int i, float sum) {
+    if (i > 0) return sum;
+    for (int64_t c = threadIdx.x; c < cols; c += kNormThreads) {
+      const float v = to_f32<T>(x[c]);
+      sum = fmaf(v, v, sum);
+    }
+    return sum;
+  });
   const float inv_rms = rsqrtf(sumsq / static_cast<float>(cols) + eps);
   for (int64_t c = threadIdx.x; c < cols; c += kNormThreads)
     out[row * cols + c] = from_f32<T>(to_f32<T>(from_f32<T>(to_f32<T>(x[c]) * inv_rms)) * to_f32<T>(weight[c]));
 }
 
-// Threads for a row: two segments to a thread, in whole warps.
-unsigned row_threads(int64_t cols) { return static_cast<unsigned>((cols / 16 + 63) / 64 * 32); }
+// Threads for a row, in whole warps: two segments to a thread, the 256 segments behind the first 256 to threads of their own.
+unsigned row_threads(int64_t cols) {
+  const unsigned segs = static_cast<unsigned>(cols / 16);
+  if (segs <= kChains) return (segs + 63) / 64 * 32;
+  if (segs <= 2 * kChains) return kChains;
+  return kChains + std::min<unsigned>(kChains, (segs - 2 * kChains + 31) / 32 * 32);
+}
 
 bool rows_kernel_fits(int64_t cols, const void* a, const void* b, const void* c) {
   return cols % 128 == 0 && cols <= 16 * kMaxRowThreads * kMaxSegs && aligned16(a) && aligned16(b) &&

@@ -6,6 +6,7 @@ flip the rounding of the intermediate `T(x * inv_rms)`, which the second roundin
 weight can widen to two units in the last place of the output, rarely; the fused forms
 must equal the unfused library calls run one after the other bit for bit; the GEMM fed with
 column-major scales must equal the GEMM fed with row-major ones bit for bit."""
+import numpy as np
 import pytest
 import torch
 
@@ -108,3 +109,25 @@ def test_rms_norm_rows_that_do_not_fill_their_threads(ks, cuda, cols, dtype):
     test_rms_norm(ks, cuda, 9, cols, dtype)
     if dtype != torch.float32:
         test_rms_norm_quant_equals_norm_then_quantize(ks, cuda, 64, cols, dtype)
+
+
+@pytest.mark.parametrize("cols", [200, 640, 2048, 2176, 4096, 4608, 7168, 8064, 8192])
+def test_rms_norm_sum_has_one_order(ks, cuda, cols):
+    """The sum of squares is 128 chains over segments c, c + 128, ... (elements, where cols % 128 != 0), whatever the number of
+    threads. Here every chain starts with 2^24 and then loses each 1 it adds, so that another order shows: 96 chains
+    more or fewer with a 2^24 are 7e-7 of the result. Bound: rsqrtf 2 ulp (2.4e-7), quotient, eps and product half an ulp."""
+    step = 16 if cols % 128 == 0 else 1
+    x = np.ones(cols, dtype=np.float32)
+    x[: min(cols, 128 * step): step] = 4096.0
+    chains = np.zeros(128, dtype=np.float32)
+    for c in range(128):
+        for first in range(c * step, cols, 128 * step):
+            for v in x[first: first + step]:
+                chains[c] += v * v
+    total = chains.sum(dtype=np.float64)     # whole numbers below 2^31: the pairs' sums round to 2^8 at most
+    want = x.astype(np.float64) / np.sqrt(total / cols + 1e-6)
+    out = torch.empty(2, cols, device=cuda)
+    ks.norm.rms_norm(out, torch.from_numpy(np.stack([x, x])).to(cuda), torch.ones(cols, device=cuda), eps=1e-6)
+    got = out.cpu().numpy().astype(np.float64)
+    assert np.array_equal(got[0], got[1])
+    assert float(np.abs(got[0] / want - 1).max()) < 4e-7
