@@ -31,7 +31,9 @@
 // part order (reproducible) and writes the tiles. (Letting the last part to arrive reduce a
 // tile inside the GEMM kernel measured 3-4 % gain instead of the 10 % the idle round costs:
 // one CTA then reads S x 128 KB behind a fence and four dependent atomics while its tensor
-// core waits.)
+// core waits.) Grouped problems, whose rounds only the device knows, are not cut: a row's sum would then depend on
+// the other rows of the call, and the call would need slots and counters, in a captured graph too (8 experts, K=14336,
+// N=4096, 16 bits: 205 us, 180 when cut).
 // What bounds it: the epilogue warps' chain per K-block (wait, TMEM loads, 64 two-wide FMAs, release) and, back to
 // back, the card's power limit. Per K-block of 128 x 256 x 128 the MMAs need 512 cycles; the loop took 872 while the
 // epilogue warps loaded scales from global memory (a load over 32 lines per warp), looked for their next tile
@@ -582,9 +584,12 @@ fp8_blockwise_umma_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
             }
           }
           float v2[16];
+          // (the columns' numbers are worked out 16 at a time: all at once they are spilled)
+          int colc = col0 + c * 16;
+          asm volatile("" : "+r"(colc));
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const int col = col0 + c * 16 + j;
+            const int col = colc + j;
             const bool col_ok = col < p.n;
             const float raw = MODE == 2 ? static_cast<float>(static_cast<int32_t>(r[j])) : __uint_as_float(r[j]);
             float v = raw;
@@ -1030,8 +1035,10 @@ ks_status_t launch_fp8_blockwise(const Fp8GemmArgs& a, cudaStream_t stream) {
   const int experts = grouped ? a.num_experts : 1;
   const int sms = sm_count();
   const int64_t tiles_m_bound = grouped ? (a.m + kBM - 1) / kBM + experts : (a.m + kBM - 1) / kBM;
-  // Tile width by estimated time: rounds of tiles over the SMs times the measured cost of a
-  // K-block of that width (~850 cycles for 128 x 256, ~550 for 128 x 128). Wide tiles win
+  // Tile width by estimated time: rounds of tiles over the SMs times the cost of a
+  // K-block of that width (850 cycles for 128 x 256, 550 for 128 x 128, measured before warps 2 and 3 took over
+  // scales and tiles; the wide loop takes ~727 since, and these figures and the 9000 and 14000 below, which
+  // stand beside them, have not been fitted again). Wide tiles win
   // as soon as they do not need more rounds than narrow ones would save.
   // (grouped: by the bound of the row tiles. Their number is on the device only; by the number to expect,
   // max(experts hit, rows / 128 + experts / 2), even routings gained up to 30 %, but 54 of 432 measured shapes lost:
