@@ -103,7 +103,7 @@ def _load_library() -> ctypes.CDLL:
             continue
     raise OSError(
         "Could not locate the kernel_set shared library (libkernel_set.so). Build it with "
-        "`python -m kernel_set_b200.build` (needs nvcc), or set KERNEL_SET_LIB to its full path / "
+        "`python kernel_set_b200/build.py` (needs nvcc), or set KERNEL_SET_LIB to its full path / "
         "KERNEL_SET_LIB_DIR to its directory. This package has no CPU fallback.\nSearched:\n  "
         + "\n  ".join(tried))
 

@@ -1,6 +1,6 @@
 """In-tree build of ``libkernel_set.so`` for sm_100a with plain nvcc.
 
-``python -m kernel_set_b200.build`` compiles every ``csrc/*.cu`` (objects are
+``python kernel_set_b200/build.py`` compiles every ``csrc/*.cu`` (objects are
 rebuilt only when a source or header is newer) and links
 ``kernel_set_b200/lib/libkernel_set.so``, the drop-in for the reference
 project's library of the same name (built there by CMake,
