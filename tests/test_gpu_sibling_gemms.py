@@ -23,6 +23,8 @@ pytestmark = pytest.mark.gpu
     (2304, 3328, 1024, "token", "channel", torch.bfloat16, "e4m3"), # several rounds, both accumulator buffers
     (77, 144, 272, "token", "tensor", torch.float32, "e5m2"),
     (33, 50, 70, "token", "channel", torch.bfloat16, "e4m3"),       # general kernel (N % 16 != 0)
+    (7, 272, 528, "token", "channel", torch.float32, "e4m3"),       # tiles of up to 32 rows load a box of 32
+    (160, 1040, 1040, "token", "channel", torch.bfloat16, "e4m3"),  # the last row tile does
 ])
 def test_gemm_fp8_per_token_per_channel(ks, cuda, m, n, k, a_mode, b_mode, out_dtype, fp8):
     g = gen(m + n + k)
@@ -48,6 +50,8 @@ def test_gemm_fp8_per_token_per_channel(ks, cuda, m, n, k, a_mode, b_mode, out_d
     (2304, 3328, 1024, "token", "channel", torch.bfloat16, True),
     (64, 128, 8192, "tensor", "tensor", torch.float32, False),      # |sum| far beyond 2^24: int32 must be exact
     (40, 72, 96, "token", "channel", torch.float16, True),          # general kernel (N % 16 != 0)
+    (1, 272, 528, "token", "channel", torch.float32, True),         # tiles of up to 32 rows load a box of 32
+    (160, 1040, 1040, "token", "channel", torch.bfloat16, True),    # the last row tile does
 ])
 def test_gemm_w8a8(ks, cuda, m, n, k, a_mode, b_mode, out_dtype, bias):
     g = gen(m * 3 + n + k)
